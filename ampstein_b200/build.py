@@ -22,9 +22,10 @@ def units():
     for name in sorted(os.listdir(CSRC)):
         if not name.endswith(".cu"):
             continue
-        if name == "exl3_gemv_inst.cu":
+        per_width = {"exl3_gemv_inst.cu": "AMP_GEMV_K", "exl3_gemm_short_inst.cu": "AMP_SHORT_K"}.get(name)
+        if per_width:                          # one object per bit width
             for k in range(1, 9):
-                out.append((name, "exl3_gemv_inst_k%d.o" % k, ["-DAMP_GEMV_K=%d" % k]))
+                out.append((name, "%s_k%d.o" % (name[:-3], k), ["-D%s=%d" % (per_width, k)]))
         else:
             out.append((name, name[:-3] + ".o", []))
     return out

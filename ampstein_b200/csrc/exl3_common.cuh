@@ -146,6 +146,105 @@ __device__ __forceinline__ void warp_had128(float& h0, float& h1, float& h2, flo
     }
 }
 
+// 128-point Hadamard with eight lanes per 128-value chunk: lane piece pc (0..7) holds the two 16-byte
+// pieces (eight values each) at elements 8 pc .. and 64 + 8 pc .. . Same butterflies in the same
+// order as warp_had128 (index bits 0..6 in turn; lower = a + b, upper = a - b), hence the same bits
+// out: bits 0-2 and 6 inside the lane, bits 3-5 across the eight lanes. 3 shuffles per value
+// instead of 5, and both the loads and the stores of a chunk are whole 128-byte lines per eight lanes.
+__device__ __forceinline__ void oct_had128(float (&h)[16], int pc)
+{
+    #pragma unroll
+    for (int b = 1; b < 8; b <<= 1)
+        #pragma unroll
+        for (int i = 0; i < 16; ++i)
+            if (!(i & b))
+            {
+                const float lo = h[i], hi = h[i | b];
+                h[i] = lo + hi;
+                h[i | b] = lo - hi;
+            }
+    #pragma unroll
+    for (int m = 1; m <= 4; m <<= 1)
+    {
+        const bool up = (pc & m) != 0;
+        #pragma unroll
+        for (int i = 0; i < 16; ++i)
+        {
+            const float p = __shfl_xor_sync(0xffffffffu, h[i], m);
+            h[i] = up ? p - h[i] : h[i] + p;
+        }
+    }
+    #pragma unroll
+    for (int i = 0; i < 8; ++i)
+    {
+        const float lo = h[i], hi = h[i + 8];
+        h[i] = lo + hi;
+        h[i + 8] = lo - hi;
+    }
+}
+
+// Two fp32 additions / multiply-adds in one instruction (sm_100 packed forms; each half rounds as the scalar one)
+__device__ __forceinline__ float2 add_f32x2(float2 a, float2 b)
+{
+    float2 d;
+    asm("{\n\t.reg .b64 x, y, z;\n\tmov.b64 x, {%2, %3};\n\tmov.b64 y, {%4, %5};\n\tadd.rn.f32x2 z, x, y;\n\tmov.b64 {%0, %1}, z;\n\t}"
+        : "=f"(d.x), "=f"(d.y) : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
+    return d;
+}
+
+__device__ __forceinline__ float2 fma_f32x2(float2 a, float2 b, float2 c)
+{
+    float2 d;
+    asm("{\n\t.reg .b64 w, x, y, z;\n\tmov.b64 w, {%2, %3};\n\tmov.b64 x, {%4, %5};\n\tmov.b64 y, {%6, %7};\n\t"
+        "fma.rn.f32x2 z, w, x, y;\n\tmov.b64 {%0, %1}, z;\n\t}"
+        : "=f"(d.x), "=f"(d.y) : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y), "f"(c.x), "f"(c.y));
+    return d;
+}
+
+// 128-point Hadamard with four lanes per 128-value chunk: lane piece pc (0..3) holds in h[4 j .. 4 j + 3] the
+// eight values at elements 8 (pc + 4 j), j = 0..3, as pairs. Same butterflies in the same order as warp_had128
+// (bits 0-2 inside the lane, 3-4 across the four lanes, 5-6 inside), hence the same bits out; two shuffles
+// per value instead of five and half the additions thanks to the packed forms (a - b = fma(b, -1, a), exact
+// up to the one rounding of the sum).
+__device__ __forceinline__ void quad_had128(float2 (&h)[16], int pc)
+{
+    const float2 neg = make_float2(-1.0f, -1.0f);
+    #pragma unroll
+    for (int i = 0; i < 16; ++i) h[i] = make_float2(h[i].x + h[i].y, h[i].x - h[i].y);
+    #pragma unroll
+    for (int b = 1; b < 4; b <<= 1)
+        #pragma unroll
+        for (int i = 0; i < 16; ++i)
+            if (!(i & b))
+            {
+                const float2 lo = h[i], hi = h[i | b];
+                h[i] = add_f32x2(lo, hi);
+                h[i | b] = fma_f32x2(hi, neg, lo);
+            }
+    #pragma unroll
+    for (int m = 1; m <= 2; m <<= 1)
+    {
+        const float s = (pc & m) ? -1.0f : 1.0f;
+        const float2 sg = make_float2(s, s);
+        #pragma unroll
+        for (int i = 0; i < 16; ++i)
+        {
+            const float2 p = make_float2(__shfl_xor_sync(0xffffffffu, h[i].x, m), __shfl_xor_sync(0xffffffffu, h[i].y, m));
+            h[i] = fma_f32x2(h[i], sg, p);
+        }
+    }
+    #pragma unroll
+    for (int b = 4; b < 16; b <<= 1)
+        #pragma unroll
+        for (int i = 0; i < 16; ++i)
+            if (!(i & b))
+            {
+                const float2 lo = h[i], hi = h[i | b];
+                h[i] = add_f32x2(lo, hi);
+                h[i | b] = fma_f32x2(hi, neg, lo);
+            }
+}
+
 struct alignas(8) half4 { __half2 x, y; };
 
 // ------------------------------------------------------------------------------------------

@@ -37,176 +37,13 @@
 // Tensor-pipe bound by design (2 * M * k * n flops). Every wait on an mbarrier is bounded; on
 // expiry the status word is set, every role leaves its loop and the CTA still frees its tensor
 // memory.
-#include "exl3_gemv_kernel.cuh"
-#include "exl3_gemv_host.h"
-#include "host_common.h"
+#include "exl3_gemm_tc.cuh"
+#include <cmath>
 #include <mutex>
 
 namespace amp {
 
-constexpr int TC_DECODE_WARPS = 16;           // two groups of eight that take alternate k steps
-constexpr int TC_THREADS = 32 * (2 + TC_DECODE_WARPS);     // warp 0 fetches, warp 1 issues the MMAs, the rest decode
-constexpr int TC_BM = 128;            // tokens per sub-tile (UMMA M)
-constexpr int TC_SUB = 4;             // sub-tiles per CTA
-constexpr int TC_BN = 128;            // output columns per CTA (UMMA N)
-constexpr int TC_BK = 64;             // k per step (one 128-byte swizzle row)
-constexpr int TC_A_SLOTS = 2, TC_B_STAGES = 3;
-constexpr int TC_A_BYTES = TC_SUB * TC_BM * TC_BK * 2;     // one slot = the x~ tile of one k step: 65536
-constexpr int TC_B_BYTES = TC_BN * TC_BK * 2;              // 16384
-// packed trellis words travel through per-lane cp.async rings this many k steps deep (the words
-// come from HBM exactly once: the ring must cover the HBM latency, a step is ~0.5 us)
-__host__ __device__ constexpr int tc_p_stages(int K) { return K <= 4 ? 4 : 3; }        // per decode group: every other step
-__host__ __device__ constexpr int tc_smem_bytes(int K)
-{
-    return 1024 + TC_A_SLOTS * TC_A_BYTES + TC_B_STAGES * TC_B_BYTES + TC_DECODE_WARPS * tc_p_stages(K) * 128 * K;
-}
-constexpr unsigned TC_SPIN_LIMIT = 1u << 22;   // try_wait polls before a wait is declared lost
-
 __device__ int g_tc_status;
-
-struct TcParams
-{
-    const unsigned char* xt;    // rotated input, k-step-major and pre-swizzled (had_tiled_kernel): [k/64][M][128 bytes]
-    const uint16_t* trellis;    // (k/16, n/16, 16K)
-    const __half* svh;          // (n)
-    void* c;                    // (M, n) fp16 or fp32
-    int M, k, n, c_fp32;        // n: row width of the trellis / output (bundle: columns per slice)
-    int sub;                    // 128-token sub-tiles per CTA: 4, or fewer when the grid would leave SMs idle
-    int* status;
-    int relay_release;          // pair form: the relay's remote arrival releases at cluster scope (slower; default relaxed)
-    // bundle (tables == 1): several matrices or equal-width column slices in one grid, identified
-    // by device pointer tables with one entry per slice, exactly as the decode kernel's table mode
-    int tables;
-    const long long* t_trellis;
-    const long long* t_svh;
-    const long long* t_c;       // may be null: outputs stacked in c as (slices, M, n)
-    const int* t_stride;        // may be null: row width = n
-    const int* t_src;           // may be null: rotated input of slice i is source i
-    // expert groups (grouped instances of the single-CTA kernel): blockIdx.y walks a tile table
-    // that a kernel in front of this one built from the routing, blockIdx.x = projection * (n / 128)
-    // + column block. A tile is up to sub * 128 consecutive rows of ONE expert in the padded,
-    // expert-sorted row space of xt / c (M = its capacity); t_trellis / t_svh hold g_kinds *
-    // g_experts entries, projection-major; projection p reads xt + p * M * k halves and writes
-    // c + p * M * n elements.
-    const int* g_ntiles;        // device: tiles in use (CTAs beyond it return at once)
-    const int* g_tile_e;        // device: expert of a tile
-    const int* g_tile_row0;     // device: first padded row of a tile (a multiple of 8)
-    const int* g_tile_rows;     // device: valid rows of a tile (1 .. sub * 128)
-    int g_experts;
-    // experts of different bit widths: per projection a device table of the experts' widths (null:
-    // all of this launch's width); a CTA whose expert has another width than this instance returns
-    const unsigned char* g_bits[2];
-};
-
-// What one CTA (pair) works on: its weight, scales, output, rotated input and column block
-struct TcSlice
-{
-    const unsigned char* trellis;
-    const __half* svh;
-    unsigned char* c;
-    const unsigned char* xt;
-    int n_row;                  // row width of trellis and output
-    int nb;                     // column block (of BW columns) inside the slice
-};
-
-template <int BW>
-__device__ __forceinline__ TcSlice tc_slice(const TcParams& P, int nbg)
-{
-    TcSlice s;
-    s.trellis = reinterpret_cast<const unsigned char*>(P.trellis);
-    s.svh = P.svh; s.c = reinterpret_cast<unsigned char*>(P.c); s.xt = P.xt; s.n_row = P.n; s.nb = nbg;
-    if (P.tables)
-    {
-        const int bps = P.n / BW, slice = nbg / bps;
-        s.nb = nbg - slice * bps;
-        s.trellis = reinterpret_cast<const unsigned char*>(P.t_trellis[slice]);
-        s.svh = reinterpret_cast<const __half*>(P.t_svh[slice]);
-        s.n_row = P.t_stride ? P.t_stride[slice] : P.n;
-        s.c = P.t_c ? reinterpret_cast<unsigned char*>(P.t_c[slice])
-                    : reinterpret_cast<unsigned char*>(P.c) + (size_t) slice * P.M * P.n * (P.c_fp32 ? 4 : 2);
-        const int src = P.t_src ? P.t_src[slice] : slice;
-        s.xt = P.xt + (size_t) src * P.M * P.k * 2;
-    }
-    return s;
-}
-
-// K-major, 128-byte swizzle, rows of 128 bytes: byte offset of (row, 16-byte chunk)
-__device__ __forceinline__ uint32_t sw128(int row, int chunk)
-{
-    return (uint32_t) (row * 128 + ((chunk ^ (row & 7)) << 4));
-}
-
-__device__ __forceinline__ uint64_t make_desc(uint32_t smem_addr)
-{
-    // start address >> 4 [0,14), LBO (1, unused for swizzled K-major) [16,30), SBO = 1024 B >> 4
-    // [32,46), descriptor version 1 [46,48), layout SWIZZLE_128B (2) [61,64)
-    return (uint64_t) ((smem_addr & 0x3ffff) >> 4) | (1ull << 16) | (64ull << 32) | (1ull << 46) | (2ull << 61);
-}
-
-__device__ __forceinline__ void umma_f16(uint32_t tmem_d, uint64_t da, uint64_t db, uint32_t idesc, uint32_t accumulate)
-{
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "setp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, {%5, %5, %5, %5}, p;\n\t}"
-        :: "r"(tmem_d), "l"(da), "l"(db), "r"(idesc), "r"(accumulate), "r"(0u) : "memory");
-}
-
-__device__ __forceinline__ void umma_commit(uint64_t* bar)
-{
-    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];"
-                 :: "r"(smem_u32(bar)) : "memory");
-}
-
-__device__ __forceinline__ void mbar_arrive(uint64_t* bar)
-{
-    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" :: "r"(smem_u32(bar)) : "memory");
-}
-
-// 4K bytes of one lane, global -> this lane's ring slot, widest cp.async the alignment allows
-template <int K>
-__device__ __forceinline__ void cp_async_chunk(uint32_t dst, const unsigned char* src)
-{
-    if constexpr (K % 4 == 0)
-    {
-        #pragma unroll
-        for (int i = 0; i < K / 4; ++i)
-            asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" :: "r"(dst + 16 * i), "l"(src + 16 * i) : "memory");
-    }
-    else if constexpr (K % 2 == 0)
-    {
-        #pragma unroll
-        for (int i = 0; i < K / 2; ++i)
-            asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" :: "r"(dst + 8 * i), "l"(src + 8 * i) : "memory");
-    }
-    else
-    {
-        #pragma unroll
-        for (int i = 0; i < K; ++i)
-            asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" :: "r"(dst + 4 * i), "l"(src + 4 * i) : "memory");
-    }
-}
-
-// two states -> two exact fp16 weights packed (a in the low half), bit-identical to the reference
-template <int CB>
-__device__ __forceinline__ uint32_t weights2(uint32_t sa, uint32_t sb)
-{
-    if constexpr (CB == 2)
-    {
-        const uint32_t raw = __byte_perm(cb2_raw(sa), cb2_raw(sb), 0x5410);
-        const __half2 kinv = __half2half2(__ushort_as_half((unsigned short) 0x1eee));
-        const __half2 kbias = __half2half2(__ushort_as_half((unsigned short) 0xc931));
-        const __half2 w = __hfma2(*reinterpret_cast<const __half2*>(&raw), kinv, kbias);
-        return *reinterpret_cast<const uint32_t*>(&w);
-    }
-    else
-    {
-        const uint32_t ya = cb_halves<CB>(sa), yb = cb_halves<CB>(sb);
-        const uint32_t lo = __byte_perm(ya, yb, 0x5410), hi = __byte_perm(ya, yb, 0x7632);
-        const __half2 w = __hadd2(*reinterpret_cast<const __half2*>(&lo), *reinterpret_cast<const __half2*>(&hi));
-        return *reinterpret_cast<const uint32_t*>(&w);
-    }
-}
 
 template <int K, int CB, bool GROUPED = false>
 __global__ __launch_bounds__(TC_THREADS, GROUPED ? 2 : 1)
@@ -937,6 +774,20 @@ void exl3_gemm_tc2_kernel(const TcParams P)
         asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" :: "r"(tmem), "r"(512u) : "memory");
 }
 
+// looked up once per device (under a lock: two host threads may make their first launch on a device
+// at the same time)
+int tc_status_ptr(int dev, int** out)
+{
+    static int* ptr[64] = {};
+    static std::mutex mu;
+    std::lock_guard<std::mutex> lock(mu);
+    int*& p = ptr[dev & 63];
+    if (!p)
+        if (cudaError_t e = cudaGetSymbolAddress((void**) &p, g_tc_status)) return cuda_rc(e, "status symbol");
+    *out = p;
+    return 0;
+}
+
 typedef void (*tc_fn)(const TcParams);
 
 #define AMP_TC_ROW(cb) { exl3_gemm_tc_kernel<1, cb>, exl3_gemm_tc_kernel<2, cb>, exl3_gemm_tc_kernel<3, cb>, exl3_gemm_tc_kernel<4, cb>, \
@@ -953,6 +804,7 @@ static const tc_fn k_tcg[3][8] = { AMP_TCG_ROW(0), AMP_TCG_ROW(1), AMP_TCG_ROW(2
 static const tc_fn k_tc2[3][8] = { AMP_TC2_ROW(0), AMP_TC2_ROW(1), AMP_TC2_ROW(2) };
 #undef AMP_TC2_ROW
 int g_tc_relay_release = 0;
+int g_tc_short = 1;       // short-batch form (exl3_gemm_short.cuh): 0 never, 1 by size, 2 always
 int g_tc_pair = 1;        // pair (cta_group::2) form: 0 never, 1 where it fills the device, 2 whenever n % 256 == 0
 
 // tiled x~ (launch_had_tiled) -> C. Called by amp_exl3_gemm for m > 16, and by amp_exl3_mgemm
@@ -982,19 +834,22 @@ int launch_gemm_tc(const void* xh, const void* trellis, void* c, const void* svh
     P.relay_release = g_tc_relay_release;
     P.t_trellis = T ? T->trellis : nullptr; P.t_svh = T ? T->svh : nullptr; P.t_c = T ? T->c : nullptr;
     P.t_stride = T ? T->stride : nullptr; P.t_src = T ? T->src : nullptr;
-    {
-        // address of the status word, looked up once per device (under a lock: two host threads
-        // may make their first launch on a device at the same time)
-        static int* status_ptr[64] = {};
-        static std::mutex status_mu;
-        std::lock_guard<std::mutex> lock(status_mu);
-        int*& sp = status_ptr[dev & 63];
-        if (!sp)
-            if (cudaError_t e = cudaGetSymbolAddress((void**) &sp, g_tc_status)) return cuda_rc(e, "status symbol");
-        P.status = sp;
-    }
+    if (int rc = tc_status_ptr(dev, &P.status)) return rc;
     int sms = 148;
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    // Short batches: the form with the weights as the M operand wins wherever its k split or its shorter tiles
+    // pay, up to about 500 rows for a wide weight and 1000 for a narrow one. The line is drawn by comparing its
+    // expected time with that of the forms below (us, measured: the pair form takes 0.60 / 0.75 per step with
+    // 128- / 256-row CTAs and 14 around the k loop, per wave of pairs; the single-CTA form about 1.1 per step).
+    if (g_tc_short == 2 || (g_tc_short && g_tc_pair == 1))
+    {
+        const double ks = k / 64, pb = (double) slices * (n / 256);
+        const double p1 = ceil(pb * ceil(M / 256.0) / (sms / 2)) * (0.60 * ks + 14), p2 = ceil(pb * ceil(M / 512.0) / (sms / 2)) * (0.75 * ks + 14);
+        const double one = ceil((double) slices * (n / 128) * ceil(M / 512.0) / sms) * (1.1 * ks + 14);
+        const double limit = g_tc_short == 2 ? 1e30 : (n % 256 ? one : (p1 < p2 ? p1 : p2));
+        const int rc = launch_gemm_short(P, K, cb, slices * (n / 128), sms, dev, limit, stream);
+        if (rc != AMP_E_UNSUPPORTED) return rc;
+    }
     // pair form (two CTAs per 256-column block) for every weight it can tile. That includes
     // batches of 17..256 tokens, where the second CTA of a pair may hold no token at all and only
     // contributes its half of the decode: 64 tokens x 14336 x 4096 0.198 -> 0.134 ms, 256 tokens x
@@ -1067,15 +922,7 @@ int launch_gemm_tc_grouped(const void* xt, void* c, long Mcap, int k, int n, int
     P.g_ntiles = G.ntiles; P.g_tile_e = G.tile_e; P.g_tile_row0 = G.tile_row0; P.g_tile_rows = G.tile_rows;
     P.g_experts = G.experts;
     P.g_bits[0] = G.bits[0]; P.g_bits[1] = G.bits[1];
-    {
-        static int* status_ptr[64] = {};
-        static std::mutex status_mu;
-        std::lock_guard<std::mutex> lock(status_mu);
-        int*& sp = status_ptr[dev & 63];
-        if (!sp)
-            if (cudaError_t e = cudaGetSymbolAddress((void**) &sp, g_tc_status)) return cuda_rc(e, "status symbol");
-        P.status = sp;
-    }
+    if (int rc = tc_status_ptr(dev, &P.status)) return rc;
     dim3 grid((unsigned) (G.kinds * (n / 128)), (unsigned) G.max_tiles);
     fn<<<grid, TC_THREADS, smem_bytes, stream>>>(P);
     return cuda_rc(cudaGetLastError(), "exl3_moe_sorted gemm launch");
@@ -1107,6 +954,18 @@ AMP_API int amp_exl3_set_gemm_relay_release(int enable)
 {
     const int old = g_tc_relay_release;
     g_tc_relay_release = enable ? 1 : 0;
+    return old;
+}
+
+// Short-batch form of the prefill GEMM: 0 = never, 1 = by size (default), 2 = always; split / tile > 0 force the
+// number of k slices (1..8) / the tokens per tile (a multiple of 16, up to 512) for tests and sweeps. Returns the
+// previous mode.
+AMP_API int amp_exl3_set_gemm_short(int mode, int split, int tile)
+{
+    const int old = g_tc_short;
+    g_tc_short = mode < 0 ? 0 : (mode > 2 ? 2 : mode);
+    g_short_split = split < 0 || split > 8 ? 0 : split;
+    g_short_tile = tile < 0 || tile > 512 ? 0 : (tile + 15) & ~15;
     return old;
 }
 

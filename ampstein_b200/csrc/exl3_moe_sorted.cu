@@ -204,43 +204,6 @@ struct MsRot
     const __half* gu; int I; const long long* d_suh; int act, gated; float act_limit;
 };
 
-// 128-point Hadamard with eight lanes per 128-value chunk: lane piece pc (0..7) holds the two 16-byte
-// pieces (eight values each) at elements 8 pc .. and 64 + 8 pc .. . Same butterflies in the same
-// order as warp_had128 (index bits 0..6 in turn; lower = a + b, upper = a - b), hence the same bits
-// out: bits 0-2 and 6 inside the lane, bits 3-5 across the eight lanes. 3 shuffles per value
-// instead of 5, and both the loads and the stores of a chunk are whole 128-byte lines per eight lanes.
-__device__ __forceinline__ void oct_had128(float (&h)[16], int pc)
-{
-    #pragma unroll
-    for (int b = 1; b < 8; b <<= 1)
-        #pragma unroll
-        for (int i = 0; i < 16; ++i)
-            if (!(i & b))
-            {
-                const float lo = h[i], hi = h[i | b];
-                h[i] = lo + hi;
-                h[i | b] = lo - hi;
-            }
-    #pragma unroll
-    for (int m = 1; m <= 4; m <<= 1)
-    {
-        const bool up = (pc & m) != 0;
-        #pragma unroll
-        for (int i = 0; i < 16; ++i)
-        {
-            const float p = __shfl_xor_sync(0xffffffffu, h[i], m);
-            h[i] = up ? p - h[i] : h[i] + p;
-        }
-    }
-    #pragma unroll
-    for (int i = 0; i < 8; ++i)
-    {
-        const float lo = h[i], hi = h[i + 8];
-        h[i] = lo + hi;
-        h[i + 8] = lo - hi;
-    }
-}
-
 // a lane's 16 rotated values -> their place in the k-step-major, swizzled layout (see
 // had_tiled_kernel): k steps 2 * chunk and 2 * chunk + 1, 16-byte piece pc ^ (row & 7) of each
 __device__ __forceinline__ void ms_store_pieces(unsigned char* xt, int mcap, int p, int cb, int pc, const float (&h)[16])

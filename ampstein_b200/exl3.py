@@ -401,19 +401,24 @@ def mgemm_rms_norm_res(x, res, norm_w, eps, y, B_ptrs, C, suh_ptrs, svh_ptrs, K,
     return C
 
 
-# Widest weight that takes the reconstruct-then-matmul form in exl3_gemm_recon. Measured on B200 at
-# 256..4096 rows (k = 4096 / 5120, 5 bits): up to 2048 columns the decode-once form is 1.25-2.2x
-# faster than the tensor-core trellis GEMM (whose k loop is as long for a narrow weight as for a
-# wide one, with most SMs idle), at 4096 columns the two are level, above it the trellis GEMM wins.
+# Widest weight that takes the reconstruct-then-matmul form in exl3_gemm_recon, for many rows: above n / 2 rows
+# (twice as many where k is 16384: the decode costs that form a pass over memory, the trellis GEMM's k split
+# hides it). Measured on B200 (us, trellis GEMM / reconstruct + matmul): 4096 x 1024 at 512 rows 19 / 21, 1024
+# rows 27 / 23, 2048 rows 39 / 27; 4096 x 2048 at 512 rows 25 / 30, 1024 rows 33 / 34, 2048 rows 48 / 44;
+# 14336 x 2048 at 1024 rows 80 / 105. Above 2048 columns the trellis GEMM wins or is level.
 RECON_MM_MAX_N = 2048
+
+
+def _recon_mm(m, k, n):
+    return n <= RECON_MM_MAX_N and m > 16 and m * 2 > n * max(1.0, k / 8192.0)
 
 
 def exl3_gemm_recon(x, trellis, suh, svh, K, mul1=False, mcg=False, out=None, scratch=None):
     """EXL3 matmul for many rows (prefill); returns a (rows, n) fp16 tensor (reference:
-    torch_exl3_gemm_recon, src/torch/amp_torch.cpp:11128-11230). Narrow weights (n <= RECON_MM_MAX_N)
+    torch_exl3_gemm_recon, src/torch/amp_torch.cpp:11128-11230). Narrow weights and many rows (_recon_mm)
     take the reference's own form of this operator -- the weight decoded ONCE into fp16 with both
     Hadamards and scales folded in (this library's reconstruct_had kernel), then one plain library
-    GEMM; wider ones the tensor-core trellis GEMM, which never writes the decoded weight to memory.
+    GEMM; everything else the tensor-core trellis GEMM, which never writes the decoded weight to memory.
     out / scratch: optional preallocated result and (k, n) fp16 buffer for the decoded weight (the
     reference allocates both per call from the caching allocator; so does this function without them)."""
     _check_cuda("exl3_gemm_recon", x, trellis, suh, svh)
@@ -424,7 +429,7 @@ def exl3_gemm_recon(x, trellis, suh, svh, K, mul1=False, mcg=False, out=None, sc
     if float(K) != float(Kt):
         raise ValueError("exl3_gemm_recon: K does not match the trellis")
     y = out if out is not None else torch.empty((x.shape[0], n), dtype=torch.float16, device=x.device)
-    if (n <= RECON_MM_MAX_N or float(Kt) != int(Kt)) and x.dtype == torch.float16 and x.shape[0] > 16:
+    if (_recon_mm(x.shape[0], k, n) or (float(Kt) != int(Kt) and x.shape[0] > 16)) and x.dtype == torch.float16:
         w = scratch if scratch is not None else torch.empty((k, n), dtype=torch.float16, device=x.device)
         exl3_reconstruct_had(w, trellis, suh, svh, K, mul1, mcg)
         return torch.mm(x, w, out=y)

@@ -122,6 +122,13 @@ int amp_exl3_gemm_bf16(const void* A, const void* trellis, void* C, const void* 
  */
 int amp_exl3_set_gemm_pair(int mode);
 /*
+ * Short-batch form of the prefill GEMM (decoded weights as the M operand, tokens as N, k split over a cluster):
+ * 0 = never, 1 = by size (default), 2 = always. split / tile > 0 force the number of k slices (1..8) / the tokens
+ * per tile (a multiple of 16, up to 512), for tests and sweeps; 0: by rule. Returns the previous mode. No
+ * counterpart in the reference.
+ */
+int amp_exl3_set_gemm_short(int mode, int split, int tile);
+/*
  * Int8-activation form of the one-row GEMV for mul1 (codebook 2) tensors up to max_k bits: the
  * rotated input is quantised to int8 with one scale per 128 rows of k and the dot product runs as
  * dp4a on the byte sum of the codebook's product, exact in int32 (about 6e-3 relative rms against
