@@ -4,11 +4,11 @@
 
 namespace amp {
 
-#define AMP_DECL(K) sh_fn sh_kernel_k##K(int cb, bool grouped);
+#define AMP_DECL(K) sh_fn sh_kernel_k##K(int cb, int grouped);
 AMP_DECL(1) AMP_DECL(2) AMP_DECL(3) AMP_DECL(4) AMP_DECL(5) AMP_DECL(6) AMP_DECL(7) AMP_DECL(8)
 #undef AMP_DECL
 
-sh_fn sh_kernel(int K, int cb, bool grouped)
+sh_fn sh_kernel(int K, int cb, int grouped)
 {
     switch (K)
     {
@@ -29,7 +29,7 @@ constexpr int SH_STATIC = 1024;          // static shared memory of the kernel (
 
 static int sh_smem(int tile, int ws, int xs)
 {
-    return 1024 + ws * SH_W_BYTES + xs * tile * TC_BK * 2;
+    return ws * SH_W_BYTES + xs * tile * TC_BK * 2;
 }
 
 // Memory plan of one tile height and number of decode groups: stages, tensor-memory columns, tokens per
@@ -42,7 +42,7 @@ static int sh_layout(ShParams& S, int tile, int ng)
     int cols = 32;
     while (cols < tile) cols <<= 1;
     S.tmem_cols = cols > SH_MAX_N ? 512 : cols;
-    const int budget = ng == 1 ? 228 * 1024 / 2 - 1024 - SH_STATIC : 227 * 1024 - SH_STATIC;     // two CTAs per SM / one
+    const int budget = 228 * 1024 / (ng == 1 ? 2 : 1) - 1024 - SH_STATIC;             // two CTAs per SM / one
     // weights are handed over a step or two behind their decode; x~ comes from L2 and wants the depth
     int ws = ng == 1 ? 3 : 5, xs = 2;
     while (ws > 2 * ng && sh_smem(tile, ws, xs) > budget) --ws;
@@ -69,7 +69,7 @@ static int sh_exchange(ShParams& S, int smem)
             S.recv_off = S.wstages * SH_W_BYTES + S.xstages * x;
         }
     }
-    const int room = (smem - 1024) / sh_row(S.split);
+    const int room = smem / sh_row(S.split);
     if (!S.recv_off && ts * S.split > room) ts = room / S.split & ~7;
     S.share = ts;
     return S.recv_off ? sh_smem(S.tile, S.wstages, S.xstages) + S.split * ts * sh_row(S.split) : smem;
@@ -85,7 +85,7 @@ static int sh_max_clusters(int c, int sms, int dev)
     if (!v)
     {
         const int smem = 227 * 1024 - SH_STATIC;
-        sh_fn fn = sh_kernel(4, 0, false);
+        sh_fn fn = sh_kernel(4, 0, 0);
         cudaLaunchConfig_t cfg = {};
         cfg.gridDim = dim3((unsigned) (c * sms), 1, 1);
         cfg.blockDim = dim3(sh_threads(2), 1, 1);
@@ -142,7 +142,7 @@ int launch_gemm_short(const TcParams& P, int K, int cb, long blocks, int sms, in
     S.pdl = g_pdl;
     const int smem = sh_plan(S, P.M, blocks, P.k / TC_BK, sms, dev, limit);
     if (!smem) return AMP_E_UNSUPPORTED;
-    sh_fn fn = sh_kernel(K, cb, false);
+    sh_fn fn = sh_kernel(K, cb, 0);
     if (cudaError_t e = ensure_smem(fn, smem, dev)) return cuda_rc(e, "exl3_gemm_short smem attribute");
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned) (blocks * S.split), (unsigned) ((P.M + S.tile - 1) / S.tile), 1);
@@ -166,6 +166,54 @@ int launch_gemm_short(const TcParams& P, int K, int cb, long blocks, int sms, in
     cfg.attrs = attr;
     cfg.numAttrs = na;
     return cuda_rc(cudaLaunchKernelEx(&cfg, fn, S), "exl3_gemm_short launch");
+}
+
+// Expert-grouped form for token-sorted MoE prefill: xt / c are (kinds, Mcap, k / n) in the padded, expert-sorted row
+// space, the tile table lives in device memory (see TcParams). One CTA per (tile, projection, 128-column block); the
+// grid is sized for G.max_tiles and the surplus returns. Eight decode warps and two CTAs per SM, so that one CTA's
+// set-up and epilogue run under the other's decode.
+int launch_gemm_short_grouped(const void* xt, void* c, long Mcap, int k, int n, int K, int cb, int c_fp32,
+                              const long long* t_trellis, const long long* t_svh, const TcGroups& G, cudaStream_t stream)
+{
+    AMP_REQUIRE(xt && c && t_trellis && t_svh && G.ntiles && G.tile_e && G.tile_row0 && G.tile_rows, "exl3_moe_sorted: null pointer");
+    AMP_REQUIRE(K >= 1 && K <= 8 && cb >= 0 && cb <= 2, "exl3_moe_sorted: unsupported bitrate / codebook");
+    AMP_REQUIRE(Mcap >= 1 && Mcap <= 0x7fffffffL && k % 128 == 0 && n % 128 == 0 && k > 0 && n > 0, "exl3_moe_sorted: k and n must be multiples of 128");
+    AMP_REQUIRE(((uintptr_t) xt & 15) == 0 && ((uintptr_t) c & 15) == 0, "exl3_moe_sorted: misaligned pointer");
+    AMP_REQUIRE(G.kinds >= 1 && G.kinds <= 2 && G.tile >= 16 && G.tile <= SH_MAX_N && G.tile % 16 == 0 && G.experts >= 1, "exl3_moe_sorted: bad grouping");
+    AMP_REQUIRE(G.max_tiles >= 1 && G.max_tiles <= 65535, "exl3_moe_sorted: too many row tiles");
+    int dev = 0;
+    if (cudaError_t e = cudaGetDevice(&dev)) return cuda_rc(e, "cudaGetDevice");
+    ShParams S = {};
+    const int smem = sh_layout(S, G.tile, 1);
+    AMP_REQUIRE(smem, "exl3_moe_sorted: tile does not fit");
+    S.x_area = smem - sh_smem(G.tile, S.wstages, 0);
+    S.split = 1;
+    S.share = smem / sh_row(1) & ~7;
+    // Dependent launch only where every grid that does anything waits for the rotation kernel: with one launch per
+    // bit width a launch whose experts all have another width would be over before that kernel, and the next
+    // launch's wait would be for it alone.
+    S.pdl = g_pdl && !G.bits[0];
+    TcParams& P = S.t;
+    P.xt = (const unsigned char*) xt; P.c = c;
+    P.M = (int) Mcap; P.k = k; P.n = n; P.c_fp32 = c_fp32;
+    P.t_trellis = t_trellis; P.t_svh = t_svh;
+    P.g_ntiles = G.ntiles; P.g_tile_e = G.tile_e; P.g_tile_row0 = G.tile_row0; P.g_tile_rows = G.tile_rows;
+    P.g_experts = G.experts;
+    P.g_bits[0] = G.bits[0]; P.g_bits[1] = G.bits[1];
+    if (int rc = tc_status_ptr(dev, &P.status)) return rc;
+    sh_fn fn = sh_kernel(K, cb, 1);
+    if (cudaError_t e = ensure_smem(fn, smem, dev)) return cuda_rc(e, "exl3_moe_sorted smem attribute");
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned) (G.kinds * (n / 128)), (unsigned) G.max_tiles, 1);
+    cfg.blockDim = dim3(sh_threads(1), 1, 1);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = stream;
+    cudaLaunchAttribute attr;
+    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr.val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = &attr;
+    cfg.numAttrs = S.pdl ? 1 : 0;
+    return cuda_rc(cudaLaunchKernelEx(&cfg, fn, S), "exl3_moe_sorted gemm launch");
 }
 
 }  // namespace amp

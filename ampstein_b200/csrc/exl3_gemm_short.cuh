@@ -40,6 +40,7 @@ struct ShParams
     int n0;                     // tokens of the first accumulator: a multiple of 16, at most 256 (the rest: the second, at column 256)
     int split;                  // CTAs per cluster = slices of k (1: no cluster)
     int wstages, xstages;       // stages of decoded weights and of x~: wstages >= 2 NG
+    int x_area;                 // expert groups: bytes of all x~ stages together (xstages then follows from the tile's rows)
     int tmem_cols;              // tensor-memory columns to allocate: a power of two >= tile, >= 32 (two accumulators: 512)
     int share;                  // tokens a CTA finishes per epilogue pass (several passes: a multiple of 8)
     int recv_off;               // where the partial sums are received: behind the stages, or 0: over them
@@ -169,7 +170,12 @@ void exl3_gemm_short_kernel(const ShParams S)
         if (bits && bits[P.g_tile_e[blockIdx.y]] != K) return;
     }
     extern __shared__ __align__(1024) unsigned char smem_raw[];
-    unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t) 1023);
+    unsigned char* smem = smem_raw;
+    if (smem_u32(smem_raw) & 1023)                           // (the swizzle needs the alignment the declaration asks for)
+    {
+        if (threadIdx.x == 0) atomicExch(P.status, 2);
+        return;
+    }
     __shared__ uint64_t x_full[SH_MAX_STAGES], w_full[SH_MAX_STAGES], done[SH_MAX_STAGES];
     __shared__ uint32_t s_tmem;
     __shared__ volatile int s_bad;
@@ -203,8 +209,9 @@ void exl3_gemm_short_kernel(const ShParams S)
     const int ksteps = P.k / TC_BK;
     const int ks0 = ksteps * crank / split, nsteps = ksteps * (crank + 1) / split - ks0;     // (split <= ksteps: never empty)
     const size_t tiles_n = (size_t) W.n_row >> 4;
-    const int x_bytes = S.tile * (TC_BK * 2);
-    const int WS = S.wstages, XS = S.xstages, DS = max(WS, XS);
+    // expert groups: the x~ stages are as tall as this tile, so that short tiles get more of them
+    const int x_bytes = (GROUPED ? (rows + 15) & ~15 : S.tile) * (TC_BK * 2);
+    const int WS = S.wstages, XS = GROUPED ? min(SH_MAX_STAGES, S.x_area / x_bytes) : S.xstages, DS = max(WS, XS);
     unsigned char* x_base = smem + WS * SH_W_BYTES;
 
     if (t == 0)
@@ -388,7 +395,7 @@ void exl3_gemm_short_kernel(const ShParams S)
     // peers write into this CTA's receive buffer from here on: where it overlaps the stages, everybody's MMAs
     // must have read theirs
     if (split > 1 && S.recv_off == 0) cluster_sync_all();
-    const int row = sh_row(split), TS = S.share;                                  // tokens this CTA finishes per pass
+    const int row = sh_row(split), n0 = S.n0, TS = S.share;                                  // tokens this CTA finishes per pass
     const uint32_t xbuf = smem_u32(smem) + (uint32_t) S.recv_off;             // [split][TS] rows of 128 fp32
     for (int p0 = 0; p0 < rows; p0 += TS * split)
     {
@@ -403,7 +410,7 @@ void exl3_gemm_short_kernel(const ShParams S)
                 uint32_t v[8];
                 asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
                              : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7])
-                             : "r"(tmem + ((uint32_t) (32 * q) << 16) + (uint32_t) (p0 + c0 + (NG > 1 && p0 + c0 >= S.n0 ? SH_MAX_N - S.n0 : 0))) : "memory");
+                             : "r"(tmem + ((uint32_t) (32 * q) << 16) + (uint32_t) (p0 + c0 + (NG > 1 && p0 + c0 >= n0 ? SH_MAX_N - n0 : 0))) : "memory");
                 asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
                 if (split == 1)
                 {
@@ -491,7 +498,7 @@ void exl3_gemm_short_kernel(const ShParams S)
 }
 
 typedef void (*sh_fn)(const ShParams);
-// kernel of a bit width and codebook: 16 decode warps, or for expert groups 8 and two CTAs per SM
-sh_fn sh_kernel(int K, int cb, bool grouped);
+// kernel of a bit width and codebook. grouped 0: dense, 16 decode warps; 1: expert groups, 8 warps and two CTAs per SM
+sh_fn sh_kernel(int K, int cb, int grouped);
 
 }  // namespace amp

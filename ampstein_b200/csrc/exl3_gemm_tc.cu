@@ -45,17 +45,10 @@ namespace amp {
 
 __device__ int g_tc_status;
 
-template <int K, int CB, bool GROUPED = false>
-__global__ __launch_bounds__(TC_THREADS, GROUPED ? 2 : 1)
+template <int K, int CB>
+__global__ __launch_bounds__(TC_THREADS, 1)
 void exl3_gemm_tc_kernel(const TcParams P)
 {
-    if constexpr (GROUPED)
-    {
-        // the whole CTA leaves, before any barrier or allocation
-        if ((int) blockIdx.y >= *P.g_ntiles || P.g_tile_rows[blockIdx.y] <= 0) return;
-        const unsigned char* bits = P.g_bits[(int) blockIdx.x / (P.n / TC_BN)];
-        if (bits && bits[P.g_tile_e[blockIdx.y]] != K) return;
-    }
     extern __shared__ __align__(1024) unsigned char smem_raw[];
     // 1024-byte alignment is required by the swizzled layout
     unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t) 1023);
@@ -64,31 +57,11 @@ void exl3_gemm_tc_kernel(const TcParams P)
     __shared__ volatile int s_bad;
 
     const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
-    // grouped instances size an x~ slot and the tensor-memory allocation by the launch's rows per
-    // tile: with 128-row tiles two CTAs share an SM (shared memory, 2 x 128 accumulator columns)
-    const int a_bytes = GROUPED ? P.sub * (TC_BM * TC_BK * 2) : TC_A_BYTES;
-    const uint32_t tmem_cols = GROUPED ? (P.sub == 1 ? 128u : (P.sub == 2 ? 256u : 512u)) : 512u;
-    TcSlice W;
-    int m0, rows;                                       // first row and valid token rows of this CTA
-    if constexpr (GROUPED)
-    {
-        const int tile = blockIdx.y, bpk = P.n / TC_BN, kind = (int) blockIdx.x / bpk;
-        const size_t idx = (size_t) kind * P.g_experts + P.g_tile_e[tile];
-        W.trellis = reinterpret_cast<const unsigned char*>(P.t_trellis[idx]);
-        W.svh = reinterpret_cast<const __half*>(P.t_svh[idx]);
-        W.c = reinterpret_cast<unsigned char*>(P.c) + (size_t) kind * P.M * P.n * (P.c_fp32 ? 4 : 2);
-        W.xt = P.xt + (size_t) kind * P.M * P.k * 2;
-        W.n_row = P.n;
-        W.nb = (int) blockIdx.x - kind * bpk;
-        m0 = P.g_tile_row0[tile];
-        rows = min(P.g_tile_rows[tile], P.sub * TC_BM);
-    }
-    else
-    {
-        W = tc_slice<TC_BN>(P, blockIdx.x);
-        m0 = (int) blockIdx.y * (P.sub * TC_BM);
-        rows = min(P.sub * TC_BM, P.M - m0);
-    }
+    constexpr int a_bytes = TC_A_BYTES;
+    constexpr uint32_t tmem_cols = 512u;
+    const TcSlice W = tc_slice<TC_BN>(P, blockIdx.x);
+    const int m0 = (int) blockIdx.y * (P.sub * TC_BM);   // first row and valid token rows of this CTA
+    const int rows = min(P.sub * TC_BM, P.M - m0);
     const int nb = W.nb;
     const int nsub = (rows + TC_BM - 1) / TC_BM;        // sub-tiles that hold any of them
     const int ksteps = P.k / TC_BK;
@@ -794,11 +767,6 @@ typedef void (*tc_fn)(const TcParams);
                          exl3_gemm_tc_kernel<5, cb>, exl3_gemm_tc_kernel<6, cb>, exl3_gemm_tc_kernel<7, cb>, exl3_gemm_tc_kernel<8, cb> }
 static const tc_fn k_tc[3][8] = { AMP_TC_ROW(0), AMP_TC_ROW(1), AMP_TC_ROW(2) };
 #undef AMP_TC_ROW
-#define AMP_TCG_ROW(cb) { exl3_gemm_tc_kernel<1, cb, true>, exl3_gemm_tc_kernel<2, cb, true>, exl3_gemm_tc_kernel<3, cb, true>, \
-                          exl3_gemm_tc_kernel<4, cb, true>, exl3_gemm_tc_kernel<5, cb, true>, exl3_gemm_tc_kernel<6, cb, true>, \
-                          exl3_gemm_tc_kernel<7, cb, true>, exl3_gemm_tc_kernel<8, cb, true> }
-static const tc_fn k_tcg[3][8] = { AMP_TCG_ROW(0), AMP_TCG_ROW(1), AMP_TCG_ROW(2) };
-#undef AMP_TCG_ROW
 #define AMP_TC2_ROW(cb) { exl3_gemm_tc2_kernel<1, cb>, exl3_gemm_tc2_kernel<2, cb>, exl3_gemm_tc2_kernel<3, cb>, exl3_gemm_tc2_kernel<4, cb>, \
                           exl3_gemm_tc2_kernel<5, cb>, exl3_gemm_tc2_kernel<6, cb>, exl3_gemm_tc2_kernel<7, cb>, exl3_gemm_tc2_kernel<8, cb> }
 static const tc_fn k_tc2[3][8] = { AMP_TC2_ROW(0), AMP_TC2_ROW(1), AMP_TC2_ROW(2) };
@@ -894,38 +862,6 @@ int launch_gemm_tc(const void* xh, const void* trellis, void* c, const void* svh
     dim3 grid((unsigned) (slices * (n / 128)), (unsigned) mblocks);
     fn<<<grid, TC_THREADS, smem_bytes, stream>>>(P);
     return cuda_rc(cudaGetLastError(), "exl3_gemm_tc launch");
-}
-
-// Expert-grouped form for token-sorted MoE prefill: xt / c are (kinds, Mcap, k / n) in the padded,
-// expert-sorted row space, the tile table lives in device memory (see TcParams). One CTA per
-// (tile, projection, 128-column block); the grid is sized for G.max_tiles and the surplus returns.
-int launch_gemm_tc_grouped(const void* xt, void* c, long Mcap, int k, int n, int K, int cb, int c_fp32,
-                           const long long* t_trellis, const long long* t_svh, const TcGroups& G, cudaStream_t stream)
-{
-    AMP_REQUIRE(xt && c && t_trellis && t_svh && G.ntiles && G.tile_e && G.tile_row0 && G.tile_rows, "exl3_moe_sorted: null pointer");
-    AMP_REQUIRE(K >= 1 && K <= 8 && cb >= 0 && cb <= 2, "exl3_moe_sorted: unsupported bitrate / codebook");
-    AMP_REQUIRE(Mcap >= 1 && Mcap <= 0x7fffffffL && k % 128 == 0 && n % 128 == 0 && k > 0 && n > 0, "exl3_moe_sorted: k and n must be multiples of 128");
-    AMP_REQUIRE(((uintptr_t) xt & 15) == 0 && ((uintptr_t) c & 15) == 0, "exl3_moe_sorted: misaligned pointer");
-    AMP_REQUIRE(G.kinds >= 1 && G.kinds <= 2 && G.sub >= 1 && G.sub <= TC_SUB && G.experts >= 1, "exl3_moe_sorted: bad grouping");
-    AMP_REQUIRE(G.max_tiles >= 1 && G.max_tiles <= 65535, "exl3_moe_sorted: too many row tiles");
-    int dev = 0;
-    if (cudaError_t e = cudaGetDevice(&dev)) return cuda_rc(e, "cudaGetDevice");
-    tc_fn fn = k_tcg[cb][K - 1];
-    // x~ slots sized by the rows per tile; never below the epilogue's 128 x 132 fp32 staging tile
-    int smem_bytes = 1024 + TC_A_SLOTS * G.sub * (TC_BM * TC_BK * 2) + TC_B_STAGES * TC_B_BYTES + TC_DECODE_WARPS * tc_p_stages(K) * 128 * K;
-    if (smem_bytes < 1024 + 128 * 132 * 4) smem_bytes = 1024 + 128 * 132 * 4;
-    if (cudaError_t e = ensure_smem(fn, smem_bytes, dev)) return cuda_rc(e, "exl3_moe_sorted smem attribute");
-    TcParams P = {};
-    P.xt = (const unsigned char*) xt; P.c = c;
-    P.M = (int) Mcap; P.k = k; P.n = n; P.c_fp32 = c_fp32; P.sub = G.sub;
-    P.t_trellis = t_trellis; P.t_svh = t_svh;
-    P.g_ntiles = G.ntiles; P.g_tile_e = G.tile_e; P.g_tile_row0 = G.tile_row0; P.g_tile_rows = G.tile_rows;
-    P.g_experts = G.experts;
-    P.g_bits[0] = G.bits[0]; P.g_bits[1] = G.bits[1];
-    if (int rc = tc_status_ptr(dev, &P.status)) return rc;
-    dim3 grid((unsigned) (G.kinds * (n / 128)), (unsigned) G.max_tiles);
-    fn<<<grid, TC_THREADS, smem_bytes, stream>>>(P);
-    return cuda_rc(cudaGetLastError(), "exl3_moe_sorted gemm launch");
 }
 
 }  // namespace amp

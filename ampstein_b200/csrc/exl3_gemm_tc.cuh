@@ -43,16 +43,16 @@ struct TcParams
     const long long* t_c;       // may be null: outputs stacked in c as (slices, M, n)
     const int* t_stride;        // may be null: row width = n
     const int* t_src;           // may be null: rotated input of slice i is source i
-    // expert groups (grouped instances of the single-CTA kernel): blockIdx.y walks a tile table
+    // expert groups (grouped instances of exl3_gemm_short_kernel): blockIdx.y walks a tile table
     // that a kernel in front of this one built from the routing, blockIdx.x = projection * (n / 128)
-    // + column block. A tile is up to sub * 128 consecutive rows of ONE expert in the padded,
+    // + column block. A tile is up to ShParams::tile consecutive rows of ONE expert in the padded,
     // expert-sorted row space of xt / c (M = its capacity); t_trellis / t_svh hold g_kinds *
     // g_experts entries, projection-major; projection p reads xt + p * M * k halves and writes
     // c + p * M * n elements.
     const int* g_ntiles;        // device: tiles in use (CTAs beyond it return at once)
     const int* g_tile_e;        // device: expert of a tile
     const int* g_tile_row0;     // device: first padded row of a tile (a multiple of 8)
-    const int* g_tile_rows;     // device: valid rows of a tile (1 .. sub * 128)
+    const int* g_tile_rows;     // device: valid rows of a tile (0: none)
     int g_experts;
     // experts of different bit widths: per projection a device table of the experts' widths (null:
     // all of this launch's width); a CTA whose expert has another width than this instance returns

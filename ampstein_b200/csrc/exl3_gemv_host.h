@@ -62,11 +62,11 @@ struct TcGroups
     const int* ntiles; const int* tile_e; const int* tile_row0; const int* tile_rows;
     int experts;         // entries per projection in the pointer tables
     int max_tiles;       // grid height: an upper bound of *ntiles
-    int sub;             // 128-row sub-tiles per tile (1..4)
+    int tile;            // most rows of a tile: a multiple of 16, at most 256
     int kinds;           // projections in one launch (gate and up: 2)
     const unsigned char* bits[2];   // per projection: device table of per-expert bit widths, or null (uniform)
 };
-int launch_gemm_tc_grouped(const void* xt, void* c, long Mcap, int k, int n, int K, int cb, int c_fp32,
+int launch_gemm_short_grouped(const void* xt, void* c, long Mcap, int k, int n, int K, int cb, int c_fp32,
                            const long long* t_trellis, const long long* t_svh, const TcGroups& G, cudaStream_t stream);
 
 // decode kernel of the half-integer bitrates (exl3_gemv_half.cu); xt = the rotated input, (m, k) fp16

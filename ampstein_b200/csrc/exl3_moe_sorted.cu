@@ -17,7 +17,7 @@
 //                                forms (gate's and up's input scales) in the k-step-major swizzled
 //                                layout the tensor-core GEMM fetches with bulk copies; notes, per
 //                                token, which padded rows belong to it.
-//   3. grouped tcgen05 GEMM      gate and up in one grid (exl3_gemm_tc_kernel<K, CB, true>): one CTA
+//   3. grouped tcgen05 GEMM      gate and up in one grid (exl3_gemm_short_kernel<..., true>): one CTA
 //                                per (tile, projection, 128 columns) decodes its weight block ONCE
 //                                for all rows of the tile; fp16 outputs as exl3_gemm gives them.
 //   4. moe_sorted_rotate_act     act(gate, up) * down's input scales, rotated, same layout.
@@ -39,7 +39,7 @@ namespace amp {
 
 constexpr int MS_GROUP_ROWS = 8;                   // rows per task of the rotation kernels: one per warp
 constexpr int MS_MAX_TOPK = 64;
-// 128-row sub-tiles per GEMM tile: 0 = chosen from the average rows per expert, 1..4 forced (A/B)
+// 128-row units per GEMM tile: 0 = by default, 1 or 2 forced (A/B)
 int g_ms_tile_sub = 0;
 
 // status bits (header word 2)
@@ -57,14 +57,12 @@ struct MsLayout
 
 static inline size_t up256(size_t v) { return (v + 255) & ~(size_t) 255; }
 
-// Rows per tile. A tile's weight block is decoded once for all its rows, so large tiles decode
-// least; but only the 128-row form leaves room for two CTAs per SM (shared memory and 2 x 128
-// accumulator columns), which hides one CTA's prologue and epilogue behind the other's main loop.
-static int ms_pick_sub(long A, long E)
+// Rows per tile in units of 128: 256-row tiles (one accumulator of the grouped GEMM, two CTAs per SM) at every chunk
+// size. Measured for 128 experts, top-8 (us, 128- / 256- / 512-row tiles): 512 tokens 289 / 290 / 442, 2048 tokens
+// 540 / 492 / 592, 8192 tokens 1742 / 1560 / 1694.
+static int ms_pick_sub()
 {
-    if (g_ms_tile_sub >= 1 && g_ms_tile_sub <= 4) return g_ms_tile_sub;
-    const long avg = A / (E > 0 ? E : 1);
-    return avg <= 192 ? 1 : 4;         // (256-row tiles lost to one of the two at every chunk size measured)
+    return g_ms_tile_sub ? g_ms_tile_sub : 2;
 }
 
 static MsLayout ms_layout(long T, long A, long E, long H, long I, int sub)
@@ -166,12 +164,16 @@ void moe_sorted_prep_kernel(const MsPrep P)
             P.sstart[e] = s0;
             P.pstart[e] = ok ? p0 : -1;
             if (ok)
+            {
+                // tiles of equal height (a multiple of 8: the swizzle phase of the rotated rows)
+                const int per = ((c + nt - 1) / nt + 7) & ~7;
                 for (int j = 0; j < nt; ++j)
                 {
                     P.tile_e[t0 + j] = e;
-                    P.tile_row0[t0 + j] = p0 + j * P.tile_cap;
-                    P.tile_rows[t0 + j] = min(P.tile_cap, c - j * P.tile_cap);
+                    P.tile_row0[t0 + j] = p0 + j * per;
+                    P.tile_rows[t0 + j] = max(0, min(per, c - j * per));
                 }
+            }
             else
                 for (int j = 0; j < nt && t0 + j < P.max_tiles; ++j)
                 {
@@ -240,6 +242,8 @@ __device__ __forceinline__ void ms_load_pieces(const __half* src, int pc, __half
 __global__ __launch_bounds__(256)
 void moe_sorted_rotate_in_kernel(const MsRot P)
 {
+    // (the GEMM behind this launch may set itself up and start its weight stream; its fetch warp waits for this grid)
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, pc = lane & 7, cl = lane >> 3;
     const int ntasks = P.hdr[0] * P.groups, chunks = P.H >> 7;
     for (int task = blockIdx.x; task < ntasks; task += gridDim.x)
@@ -302,6 +306,7 @@ void moe_sorted_rotate_in_kernel(const MsRot P)
 __global__ __launch_bounds__(256)
 void moe_sorted_rotate_act_kernel(const MsRot P)
 {
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, pc = lane & 7, cl = lane >> 3;
     const int ntasks = P.hdr[0] * P.groups, chunks = P.I >> 7;
     const __half* gbase = P.gu;                                                     // gate outputs (projection 0)
@@ -502,7 +507,7 @@ AMP_API int amp_exl3_moe_sorted(const amp_moe_sorted_args* a, cudaStream_t strea
     AMP_REQUIRE(a->act >= 0 && a->act <= 3, "exl3_moe_sorted: unknown activation");
     // (16 bytes also for every scale vector the tables point to: the rotation kernels load them in 16-byte pieces)
     AMP_REQUIRE(((uintptr_t) a->y & 15) == 0 && ((uintptr_t) a->out & 15) == 0, "exl3_moe_sorted: misaligned tensor");
-    const MsLayout L = ms_layout(a->T, a->A, a->E, a->H, a->I, ms_pick_sub(a->A, a->E));
+    const MsLayout L = ms_layout(a->T, a->A, a->E, a->H, a->I, ms_pick_sub());
     AMP_REQUIRE(a->workspace && ((uintptr_t) a->workspace & 255) == 0 &&
                 a->workspace_bytes >= amp_exl3_moe_sorted_workspace(a->T, a->A, a->E, a->H, a->I),
                 "exl3_moe_sorted: workspace missing, misaligned (256) or smaller than amp_exl3_moe_sorted_workspace()");
@@ -547,7 +552,7 @@ AMP_API int amp_exl3_moe_sorted(const amp_moe_sorted_args* a, cudaStream_t strea
 
     TcGroups G = {};
     G.ntiles = Pp.hdr; G.tile_e = Pp.tile_e; G.tile_row0 = Pp.tile_row0; G.tile_rows = Pp.tile_rows;
-    G.experts = E; G.max_tiles = L.max_tiles; G.sub = L.sub;
+    G.experts = E; G.max_tiles = L.max_tiles; G.tile = 128 * L.sub;
     const long long* tab = Pp.tab;
     __half* gu = (__half*) (ws + L.gu);
     const bool mixed = a->g_bits || a->u_bits || a->d_bits;
@@ -559,21 +564,21 @@ AMP_API int amp_exl3_moe_sorted(const amp_moe_sorted_args* a, cudaStream_t strea
         G.bits[0] = gated ? (const unsigned char*) a->g_bits : ub; G.bits[1] = ub;
         for (int K = 1; K <= 8; ++K)
             if (a->kmask_gu & (1 << (K - 1)))
-                if (int rc = launch_gemm_tc_grouped(ws + L.xt_gu, gu, L.mcap, a->H, a->I, K, a->cb, 0,
+                if (int rc = launch_gemm_short_grouped(ws + L.xt_gu, gu, L.mcap, a->H, a->I, K, a->cb, 0,
                                                     gated ? tab : tab + E, gated ? tab + 2 * E : tab + 3 * E, G, stream)) return rc;
     }
     else if (gated && a->Kg == a->Ku)
     {
         G.kinds = 2;
-        if (int rc = launch_gemm_tc_grouped(ws + L.xt_gu, gu, L.mcap, a->H, a->I, a->Ku, a->cb, 0, tab, tab + 2 * E, G, stream)) return rc;
+        if (int rc = launch_gemm_short_grouped(ws + L.xt_gu, gu, L.mcap, a->H, a->I, a->Ku, a->cb, 0, tab, tab + 2 * E, G, stream)) return rc;
     }
     else
     {
         G.kinds = 1;
         if (gated)
-            if (int rc = launch_gemm_tc_grouped(ws + L.xt_gu, gu, L.mcap, a->H, a->I, a->Kg, a->cb, 0, tab, tab + 2 * E, G, stream)) return rc;
+            if (int rc = launch_gemm_short_grouped(ws + L.xt_gu, gu, L.mcap, a->H, a->I, a->Kg, a->cb, 0, tab, tab + 2 * E, G, stream)) return rc;
         const size_t po = gated ? (size_t) L.mcap : 0;       // up is projection 1 when gated
-        if (int rc = launch_gemm_tc_grouped(ws + L.xt_gu + po * a->H * 2, gu + po * a->I, L.mcap, a->H, a->I, a->Ku, a->cb, 0,
+        if (int rc = launch_gemm_short_grouped(ws + L.xt_gu + po * a->H * 2, gu + po * a->I, L.mcap, a->H, a->I, a->Ku, a->cb, 0,
                                             tab + E, tab + 3 * E, G, stream)) return rc;
     }
 
@@ -587,7 +592,7 @@ AMP_API int amp_exl3_moe_sorted(const amp_moe_sorted_args* a, cudaStream_t strea
     G.bits[0] = G.bits[1] = mixed ? (const unsigned char*) a->d_bits : nullptr;
     for (int K = 1; K <= 8; ++K)
         if (mixed ? (a->kmask_d & (1 << (K - 1))) != 0 : K == a->Kd)
-            if (int rc = launch_gemm_tc_grouped(ws + L.xt_d, ws + L.dout, L.mcap, a->I, a->H, K, a->cb, 1, tab + 4 * E, tab + 5 * E, G, stream)) return rc;
+            if (int rc = launch_gemm_short_grouped(ws + L.xt_d, ws + L.dout, L.mcap, a->I, a->H, K, a->cb, 1, tab + 4 * E, tab + 5 * E, G, stream)) return rc;
 
     if (a->scratch)
     {
@@ -616,12 +621,12 @@ AMP_API int amp_exl3_moe_gather(float* out, const float* scratch, const void* fl
     return cuda_rc(cudaGetLastError(), "exl3_moe_gather launch");
 }
 
-// Rows per GEMM tile of amp_exl3_moe_sorted in units of 128: 0 (default) = chosen per call from the
-// average rows per expert, 1..4 = forced. For A/B measurements. Returns the previous setting.
+// Rows per GEMM tile of amp_exl3_moe_sorted in units of 128: 0 = default (2), 1 or 2 = forced (3 and 4 are taken
+// as 2). For A/B measurements. Returns the previous setting.
 AMP_API int amp_exl3_set_moe_sorted_tile(int sub)
 {
     const int prev = g_ms_tile_sub;
-    g_ms_tile_sub = (sub >= 0 && sub <= 4) ? sub : 0;
+    g_ms_tile_sub = sub <= 0 || sub > 4 ? 0 : (sub > 2 ? 2 : sub);
     return prev;
 }
 
