@@ -10,6 +10,7 @@
 #include <cuda_fp16.h>
 #include <cuda_runtime.h>
 #include <stdint.h>
+#include <type_traits>
 
 namespace amp {
 
@@ -146,43 +147,6 @@ __device__ __forceinline__ void warp_had128(float& h0, float& h1, float& h2, flo
     }
 }
 
-// 128-point Hadamard with eight lanes per 128-value chunk: lane piece pc (0..7) holds the two 16-byte
-// pieces (eight values each) at elements 8 pc .. and 64 + 8 pc .. . Same butterflies in the same
-// order as warp_had128 (index bits 0..6 in turn; lower = a + b, upper = a - b), hence the same bits
-// out: bits 0-2 and 6 inside the lane, bits 3-5 across the eight lanes. 3 shuffles per value
-// instead of 5, and both the loads and the stores of a chunk are whole 128-byte lines per eight lanes.
-__device__ __forceinline__ void oct_had128(float (&h)[16], int pc)
-{
-    #pragma unroll
-    for (int b = 1; b < 8; b <<= 1)
-        #pragma unroll
-        for (int i = 0; i < 16; ++i)
-            if (!(i & b))
-            {
-                const float lo = h[i], hi = h[i | b];
-                h[i] = lo + hi;
-                h[i | b] = lo - hi;
-            }
-    #pragma unroll
-    for (int m = 1; m <= 4; m <<= 1)
-    {
-        const bool up = (pc & m) != 0;
-        #pragma unroll
-        for (int i = 0; i < 16; ++i)
-        {
-            const float p = __shfl_xor_sync(0xffffffffu, h[i], m);
-            h[i] = up ? p - h[i] : h[i] + p;
-        }
-    }
-    #pragma unroll
-    for (int i = 0; i < 8; ++i)
-    {
-        const float lo = h[i], hi = h[i + 8];
-        h[i] = lo + hi;
-        h[i + 8] = lo - hi;
-    }
-}
-
 // Two fp32 additions / multiply-adds in one instruction (sm_100 packed forms; each half rounds as the scalar one)
 __device__ __forceinline__ float2 add_f32x2(float2 a, float2 b)
 {
@@ -203,16 +167,17 @@ __device__ __forceinline__ float2 fma_f32x2(float2 a, float2 b, float2 c)
 
 // 128-point Hadamard with four lanes per 128-value chunk: lane piece pc (0..3) holds in h[4 j .. 4 j + 3] the
 // eight values at elements 8 (pc + 4 j), j = 0..3, as pairs. Same butterflies in the same order as warp_had128
-// (bits 0-2 inside the lane, 3-4 across the four lanes, 5-6 inside), hence the same bits out; two shuffles
-// per value instead of five and half the additions thanks to the packed forms (a - b = fma(b, -1, a), exact
-// up to the one rounding of the sum).
+// (bits 0-2 inside the lane, 3-4 across the four lanes, 5-6 inside), hence the same bits out; two shuffles per
+// value instead of five and half the additions thanks to the packed forms (a - b = fma(b, -1, a), exact up to
+// the one rounding of the sum).
 __device__ __forceinline__ void quad_had128(float2 (&h)[16], int pc)
 {
     const float2 neg = make_float2(-1.0f, -1.0f);
     #pragma unroll
     for (int i = 0; i < 16; ++i) h[i] = make_float2(h[i].x + h[i].y, h[i].x - h[i].y);
-    #pragma unroll
-    for (int b = 1; b < 4; b <<= 1)
+    auto stage = [&](auto bit)
+    {
+        constexpr int b = decltype(bit)::value;
         #pragma unroll
         for (int i = 0; i < 16; ++i)
             if (!(i & b))
@@ -221,6 +186,8 @@ __device__ __forceinline__ void quad_had128(float2 (&h)[16], int pc)
                 h[i] = add_f32x2(lo, hi);
                 h[i | b] = fma_f32x2(hi, neg, lo);
             }
+    };
+    stage(std::integral_constant<int, 1>()); stage(std::integral_constant<int, 2>());
     #pragma unroll
     for (int m = 1; m <= 2; m <<= 1)
     {
@@ -233,16 +200,7 @@ __device__ __forceinline__ void quad_had128(float2 (&h)[16], int pc)
             h[i] = fma_f32x2(h[i], sg, p);
         }
     }
-    #pragma unroll
-    for (int b = 4; b < 16; b <<= 1)
-        #pragma unroll
-        for (int i = 0; i < 16; ++i)
-            if (!(i & b))
-            {
-                const float2 lo = h[i], hi = h[i | b];
-                h[i] = add_f32x2(lo, hi);
-                h[i | b] = fma_f32x2(hi, neg, lo);
-            }
+    stage(std::integral_constant<int, 4>()); stage(std::integral_constant<int, 8>());
 }
 
 struct alignas(8) half4 { __half2 x, y; };

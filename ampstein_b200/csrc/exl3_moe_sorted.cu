@@ -37,7 +37,6 @@
 
 namespace amp {
 
-constexpr int MS_GROUP_ROWS = 8;                   // rows per task of the rotation kernels: one per warp
 constexpr int MS_MAX_TOPK = 64;
 // 128-row units per GEMM tile: 0 = by default, 1 or 2 forced (A/B)
 int g_ms_tile_sub = 0;
@@ -52,7 +51,7 @@ constexpr int MS_E_SLOT = 16;                      // deferred sum: a slot index
 struct MsLayout
 {
     long mcap; int max_tiles, topk, sub;
-    size_t hdr, pstart, sstart, tile_e, tile_row0, tile_rows, fill, list, tab, xt_gu, gu, xt_d, dout, total;
+    size_t hdr, pstart, sstart, grp, tile_e, tile_row0, tile_rows, fill, list, tab, xt_gu, gu, xt_d, dout, total;
 };
 
 static inline size_t up256(size_t v) { return (v + 255) & ~(size_t) 255; }
@@ -79,6 +78,7 @@ static MsLayout ms_layout(long T, long A, long E, long H, long I, int sub)
     L.hdr = o;       o = up256(o + 4 * sizeof(int));
     L.pstart = o;    o = up256(o + (size_t) E * sizeof(int));
     L.sstart = o;    o = up256(o + (size_t) E * sizeof(int));
+    L.grp = o;       o = up256(o + (size_t) (L.mcap / 8) * sizeof(int));
     L.tile_e = o;    o = up256(o + (size_t) L.max_tiles * sizeof(int));
     L.tile_row0 = o; o = up256(o + (size_t) L.max_tiles * sizeof(int));
     L.tile_rows = o; o = up256(o + (size_t) L.max_tiles * sizeof(int));
@@ -97,7 +97,7 @@ static MsLayout ms_layout(long T, long A, long E, long H, long I, int sub)
 struct MsPrep
 {
     const long long* count; int E, lo, hi, T; long A; int mcap, max_tiles, tile_cap;
-    int* hdr; int* pstart; int* sstart; int* tile_e; int* tile_row0; int* tile_rows; int* fill;
+    int* hdr; int* pstart; int* sstart; int* grp; int* tile_e; int* tile_row0; int* tile_rows; int* fill;
     const long long* src[6];        // g_trellis, u_trellis, g_svh, u_svh, d_trellis, d_svh (g_* null when not gated)
     long long* tab;                 // [trellis: gate E, up E][svh: gate E, up E][down trellis E][down svh E]
 };
@@ -163,6 +163,8 @@ void moe_sorted_prep_kernel(const MsPrep P)
             if (ok && t0 + nt > P.max_tiles) { ok = false; status |= MS_E_TILES; }
             P.sstart[e] = s0;
             P.pstart[e] = ok ? p0 : -1;
+            if (!ok && pad)          // (rows that nobody owns: a group without rows)
+                for (int g = p0 >> 3; g < (p0 + pad) >> 3 && g < P.mcap >> 3; ++g) P.grp[g] = 0;
             if (ok)
             {
                 // tiles of equal height (a multiple of 8: the swizzle phase of the rotated rows)
@@ -183,6 +185,16 @@ void moe_sorted_prep_kernel(const MsPrep P)
         carry_s += tot_s; carry_p += tot_p; carry_t += tot_t;
     }
     status = __syncthreads_or(status);
+    // expert and valid rows of every 8-row group of the padded row space (what the row-wise kernels walk)
+    for (int e = t >> 5; e < P.E; e += 32)
+    {
+        const int p0 = P.pstart[e];
+        if (p0 < 0) continue;
+        const long long cl = P.count[e];
+        const int c = cl > 0 ? (int) cl : 0;
+        if (c < P.lo || c > P.hi) continue;
+        for (int g = t & 31; 8 * g < c; g += 32) P.grp[(p0 >> 3) + g] = e | (min(8, c - 8 * g) << 24);
+    }
     if (t == 0)
     {
         P.hdr[0] = min(carry_t, P.max_tiles);
@@ -194,69 +206,71 @@ void moe_sorted_prep_kernel(const MsPrep P)
 struct MsRot
 {
     const int* hdr; const int* pstart; const int* sstart;
-    const int* tile_e; const int* tile_row0; const int* tile_rows;
+    const int* grp;                                  // per 8-row group of the padded row space: expert | valid rows << 24
     int* status;
     const long long* tok_sorted; long A; int T, topk;
     const __half* y; int H;                          // gather source (T, H)
     const long long* g_suh; const long long* u_suh;  // g_suh null: not gated
     unsigned char* xt;                               // (kinds, k / 64, mcap, 128 bytes)
-    int mcap, groups;                                // groups: 8-row groups per tile
+    int mcap;
     int* fill; int2* list;
     // activation stage
     const __half* gu; int I; const long long* d_suh; int act, gated; float act_limit;
 };
 
-// a lane's 16 rotated values -> their place in the k-step-major, swizzled layout (see
-// had_tiled_kernel): k steps 2 * chunk and 2 * chunk + 1, 16-byte piece pc ^ (row & 7) of each
-__device__ __forceinline__ void ms_store_pieces(unsigned char* xt, int mcap, int p, int cb, int pc, const float (&h)[16])
+// a lane's 32 rotated values (quad_had128's layout) -> their place in the k-step-major, swizzled layout (see
+// had_tiled_kernel): piece pc + 4 j of the chunk is piece (pc + 4 j) % 8 of k step 2 * chunk + j / 2
+__device__ __forceinline__ void ms_store_pieces(unsigned char* xt, int mcap, int p, int cb, int pc, const float2 (&h)[16])
 {
     #pragma unroll
-    for (int j = 0; j < 2; ++j)
+    for (int j = 0; j < 4; ++j)
     {
-        const __half2 a = __floats2half2_rn(h[8 * j + 0] * kRScale, h[8 * j + 1] * kRScale);
-        const __half2 b = __floats2half2_rn(h[8 * j + 2] * kRScale, h[8 * j + 3] * kRScale);
-        const __half2 c = __floats2half2_rn(h[8 * j + 4] * kRScale, h[8 * j + 5] * kRScale);
-        const __half2 d = __floats2half2_rn(h[8 * j + 6] * kRScale, h[8 * j + 7] * kRScale);
         uint4 o;
-        o.x = *reinterpret_cast<const uint32_t*>(&a); o.y = *reinterpret_cast<const uint32_t*>(&b);
-        o.z = *reinterpret_cast<const uint32_t*>(&c); o.w = *reinterpret_cast<const uint32_t*>(&d);
-        unsigned char* row = xt + (((size_t) (2 * cb + j) * (size_t) mcap + (size_t) p) << 7);
-        *reinterpret_cast<uint4*>(row + ((pc ^ (p & 7)) << 4)) = o;
+        __half2* o2 = reinterpret_cast<__half2*>(&o);
+        #pragma unroll
+        for (int q = 0; q < 4; ++q) o2[q] = __floats2half2_rn(h[4 * j + q].x * kRScale, h[4 * j + q].y * kRScale);
+        unsigned char* row = xt + (((size_t) (2 * cb + (j >> 1)) * (size_t) mcap + (size_t) p) << 7);
+        *reinterpret_cast<uint4*>(row + (((pc + 4 * (j & 1)) ^ (p & 7)) << 4)) = o;
     }
 }
 
-// the lane's two pieces of a chunk (src = first value of the chunk): elements 8 pc .. and 64 + 8 pc ..
-__device__ __forceinline__ void ms_load_pieces(const __half* src, int pc, __half2 (&v)[8])
+// the lane's four 16-byte pieces of a chunk (src = first value of the chunk): elements 8 (pc + 4 j) ..
+__device__ __forceinline__ void ms_load_pieces(const __half* src, int pc, uint4 (&v)[4])
 {
     #pragma unroll
-    for (int j = 0; j < 2; ++j)
+    for (int j = 0; j < 4; ++j) v[j] = *reinterpret_cast<const uint4*>(src + 8 * (pc + 4 * j));
+}
+
+__device__ __forceinline__ void ms_scale(const uint4 (&v)[4], const uint4 (&s)[4], float2 (&h)[16])
+{
+    #pragma unroll
+    for (int j = 0; j < 4; ++j)
     {
-        const uint4 r = *reinterpret_cast<const uint4*>(src + 64 * j + 8 * pc);
-        v[4 * j + 0] = *reinterpret_cast<const __half2*>(&r.x); v[4 * j + 1] = *reinterpret_cast<const __half2*>(&r.y);
-        v[4 * j + 2] = *reinterpret_cast<const __half2*>(&r.z); v[4 * j + 3] = *reinterpret_cast<const __half2*>(&r.w);
+        const __half2* a = reinterpret_cast<const __half2*>(&v[j]);
+        const __half2* b = reinterpret_cast<const __half2*>(&s[j]);
+        #pragma unroll
+        for (int q = 0; q < 4; ++q) h[4 * j + q] = __half22float2(__hmul2(a[q], b[q]));
     }
 }
 
-// task = (tile, group of 8 rows): one row per warp; a warp takes four 128-value chunks of its row
-// per pass, eight lanes each.
-__global__ __launch_bounds__(256)
+// One row per warp; a warp takes eight 128-value chunks of its row per pass, four lanes each.
+// Bound by instruction issue (two rotations per assignment): the packed butterflies took 12000 rows of 2048 from
+// 47 to 29 us.
+__global__ __launch_bounds__(128, 5)
 void moe_sorted_rotate_in_kernel(const MsRot P)
 {
     // (the GEMM behind this launch may set itself up and start its weight stream; its fetch warp waits for this grid)
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, pc = lane & 7, cl = lane >> 3;
-    const int ntasks = P.hdr[0] * P.groups, chunks = P.H >> 7;
-    for (int task = blockIdx.x; task < ntasks; task += gridDim.x)
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, pc = lane & 3, cl = lane >> 2;
+    const int nrows = P.hdr[1], chunks = P.H >> 7;
+    for (int p = (int) blockIdx.x * 4 + warp; p < nrows; p += (int) gridDim.x * 4)
     {
-        const int tile = task / P.groups, rg = task - tile * P.groups;
-        const int rows = P.tile_rows[tile];
-        const int r = rg * MS_GROUP_ROWS + warp;
-        if (r >= rows) continue;
-        const int e = P.tile_e[tile], row0 = P.tile_row0[tile];
+        const int rec = P.grp[p >> 3], e = rec & 0xffffff;
+        if ((p & 7) >= (rec >> 24)) continue;
+        const int s = P.sstart[e] + (p - P.pstart[e]);
+        const long long tok = (s >= 0 && s < P.A) ? P.tok_sorted[s] : -1;
         const __half* gs = P.g_suh ? reinterpret_cast<const __half*>(P.g_suh[e]) : nullptr;
         const __half* us = reinterpret_cast<const __half*>(P.u_suh[e]);
-        const int p = row0 + r, s = P.sstart[e] + (row0 - P.pstart[e]) + r;
-        const long long tok = (s >= 0 && s < P.A) ? P.tok_sorted[s] : -1;
         if (tok < 0 || tok >= P.T)
         {
             if (lane == 0) atomicOr(P.status, MS_E_TOKEN);
@@ -270,74 +284,69 @@ void moe_sorted_rotate_in_kernel(const MsRot P)
         }
         const __half* src = P.y + (size_t) tok * P.H;
         unsigned char* xu = P.xt + (gs ? (size_t) P.mcap * P.H * 2 : 0);
-        for (int c0 = 0; c0 < chunks; c0 += 4)
+        #pragma unroll 1
+        for (int c0 = 0; c0 < chunks; c0 += 8)
         {
             const int cb = c0 + cl;
             const bool live = cb < chunks;                 // (idle lanes still take part in the shuffles)
             const int off = (live ? cb : 0) * 128;
-            __half2 v[8], su[8], sg[8];
-            float h[16];
+            uint4 v[4], sc[4];
+            float2 h[16];
             ms_load_pieces(src + off, pc, v);
-            ms_load_pieces(us + off, pc, su);
-            if (gs) ms_load_pieces(gs + off, pc, sg);
-            #pragma unroll
-            for (int i = 0; i < 8; ++i)
-            {
-                const __half2 a = __hmul2(v[i], su[i]);
-                h[2 * i] = __low2float(a); h[2 * i + 1] = __high2float(a);
-            }
-            oct_had128(h, pc);
+            ms_load_pieces(us + off, pc, sc);
+            ms_scale(v, sc, h);
+            if (gs) ms_load_pieces(gs + off, pc, sc);
+            quad_had128(h, pc);
             if (live) ms_store_pieces(xu, P.mcap, p, cb, pc, h);
             if (gs)
             {
-                #pragma unroll
-                for (int i = 0; i < 8; ++i)
-                {
-                    const __half2 a = __hmul2(v[i], sg[i]);
-                    h[2 * i] = __low2float(a); h[2 * i + 1] = __high2float(a);
-                }
-                oct_had128(h, pc);
+                ms_scale(v, sc, h);
+                quad_had128(h, pc);
                 if (live) ms_store_pieces(P.xt, P.mcap, p, cb, pc, h);
             }
         }
     }
 }
 
-__global__ __launch_bounds__(256)
+// task = 128-value chunks of a row: a warp takes eight consecutive (row, chunk) pairs of an expert's 8-row group, four
+// lanes each
+__global__ __launch_bounds__(256, 3)
 void moe_sorted_rotate_act_kernel(const MsRot P)
 {
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, pc = lane & 7, cl = lane >> 3;
-    const int ntasks = P.hdr[0] * P.groups, chunks = P.I >> 7;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, pc = lane & 3, cl = lane >> 2;
+    const int ngroups = P.hdr[1] >> 3, chunks = P.I >> 7;
     const __half* gbase = P.gu;                                                     // gate outputs (projection 0)
     const __half* ubase = P.gu + (P.gated ? (size_t) P.mcap * P.I : 0);              // up outputs
-    for (int task = blockIdx.x; task < ntasks; task += gridDim.x)
+    for (int g = blockIdx.x; g < ngroups; g += gridDim.x)
     {
-        const int tile = task / P.groups, rg = task - tile * P.groups;
-        const int rows = P.tile_rows[tile];
-        const int r = rg * MS_GROUP_ROWS + warp;
-        if (r >= rows) continue;
-        const int e = P.tile_e[tile], p = P.tile_row0[tile] + r;
+        const int rec = P.grp[g], e = rec & 0xffffff, rows = rec >> 24;
+        if (rows == 0) continue;
         const __half* ds = reinterpret_cast<const __half*>(P.d_suh[e]);
-        const __half* ur = ubase + (size_t) p * P.I;
-        const __half* gr = gbase + (size_t) p * P.I;
-        for (int c0 = 0; c0 < chunks; c0 += 4)
+        #pragma unroll 1
+        for (int cb = warp; cb < chunks; cb += 8)          // lane group cl: row cl of the group, chunk cb
         {
-            const int cb = c0 + cl;
-            const bool live = cb < chunks;
-            const int off = (live ? cb : 0) * 128;
-            __half2 u[8], g[8], sc[8];
-            float h[16];
-            ms_load_pieces(ur + off, pc, u);
-            ms_load_pieces((P.gated ? gr : ur) + off, pc, g);
-            ms_load_pieces(ds + off, pc, sc);
+            const bool live = cl < rows;                   // (idle lanes still take part in the shuffles)
+            const int p = 8 * g + (live ? cl : 0);
+            const __half* ur = ubase + (size_t) p * P.I + cb * 128;
+            const __half* gr = gbase + (size_t) p * P.I + cb * 128;
+            uint4 u[4], gt[4], sc[4];
+            float2 h[16];
+            ms_load_pieces(ur, pc, u);
+            ms_load_pieces(P.gated ? gr : ur, pc, gt);
+            ms_load_pieces(ds + cb * 128, pc, sc);
             #pragma unroll
-            for (int i = 0; i < 8; ++i)
+            for (int j = 0; j < 4; ++j)
             {
-                h[2 * i] = moe_act_gate(P.act, P.gated, __low2float(g[i]), __low2float(u[i]), P.act_limit) * __low2float(sc[i]);
-                h[2 * i + 1] = moe_act_gate(P.act, P.gated, __high2float(g[i]), __high2float(u[i]), P.act_limit) * __high2float(sc[i]);
+                const __half2* a = reinterpret_cast<const __half2*>(&gt[j]);
+                const __half2* b = reinterpret_cast<const __half2*>(&u[j]);
+                const __half2* c = reinterpret_cast<const __half2*>(&sc[j]);
+                #pragma unroll
+                for (int q = 0; q < 4; ++q)
+                    h[4 * j + q] = make_float2(moe_act_gate(P.act, P.gated, __low2float(a[q]), __low2float(b[q]), P.act_limit) * __low2float(c[q]),
+                                               moe_act_gate(P.act, P.gated, __high2float(a[q]), __high2float(b[q]), P.act_limit) * __high2float(c[q]));
             }
-            oct_had128(h, pc);
+            quad_had128(h, pc);
             if (live) ms_store_pieces(P.xt, P.mcap, p, cb, pc, h);
         }
     }
@@ -371,7 +380,7 @@ void moe_sorted_combine_kernel(const int* __restrict__ fill, const int2* __restr
     for (int c = t; c < (H >> 2); c += 256)
     {
         float4 acc = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-        #pragma unroll 4
+        #pragma unroll 8
         for (int j = 0; j < n; ++j)
         {
             const float4 v = __ldcs(reinterpret_cast<const float4*>(dout + (size_t) s_row[j] * H) + c);
@@ -393,15 +402,12 @@ void moe_sorted_to_slots_kernel(const MsRot P, const float* __restrict__ dout, c
                                 float* __restrict__ scratch, const long long* __restrict__ slot_base, long scratch_rows)
 {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int ntasks = P.hdr[0] * P.groups;
-    for (int task = blockIdx.x; task < ntasks; task += gridDim.x)
+    const int ngroups = P.hdr[1] >> 3;
+    for (int g = blockIdx.x; g < ngroups; g += gridDim.x)
     {
-        const int tile = task / P.groups, rg = task - tile * P.groups;
-        const int rows = P.tile_rows[tile];
-        const int r = rg * MS_GROUP_ROWS + warp;
-        if (r >= rows) continue;
-        const int e = P.tile_e[tile], row0 = P.tile_row0[tile];
-        const int in_expert = (row0 - P.pstart[e]) + r, p = row0 + r, s = P.sstart[e] + in_expert;
+        const int rec = P.grp[g], e = rec & 0xffffff;
+        if (warp >= (rec >> 24)) continue;
+        const int p = 8 * g + warp, in_expert = p - P.pstart[e], s = P.sstart[e] + in_expert;
         const long long slot = slot_base[e] + in_expert;
         if (slot < 0 || slot >= scratch_rows || s < 0 || s >= P.A)
         {
@@ -522,6 +528,7 @@ AMP_API int amp_exl3_moe_sorted(const amp_moe_sorted_args* a, cudaStream_t strea
     Pp.hi = a->count_hi <= 0 ? 0x3fffffff : a->count_hi;
     Pp.mcap = (int) L.mcap; Pp.max_tiles = L.max_tiles; Pp.tile_cap = 128 * L.sub;
     Pp.hdr = (int*) (ws + L.hdr); Pp.pstart = (int*) (ws + L.pstart); Pp.sstart = (int*) (ws + L.sstart);
+    Pp.grp = (int*) (ws + L.grp);
     Pp.tile_e = (int*) (ws + L.tile_e); Pp.tile_row0 = (int*) (ws + L.tile_row0); Pp.tile_rows = (int*) (ws + L.tile_rows);
     Pp.fill = (int*) (ws + L.fill);
     Pp.src[0] = gated ? (const long long*) a->g_trellis : nullptr; Pp.src[1] = (const long long*) a->u_trellis;
@@ -534,20 +541,20 @@ AMP_API int amp_exl3_moe_sorted(const amp_moe_sorted_args* a, cudaStream_t strea
     int dev = 0, sms = 148;
     if (cudaError_t e = cudaGetDevice(&dev)) return cuda_rc(e, "cudaGetDevice");
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    const int groups = 128 * L.sub / MS_GROUP_ROWS;
-    const long tasks_max = (long) L.max_tiles * groups;
-    const int rot_blocks = (int) (tasks_max < (long) sms * 8 ? tasks_max : (long) sms * 8);
+    const long groups_max = L.mcap / 8;
+    const int rot_blocks = (int) (groups_max < (long) sms * 8 ? groups_max : (long) sms * 8);
 
     MsRot R = {};
     R.hdr = Pp.hdr; R.pstart = Pp.pstart; R.sstart = Pp.sstart;
-    R.tile_e = Pp.tile_e; R.tile_row0 = Pp.tile_row0; R.tile_rows = Pp.tile_rows;
+    R.grp = Pp.grp;
     R.status = Pp.hdr + 2;
     R.tok_sorted = (const long long*) a->tok_sorted; R.A = a->A; R.T = a->T; R.topk = (int) (a->A / a->T);
     R.y = (const __half*) a->y; R.H = a->H;
     R.g_suh = gated ? (const long long*) a->g_suh : nullptr; R.u_suh = (const long long*) a->u_suh;
-    R.xt = ws + L.xt_gu; R.mcap = (int) L.mcap; R.groups = groups;
+    R.xt = ws + L.xt_gu; R.mcap = (int) L.mcap;
     R.fill = Pp.fill; R.list = (int2*) (ws + L.list);
-    moe_sorted_rotate_in_kernel<<<rot_blocks, 256, 0, stream>>>(R);
+    const long in_blocks = L.mcap / 4;                 // (a row per warp)
+    moe_sorted_rotate_in_kernel<<<(unsigned) (in_blocks < (long) sms * 20 ? in_blocks : (long) sms * 20), 128, 0, stream>>>(R);
     if (cudaError_t e = cudaGetLastError()) return cuda_rc(e, "exl3_moe_sorted input rotation launch");
 
     TcGroups G = {};
