@@ -7,6 +7,7 @@ _HERE = os.path.dirname(os.path.abspath(__file__))
 LIB_PATH = os.path.join(_HERE, "libampstein_b200.so")
 
 _lib = None
+_fast = {}        # entries bound as builtins (csrc_py/fast_call.c); the others go through ctypes
 
 _vp = ctypes.c_void_p
 _i = ctypes.c_int
@@ -101,6 +102,11 @@ def lib():
         L.amp_comm_ctl_bytes.restype = ctypes.c_long
         L.amp_b200_last_error.restype = ctypes.c_char_p
         L.amp_b200_last_error.argtypes = []
+        try:
+            from . import _fast as builtins_
+        except ImportError as e:
+            raise ImportError("ampstein_b200: _fast.so is missing or stale; build it with `python -m ampstein_b200.build` (%s)" % e)
+        _fast.update({n: getattr(builtins_, n) for n in SIGNATURES if hasattr(builtins_, n)})
         _lib = L
     return _lib
 
@@ -111,7 +117,10 @@ def last_error():
 
 def call(name, *args):
     """Call a C-ABI entry point; raise AmpError on a non-zero return code."""
-    rc = getattr(lib(), name)(*args)
+    f = _fast.get(name)
+    if f is None:
+        f = getattr(lib(), name)            # (loads the library and fills _fast on the first call)
+    rc = f(*args)
     if rc != 0:
         raise AmpError(name, rc, last_error())
     return rc

@@ -62,7 +62,27 @@ def build(force=False, verbose=False):
         r = subprocess.run(cmd, capture_output=True, text=True)
         if r.returncode != 0:
             raise RuntimeError("link failed:\n%s\n%s" % (r.stdout, r.stderr))
+    build_fast_call(force)
     return LIB
+
+
+FAST_SRC = os.path.join(HERE, "csrc_py", "fast_call.c")
+FAST = os.path.join(HERE, "_fast.so")
+
+
+def build_fast_call(force=False):
+    """Builds ampstein_b200/_fast.so: the per-token entries of the C ABI as builtins (plain gcc)."""
+    header = os.path.join(HERE, "..", "include", "ampstein_b200.h")
+    if not force and os.path.exists(FAST) and os.path.getmtime(FAST) >= max(os.path.getmtime(FAST_SRC), os.path.getmtime(header)):
+        return FAST
+    import sysconfig
+    cuda = os.environ.get("CUDA_HOME", "/usr/local/cuda")
+    cmd = [os.environ.get("CC", "gcc"), "-O2", "-fPIC", "-shared", "-I" + sysconfig.get_paths()["include"], "-I" + os.path.join(cuda, "include"),
+           FAST_SRC, "-o", FAST, "-L" + HERE, "-lampstein_b200", "-Wl,-rpath,$ORIGIN"]
+    r = subprocess.run(cmd, capture_output=True, text=True)
+    if r.returncode != 0:
+        raise RuntimeError("fast-call build failed:\n%s\n%s" % (r.stdout, r.stderr))
+    return FAST
 
 
 GLUE_SRC = os.path.join(HERE, "csrc_torch", "torch_glue.cpp")

@@ -10,8 +10,21 @@ import torch
 from . import _lib
 
 
+_raw_stream = torch._C._cuda_getCurrentRawStream       # (torch.cuda.current_stream builds a Stream object: 2 us)
+_get_device = torch._C._cuda_getDevice
+
+
 def _stream(t):
-    return torch.cuda.current_stream(t.device).cuda_stream
+    return _raw_stream(t.get_device())
+
+
+def _launch(t, name, *args):
+    """One call of the C ABI on t's device and its current stream (appended as the last argument)."""
+    dev = t.get_device()
+    if _get_device() == dev:
+        return _lib.call(name, *args, _raw_stream(dev))
+    with torch.cuda.device(dev):
+        return _lib.call(name, *args, _raw_stream(dev))
 
 
 def _check_cuda(name, *ts):
@@ -65,9 +78,8 @@ def exl3_reconstruct(unpacked, packed, K, mul1=False, mcg=False):
         raise TypeError("exl3_reconstruct: unpacked must be 2-D float16")
     if unpacked.shape[0] != k or unpacked.shape[1] != n:
         raise ValueError("exl3_reconstruct: unpacked must be (%d, %d)" % (k, n))
-    with torch.cuda.device(packed.device):
-        _lib.call("amp_exl3_reconstruct", unpacked.data_ptr(), packed.data_ptr(), k, n, _kcode("exl3_reconstruct", Kt, mul1),
-                  _cb(mul1, mcg), 0, n, _stream(packed))
+    _launch(packed, "amp_exl3_reconstruct", unpacked.data_ptr(), packed.data_ptr(), k, n, _kcode("exl3_reconstruct", Kt, mul1),
+                  _cb(mul1, mcg), 0, n)
     return unpacked
 
 
@@ -140,11 +152,10 @@ def had_r_128(input, output, pre_scale=None, post_scale=None, scale=1.0):
     for s in (pre_scale, post_scale):
         if s is not None and (s.dtype != torch.float16 or s.numel() < cols):
             raise ValueError("had_r_128: scale vectors must be float16 with one value per column")
-    with torch.cuda.device(input.device):
-        _lib.call("amp_had_r_128", input.data_ptr(), output.data_ptr(),
+    _launch(input, "amp_had_r_128", input.data_ptr(), output.data_ptr(),
                   pre_scale.data_ptr() if pre_scale is not None else None,
                   post_scale.data_ptr() if post_scale is not None else None,
-                  rows, cols, 3 if mixed else (1 if input.dtype == torch.float32 else 0), float(scale), _stream(input))
+                  rows, cols, 3 if mixed else (1 if input.dtype == torch.float32 else 0), float(scale))
     return output
 
 
@@ -185,11 +196,46 @@ def exl3_gemm(A, B, C, suh, svh, mul1=False, mcg=False):
     # (from five rows on it lets the input be rotated once instead of by every CTA; the half-rate
     # kernel always takes its input rotated)
     A_had = torch.empty(A.shape, dtype=torch.float16, device=A.device) if (m >= 5 or bf16 or half_rate) else None
-    with torch.cuda.device(A.device):
-        _lib.call("amp_exl3_gemm_bf16" if bf16 else "amp_exl3_gemm", A.data_ptr(), B.data_ptr(), C.data_ptr(),
+    _launch(A, "amp_exl3_gemm_bf16" if bf16 else "amp_exl3_gemm", A.data_ptr(), B.data_ptr(), C.data_ptr(),
                   suh.data_ptr(), A_had.data_ptr() if A_had is not None else None, svh.data_ptr(), m, k, n, K,
-                  _cb(mul1, mcg), 1 if C.dtype == torch.float32 else 0, _stream(A))
+                  _cb(mul1, mcg), 1 if C.dtype == torch.float32 else 0)
     return C
+
+
+class GemmPlan:
+    """A checked weight (trellis, suh, svh) as exl3_gemm takes it, for callers that apply it many times: run()
+    checks only the activations (the full check costs as much host time as a small launch). Holds the tensors it
+    was made from; matches() tells whether they are still the caller's."""
+
+    __slots__ = ("tensors", "k", "n", "K", "cb")
+
+    def __init__(self, trellis, suh, svh, mul1=False, mcg=False):
+        _check_cuda("exl3_gemm", trellis, suh, svh)
+        self.k, self.n, self.K = _trellis_dims("exl3_gemm", trellis)
+        if suh.dtype != torch.float16 or svh.dtype != torch.float16 or suh.numel() != self.k or svh.numel() != self.n:
+            raise ValueError("exl3_gemm: incompatible shapes")
+        self.cb = _cb(mul1, mcg)
+        self.tensors = (trellis, suh, svh)
+
+    def matches(self, trellis, suh, svh):
+        t = self.tensors
+        return t[0] is trellis and t[1] is suh and t[2] is svh
+
+    def run(self, x):
+        """The (m, n) fp16 result for a contiguous (m, k) fp16 CUDA tensor of at least one row on the weight's
+        device; None where x is anything else (the caller then takes exl3_gemm, which says what is wrong)."""
+        t, s, v = self.tensors
+        if x.dtype is not torch.float16 or x.dim() != 2 or not x.is_contiguous():
+            return None
+        m, k = x.shape
+        dev = x.get_device()
+        if k != self.k or m < 1 or dev < 0 or dev != t.get_device() or _get_device() != dev:
+            return None
+        y = x.new_empty((m, self.n))
+        had = x.new_empty((m, k)) if m >= 5 else None            # rotation scratch, as in exl3_gemm
+        _lib.call("amp_exl3_gemm", x.data_ptr(), t.data_ptr(), y.data_ptr(), s.data_ptr(), had.data_ptr() if m >= 5 else None, v.data_ptr(), m, k, self.n, self.K,
+                  self.cb, 0, _raw_stream(dev))
+        return y
 
 
 def exl3_gemm_silu_mul(gate, up, B, C, suh, svh, mul1=False, mcg=False):
@@ -210,9 +256,8 @@ def exl3_gemm_silu_mul(gate, up, B, C, suh, svh, mul1=False, mcg=False):
         raise ValueError("exl3_gemm_silu_mul: 1..16 rows (larger batches: silu_mul, then exl3_gemm)")
     if C.numel() != m * n or suh.numel() != k or svh.numel() != n:
         raise ValueError("exl3_gemm_silu_mul: incompatible shapes")
-    with torch.cuda.device(gate.device):
-        _lib.call("amp_exl3_gemv_silu_mul", gate.data_ptr(), up.data_ptr(), B.data_ptr(), C.data_ptr(), suh.data_ptr(),
-                  svh.data_ptr(), m, k, n, K, _cb(mul1, mcg), 1 if C.dtype == torch.float32 else 0, _stream(gate))
+    _launch(gate, "amp_exl3_gemv_silu_mul", gate.data_ptr(), up.data_ptr(), B.data_ptr(), C.data_ptr(), suh.data_ptr(),
+                  svh.data_ptr(), m, k, n, K, _cb(mul1, mcg), 1 if C.dtype == torch.float32 else 0)
     return C
 
 
@@ -239,10 +284,9 @@ def exl3_gemm_rms_norm_res(x, res, norm_w, eps, y, B, C, suh, svh, mul1=False, m
     m = x.numel() // k
     if x.shape[-1] != k or not 1 <= m <= 16 or C.numel() != m * n or suh.numel() != k or svh.numel() != n:
         raise ValueError("exl3_gemm_rms_norm_res: incompatible shapes (1..16 rows)")
-    with torch.cuda.device(x.device):
-        _lib.call("amp_exl3_gemv_rms_norm_res", x.data_ptr(), res.data_ptr(), norm_w.data_ptr(), float(eps), y.data_ptr(),
+    _launch(x, "amp_exl3_gemv_rms_norm_res", x.data_ptr(), res.data_ptr(), norm_w.data_ptr(), float(eps), y.data_ptr(),
                   B.data_ptr(), C.data_ptr(), suh.data_ptr(), svh.data_ptr(), m, k, n, K, _cb(mul1, mcg),
-                  1 if C.dtype == torch.float32 else 0, _stream(x))
+                  1 if C.dtype == torch.float32 else 0)
     return C
 
 
@@ -258,9 +302,8 @@ def exl3_gemm_add_res(x, B, suh, svh, h, y, ssq, mul1=False, mcg=False):
     if x.shape[-1] != k or not 1 <= m <= 16 or h.numel() != m * n or y.numel() != m * n or ssq.numel() < m * (n // 128) \
             or y.data_ptr() == h.data_ptr():
         raise ValueError("exl3_gemm_add_res: incompatible shapes (1..16 rows), or y aliases h")
-    with torch.cuda.device(x.device):
-        _lib.call("amp_exl3_gemv_add_res", x.data_ptr(), B.data_ptr(), suh.data_ptr(), svh.data_ptr(), h.data_ptr(), y.data_ptr(),
-                  ssq.data_ptr(), m, k, n, K, _cb(mul1, mcg), _stream(x))
+    _launch(x, "amp_exl3_gemv_add_res", x.data_ptr(), B.data_ptr(), suh.data_ptr(), svh.data_ptr(), h.data_ptr(), y.data_ptr(),
+                  ssq.data_ptr(), m, k, n, K, _cb(mul1, mcg))
     return y, ssq
 
 
@@ -273,9 +316,8 @@ def exl3_gemm_normed(y, ssq, norm_w, eps, B, C, suh, svh, mul1=False, mcg=False)
         raise TypeError("exl3_gemm_normed: y, norm_w fp16; ssq fp32; C fp16 or fp32")
     if y.shape[-1] != k or not 1 <= m <= 16 or C.numel() != m * n or ssq.numel() < m * (k // 128) or norm_w.numel() != k:
         raise ValueError("exl3_gemm_normed: incompatible shapes (1..16 rows)")
-    with torch.cuda.device(y.device):
-        _lib.call("amp_exl3_gemv_normed", y.data_ptr(), ssq.data_ptr(), norm_w.data_ptr(), float(eps), B.data_ptr(), C.data_ptr(),
-                  suh.data_ptr(), svh.data_ptr(), m, k, n, K, _cb(mul1, mcg), 1 if C.dtype == torch.float32 else 0, _stream(y))
+    _launch(y, "amp_exl3_gemv_normed", y.data_ptr(), ssq.data_ptr(), norm_w.data_ptr(), float(eps), B.data_ptr(), C.data_ptr(),
+                  suh.data_ptr(), svh.data_ptr(), m, k, n, K, _cb(mul1, mcg), 1 if C.dtype == torch.float32 else 0)
     return C
 
 
@@ -293,13 +335,12 @@ def mgemm_normed(y, ssq, norm_w, eps, B_ptrs, C, suh_ptrs, svh_ptrs, K, mcg, mul
     c_ptrs = n_stride = had_src = None
     if opts is not None:
         c_ptrs, n_stride, had_src = opts["c_ptrs"], opts["n_stride_list"], opts["had_src_list"]
-    with torch.cuda.device(y.device):
-        _lib.call("amp_exl3_mgemm_normed", y.data_ptr(), ssq.data_ptr(), norm_w.data_ptr(), float(eps),
+    _launch(y, "amp_exl3_mgemm_normed", y.data_ptr(), ssq.data_ptr(), norm_w.data_ptr(), float(eps),
                   B_ptrs.data_ptr(), C.data_ptr(), suh_ptrs.data_ptr(), svh_ptrs.data_ptr(), num, m, k, width,
                   int(K), _cb(mul1, mcg), 1 if C.dtype == torch.float32 else 0,
                   c_ptrs.data_ptr() if c_ptrs is not None else None,
                   n_stride.data_ptr() if n_stride is not None else None,
-                  had_src.data_ptr() if had_src is not None else None, _stream(y))
+                  had_src.data_ptr() if had_src is not None else None)
     return C
 
 
@@ -313,9 +354,8 @@ def rms_norm_res(x, res, norm_w, eps, y=None, n=None):
     if any(t.dtype != torch.float16 for t in (x, res, norm_w, y, n)) or x.shape != res.shape or norm_w.numel() != x.shape[-1]:
         raise TypeError("rms_norm_res: float16 tensors of one shape, norm_w one value per column")
     dim = x.shape[-1]
-    with torch.cuda.device(x.device):
-        _lib.call("amp_b200_rms_norm_res", x.data_ptr(), res.data_ptr(), norm_w.data_ptr(), y.data_ptr(), n.data_ptr(),
-                  x.numel() // dim, dim, float(eps), _stream(x))
+    _launch(x, "amp_b200_rms_norm_res", x.data_ptr(), res.data_ptr(), norm_w.data_ptr(), y.data_ptr(), n.data_ptr(),
+                  x.numel() // dim, dim, float(eps))
     return y, n
 
 
@@ -325,8 +365,7 @@ def silu_mul(g, u, out=None):
     _check_cuda("silu_mul", g, u, out)
     if g.dtype != torch.float16 or u.dtype != torch.float16 or out.dtype != torch.float16 or g.shape != u.shape:
         raise TypeError("silu_mul: float16 tensors of one shape")
-    with torch.cuda.device(g.device):
-        _lib.call("amp_b200_silu_mul", g.data_ptr(), u.data_ptr(), out.data_ptr(), g.numel(), _stream(g))
+    _launch(g, "amp_b200_silu_mul", g.data_ptr(), u.data_ptr(), out.data_ptr(), g.numel())
     return out
 
 
@@ -336,9 +375,8 @@ def argmax_advance(logits, ids, pos, log, ws):
     _check_cuda("argmax_advance", logits, ids, pos, log, ws)
     if logits.dtype != torch.float16 or ids.dtype != torch.int64 or pos.dtype != torch.int64 or log.dtype != torch.int64:
         raise TypeError("argmax_advance: logits float16; ids, pos, log int64")
-    with torch.cuda.device(logits.device):
-        _lib.call("amp_b200_argmax_advance", logits.data_ptr(), logits.numel(), ids.data_ptr(), pos.data_ptr(), log.data_ptr(),
-                  log.numel(), ws.data_ptr(), _stream(logits))
+    _launch(logits, "amp_b200_argmax_advance", logits.data_ptr(), logits.numel(), ids.data_ptr(), pos.data_ptr(), log.data_ptr(),
+                  log.numel(), ws.data_ptr())
 
 
 def lm_head_argmax(x, res, norm_w, eps, y, B, logits, suh, svh, ids, pos, log, ws, vocab=None, mul1=False, mcg=False):
@@ -361,10 +399,9 @@ def lm_head_argmax(x, res, norm_w, eps, y, B, logits, suh, svh, ids, pos, log, w
     vocab = n if vocab is None else int(vocab)
     if not 1 <= vocab <= n:
         raise ValueError("lm_head_argmax: vocab out of range")
-    with torch.cuda.device(x.device):
-        _lib.call("amp_exl3_lm_head_argmax", x.data_ptr(), res.data_ptr(), norm_w.data_ptr(), float(eps), y.data_ptr(),
+    _launch(x, "amp_exl3_lm_head_argmax", x.data_ptr(), res.data_ptr(), norm_w.data_ptr(), float(eps), y.data_ptr(),
                   B.data_ptr(), logits.data_ptr(), suh.data_ptr(), svh.data_ptr(), k, n, K, _cb(mul1, mcg), vocab,
-                  ids.data_ptr(), pos.data_ptr(), log.data_ptr(), log.numel(), ws.data_ptr(), _stream(x))
+                  ids.data_ptr(), pos.data_ptr(), log.data_ptr(), log.numel(), ws.data_ptr())
     return logits
 
 
@@ -391,13 +428,12 @@ def mgemm_rms_norm_res(x, res, norm_w, eps, y, B_ptrs, C, suh_ptrs, svh_ptrs, K,
             raise ValueError("mgemm_rms_norm_res: slice tables do not match C")
     if B_ptrs.numel() < num or svh_ptrs.numel() < num:
         raise ValueError("mgemm_rms_norm_res: pointer tables shorter than the matrix count")
-    with torch.cuda.device(x.device):
-        _lib.call("amp_exl3_mgemm_rms_norm_res", x.data_ptr(), res.data_ptr(), norm_w.data_ptr(), float(eps), y.data_ptr(),
+    _launch(x, "amp_exl3_mgemm_rms_norm_res", x.data_ptr(), res.data_ptr(), norm_w.data_ptr(), float(eps), y.data_ptr(),
                   B_ptrs.data_ptr(), C.data_ptr(), suh_ptrs.data_ptr(), svh_ptrs.data_ptr(), num, m, k, width,
                   int(K), _cb(mul1, mcg), 1 if C.dtype == torch.float32 else 0,
                   c_ptrs.data_ptr() if c_ptrs is not None else None,
                   n_stride.data_ptr() if n_stride is not None else None,
-                  had_src.data_ptr() if had_src is not None else None, _stream(x))
+                  had_src.data_ptr() if had_src is not None else None)
     return C
 
 
@@ -496,13 +532,12 @@ def mgemm(x, B_ptrs, C, suh_ptrs, A_had, svh_ptrs, K, mcg, mul1, opts=None):
             raise ValueError("mgemm: A_had must be a contiguous float16 tensor of (sources, m, k)")
         if not x.is_contiguous():
             raise ValueError("mgemm: x must be contiguous")
-    with torch.cuda.device(x.device):
-        _lib.call("amp_exl3_mgemm_bf16" if bf16 else "amp_exl3_mgemm", x.data_ptr(), B_ptrs.data_ptr(), C.data_ptr(), suh_ptrs.data_ptr(),
+    _launch(x, "amp_exl3_mgemm_bf16" if bf16 else "amp_exl3_mgemm", x.data_ptr(), B_ptrs.data_ptr(), C.data_ptr(), suh_ptrs.data_ptr(),
                   A_had.data_ptr() if A_had is not None else None, svh_ptrs.data_ptr(), num, m, k, width,
                   int(K), _cb(mul1, mcg), 1 if C.dtype == torch.float32 else 0,
                   c_ptrs.data_ptr() if c_ptrs is not None else None,
                   n_stride.data_ptr() if n_stride is not None else None,
-                  had_src.data_ptr() if had_src is not None else None, num_had_src, _stream(x))
+                  had_src.data_ptr() if had_src is not None else None, num_had_src)
     return C
 
 
@@ -634,8 +669,7 @@ def moe_coop(x, sel, rw, cfg, sh_out=None):
         _moe_bit_masks("exl3_moe_coop", cfg, a.n_local, gated)
         a.g_bits, a.u_bits, a.d_bits = p(cfg["g_bits"]), p(cfg["u_bits"]), p(cfg["d_bits"])
         a.kmask_gu, a.kmask_d = cfg["_kmask"]
-    with torch.cuda.device(x.device):
-        _lib.call("amp_exl3_moe_coop", ctypes.byref(a), _stream(x))
+    _launch(x, "amp_exl3_moe_coop", ctypes.addressof(a))
     return None
 
 
@@ -701,9 +735,8 @@ def exl3_shard_cols(trellis, svh, ranges):
     out = torch.empty((k // 16, total // 16, trellis.shape[2]), dtype=trellis.dtype, device=trellis.device)
     out_svh = torch.empty(total, dtype=torch.float16, device=trellis.device)
     flat = (ctypes.c_int * (2 * len(ranges)))(*[v for r in ranges for v in r])
-    with torch.cuda.device(trellis.device):
-        _lib.call("amp_exl3_shard_cols", trellis.data_ptr(), svh.data_ptr(), out.data_ptr(), out_svh.data_ptr(), k, n, K,
-                  ctypes.cast(flat, ctypes.c_void_p), len(ranges), _stream(trellis))
+    _launch(trellis, "amp_exl3_shard_cols", trellis.data_ptr(), svh.data_ptr(), out.data_ptr(), out_svh.data_ptr(), k, n, K,
+                  ctypes.cast(flat, ctypes.c_void_p), len(ranges))
     return out, out_svh
 
 
@@ -720,9 +753,8 @@ def exl3_shard_rows(trellis, suh, k0, klen):
         raise ValueError("models.rows: range [%d, %d] not 128-aligned/in bounds" % (k0, klen))
     out = torch.empty((klen // 16, n // 16, trellis.shape[2]), dtype=trellis.dtype, device=trellis.device)
     out_suh = torch.empty(klen, dtype=torch.float16, device=trellis.device)
-    with torch.cuda.device(trellis.device):
-        _lib.call("amp_exl3_shard_rows", trellis.data_ptr(), suh.data_ptr(), out.data_ptr(), out_suh.data_ptr(), k, n, K,
-                  k0, klen, _stream(trellis))
+    _launch(trellis, "amp_exl3_shard_rows", trellis.data_ptr(), suh.data_ptr(), out.data_ptr(), out_suh.data_ptr(), k, n, K,
+                  k0, klen)
     return out, out_suh
 
 
@@ -743,9 +775,8 @@ def moe_prep(idx, w, n_experts, e0=0):
     count, start, kind = torch.empty(E + 1, **lo), torch.empty(E + 1, **lo), torch.empty(E, **lo)
     if A == 0:
         return [fe, order, tok, wts, count.zero_(), start.zero_(), inv, kind.zero_()]
-    with torch.cuda.device(idx.device):
-        _lib.call("amp_moe_prep", idx.data_ptr(), w.data_ptr(), A, K, E, int(e0), fe.data_ptr(), order.data_ptr(),
-                  tok.data_ptr(), wts.data_ptr(), count.data_ptr(), start.data_ptr(), inv.data_ptr(), kind.data_ptr(), _stream(idx))
+    _launch(idx, "amp_moe_prep", idx.data_ptr(), w.data_ptr(), A, K, E, int(e0), fe.data_ptr(), order.data_ptr(),
+                  tok.data_ptr(), wts.data_ptr(), count.data_ptr(), start.data_ptr(), inv.data_ptr(), kind.data_ptr())
     return [fe, order, tok, wts, count, start, inv, kind]
 
 
@@ -820,8 +851,7 @@ def moe_fused(y, out, count, tok_sorted, w_sorted, cfg, num_active=-1, lo=1, hi=
                 or slot_base.numel() < E:
             raise TypeError("moe_fused: scratch must be fp32 [slots, hidden], slot_base int64 with one entry per expert")
         a.scratch, a.slot_base, a.scratch_rows = p(scratch), p(slot_base), scratch.shape[0]
-    with torch.cuda.device(y.device):
-        _lib.call("amp_exl3_moe_sorted", ctypes.byref(a), _stream(y))
+    _launch(y, "amp_exl3_moe_sorted", ctypes.addressof(a))
     return None
 
 
@@ -833,8 +863,7 @@ def moe_fused_status(cfg, device=None):
     if ws is None:
         return 0
     out = ctypes.c_int(0)
-    with torch.cuda.device(ws.device):
-        _lib.call("amp_exl3_moe_sorted_status", ws.data_ptr(), ctypes.byref(out), _stream(ws))
+    _launch(ws, "amp_exl3_moe_sorted_status", ws.data_ptr(), ctypes.byref(out))
     return out.value
 
 
@@ -861,8 +890,7 @@ def moe_gather(out, scratch, flat_expert, inv_order, expert_start, slot_base, sl
     E = slot_kind.numel()
     if slot_base.numel() < E or expert_start.numel() < E:
         raise ValueError("moe_gather: table sizes")
-    with torch.cuda.device(out.device):
-        _lib.call("amp_exl3_moe_gather", out.data_ptr(), scratch.data_ptr(), flat_expert.data_ptr(), inv_order.data_ptr(),
+    _launch(out, "amp_exl3_moe_gather", out.data_ptr(), scratch.data_ptr(), flat_expert.data_ptr(), inv_order.data_ptr(),
                   expert_start.data_ptr(), slot_base.data_ptr(), slot_kind.data_ptr(), w_sorted.data_ptr(),
-                  T, H, flat_expert.numel() // T, E, scratch.shape[0], _stream(out))
+                  T, H, flat_expert.numel() // T, E, scratch.shape[0])
     return None

@@ -29,15 +29,25 @@ class LinearEXL3:
         self.mul1, self.mcg = mul1, mcg
         self.in_features = trellis.shape[0] * 16
         self.out_features = trellis.shape[1] * 16
+        self._plan = None
 
     def forward(self, x, out=None):
         m = x.shape[0]
+        if out is None and m <= RECON_ROWS:
+            # the per-token call: the weight is checked once, the activations each time
+            plan = self._plan
+            if plan is None or not plan.matches(self.trellis, self.suh, self.svh):
+                plan = self._plan = exl3.GemmPlan(self.trellis, self.suh, self.svh, self.mul1, self.mcg) if float(self.K) == int(self.K) else None
+            if plan is not None:
+                out = plan.run(x)
+                if out is not None:
+                    return out if self.bias is None else out.add(self.bias)
         if out is None and m > RECON_ROWS and self.out_features <= RECON_MAX_N:
             out = exl3.exl3_gemm_recon(x.contiguous(), self.trellis, self.suh, self.svh, self.K,
                                        self.mul1, self.mcg)
         else:
             if out is None:
-                out = torch.empty((m, self.out_features), dtype=torch.float16, device=x.device)
+                out = x.new_empty((m, self.out_features), dtype=torch.float16)
             exl3.exl3_gemm(x, self.trellis, out, self.suh, self.svh, self.mul1, self.mcg)
         if self.bias is not None:
             out = out.add(self.bias)
