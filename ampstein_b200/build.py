@@ -24,7 +24,7 @@ def units():
             continue
         per_width = {"exl3_gemv_inst.cu": "AMP_GEMV_K", "exl3_gemm_short_inst.cu": "AMP_SHORT_K"}.get(name)
         if per_width:                          # one object per bit width
-            for k in range(1, 9):
+            for k in list(range(1, 9)) + ([17, 18, 19] if per_width == "AMP_GEMV_K" else []):      # 16 + KA: KA + 0.5 bits
                 out.append((name, "%s_k%d.o" % (name[:-3], k), ["-D%s=%d" % (per_width, k)]))
         else:
             out.append((name, name[:-3] + ".o", []))

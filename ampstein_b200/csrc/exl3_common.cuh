@@ -99,15 +99,13 @@ __device__ __forceinline__ uint32_t mask16_fma(uint32_t x)
     return d;
 }
 
-// compile-time position inside a register chunk w[0..NW) preceded by `prev`; bit 0 of the chunk
-// is the MSB of w[0]. I = index of the weight inside the chunk. FMA: do the 16-bit mask on the
-// FMA-heavy pipe instead of the ALU.
-template <int K, int I, int NW, bool FMA = true>
-__device__ __forceinline__ uint32_t window_ct(const uint32_t (&w)[NW], uint32_t prev)
+// The 16 bits that end with bit LAST of a register chunk w[0..NW) preceded by `prev`; bit 0 of the chunk is the MSB
+// of w[0]. FMA: do the 16-bit mask on the FMA-heavy pipe instead of the ALU.
+template <int LAST, int NW, bool FMA = true>
+__device__ __forceinline__ uint32_t window_end_ct(const uint32_t (&w)[NW], uint32_t prev)
 {
-    constexpr int last = (I + 1) * K - 1;
-    constexpr int j1 = last / 32;
-    constexpr int sh = 31 - (last % 32);
+    constexpr int j1 = LAST / 32;
+    constexpr int sh = 31 - (LAST % 32);
     static_assert(j1 < NW, "window outside the chunk");
     if constexpr (sh + 16 <= 32)
     {
@@ -121,6 +119,13 @@ __device__ __forceinline__ uint32_t window_ct(const uint32_t (&w)[NW], uint32_t 
         const uint32_t v = __funnelshift_r(w[j1], hi, sh);
         return FMA ? mask16_fma(v) : (v & 0xffffu);
     }
+}
+
+// window of weight I of the chunk at K bits per weight
+template <int K, int I, int NW, bool FMA = true>
+__device__ __forceinline__ uint32_t window_ct(const uint32_t (&w)[NW], uint32_t prev)
+{
+    return window_end_ct<(I + 1) * K - 1, NW, FMA>(w, prev);
 }
 
 // ------------------------------------------------------------------------------------------

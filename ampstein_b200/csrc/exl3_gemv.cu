@@ -41,6 +41,9 @@ static gemv_fn gemv_kernel_for(int K, int cb, int MB, int mode, int gin)
         case 6: return gemv_kernel_k6(cb, MB, mode, gin);
         case 7: return gemv_kernel_k7(cb, MB, mode, gin);
         case 8: return gemv_kernel_k8(cb, MB, mode, gin);
+        case GEMV_HALF + 1: return gemv_kernel_k17(cb, MB, mode, gin);
+        case GEMV_HALF + 2: return gemv_kernel_k18(cb, MB, mode, gin);
+        case GEMV_HALF + 3: return gemv_kernel_k19(cb, MB, mode, gin);
     }
     return nullptr;
 }
@@ -172,7 +175,9 @@ int g_int8_max_k = int8_env("EXL3_INT8_GEMV_MAX_K", 6);
 int launch_gemv(const GemvLaunch& A, cudaStream_t stream)
 {
     const int m = A.m, k = A.k, K = A.K;
-    AMP_REQUIRE(K >= 1 && K <= 8, "exl3_gemv: unsupported EXL3 bitrate %d (integer 1..8)", K);
+    const bool half_rate = K > GEMV_HALF;
+    AMP_REQUIRE((K >= 1 && K <= 8) || (K <= GEMV_HALF + 3 && half_rate && A.cb == 2 && !A.mode && !A.tables),
+                "exl3_gemv: unsupported EXL3 bitrate %d (integer 1..8)", K);
     AMP_REQUIRE(A.cb >= 0 && A.cb <= 2, "exl3_gemv: codebook index %d out of range", A.cb);
     AMP_REQUIRE(m >= 1 && m <= 16, "exl3_gemv: m must be 1..16 (got %d)", m);
     AMP_REQUIRE(k > 0 && A.width > 0 && k % 128 == 0 && A.width % 128 == 0 && A.stride % 128 == 0,
@@ -201,7 +206,7 @@ int launch_gemv(const GemvLaunch& A, cudaStream_t stream)
     const DevInfo& D = dev_info(dev);
 
     const int MB = m <= 8 ? 1 : 2;
-    const bool tc = !A.mode && m <= TCV_MAX_M && g_gemv_tc && !A.arin.N && !A.ar.push_only && !A.x2 && !A.h_in && !A.norm_w;
+    const bool tc = !A.mode && !half_rate && m <= TCV_MAX_M && g_gemv_tc && !A.arin.N && !A.ar.push_only && !A.x2 && !A.h_in && !A.norm_w;
     // five rows or more with a scratch for the rotated input: rotate once, in a launch of its own
     const bool norm_producer = A.h_in != nullptr;                       // split norm, producer side
     const bool norm_consumer = A.norm_w != nullptr && A.ssq != nullptr && !A.x2;   // ... consumer side
@@ -776,19 +781,14 @@ static int gemm_any(const void* A, int a_bf16, const void* trellis, void* C, con
     if (m == 0) return 0;
     if (K > 256)
     {
-        // half-integer bitrate KA + 0.5 (K = AMP_EXL3_HALF_RATE(KA)), mul1 codebook: the input is rotated into
-        // A_had by the Hadamard kernel, then the half-rate decode kernel runs (up to 16 rows; the
-        // many-rows operator reconstructs the weight once instead, see exl3_gemm_recon)
+        // half-integer bitrate KA + 0.5 (K = AMP_EXL3_HALF_RATE(KA)), mul1 codebook: up to 16 rows on the decode
+        // kernel (the many-rows operator reconstructs the weight once instead, see exl3_gemm_recon)
         AMP_REQUIRE(K <= 256 + 3 && cb == 2, "exl3_gemm: half-integer bitrates are 1.5 / 2.5 / 3.5 with the mul1 codebook");
         AMP_REQUIRE(m <= 16 && !a_bf16, "exl3_gemm: half-integer bitrates take up to 16 fp16 rows here");
         AMP_REQUIRE(A && suh && A_had && k > 0 && k % 128 == 0, "exl3_gemm: half-integer bitrates need the A_had scratch (same shape as A)");
-        if (int rc = amp_had_r_128(A, A_had, suh, nullptr, m, k, 0, 1.0f, stream)) return rc;
-        int dev = 0;
-        if (cudaError_t e = cudaGetDevice(&dev)) return cuda_rc(e, "cudaGetDevice");
-        int* counters = nullptr; float* scratch = nullptr;
-        if (int rc = workspace_region(dev, stream, &counters, &scratch)) return rc;
-        return launch_gemv_half(A_had, trellis, svh, C, m, k, n, K - 256, c_fp32, counters, scratch, GEMV_SCRATCH_BYTES,
-                                GEMV_MAX_BLOCKS, dev_info(dev).sms, stream);
+        GemvLaunch L = direct(A, trellis, C, suh, svh, m, k, n, GEMV_HALF + K - 256, cb, c_fp32, 0, 0);
+        L.x_rot = A_had; L.num_src = 1;
+        return launch_gemv(L, stream);
     }
     if (m <= 16 && !a_bf16)
     {

@@ -1,5 +1,5 @@
 // Kernel instances of the trellis-decode GEMV for one bitrate; compiled once per K with
-// -DAMP_GEMV_K=<1..8> so the eight translation units build in parallel.
+// -DAMP_GEMV_K=<1..8, 17..19> (17..19: the half-integer rates) so the translation units build in parallel.
 #include "exl3_gemv_kernel.cuh"
 #include "exl3_gemv_tc.cuh"
 
@@ -12,6 +12,19 @@
 
 namespace amp {
 
+#if AMP_GEMV_K > 8
+// half-integer bitrates (mul1 codebook): single matrices, fp16 activations
+gemv_fn AMP_CAT(gemv_kernel_k, AMP_GEMV_K)(int cb, int MB, int mode, int gin)
+{
+    static const gemv_fn fn[2][2] =
+    {
+        { exl3_gemv_kernel<AMP_GEMV_K, 2, 1>, exl3_gemv_kernel<AMP_GEMV_K, 2, 2> },
+        { exl3_gemv_kernel<AMP_GEMV_K, 2, 1, 0, 2>, exl3_gemv_kernel<AMP_GEMV_K, 2, 2, 0, 2> },
+    };
+    if (cb != 2 || mode || (gin != 0 && gin != 2) || MB < 1 || MB > 2) return nullptr;
+    return fn[gin / 2][MB - 1];
+}
+#else
 gemv_fn AMP_CAT(gemv_kernel_k, AMP_GEMV_K)(int cb, int MB, int mode, int gin)
 {
     // input gathered from the all-reduce buffers (split exchange)
@@ -90,5 +103,6 @@ gemv_fn AMP_CAT(gemv_tc_kernel_k, AMP_GEMV_K)(int cb, int ar)
     if (cb < 0 || cb > 2) return nullptr;
     return fn[cb][ar ? 1 : 0];
 }
+#endif
 
 }  // namespace amp

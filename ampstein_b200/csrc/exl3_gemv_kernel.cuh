@@ -250,13 +250,24 @@ struct GemvParams
     int am_vocab;               // columns that take part (<= n)
 };
 
+// Bitrate parameter K of the kernels: 1..8 bits per weight, or GEMV_HALF + KA for the half-integer rate KA + 0.5
+// (positions alternate KA and KA + 1 bits: 2 KA + 1 bits a pair, mul1 codebook).
+constexpr int GEMV_HALF = 16;
+__host__ __device__ constexpr int gemv_tile_bytes(int K) { return K <= 8 ? 32 * K : 16 * (2 * (K - GEMV_HALF) + 1); }
+// registers that hold the packed words of a lane's 32 weights (a half rate: 16 (2 KA + 1) bits, the last word half used)
+__host__ __device__ constexpr int gemv_words(int K) { return K <= 8 ? K : K - GEMV_HALF + 1; }
+
 // A ring slot holds one unit of one warp: four tile rows (the 64-row group) of GEMV_NT adjacent
-// tiles, each row padded by 32 bytes so that the four rows start in different banks.
-__host__ __device__ constexpr int gemv_row_pitch(int K) { return GEMV_NT * 32 * K + 32; }   // bytes per tile row inside a slot
+// tiles, each row padded to 32 bytes more than a multiple of 128 (integer rates: to an odd multiple of 32) so
+// that the four rows start in different banks.
+__host__ __device__ constexpr int gemv_row_pitch(int K)        // bytes per tile row inside a slot
+{
+    return K <= 8 ? GEMV_NT * 32 * K + 32 : (GEMV_NT * gemv_tile_bytes(K) + 95) / 128 * 128 + 32;
+}
 __host__ __device__ constexpr int gemv_slot_bytes(int K) { return 4 * gemv_row_pitch(K); }
 // ring depth per warp: deep enough that a layer-sized matrix is requested almost whole when the
 // grid starts (a CTA's range is then 4-30 units), so HBM streams from the first microsecond on
-__host__ __device__ constexpr int gemv_stages(int K) { return K <= 4 ? 8 : (K <= 6 ? 6 : 5); }
+__host__ __device__ constexpr int gemv_stages(int K) { return K <= 4 || K > 8 ? 8 : (K <= 6 ? 6 : 5); }
 
 // byte offsets inside dynamic shared memory
 struct GemvSmem
@@ -294,6 +305,25 @@ __device__ __forceinline__ uint32_t lds32(uint32_t addr)
     uint32_t v;
     asm volatile("ld.shared.u32 %0, [%1];" : "=r"(v) : "r"(addr) : "memory");
     return v;
+}
+
+// The packed words of one lane at a half-integer rate, aligned to the start of its 32 weights: piece gq of a tile
+// starts at bit 16 (2 KA + 1) gq, in the middle of a word for odd gq. tile: shared address of the tile's words
+// (a ring of 4 (2 KA + 1)); prev: the 32 bits in front of the piece.
+template <int KA>
+__device__ __forceinline__ void load_chunk_half(uint32_t tile, int gq, uint32_t (&w)[KA + 1], uint32_t& prev)
+{
+    constexpr int B2 = 2 * KA + 1, W = 4 * B2;
+    const int first = (gq * B2) >> 1;
+    const uint32_t sel = (gq & 1) ? 0x1076u : 0x3210u;        // odd: each word moves up by 16 bits
+    uint32_t r[KA + 2];
+    r[0] = lds32(tile + 4 * (first == 0 ? W - 1 : first - 1));
+    #pragma unroll
+    for (int i = 0; i <= KA; ++i) r[i + 1] = lds32(tile + 4 * (first + i));
+    prev = __byte_perm(r[0], r[1], sel);
+    #pragma unroll
+    for (int i = 0; i < KA; ++i) w[i] = __byte_perm(r[i + 1], r[i + 2], sel);
+    w[KA] = __byte_perm(r[KA + 1], 0u, sel);
 }
 
 // K words of one lane's chunk from shared memory, widest loads the alignment allows
@@ -360,9 +390,22 @@ __device__ __forceinline__ uint32_t hi16_fma(uint32_t r)
 // word cut from the stream holds two states (high and low half): one funnel shift serves two
 // weights. Other bitrates cut each window on its own (shift on the ALU, mask on the FMA pipe).
 template <int K, int R, bool FMA = true>
-__device__ __forceinline__ void states8(const uint32_t (&w)[K], uint32_t prev, uint32_t (&s)[8])
+__device__ __forceinline__ void states8(const uint32_t (&w)[gemv_words(K)], uint32_t prev, uint32_t (&s)[8])
 {
-    if constexpr (K == 4 || K == 8)
+    if constexpr (K > 8)
+    {
+        // half-integer rate: pairs of positions of 2 KA + 1 bits, the first of a pair KA bits long
+        auto cut = [&](auto tag)
+        {
+            constexpr int I = R * 8 + decltype(tag)::value, KA = K - GEMV_HALF, B2 = 2 * KA + 1;
+            return window_end_ct<(I & 1) ? (I / 2 + 1) * B2 - 1 : (I / 2) * B2 + KA - 1, gemv_words(K), FMA>(w, prev);
+        };
+        s[0] = cut(std::integral_constant<int, 0>()); s[1] = cut(std::integral_constant<int, 1>());
+        s[2] = cut(std::integral_constant<int, 2>()); s[3] = cut(std::integral_constant<int, 3>());
+        s[4] = cut(std::integral_constant<int, 4>()); s[5] = cut(std::integral_constant<int, 5>());
+        s[6] = cut(std::integral_constant<int, 6>()); s[7] = cut(std::integral_constant<int, 7>());
+    }
+    else if constexpr (K == 4 || K == 8)
     {
         constexpr int D = 16 / K;                       // pair distance in positions
         int pair = 0;
@@ -395,11 +438,12 @@ __device__ __forceinline__ void states8(const uint32_t (&w)[K], uint32_t prev, u
 // word before them. xb: duplicated activations of the tile's 16 rows for this lane's batch
 // row(s), xb[r] = row r.
 template <int K, int CB, int MB, int R>
-__device__ __forceinline__ void decode_mma_r(const uint32_t (&w)[K], uint32_t prev, const uint32_t (&xb)[MB][16],
+__device__ __forceinline__ void decode_mma_r(const uint32_t (&w)[gemv_words(K)], uint32_t prev, const uint32_t (&xb)[MB][16],
                                              float (&acc0)[MB][4], float (&acc1)[MB][4])
 {
     uint32_t s[8], a[8];
-    states8<K, R>(w, prev, s);
+    // (codebook 2 already has the multiply and the byte sum on the FMA-heavy pipe: its fields are cut on the ALU)
+    states8<K, R, CB != 2>(w, prev, s);
     #pragma unroll
     for (int j = 0; j < 8; ++j) a[j] = a_word<CB>(s[j]);
     #pragma unroll
@@ -426,7 +470,7 @@ __device__ __forceinline__ int dp4a_us(uint32_t a, uint32_t b, int c)
 // code of tile row r; a0 / a1: columns gq and gq + 8 of the tile (two chains each). The multiply
 // and the dp4a both run on the FMA-heavy pipe, so the field extraction stays on the ALU.
 template <int K, int R>
-__device__ __forceinline__ void decode_dp4a_r(const uint32_t (&w)[K], uint32_t prev, const uint32_t (&xs)[16],
+__device__ __forceinline__ void decode_dp4a_r(const uint32_t (&w)[gemv_words(K)], uint32_t prev, const uint32_t (&xs)[16],
                                               int (&a0)[2], int (&a1)[2])
 {
     uint32_t s[8];
@@ -444,7 +488,7 @@ __device__ __forceinline__ void decode_dp4a_r(const uint32_t (&w)[K], uint32_t p
 // The same with a second set of activation codes (the int8 rounding error of the first set, quantised
 // again): the decoded products are shared, each costs one more dp4a.
 template <int K, int R>
-__device__ __forceinline__ void decode_dp4a2_r(const uint32_t (&w)[K], uint32_t prev, const uint32_t (&xs)[16], const uint32_t (&xr)[16],
+__device__ __forceinline__ void decode_dp4a2_r(const uint32_t (&w)[gemv_words(K)], uint32_t prev, const uint32_t (&xs)[16], const uint32_t (&xr)[16],
                                                int (&a0)[2], int (&a1)[2], int (&b0)[2], int (&b1)[2])
 {
     uint32_t s[8];
@@ -691,9 +735,9 @@ void exl3_gemv_kernel(const GemvParams P)
     constexpr int S = gemv_stages(K);
     constexpr int RP = gemv_row_pitch(K);
     constexpr int SLOT = gemv_slot_bytes(K);
-    constexpr int TILE_BYTES = 32 * K;
+    constexpr int TILE_BYTES = gemv_tile_bytes(K);
     constexpr int NT = GEMV_NT;
-    constexpr int ROWP = NT * 2 * K;                   // 16-byte pieces per tile row of a unit
+    constexpr int ROWP = NT * TILE_BYTES / 16;         // 16-byte pieces per tile row of a unit
     constexpr int PIECES = 4 * ROWP;                   // ... and per unit
     constexpr int NP = (PIECES + 31) / 32;             // copy instructions per unit and lane
 
@@ -1001,7 +1045,7 @@ void exl3_gemv_kernel(const GemvParams P)
     int xrow[MB];                                      // word offset of this lane's batch row in xd
     #pragma unroll
     for (int mb = 0; mb < MB; ++mb) xrow[mb] = min(mb * 8 + gq, m - 1) * XPITCH + pq * 4;
-    const uint32_t w_off = ring_s + pq * RP + gq * K * 4;                             // this lane's K words of the first tile
+    const uint32_t w_off = ring_s + pq * RP + (K <= 8 ? gq * K * 4 : 0);              // this lane's K words of the first tile (half rates: the tile)
     const uint32_t p_off = ring_s + pq * RP + ((gq * K + 8 * K - 1) % (8 * K)) * 4;   // the word before them (ring)
     const uint32_t xd_s = smem_u32(xd);
 
@@ -1535,12 +1579,20 @@ void exl3_gemv_kernel(const GemvParams P)
                     for (int i = 0; i < 4; ++i)
                         lds128(xaddr + xrow[mb] * 4 + i * 64, xb[mb][4 * i], xb[mb][4 * i + 1], xb[mb][4 * i + 2], xb[mb][4 * i + 3]);
 
-                uint32_t w[NT][K], prev[NT];
+                uint32_t w[NT][gemv_words(K)], prev[NT];
                 #pragma unroll
                 for (int nt = 0; nt < NT; ++nt)
                 {
+                    if constexpr (K > 8)
+                    {
+                        load_chunk_half<K - GEMV_HALF>(w_off + cslot + nt * TILE_BYTES, gq, w[nt], prev[nt]);
+                        continue;
+                    }
+                    else
+                    {
                     load_chunk_s<K>(w_off + cslot + nt * TILE_BYTES, w[nt]);
                     prev[nt] = lds32(p_off + cslot + nt * TILE_BYTES);
+                    }
                 }
                 if constexpr (CB == 4)
                 {
@@ -1912,6 +1964,7 @@ typedef void (*gemv_fn)(const GemvParams);
 #define AMP_GEMV_LOOKUP_DECL(K) gemv_fn gemv_kernel_k##K(int cb, int MB, int mode, int gin);
 AMP_GEMV_LOOKUP_DECL(1) AMP_GEMV_LOOKUP_DECL(2) AMP_GEMV_LOOKUP_DECL(3) AMP_GEMV_LOOKUP_DECL(4)
 AMP_GEMV_LOOKUP_DECL(5) AMP_GEMV_LOOKUP_DECL(6) AMP_GEMV_LOOKUP_DECL(7) AMP_GEMV_LOOKUP_DECL(8)
+AMP_GEMV_LOOKUP_DECL(17) AMP_GEMV_LOOKUP_DECL(18) AMP_GEMV_LOOKUP_DECL(19)
 #undef AMP_GEMV_LOOKUP_DECL
 
 }  // namespace amp
