@@ -440,6 +440,7 @@ void exl3_gemm_short_kernel(const ShParams S)
             // four lanes per token, eight tokens per warp in flight
             const int pc = lane & 3, cl = lane >> 2;
             const __half* svp = W.svh + (size_t) nb * 128 + 8 * pc;
+            const bool wide = (reinterpret_cast<uintptr_t>(W.c) & 15) == 0;      // (a bundle's outputs may be 8-byte aligned)
             for (int r0 = warp * 8; r0 < nt; r0 += NDEC * 8)
             {
                 const int r = r0 + cl;
@@ -465,8 +466,9 @@ void exl3_gemm_short_kernel(const ShParams S)
                 #pragma unroll
                 for (int j = 0; j < 4; ++j)
                 {
-                    const uint4 sv = *reinterpret_cast<const uint4*>(svp + 32 * j);
-                    const __half2* s2 = reinterpret_cast<const __half2*>(&sv);
+                    // (scale vectors are 8-byte aligned)
+                    const uint2 sv[2] = { *reinterpret_cast<const uint2*>(svp + 32 * j), *reinterpret_cast<const uint2*>(svp + 32 * j + 4) };
+                    const __half2* s2 = reinterpret_cast<const __half2*>(sv);
                     float2* v = h + 4 * j;
                     #pragma unroll
                     for (int q = 0; q < 4; ++q) { v[q].x *= kRScale; v[q].y *= kRScale; }
@@ -482,7 +484,9 @@ void exl3_gemm_short_kernel(const ShParams S)
                         __half2* o2 = reinterpret_cast<__half2*>(&o);
                         #pragma unroll
                         for (int q = 0; q < 4; ++q) o2[q] = __hmul2(__floats2half2_rn(v[q].x, v[q].y), s2[q]);
-                        *reinterpret_cast<uint4*>(reinterpret_cast<__half*>(W.c) + at + 32 * j) = o;
+                        __half* dst = reinterpret_cast<__half*>(W.c) + at + 32 * j;
+                        if (wide) *reinterpret_cast<uint4*>(dst) = o;
+                        else { reinterpret_cast<uint2*>(dst)[0] = make_uint2(o.x, o.y); reinterpret_cast<uint2*>(dst)[1] = make_uint2(o.z, o.w); }
                     }
                 }
             }

@@ -774,6 +774,30 @@ extern "C" int amp_had_r_128(const void* in, void* out, const void* pre, const v
 // a small launch of its own rotates the input into A_had once); more rows take the
 // tensor-core path: x~ is written into A_had (same shape as A, fp16: required) by the Hadamard
 // kernel and the tcgen05 GEMM consumes it. a_bf16: A holds bf16 instead of fp16 (m > 16 only).
+// Nine to sixteen rows: the decode kernel repeats the MMA of every weight for the second eight rows, the short-batch
+// tensor-core kernel takes the same time from 2 to 16 rows. Measured (us, tensor cores / decode kernel): 4096 x 4096
+// at 4 bits 9 rows 13.9 / 32.1, 16 rows 14.0 / 39.0; 4096 x 14336 8 rows 30.3 / 23.3, 9 rows 30.1 / 41.6; 25600 x
+// 5120 at 3 bits 8 rows 55.4 / 50.5, 16 rows 55.6 / 103. (Small matrices would gain from five rows on, 4096 x 4096
+// 8 rows 13.8 / 20.2, but up to eight rows every form of a linear -- fused norm, activation, all-reduce -- is one
+// kernel and gives the same bits. A_had plays no part: results do not depend on it.)
+static bool few_rows_on_tensor_cores(int m, long k, long n)
+{
+    return g_tc_short && m >= 9 && k * m * 6 <= (long) GEMV_SCRATCH_BYTES;
+}
+
+// Scratch for the rotated input where the caller gives none: the stream's workspace (ordered with everything else
+// on the stream that uses it)
+static int rotation_scratch(size_t values, cudaStream_t stream, void** out)
+{
+    int dev = 0;
+    if (cudaError_t e = cudaGetDevice(&dev)) return cuda_rc(e, "cudaGetDevice");
+    int* counters = nullptr; float* scratch = nullptr;
+    if (int rc = workspace_region(dev, stream, &counters, &scratch)) return rc;
+    AMP_REQUIRE(values * 2 <= (size_t) GEMV_SCRATCH_BYTES, "exl3_gemm: input too large for the workspace");
+    *out = scratch;
+    return 0;
+}
+
 static int gemm_any(const void* A, int a_bf16, const void* trellis, void* C, const void* suh, void* A_had,
                     const void* svh, int m, int k, int n, int K, int cb, int c_fp32, cudaStream_t stream)
 {
@@ -790,14 +814,16 @@ static int gemm_any(const void* A, int a_bf16, const void* trellis, void* C, con
         L.x_rot = A_had; L.num_src = 1;
         return launch_gemv(L, stream);
     }
-    if (m <= 16 && !a_bf16)
+    if (m <= 16 && !a_bf16 && !(few_rows_on_tensor_cores(m, k, n) && ((uintptr_t) C & 15) == 0 && ((uintptr_t) A_had & 15) == 0))
     {
         GemvLaunch L = direct(A, trellis, C, suh, svh, m, k, n, K, cb, c_fp32, 0, 0);
         L.x_rot = A_had;                               // optional: used from five rows up
         return launch_gemv(L, stream);
     }
-    AMP_REQUIRE(A_had, "exl3_gemm: A_had scratch (same shape as A, fp16) is required above 16 rows");
+    AMP_REQUIRE(A_had || (m <= 16 && !a_bf16), "exl3_gemm: A_had scratch (same shape as A, fp16) is required above 16 rows");
     AMP_REQUIRE(A && suh && k > 0 && k % 128 == 0, "exl3_gemm: bad input");
+    if (!A_had)
+        if (int rc = rotation_scratch((size_t) m * k, stream, &A_had)) return rc;
     if (int rc = launch_had_tiled(A, A_had, suh, m, k, a_bf16, stream)) return rc;
     return launch_gemm_tc(A_had, trellis, C, svh, m, k, n, K, cb, c_fp32, stream);
 }
@@ -835,12 +861,15 @@ static int mgemm_any(const void* x, int x_bf16, const void* trellis_ptrs, void* 
 {
     if (num == 0 || m == 0) return 0;
     AMP_REQUIRE(num > 0 && m > 0, "exl3_mgemm: negative matrix or row count");
-    if (m > 16 || x_bf16)
+    const int sources = had_src_list ? num_had_src : num;
+    const bool few = m <= 16 && !x_bf16;
+    if (!few || (sources >= 1 && sources <= 3 && ((uintptr_t) C & 15) == 0 && ((uintptr_t) A_had & 15) == 0 && few_rows_on_tensor_cores(m, k, (long) num * width)))
     {
         AMP_REQUIRE(x && trellis_ptrs && suh_ptrs && svh_ptrs && (C || c_ptrs), "exl3_mgemm: pointer tables are required");
-        AMP_REQUIRE(A_had, "exl3_mgemm: A_had scratch ((sources, m, k) fp16) is required above 16 rows");
+        AMP_REQUIRE(A_had || few, "exl3_mgemm: A_had scratch ((sources, m, k) fp16) is required above 16 rows");
         AMP_REQUIRE(!had_src_list || num_had_src >= 1, "exl3_mgemm: num_had_src missing");
-        const int sources = had_src_list ? num_had_src : num;
+        if (!A_had)
+            if (int rc = rotation_scratch((size_t) sources * m * k, stream, &A_had)) return rc;
         if (int rc = launch_had_tiled(x, A_had, nullptr, m, k, x_bf16, stream, (const long long*) suh_ptrs, sources)) return rc;
         TcTables T;
         T.num = num; T.trellis = (const long long*) trellis_ptrs; T.svh = (const long long*) svh_ptrs;

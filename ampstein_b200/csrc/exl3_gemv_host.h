@@ -70,5 +70,6 @@ int launch_gemm_short_grouped(const void* xt, void* c, long Mcap, int k, int n, 
                            const long long* t_trellis, const long long* t_svh, const TcGroups& G, cudaStream_t stream);
 
 extern int g_pdl;
+extern int g_tc_short;     // short-batch GEMM: 0 never, 1 by size, 2 always (exl3_gemm_tc.cu)
 
 }  // namespace amp
