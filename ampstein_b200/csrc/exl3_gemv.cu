@@ -126,7 +126,7 @@ int g_cluster = 1;        // cluster form of the partial-sum exchange
 // cycles per mma.sync it saves); kept for A/B runs (amp_exl3_set_gemv_tc).
 int g_gemv_tc = 0;
 // (with more than 16 units per CTA the grid of 8 x blocks CTAs is too coarse: measured slower)
-constexpr int GEMV_CLUSTER = 8, GEMV_CLUSTER_MAX_M = 4, GEMV_CLUSTER_MAX_UNITS = 16;
+constexpr int GEMV_CLUSTER = 8, GEMV_CLUSTER_MAX_M = 8, GEMV_CLUSTER_MAX_UNITS = 16;
 
 // x~ = fp16(H(x * suh) / sqrt(128)) of every source, (sources, m, k) fp16 row-major: one warp per
 // 128 values, the arithmetic of the GEMV kernel's own prologue (fp16 scale, fp32 butterfly, one
@@ -295,12 +295,20 @@ int launch_gemv(const GemvLaunch& A, cudaStream_t stream)
         if (S >= 1) ncta = col_blocks * S;
         else { ncta = (long) D.sms * ctas_per_sm; while (ncta > D.sms && units / ncta < 4) ncta -= D.sms; }
     }
-    // Layer-sized single matrices at small batch: one cluster of eight CTAs per column block. The
-    // partial sums then travel through distributed shared memory and a cluster barrier (about a
+    // Layer-sized single matrices at up to eight rows (4096 x 1024 at 8 rows 16.3 -> 9.8 us, 4096 x 4096 20.2 ->
+    // 17.0): one cluster of eight CTAs per column block. The partial sums then travel through distributed shared memory and a cluster barrier (about a
     // microsecond) instead of global memory, a fence, an atomic and a read-back (about three).
     int cluster = 0;
+    // (five rows and more: the exchange area and x~ of all rows may leave room for fewer CTAs per SM)
+    int cluster_ctas = ctas_per_sm;
+    if (m > 4 && !A.mode)
+    {
+        const int need = (G / GEMV_CLUSTER + 1 + 3) / 4 * 4;
+        const int fit = smem_per_sm / (gemv_smem_layout(K, m, need < xcap ? need : xcap, GEMV_CLUSTER).total + 1024);
+        if (fit < cluster_ctas) cluster_ctas = fit;
+    }
     if (!A.mode && !A.ws_counters && A.force_split == 0 && A.force_xgroups == 0 && m <= GEMV_CLUSTER_MAX_M && G % GEMV_CLUSTER == 0 &&
-        G / GEMV_CLUSTER >= 2 && G / GEMV_CLUSTER <= GEMV_CLUSTER_MAX_UNITS && col_blocks * GEMV_CLUSTER <= (long) D.sms * ctas_per_sm && g_cluster)
+        G / GEMV_CLUSTER >= 2 && G / GEMV_CLUSTER <= GEMV_CLUSTER_MAX_UNITS && col_blocks * GEMV_CLUSTER <= (long) D.sms * cluster_ctas && g_cluster)
     {
         cluster = GEMV_CLUSTER;
         ncta = col_blocks * GEMV_CLUSTER;
