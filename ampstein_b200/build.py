@@ -22,7 +22,7 @@ def units():
     for name in sorted(os.listdir(CSRC)):
         if not name.endswith(".cu"):
             continue
-        per_width = {"exl3_gemv_inst.cu": "AMP_GEMV_K", "exl3_gemm_short_inst.cu": "AMP_SHORT_K"}.get(name)
+        per_width = {"exl3_gemv_inst.cu": "AMP_GEMV_K", "exl3_gemm_tc_inst.cu": "AMP_TC_K"}.get(name)
         if per_width:                          # one object per bit width
             for k in list(range(1, 9)) + ([17, 18, 19] if per_width == "AMP_GEMV_K" else []):      # 16 + KA: KA + 0.5 bits
                 out.append((name, "%s_k%d.o" % (name[:-3], k), ["-D%s=%d" % (per_width, k)]))

@@ -790,7 +790,7 @@ extern "C" int amp_had_r_128(const void* in, void* out, const void* pre, const v
 // kernel and gives the same bits. A_had plays no part: results do not depend on it.)
 static bool few_rows_on_tensor_cores(int m, long k, long n)
 {
-    return g_tc_short && m >= 9 && k * m * 6 <= (long) GEMV_SCRATCH_BYTES;
+    return m >= 9 && k * m * 6 <= (long) GEMV_SCRATCH_BYTES;
 }
 
 // Scratch for the rotated input where the caller gives none: the stream's workspace (ordered with everything else

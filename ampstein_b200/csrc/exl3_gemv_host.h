@@ -66,10 +66,9 @@ struct TcGroups
     int kinds;           // projections in one launch (gate and up: 2)
     const unsigned char* bits[2];   // per projection: device table of per-expert bit widths, or null (uniform)
 };
-int launch_gemm_short_grouped(const void* xt, void* c, long Mcap, int k, int n, int K, int cb, int c_fp32,
+int launch_gemm_tc_grouped(const void* xt, void* c, long Mcap, int k, int n, int K, int cb, int c_fp32,
                            const long long* t_trellis, const long long* t_svh, const TcGroups& G, cudaStream_t stream);
 
 extern int g_pdl;
-extern int g_tc_short;     // short-batch GEMM: 0 never, 1 by size, 2 always (exl3_gemm_tc.cu)
 
 }  // namespace amp

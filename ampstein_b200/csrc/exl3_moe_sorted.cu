@@ -17,7 +17,7 @@
 //                                forms (gate's and up's input scales) in the k-step-major swizzled
 //                                layout the tensor-core GEMM fetches with bulk copies; notes, per
 //                                token, which padded rows belong to it.
-//   3. grouped tcgen05 GEMM      gate and up in one grid (exl3_gemm_short_kernel<..., true>): one CTA
+//   3. grouped tcgen05 GEMM      gate and up in one grid (exl3_gemm_tc_kernel<..., true>): one CTA
 //                                per (tile, projection, 128 columns) decodes its weight block ONCE
 //                                for all rows of the tile; fp16 outputs as exl3_gemm gives them.
 //   4. moe_sorted_rotate_act     act(gate, up) * down's input scales, rotated, same layout.
@@ -571,21 +571,21 @@ AMP_API int amp_exl3_moe_sorted(const amp_moe_sorted_args* a, cudaStream_t strea
         G.bits[0] = gated ? (const unsigned char*) a->g_bits : ub; G.bits[1] = ub;
         for (int K = 1; K <= 8; ++K)
             if (a->kmask_gu & (1 << (K - 1)))
-                if (int rc = launch_gemm_short_grouped(ws + L.xt_gu, gu, L.mcap, a->H, a->I, K, a->cb, 0,
+                if (int rc = launch_gemm_tc_grouped(ws + L.xt_gu, gu, L.mcap, a->H, a->I, K, a->cb, 0,
                                                     gated ? tab : tab + E, gated ? tab + 2 * E : tab + 3 * E, G, stream)) return rc;
     }
     else if (gated && a->Kg == a->Ku)
     {
         G.kinds = 2;
-        if (int rc = launch_gemm_short_grouped(ws + L.xt_gu, gu, L.mcap, a->H, a->I, a->Ku, a->cb, 0, tab, tab + 2 * E, G, stream)) return rc;
+        if (int rc = launch_gemm_tc_grouped(ws + L.xt_gu, gu, L.mcap, a->H, a->I, a->Ku, a->cb, 0, tab, tab + 2 * E, G, stream)) return rc;
     }
     else
     {
         G.kinds = 1;
         if (gated)
-            if (int rc = launch_gemm_short_grouped(ws + L.xt_gu, gu, L.mcap, a->H, a->I, a->Kg, a->cb, 0, tab, tab + 2 * E, G, stream)) return rc;
+            if (int rc = launch_gemm_tc_grouped(ws + L.xt_gu, gu, L.mcap, a->H, a->I, a->Kg, a->cb, 0, tab, tab + 2 * E, G, stream)) return rc;
         const size_t po = gated ? (size_t) L.mcap : 0;       // up is projection 1 when gated
-        if (int rc = launch_gemm_short_grouped(ws + L.xt_gu + po * a->H * 2, gu + po * a->I, L.mcap, a->H, a->I, a->Ku, a->cb, 0,
+        if (int rc = launch_gemm_tc_grouped(ws + L.xt_gu + po * a->H * 2, gu + po * a->I, L.mcap, a->H, a->I, a->Ku, a->cb, 0,
                                             tab + E, tab + 3 * E, G, stream)) return rc;
     }
 
@@ -599,7 +599,7 @@ AMP_API int amp_exl3_moe_sorted(const amp_moe_sorted_args* a, cudaStream_t strea
     G.bits[0] = G.bits[1] = mixed ? (const unsigned char*) a->d_bits : nullptr;
     for (int K = 1; K <= 8; ++K)
         if (mixed ? (a->kmask_d & (1 << (K - 1))) != 0 : K == a->Kd)
-            if (int rc = launch_gemm_short_grouped(ws + L.xt_d, ws + L.dout, L.mcap, a->I, a->H, K, a->cb, 1, tab + 4 * E, tab + 5 * E, G, stream)) return rc;
+            if (int rc = launch_gemm_tc_grouped(ws + L.xt_d, ws + L.dout, L.mcap, a->I, a->H, K, a->cb, 1, tab + 4 * E, tab + 5 * E, G, stream)) return rc;
 
     if (a->scratch)
     {

@@ -533,7 +533,7 @@ def measure_prefill(steps, warmup, bundles=True):
         "gpu_launches": launches * steps, "clocks": clocks,
         "roofline": {"bound": "tensor", "achieved": round(tf, 1), "peak": peak, "unit": "TFLOP/s", "frac": round(tf / peak, 4),
                      "peak_source": "measured burst (MEASURED_PEAKS.json)" if "bf16_tflops" in peaks else "fallback",
-                     "kernel": "exl3_gemm_tc2_kernel", "traffic": None}}
+                     "kernel": "exl3_gemm_tc_kernel", "traffic": None}}
 
 
 def moe_launches(T):
@@ -661,7 +661,7 @@ def measure_moe_prefill(steps, warmup, T=2048):
         "gpu_launches": 6 * len(sets) * steps, "clocks": clocks,
         "roofline": {"bound": "tensor", "achieved": round(tf, 1), "peak": peak, "unit": "TFLOP/s", "frac": round(tf / peak, 4),
                      "peak_source": "measured (MEASURED_PEAKS.json), burst" if "bf16_tflops" in peaks else "fallback",
-                     "kernel": "exl3_gemm_tc_kernel<K, CB, grouped>", "flops_per_layer": int(flops), "traffic": None}}
+                     "kernel": "exl3_gemm_tc_kernel (grouped)", "flops_per_layer": int(flops), "traffic": None}}
 
 
 def measure_gemm(steps, warmup, shape, rows):

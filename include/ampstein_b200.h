@@ -114,20 +114,16 @@ int amp_exl3_gemm_bf16(const void* A, const void* trellis, void* C, const void* 
                        cudaStream_t stream);
 
 /*
- * Form of the prefill GEMM: 0 = one CTA per tile only, 1 = by shape (default: CTA pairs with
- * tcgen05 cta_group::2 whenever n is a multiple of 256: 256 tokens x 256 columns per pair while
- * that grid fits one wave, 512 tokens beyond; single CTAs otherwise), 2 / 3 = pairs of
- * 512 / 256 tokens whenever n is a multiple of 256 (for tests). Returns the previous setting. No
+ * Pair form of the tensor-core GEMM (two CTAs per 256 columns, tcgen05 cta_group::2): 0 = never, 1 = by plan (default),
+ * 2 / 3 = pairs of 512 / 256 tokens whenever n is a multiple of 256 (for tests). Returns the previous setting. No
  * counterpart in the reference.
  */
 int amp_exl3_set_gemm_pair(int mode);
 /*
- * Short-batch form of the prefill GEMM (decoded weights as the M operand, tokens as N, k split over a cluster):
- * 0 = never, 1 = by size (default), 2 = always. split / tile > 0 force the number of k slices (1..8) / the tokens
- * per tile (a multiple of 16, up to 512), for tests and sweeps; 0: by rule. Returns the previous mode. No
- * counterpart in the reference.
+ * Plan of the tensor-core GEMM for tests and sweeps: the number of k slices (1..8) and / or the tokens per tile (a
+ * multiple of 16, up to 512); 0: by rule (default). Returns 0. No counterpart in the reference.
  */
-int amp_exl3_set_gemm_short(int mode, int split, int tile);
+int amp_exl3_set_gemm_plan(int split, int tile);
 /*
  * Int8-activation form of the one-row GEMV for mul1 (codebook 2) tensors up to max_k bits: the
  * rotated input is quantised to int8 with one scale per 128 rows of k and the dot product runs as
@@ -461,10 +457,9 @@ int amp_exl3_moe_gather(float* out, const float* scratch, const void* flat_exper
                         int T, int H, int topk, int E, long scratch_rows, cudaStream_t stream);
 /* bytes of workspace for a chunk of T tokens with A picks over E experts (0: bad sizes) */
 long amp_exl3_moe_sorted_workspace(long T, long A, long E, long H, long I);
-/* Rows per GEMM tile of amp_exl3_moe_sorted in units of 128 (one tile = rows of one expert whose
- * weight block a CTA decodes once): 0 (default) = chosen per call from the average rows per expert,
- * 1..4 forced; for A/B measurements. Returns the previous setting. No reference counterpart (its
- * row tiers are the caller's m_tile argument). */
+/* Rows per GEMM tile of amp_exl3_moe_sorted in units of 128 (one tile = rows of one expert whose weight block a CTA
+ * decodes once): 0 = default (2), 1 or 2 forced (3 and 4 are taken as 2); for A/B measurements. Returns the previous
+ * setting. No reference counterpart (its row tiers are the caller's m_tile argument). */
 int amp_exl3_set_moe_sorted_tile(int sub);
 /* Reads the status word the last call left in its workspace: 0 = clean, bits 0 / 1 = count[]
  * describes more rows than the sorted list holds, bit 2 = a token index outside [0, T), bit 3 = a
