@@ -152,34 +152,58 @@ __device__ __forceinline__ void warp_had128(float& h0, float& h1, float& h2, flo
     }
 }
 
-// Two fp32 additions / multiply-adds in one instruction (sm_100 packed forms; each half rounds as the scalar one)
-__device__ __forceinline__ float2 add_f32x2(float2 a, float2 b)
+// Two fp32 values in one 64-bit register and the packed operations on them (sm_100; each half rounds as the scalar one)
+typedef unsigned long long f32x2;
+
+__device__ __forceinline__ f32x2 pack_f32x2(float x, float y)
 {
-    float2 d;
-    asm("{\n\t.reg .b64 x, y, z;\n\tmov.b64 x, {%2, %3};\n\tmov.b64 y, {%4, %5};\n\tadd.rn.f32x2 z, x, y;\n\tmov.b64 {%0, %1}, z;\n\t}"
-        : "=f"(d.x), "=f"(d.y) : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
+    f32x2 d;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(d) : "f"(x), "f"(y));
     return d;
 }
 
-__device__ __forceinline__ float2 fma_f32x2(float2 a, float2 b, float2 c)
+__device__ __forceinline__ float2 unpack_f32x2(f32x2 v)
 {
     float2 d;
-    asm("{\n\t.reg .b64 w, x, y, z;\n\tmov.b64 w, {%2, %3};\n\tmov.b64 x, {%4, %5};\n\tmov.b64 y, {%6, %7};\n\t"
-        "fma.rn.f32x2 z, w, x, y;\n\tmov.b64 {%0, %1}, z;\n\t}"
-        : "=f"(d.x), "=f"(d.y) : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y), "f"(c.x), "f"(c.y));
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(d.x), "=f"(d.y) : "l"(v));
+    return d;
+}
+
+__device__ __forceinline__ f32x2 add_f32x2(f32x2 a, f32x2 b)
+{
+    f32x2 d;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+    return d;
+}
+
+__device__ __forceinline__ f32x2 mul_f32x2(f32x2 a, f32x2 b)
+{
+    f32x2 d;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+    return d;
+}
+
+__device__ __forceinline__ f32x2 fma_f32x2(f32x2 a, f32x2 b, f32x2 c)
+{
+    f32x2 d;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
     return d;
 }
 
 // 128-point Hadamard with four lanes per 128-value chunk: lane piece pc (0..3) holds in h[4 j .. 4 j + 3] the
 // eight values at elements 8 (pc + 4 j), j = 0..3, as pairs. Same butterflies in the same order as warp_had128
-// (bits 0-2 inside the lane, 3-4 across the four lanes, 5-6 inside), hence the same bits out; two shuffles per
-// value instead of five and half the additions thanks to the packed forms (a - b = fma(b, -1, a), exact up to
+// (bits 0-2 inside the lane, 3-4 across the four lanes, 5-6 inside), hence the same bits out; two shuffles
+// per value instead of five and half the additions thanks to the packed forms (a - b = fma(b, -1, a), exact up to
 // the one rounding of the sum).
-__device__ __forceinline__ void quad_had128(float2 (&h)[16], int pc)
+__device__ __forceinline__ void quad_had128(f32x2 (&h)[16], int pc)
 {
-    const float2 neg = make_float2(-1.0f, -1.0f);
+    const f32x2 neg = pack_f32x2(-1.0f, -1.0f);
     #pragma unroll
-    for (int i = 0; i < 16; ++i) h[i] = make_float2(h[i].x + h[i].y, h[i].x - h[i].y);
+    for (int i = 0; i < 16; ++i)
+    {
+        const float2 v = unpack_f32x2(h[i]);
+        h[i] = pack_f32x2(v.x + v.y, v.x - v.y);
+    }
     auto stage = [&](auto bit)
     {
         constexpr int b = decltype(bit)::value;
@@ -187,7 +211,7 @@ __device__ __forceinline__ void quad_had128(float2 (&h)[16], int pc)
         for (int i = 0; i < 16; ++i)
             if (!(i & b))
             {
-                const float2 lo = h[i], hi = h[i | b];
+                const f32x2 lo = h[i], hi = h[i | b];
                 h[i] = add_f32x2(lo, hi);
                 h[i | b] = fma_f32x2(hi, neg, lo);
             }
@@ -197,12 +221,12 @@ __device__ __forceinline__ void quad_had128(float2 (&h)[16], int pc)
     for (int m = 1; m <= 2; m <<= 1)
     {
         const float s = (pc & m) ? -1.0f : 1.0f;
-        const float2 sg = make_float2(s, s);
+        const f32x2 sg = pack_f32x2(s, s);
         #pragma unroll
         for (int i = 0; i < 16; ++i)
         {
-            const float2 p = make_float2(__shfl_xor_sync(0xffffffffu, h[i].x, m), __shfl_xor_sync(0xffffffffu, h[i].y, m));
-            h[i] = fma_f32x2(h[i], sg, p);
+            const float2 v = unpack_f32x2(h[i]);
+            h[i] = fma_f32x2(h[i], sg, pack_f32x2(__shfl_xor_sync(0xffffffffu, v.x, m), __shfl_xor_sync(0xffffffffu, v.y, m)));
         }
     }
     stage(std::integral_constant<int, 4>()); stage(std::integral_constant<int, 8>());

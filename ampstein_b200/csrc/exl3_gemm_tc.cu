@@ -90,7 +90,7 @@ static int tg_exchange(TgParams& S, int smem)
         }
     }
     const int room = smem / tg_row(S.split);
-    if (!S.recv_off && ts * S.split > room) ts = room / S.split & ~7;
+    if (!S.recv_off && ts * S.split > room) ts = room / S.split & ~15;
     S.share = ts;
     return S.recv_off ? tg_smem(S.tile, S.wstages, S.xstages) + S.split * ts * tg_row(S.split) : smem;
 }
@@ -239,7 +239,7 @@ int launch_gemm_tc_grouped(const void* xt, void* c, long Mcap, int k, int n, int
     AMP_REQUIRE(smem, "exl3_moe_sorted: tile does not fit");
     S.x_area = smem - tg_smem(0, S.wstages, 0);
     S.split = 1;
-    S.share = smem / tg_row(1) & ~7;
+    S.share = smem / tg_row(1) & ~15;
     // Dependent launch only where every grid that does anything waits for the rotation kernel: with one launch per
     // bit width a launch whose experts all have another width would be over before that kernel, and the next
     // launch's wait would be for it alone.

@@ -163,7 +163,7 @@ struct TgParams
     int wstages, xstages;       // stages of decoded weights and of x~: wstages >= 2 NG
     int x_area;                 // expert groups: bytes of all x~ stages together (xstages then follows from the tile's rows)
     int tmem_cols;              // tensor-memory columns to allocate: a power of two >= tile, >= 32 (two accumulators: 512)
-    int share;                  // tokens a CTA finishes per epilogue pass (several passes: a multiple of 8)
+    int share;                  // tokens a CTA finishes per epilogue pass (no split, or several passes: a multiple of 16)
     int recv_off;               // where the partial sums are received: behind the stages, or 0: over them
     int pdl;                    // launched as a programmatic dependent of the kernel that writes x~
 };
@@ -205,9 +205,9 @@ __device__ __forceinline__ void sts128(uint32_t addr, uint32_t a, uint32_t b, ui
     asm volatile("st.shared.v4.u32 [%0], {%1, %2, %3, %4};" :: "r"(addr), "r"(a), "r"(b), "r"(c), "r"(d) : "memory");
 }
 
-__device__ __forceinline__ void lds128f(uint32_t addr, float2& a, float2& b)
+__device__ __forceinline__ void lds_f32x2(uint32_t addr, f32x2& a, f32x2& b)
 {
-    asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(a.x), "=f"(a.y), "=f"(b.x), "=f"(b.y) : "r"(addr) : "memory");
+    asm volatile("ld.shared.v2.b64 {%0, %1}, [%2];" : "=l"(a), "=l"(b) : "r"(addr) : "memory");
 }
 
 // Two states -> two exact fp16 weights, packed. As weights2, with the halves of each word added by one
@@ -333,6 +333,7 @@ void exl3_gemm_tc_kernel(const TgParams S)
     __shared__ uint64_t x_full[TG_MAX_STAGES], w_full[TG_MAX_STAGES], done[TG_MAX_STAGES], peer[PAIR ? TG_MAX_STAGES : 1];
     __shared__ uint32_t s_tmem;
     __shared__ volatile int s_bad;
+    __shared__ __align__(16) uint2 s_svh[32];                    // the block's output scales
     constexpr int NDEC = 8 * NG, NGR = NDEC / TG_GROUP_WARPS;    // decode warps; groups of them that take alternate steps
 
     const int t = threadIdx.x, lane = t & 31, warp = __shfl_sync(0xffffffffu, t >> 5, 0);
@@ -398,6 +399,7 @@ void exl3_gemm_tc_kernel(const TgParams S)
             asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
         }
     }
+    if (warp == NDEC + 1) s_svh[lane] = reinterpret_cast<const uint2*>(W.svh + (size_t) nb * 128)[lane];      // (8-byte aligned)
     // The decode warps' packed words go straight into registers, one step ahead of their use (two: no gain). (Not through
     // cp.async rings: the release of a step's barrier waits for the warp's copies in flight, so that every
     // step paid the HBM latency -- 1.1 us per step and warp, 20 us for 77 x 4096 x 4096 at 4 bits.)
@@ -585,7 +587,10 @@ void exl3_gemm_tc_kernel(const TgParams S)
     // peers write into this CTA's receive buffer from here on: where it overlaps the stages, everybody's MMAs
     // must have read theirs
     if (split > 1 && S.recv_off == 0) cluster_sync_all();
-    const int row = tg_row(split), n0 = S.n0, TS = S.share;                                  // tokens this CTA finishes per pass
+    const int row = tg_row(split), n0 = S.n0;
+    // passes of equal length, each CTA of the cluster finishing TS tokens of a pass
+    const int npass = (rows + S.share * split - 1) / (S.share * split);
+    const int TS = npass > 1 ? ((rows + npass * split - 1) / (npass * split) + 15) & ~15 : S.share;
     const uint32_t xbuf = smem_u32(smem) + (uint32_t) S.recv_off;             // [split][TS] rows of 128 fp32
     for (int p0 = 0; p0 < rows; p0 += TS * split)
     {
@@ -595,23 +600,25 @@ void exl3_gemm_tc_kernel(const TgParams S)
             // rows of the accumulator (output columns) 32 q .. + 31 belong to the warps with warp % 4 == q
             const int q = warp & 3;
             const uint32_t col = xbuf + (uint32_t) (crank * TS * row + (q * 32 + lane) * 4);
-            for (int c0 = (warp >> 2) * 8; c0 < np; c0 += NDEC * 2)
+            for (int c0 = (warp >> 2) * 16; c0 < np; c0 += NDEC * 4)
             {
-                uint32_t v[8];
-                asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
-                             : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7])
+                uint32_t v[16];
+                asm volatile("tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
+                             : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]),
+                               "=r"(v[8]), "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15])
                              : "r"(tmem + ((uint32_t) (32 * q) << 16) + (uint32_t) (p0 + c0 + (NG > 1 && p0 + c0 >= n0 ? TG_MAX_N - n0 : 0))) : "memory");
                 asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
                 if (split == 1)
                 {
+                    // (a last chunk stores what lies behind its tokens too: the buffer has room for whole chunks)
+                    const uint32_t at = col + (uint32_t) (c0 * 528);
                     #pragma unroll
-                    for (int j = 0; j < 8; ++j)
-                        if (c0 + j < np) asm volatile("st.shared.u32 [%0], %1;" :: "r"(col + (uint32_t) ((c0 + j) * row)), "r"(v[j]) : "memory");
+                    for (int j = 0; j < 16; ++j) asm volatile("st.shared.u32 [%0], %1;" :: "r"(at + (uint32_t) (j * 528)), "r"(v[j]) : "memory");
                     continue;
                 }
                 int dest = c0 / TS, tl = c0 - dest * TS;
                 #pragma unroll
-                for (int j = 0; j < 8; ++j)
+                for (int j = 0; j < 16; ++j)
                 {
                     if (c0 + j < np)
                     {
@@ -629,24 +636,26 @@ void exl3_gemm_tc_kernel(const TgParams S)
         {
             // four lanes per token, eight tokens per warp in flight
             const int pc = lane & 3, cl = lane >> 2;
-            const __half* svp = W.svh + (size_t) nb * 128 + 8 * pc;
+            const uint32_t svp = smem_u32(s_svh) + 16 * pc;
             const bool wide = (reinterpret_cast<uintptr_t>(W.c) & 15) == 0;      // (a bundle's outputs may be 8-byte aligned)
+            const f32x2 rs = pack_f32x2(kRScale, kRScale);
+            #pragma unroll 1
             for (int r0 = warp * 8; r0 < nt; r0 += NDEC * 8)
             {
                 const int r = r0 + cl;
                 // partial sums of the cluster's CTAs in ascending k order
                 uint32_t at_s = xbuf + (uint32_t) (min(r, nt - 1) * row + 32 * pc);
-                float2 h[16];
+                f32x2 h[16];
                 #pragma unroll
-                for (int j = 0; j < 8; ++j) lds128f(at_s + (j & 1) * 16 + (j >> 1) * 128, h[2 * j], h[2 * j + 1]);
+                for (int j = 0; j < 8; ++j) lds_f32x2(at_s + (j & 1) * 16 + (j >> 1) * 128, h[2 * j], h[2 * j + 1]);
                 for (int i = 1; i < split; ++i)
                 {
                     at_s += (uint32_t) (TS * row);
                     #pragma unroll
                     for (int j = 0; j < 8; ++j)
                     {
-                        float2 u, v;
-                        lds128f(at_s + (j & 1) * 16 + (j >> 1) * 128, u, v);
+                        f32x2 u, v;
+                        lds_f32x2(at_s + (j & 1) * 16 + (j >> 1) * 128, u, v);
                         h[2 * j] = add_f32x2(h[2 * j], u); h[2 * j + 1] = add_f32x2(h[2 * j + 1], v);
                     }
                 }
@@ -656,12 +665,12 @@ void exl3_gemm_tc_kernel(const TgParams S)
                 #pragma unroll
                 for (int j = 0; j < 4; ++j)
                 {
-                    // (scale vectors are 8-byte aligned)
-                    const uint2 sv[2] = { *reinterpret_cast<const uint2*>(svp + 32 * j), *reinterpret_cast<const uint2*>(svp + 32 * j + 4) };
-                    const __half2* s2 = reinterpret_cast<const __half2*>(sv);
-                    float2* v = h + 4 * j;
+                    uint4 sv;
+                    lds128(svp + 64 * j, sv.x, sv.y, sv.z, sv.w);
+                    const __half2* s2 = reinterpret_cast<const __half2*>(&sv);
+                    float2 v[4];
                     #pragma unroll
-                    for (int q = 0; q < 4; ++q) { v[q].x *= kRScale; v[q].y *= kRScale; }
+                    for (int q = 0; q < 4; ++q) v[q] = unpack_f32x2(mul_f32x2(h[4 * j + q], rs));
                     if (P.c_fp32)
                     {
                         float4* o = reinterpret_cast<float4*>(reinterpret_cast<float*>(W.c) + at + 32 * j);
@@ -673,7 +682,7 @@ void exl3_gemm_tc_kernel(const TgParams S)
                         uint4 o;
                         __half2* o2 = reinterpret_cast<__half2*>(&o);
                         #pragma unroll
-                        for (int q = 0; q < 4; ++q) o2[q] = __hmul2(__floats2half2_rn(v[q].x, v[q].y), s2[q]);
+                        for (int q = 0; q < 4; ++q) o2[q] = __hmul2(__float22half2_rn(v[q]), s2[q]);
                         __half* dst = reinterpret_cast<__half*>(W.c) + at + 32 * j;
                         if (wide) *reinterpret_cast<uint4*>(dst) = o;
                         else { reinterpret_cast<uint2*>(dst)[0] = make_uint2(o.x, o.y); reinterpret_cast<uint2*>(dst)[1] = make_uint2(o.z, o.w); }

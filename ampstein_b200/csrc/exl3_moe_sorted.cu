@@ -220,7 +220,7 @@ struct MsRot
 
 // a lane's 32 rotated values (quad_had128's layout) -> their place in the k-step-major, swizzled layout (see
 // had_tiled_kernel): piece pc + 4 j of the chunk is piece (pc + 4 j) % 8 of k step 2 * chunk + j / 2
-__device__ __forceinline__ void ms_store_pieces(unsigned char* xt, int mcap, int p, int cb, int pc, const float2 (&h)[16])
+__device__ __forceinline__ void ms_store_pieces(unsigned char* xt, int mcap, int p, int cb, int pc, const f32x2 (&h)[16])
 {
     #pragma unroll
     for (int j = 0; j < 4; ++j)
@@ -228,7 +228,7 @@ __device__ __forceinline__ void ms_store_pieces(unsigned char* xt, int mcap, int
         uint4 o;
         __half2* o2 = reinterpret_cast<__half2*>(&o);
         #pragma unroll
-        for (int q = 0; q < 4; ++q) o2[q] = __floats2half2_rn(h[4 * j + q].x * kRScale, h[4 * j + q].y * kRScale);
+        for (int q = 0; q < 4; ++q) o2[q] = __float22half2_rn(unpack_f32x2(mul_f32x2(h[4 * j + q], pack_f32x2(kRScale, kRScale))));
         unsigned char* row = xt + (((size_t) (2 * cb + (j >> 1)) * (size_t) mcap + (size_t) p) << 7);
         *reinterpret_cast<uint4*>(row + (((pc + 4 * (j & 1)) ^ (p & 7)) << 4)) = o;
     }
@@ -241,7 +241,7 @@ __device__ __forceinline__ void ms_load_pieces(const __half* src, int pc, uint4 
     for (int j = 0; j < 4; ++j) v[j] = *reinterpret_cast<const uint4*>(src + 8 * (pc + 4 * j));
 }
 
-__device__ __forceinline__ void ms_scale(const uint4 (&v)[4], const uint4 (&s)[4], float2 (&h)[16])
+__device__ __forceinline__ void ms_scale(const uint4 (&v)[4], const uint4 (&s)[4], f32x2 (&h)[16])
 {
     #pragma unroll
     for (int j = 0; j < 4; ++j)
@@ -249,7 +249,11 @@ __device__ __forceinline__ void ms_scale(const uint4 (&v)[4], const uint4 (&s)[4
         const __half2* a = reinterpret_cast<const __half2*>(&v[j]);
         const __half2* b = reinterpret_cast<const __half2*>(&s[j]);
         #pragma unroll
-        for (int q = 0; q < 4; ++q) h[4 * j + q] = __half22float2(__hmul2(a[q], b[q]));
+        for (int q = 0; q < 4; ++q)
+        {
+            const float2 v = __half22float2(__hmul2(a[q], b[q]));
+            h[4 * j + q] = pack_f32x2(v.x, v.y);
+        }
     }
 }
 
@@ -291,7 +295,7 @@ void moe_sorted_rotate_in_kernel(const MsRot P)
             const bool live = cb < chunks;                 // (idle lanes still take part in the shuffles)
             const int off = (live ? cb : 0) * 128;
             uint4 v[4], sc[4];
-            float2 h[16];
+            f32x2 h[16];
             ms_load_pieces(src + off, pc, v);
             ms_load_pieces(us + off, pc, sc);
             ms_scale(v, sc, h);
@@ -331,7 +335,7 @@ void moe_sorted_rotate_act_kernel(const MsRot P)
             const __half* ur = ubase + (size_t) p * P.I + cb * 128;
             const __half* gr = gbase + (size_t) p * P.I + cb * 128;
             uint4 u[4], gt[4], sc[4];
-            float2 h[16];
+            f32x2 h[16];
             ms_load_pieces(ur, pc, u);
             ms_load_pieces(P.gated ? gr : ur, pc, gt);
             ms_load_pieces(ds + cb * 128, pc, sc);
@@ -343,7 +347,7 @@ void moe_sorted_rotate_act_kernel(const MsRot P)
                 const __half2* c = reinterpret_cast<const __half2*>(&sc[j]);
                 #pragma unroll
                 for (int q = 0; q < 4; ++q)
-                    h[4 * j + q] = make_float2(moe_act_gate(P.act, P.gated, __low2float(a[q]), __low2float(b[q]), P.act_limit) * __low2float(c[q]),
+                    h[4 * j + q] = pack_f32x2(moe_act_gate(P.act, P.gated, __low2float(a[q]), __low2float(b[q]), P.act_limit) * __low2float(c[q]),
                                                moe_act_gate(P.act, P.gated, __high2float(a[q]), __high2float(b[q]), P.act_limit) * __high2float(c[q]));
             }
             quad_had128(h, pc);
