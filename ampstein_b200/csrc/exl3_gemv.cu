@@ -228,7 +228,7 @@ int launch_gemv(const GemvLaunch& A, cudaStream_t stream)
     const int i8 = (!tc && !A.mode && !A.arin.N && !special_in && A.cb == 2 && m == 1 && K <= g_int8_max_k)
                        ? (g_int8_gemv == 2 ? 3 : (g_int8_gemv == 1 ? 4 : 0)) : 0;
     gemv_fn fn = tc ? gemv_tc_kernel_for(K, A.cb, A.ar.N != 0)
-                    : gemv_kernel_for(K, i8 ? i8 : A.cb, MB, A.mode, A.arin.N ? 1 : (norm_producer ? 5 : (norm_consumer ? 6 : (fused_norm ? 4 : (fused_act ? 3 : (prerot ? 2 : 0))))));
+                    : gemv_kernel_for(K, i8 ? i8 : A.cb, MB, A.mode, A.mode ? (A.moe.inline_runs ? 7 : 0) : A.arin.N ? 1 : (norm_producer ? 5 : (norm_consumer ? 6 : (fused_norm ? 4 : (fused_act ? 3 : (prerot ? 2 : 0))))));
     if (!fn) return fail(AMP_E_UNSUPPORTED, "exl3_gemv: no kernel for K=%d cb=%d", K, A.cb);
 
     // x~ rows resident at a time: at most 16 KB of shared memory (whole segments for small
@@ -246,11 +246,11 @@ int launch_gemv(const GemvLaunch& A, cudaStream_t stream)
         return c < 4 ? 4 : c;
     };
     int xcap = xcap_for(16);
-    if (m > 4 && !A.mode)
+    if (m > 4 && !A.moe.inline_runs)
     {
-        // several batch rows: twice the x~ budget (half as many block-wide x~ passes per range)
-        // where that does not cost a resident CTA (not for the grouped modes: their runs mostly hold
-        // one or two rows, and the single-token form also needs room for the cluster exchange)
+        // several batch rows: twice the x~ budget (half as many block-wide x~ passes per range; runs of experts:
+        // all of k resident for more rows) where that does not cost a resident CTA (not for the single-token
+        // grouped form, which needs the room for its cluster exchange)
         const int big = xcap_for(32);
         if (smem_per_sm / (gemv_smem_layout(K, m, big).total + 1024) >= reg_ctas) xcap = big;
     }

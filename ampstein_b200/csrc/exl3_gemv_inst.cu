@@ -74,17 +74,24 @@ gemv_fn AMP_CAT(gemv_kernel_k, AMP_GEMV_K)(int cb, int MB, int mode, int gin)
         { exl3_gemv_kernel<AMP_GEMV_K, 1, 1>, exl3_gemv_kernel<AMP_GEMV_K, 1, 2> },
         { exl3_gemv_kernel<AMP_GEMV_K, 2, 1>, exl3_gemv_kernel<AMP_GEMV_K, 2, 2> },
     };
+    // grouped experts: runs from a table, and a single token (gin 7)
     static const gemv_fn moe[3][2] =
     {
         { exl3_gemv_kernel<AMP_GEMV_K, 0, 1, 1>, exl3_gemv_kernel<AMP_GEMV_K, 0, 1, 2> },
         { exl3_gemv_kernel<AMP_GEMV_K, 1, 1, 1>, exl3_gemv_kernel<AMP_GEMV_K, 1, 1, 2> },
         { exl3_gemv_kernel<AMP_GEMV_K, 2, 1, 1>, exl3_gemv_kernel<AMP_GEMV_K, 2, 1, 2> },
     };
+    static const gemv_fn one[3][2] =
+    {
+        { exl3_gemv_kernel<AMP_GEMV_K, 0, 1, 1, 7>, exl3_gemv_kernel<AMP_GEMV_K, 0, 1, 2, 7> },
+        { exl3_gemv_kernel<AMP_GEMV_K, 1, 1, 1, 7>, exl3_gemv_kernel<AMP_GEMV_K, 1, 1, 2, 7> },
+        { exl3_gemv_kernel<AMP_GEMV_K, 2, 1, 1, 7>, exl3_gemv_kernel<AMP_GEMV_K, 2, 1, 2, 7> },
+    };
     // cb 3 = the mul1 codebook with int8 activations: one batch row, plain launches only
     if (cb == 3) return (MB == 1 && !mode && !gin) ? exl3_gemv_kernel<AMP_GEMV_K, 3, 1> : nullptr;
     if (cb == 4) return (MB == 1 && !mode && !gin) ? exl3_gemv_kernel<AMP_GEMV_K, 4, 1> : nullptr;
     if (cb < 0 || cb > 2 || MB < 1 || MB > 2 || mode < 0 || mode > 2) return nullptr;
-    if (mode) return (MB == 1 && !gin) ? moe[cb][mode - 1] : nullptr;
+    if (mode) return (MB == 1 && (!gin || gin == 7)) ? (gin ? one : moe)[cb][mode - 1] : nullptr;
     if (gin == 4) return fnn[cb][MB - 1];
     if (gin == 5) return fnp[cb][MB - 1];
     if (gin == 6) return fnc[cb][MB - 1];

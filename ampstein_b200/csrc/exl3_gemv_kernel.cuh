@@ -722,8 +722,8 @@ void exl3_gemv_kernel(const GemvParams P)
 {
     extern __shared__ __align__(128) unsigned char smem[];
     const GemvSmem L = gemv_smem_layout(K, P.m, P.xgroups, P.cluster, GIN == 1, (GIN == 4 || CB == 4) ? P.rowbuf : 0);
-    const int XPITCH = gemv_xpitch(P.xgroups);
-    const int XG = P.xgroups;
+    int XPITCH = gemv_xpitch(P.xgroups);               // (grouped modes: per segment)
+    int XG = P.xgroups;
     float* part = reinterpret_cast<float*>(smem + L.part);
     uint32_t* xd = reinterpret_cast<uint32_t*>(smem + L.xd);
     float* gsum = reinterpret_cast<float*>(smem + L.gsum);
@@ -732,6 +732,10 @@ void exl3_gemv_kernel(const GemvParams P)
     (void) xd2;
     __shared__ int s_last;
 
+    // grouped modes: the instance of a single token, whose runs of one row every CTA derives itself and whose launch
+    // may have clusters, and the instance that reads a run table (GIN 0). Apart because the code of one costs the
+    // other microseconds per launch (a cold CTA fetches it instruction line by line).
+    constexpr bool ONE = MODE != 0 && GIN == 7, RUNS = MODE != 0 && GIN != 7;
     constexpr int S = gemv_stages(K);
     constexpr int RP = gemv_row_pitch(K);
     constexpr int SLOT = gemv_slot_bytes(K);
@@ -764,7 +768,7 @@ void exl3_gemv_kernel(const GemvParams P)
     int inline_active = 0;
     if constexpr (MODE != 0)
     {
-        if (P.moe.inline_runs)
+        if constexpr (ONE)
         {
             // one token: its active picks, in pick order, are the runs (one row each); lane i of
             // the first warp reads pick i
@@ -820,7 +824,7 @@ void exl3_gemv_kernel(const GemvParams P)
     if constexpr (MODE == 2)
     {
         // a single token without any local pick: nobody will deliver a slot, the row is still due
-        if (P.moe.inline_runs && inline_active == 0 && cta == 0 && P.moe.first_down)
+        if (ONE && inline_active == 0 && cta == 0 && P.moe.first_down)
             for (int c = warp; c < (P.moe.Ho >> 7); c += GEMV_WARPS) moe_combine_chunk(P.moe, 0, c, lane);
     }
     if (cta >= ncta) return;                           // an exited CTA counts as having released its dependents
@@ -828,7 +832,19 @@ void exl3_gemv_kernel(const GemvParams P)
     split.q = U / ncta;
     split.r = U - split.q * ncta;
     int u0 = split.begin(cta), u1 = split.begin(cta + 1);
-    if constexpr (MODE != 0)
+    if constexpr (RUNS)
+    {
+        // ranges of whole column blocks where the longest is no more than three units longer: nothing to exchange then
+        // (an exchange costs about that: 16 tokens of 128 experts, 768 rows down, 135.5 -> 132.2 us per layer)
+        const int nblocks = U / G, bq = nblocks / ncta, br = nblocks - bq * ncta;
+        if ((bq + (br > 0 ? 1 : 0)) * G <= split.q + 3)
+        {
+            u0 = (bq * cta + min(cta, br)) * G;
+            u1 = u0 + (bq + (cta < br ? 1 : 0)) * G;
+            if (u0 >= u1) return;
+        }
+    }
+    if constexpr (ONE)
     {
         if (P.cluster)
         {
@@ -1050,6 +1066,11 @@ void exl3_gemv_kernel(const GemvParams P)
     const uint32_t xd_s = smem_u32(xd);
 
     uint32_t cslot = 0;                                // byte offset of the next slot to consume
+    // Grouped modes: x~ kept from one column block of the range to the next of the same run, where the x~ area holds
+    // all of k (then at its place in k): whose input it is and the first group there (up to the last one). A range of two
+    // to four blocks rotated the run's rows for each (16 tokens of 128 experts: 153.6 -> 136.8 us per layer)
+    constexpr bool KEEP = RUNS;
+    int kept_of = -1, kept_g = 0;
     int useg = u0;
     while (useg < u1)
     {
@@ -1072,7 +1093,7 @@ void exl3_gemv_kernel(const GemvParams P)
             const int run = filtered ? s_sel[srun] : srun;
             const int* rec = runs + 2 + run * MOE_RUN_INTS;
             const int expert = rec[0];
-            nrows = rec[1];
+            nrows = ONE ? 1 : rec[1];
             run_slots = reinterpret_cast<const unsigned char*>(rec + 2);
             suh = reinterpret_cast<const __half*>(P.moe.suh[proj][expert]);
             svh = reinterpret_cast<const __half*>(P.moe.svh[proj][expert]);
@@ -1081,6 +1102,12 @@ void exl3_gemv_kernel(const GemvParams P)
             stride = P.width;
             // the expert's output scales are needed at the very end: pull their lines into L2 now
             if (t < 2) asm volatile("prefetch.global.L2 [%0];" :: "l"(svh + (size_t) nb * 128 + t * 64));
+            // the x~ area is cut by the rows of the run at hand: most have one or two of the eight it could hold
+            if constexpr (RUNS)
+            {
+                XG = min((m * P.xgroups / nrows) & ~3, (G + 3) & ~3);
+                XPITCH = gemv_xpitch(XG);
+            }
             #pragma unroll
             for (int mb = 0; mb < MB; ++mb) xrow[mb] = min(mb * 8 + gq, nrows - 1) * XPITCH + pq * 4;
         }
@@ -1112,8 +1139,22 @@ void exl3_gemv_kernel(const GemvParams P)
         for (int cg0 = g0 & ~1; cg0 < g1; cg0 += XG)
         {
             const int cg1 = min(cg0 + XG, g1);
-            const int nblk = (cg1 - cg0 + 1) >> 1;      // 128-row blocks in this chunk
-            __syncthreads();                            // previous x~ fully consumed
+            // in the x~ area: the chunk's first group (0: every group at its place in k) and the end of the groups
+            // that are still to be rotated
+            int base = cg0, fill1 = cg1;
+            if constexpr (KEEP)
+                if (XG >= G)
+                {
+                    base = 0;
+                    if (kept_of == slice) fill1 = min(fill1, kept_g);
+                    kept_of = slice;
+                    kept_g = cg0;
+                }
+            const int nblk = (fill1 - cg0 + 1) >> 1;    // 128-row blocks to rotate
+            const int xo = (cg0 - base) * 64;           // ... and the word of the area they start at
+            __syncthreads();                            // previous x~ (and finished block) fully consumed
+            if (!KEEP || nblk > 0)
+            {
 
             // x~ = fp16(H(x * suh) / sqrt(128)), stored duplicated ((v, v) per word) and in the
             // order the B fragments are read: word = group*64 + (row%16 / 4)*16 + (row%64 / 16)*4 + row%4.
@@ -1136,7 +1177,7 @@ void exl3_gemv_kernel(const GemvParams P)
                     d.x = (uint32_t) (i0 & 0xff) * 0x01010101u; d.y = (uint32_t) (i1 & 0xff) * 0x01010101u;
                     d.z = (uint32_t) (i2 & 0xff) * 0x01010101u; d.w = (uint32_t) (i3 & 0xff) * 0x01010101u;
                     const int r = jb * 128 + lane * 4;
-                    const int word = (r >> 6) * 64 + ((r & 15) >> 2) * 16 + ((r & 63) >> 4) * 4;
+                    const int word = xo + (r >> 6) * 64 + ((r & 15) >> 2) * 16 + ((r & 63) >> 4) * 4;
                     *reinterpret_cast<uint4*>(xd + b * XPITCH + word) = d;
                     const float q = __fdiv_rn(mx, 127.0f);
                     // per 64-row group (lanes 0-15 / 16-31): the dequantised sum of the codes and the scale
@@ -1162,8 +1203,8 @@ void exl3_gemv_kernel(const GemvParams P)
                     }
                     if ((lane & 15) == 0)
                     {
-                        gsum[b * XG + 2 * jb + (lane >> 4)] = gs;
-                        qs[b * XG + 2 * jb + (lane >> 4)] = q;
+                        gsum[b * XG + (xo >> 6) + 2 * jb + (lane >> 4)] = gs;
+                        qs[b * XG + (xo >> 6) + 2 * jb + (lane >> 4)] = q;
                     }
                     return;
                 }
@@ -1173,7 +1214,7 @@ void exl3_gemv_kernel(const GemvParams P)
                 d.x = __byte_perm(u01, u01, 0x1010); d.y = __byte_perm(u01, u01, 0x3232);
                 d.z = __byte_perm(u23, u23, 0x1010); d.w = __byte_perm(u23, u23, 0x3232);
                 const int r = jb * 128 + lane * 4;      // row inside the chunk
-                const int word = (r >> 6) * 64 + ((r & 15) >> 2) * 16 + ((r & 63) >> 4) * 4;
+                const int word = xo + (r >> 6) * 64 + ((r & 15) >> 2) * 16 + ((r & 63) >> 4) * 4;
                 *reinterpret_cast<uint4*>(xd + b * XPITCH + word) = d;
                 if constexpr (CB == 2)
                 {
@@ -1181,7 +1222,7 @@ void exl3_gemv_kernel(const GemvParams P)
                     float sg = (__low2float(o01) + __high2float(o01)) + (__low2float(o23) + __high2float(o23));
                     #pragma unroll
                     for (int i = 1; i < 16; i <<= 1) sg += __shfl_xor_sync(0xffffffffu, sg, i);
-                    if ((lane & 15) == 0) gsum[b * XG + 2 * jb + (lane >> 4)] = sg;
+                    if ((lane & 15) == 0) gsum[b * XG + (xo >> 6) + 2 * jb + (lane >> 4)] = sg;
                 }
             };
             auto had_store = [&](int b, int jb, float h0, float h1, float h2, float h3)
@@ -1545,6 +1586,7 @@ void exl3_gemv_kernel(const GemvParams P)
                 }
             }
             __syncthreads();
+            }
 
             const int c0 = max(cg0, g0);                // first group of the chunk that belongs to the range
             if constexpr (CB == 2 || CB == 3 || CB == 4)
@@ -1556,13 +1598,13 @@ void exl3_gemv_kernel(const GemvParams P)
                     {
                         const int b = min(mb * 8 + 2 * pq + e, nrows - 1);
                         float sacc = xsum[mb][e];
-                        for (int g = c0; g < cg1; ++g) sacc += gsum[b * XG + (g - cg0)];
+                        for (int g = c0; g < cg1; ++g) sacc += gsum[b * XG + (g - base)];
                         xsum[mb][e] = sacc;
                     }
             }
 
             // every warp walks the chunk's units c0 .. cg1-1
-            uint32_t xaddr = xd_s + (c0 - cg0) * 256;   // shared address of the unit's x~ (64 words a group)
+            uint32_t xaddr = xd_s + (c0 - base) * 256;   // shared address of the unit's x~ (64 words a group)
             for (int n = cg1 - c0; n > 0; --n, xaddr += 256)
             {
                 cp_async_wait_n<S - 2>();               // the unit has landed (this lane's pieces)
@@ -1601,7 +1643,7 @@ void exl3_gemv_kernel(const GemvParams P)
                     #pragma unroll
                     for (int i = 0; i < 4; ++i)
                         lds128(xaddr + (uint32_t) ((xd2 - xd) * 4) + xrow[0] * 4 + i * 64, xr[4 * i], xr[4 * i + 1], xr[4 * i + 2], xr[4 * i + 3]);
-                    const float q = qs[(c0 - cg0) + (cg1 - c0 - n)], q2 = q * (1.0f / 254.0f);
+                    const float q = qs[(c0 - base) + (cg1 - c0 - n)], q2 = q * (1.0f / 254.0f);
                     #pragma unroll
                     for (int nt = 0; nt < NT; ++nt)
                     {
@@ -1620,7 +1662,7 @@ void exl3_gemv_kernel(const GemvParams P)
                 {
                     // int8 activations (one batch row): exact integer sums over the unit, scaled by
                     // the unit's block scale into the fp32 sums of the segment
-                    const float q = qs[(c0 - cg0) + (cg1 - c0 - n)];
+                    const float q = qs[(c0 - base) + (cg1 - c0 - n)];
                     #pragma unroll
                     for (int nt = 0; nt < NT; ++nt)
                     {
@@ -1661,7 +1703,7 @@ void exl3_gemv_kernel(const GemvParams P)
         const int my_slot = 2 * cta + (blk * G > u0 ? 1 : 0);
         float* dst = whole ? part : slots + (size_t) my_slot * m * 128;
         // cluster form: the partial goes straight into the shared memory of the cluster's first CTA
-        const bool clustered = P.cluster > 0;
+        const bool clustered = !RUNS && P.cluster > 0;
         uint32_t xdst = 0;
         if (clustered) xdst = cluster_map(smem_u32(smem + L.xchg), 0) + cluster_rank() * (m * 128 * 4);
         #pragma unroll
@@ -1813,7 +1855,7 @@ void exl3_gemv_kernel(const GemvParams P)
                         if (lane == 0)
                         {
                             __threadfence();
-                            const int need = P.moe.inline_runs ? inline_active : P.moe.need[row];
+                            const int need = ONE ? inline_active : P.moe.need[row];
                             if (atomicAdd(cnt, 1) == need - 1)
                             {
                                 *cnt = 0;                            // zero again for the next call
