@@ -158,7 +158,7 @@ void gemv_prerotate_kernel(const __half* __restrict__ x, __half* __restrict__ ou
     *reinterpret_cast<half4*>(out + ((size_t) blockIdx.y * m + b) * k + (size_t) jb * 128 + lane * 4) = o;
 }
 
-constexpr int GEMV_PREROTATE_MIN_M = 5;
+constexpr int GEMV_PREROTATE_MIN_M = 5, GEMV_PREROTATE_MIN_PER = 60;
 
 // Int8-activation form of the one-row GEMV for mul1 (codebook 2) tensors, as the reference's
 // EXL3_INT8_GEMV switch (vendor/exl3/exllamav3_ext/quant/exl3_gemv_int8.cu:20-52): 0 = off, 2 = plain
@@ -207,7 +207,6 @@ int launch_gemv(const GemvLaunch& A, cudaStream_t stream)
 
     const int MB = m <= 8 ? 1 : 2;
     const bool tc = !A.mode && !half_rate && m <= TCV_MAX_M && g_gemv_tc && !A.arin.N && !A.ar.push_only && !A.x2 && !A.h_in && !A.norm_w;
-    // five rows or more with a scratch for the rotated input: rotate once, in a launch of its own
     const bool norm_producer = A.h_in != nullptr;                       // split norm, producer side
     const bool norm_consumer = A.norm_w != nullptr && A.ssq != nullptr && !A.x2;   // ... consumer side
     AMP_REQUIRE(!norm_producer || (!A.mode && !A.arin.N && !A.ar.N && !A.tables && !A.c_fp32 && A.y && A.ssq && !A.norm_w && !A.x2 &&
@@ -223,10 +222,17 @@ int launch_gemv(const GemvLaunch& A, cudaStream_t stream)
                                 (((uintptr_t) A.x2 | (uintptr_t) A.norm_w | (uintptr_t) A.y) & 7) == 0),
                 "exl3_gemv: the fused norm takes x, residual, weight and a separate output for the residual stream, 8-byte aligned");
     const bool special_in = fused_act || fused_norm || norm_producer || norm_consumer;
-    const bool prerot = !tc && !A.mode && !A.arin.N && !special_in && m >= GEMV_PREROTATE_MIN_M && A.x_rot && A.x;
     // mul1, one row: int8 activations (kernel instance 3), or int8 with error-feedback codes (instance 4)
     const int i8 = (!tc && !A.mode && !A.arin.N && !special_in && A.cb == 2 && m == 1 && K <= g_int8_max_k)
                        ? (g_int8_gemv == 2 ? 3 : (g_int8_gemv == 1 ? 4 : 0)) : 0;
+    // with a scratch for the rotated input: rotate once, in a launch of its own, instead of in every CTA for each column
+    // block of its range. From five rows on, and with fewer where a range (`per` 64-row groups of three CTAs per SM)
+    // is long enough. Measured (us, rotated in the CTAs / once): 4096 x 128256 (per 144) at 1 row 127.5 / 121.6, 2 rows
+    // 137 / 124, 3 rows 148 / 128, 4 rows 158 / 130; 5120 x 25600 (36) at 1 row 37.4 / 38.6, 2 rows level, 3 rows 43.2 /
+    // 41.3; 4096 x 28672 (32) at 1 row 28.3 / 29.5, 2 rows 30.5 / 31.4, 3 rows 32.9 / 32.0; 14336 x 4096 (16) at 3 rows 21.1 / 23.4, 4 rows level.
+    const long per = (long) A.slices * (A.width / 128) * (k / 64) / (3 * D.sms);
+    const bool prerot = !tc && !A.mode && !A.arin.N && !special_in && A.x_rot && A.x &&
+                        (m >= GEMV_PREROTATE_MIN_M || (m >= 2 && (m - 1) * per >= GEMV_PREROTATE_MIN_PER) || (m == 1 && !i8 && per >= 100));
     gemv_fn fn = tc ? gemv_tc_kernel_for(K, A.cb, A.ar.N != 0)
                     : gemv_kernel_for(K, i8 ? i8 : A.cb, MB, A.mode, A.mode ? (A.moe.inline_runs ? 7 : 0) : A.arin.N ? 1 : (norm_producer ? 5 : (norm_consumer ? 6 : (fused_norm ? 4 : (fused_act ? 3 : (prerot ? 2 : 0))))));
     if (!fn) return fail(AMP_E_UNSUPPORTED, "exl3_gemv: no kernel for K=%d cb=%d", K, A.cb);
@@ -617,7 +623,7 @@ AMP_API int amp_exl3_gemv_allreduce(const void* x, const void* trellis, void* ou
     return launch_gemv(A, stream);
 }
 
-// The same with a scratch for the rotated input ((m, k) fp16, nullable): from five rows on the input
+// The same with a scratch for the rotated input ((m, k) fp16, nullable): the input
 // is then rotated once by a small launch of its own instead of by every CTA (as amp_exl3_gemm's A_had).
 AMP_API int amp_exl3_gemv_allreduce_rot(const void* x, const void* trellis, void* out, const void* suh, const void* svh,
                                         int m, int k, int n, int K, int cb, void* const* bufs, int* const* ctls,
@@ -778,7 +784,7 @@ extern "C" int amp_had_r_128(const void* in, void* out, const void* pre, const v
                              long rows, int cols, int dtype, float scale, cudaStream_t stream);
 
 // C = had(A*suh) @ W_hat -> had(.)*svh for any m. Up to 16 rows run on the decode kernel (the input
-// transform lives in the kernel's prologue up to four rows; from five rows on, when A_had is given,
+// transform lives in the kernel's prologue; from five rows on, large weights from fewer, when A_had is given,
 // a small launch of its own rotates the input into A_had once); more rows take the
 // tensor-core path: x~ is written into A_had (same shape as A, fp16: required) by the Hadamard
 // kernel and the tcgen05 GEMM consumes it. a_bf16: A holds bf16 instead of fp16 (m > 16 only).
@@ -825,7 +831,7 @@ static int gemm_any(const void* A, int a_bf16, const void* trellis, void* C, con
     if (m <= 16 && !a_bf16 && !(few_rows_on_tensor_cores(m, k, n) && ((uintptr_t) C & 15) == 0 && ((uintptr_t) A_had & 15) == 0))
     {
         GemvLaunch L = direct(A, trellis, C, suh, svh, m, k, n, K, cb, c_fp32, 0, 0);
-        L.x_rot = A_had;                               // optional: used from five rows up
+        L.x_rot = A_had;                               // optional
         return launch_gemv(L, stream);
     }
     AMP_REQUIRE(A_had || (m <= 16 && !a_bf16), "exl3_gemm: A_had scratch (same shape as A, fp16) is required above 16 rows");
@@ -892,7 +898,7 @@ static int mgemm_any(const void* x, int x_bf16, const void* trellis_ptrs, void* 
     A.tables = 1; A.slices = num; A.width = width; A.stride = width;
     A.m = m; A.k = k; A.K = K; A.cb = cb; A.c_fp32 = c_fp32;
     A.num_src = had_src_list ? num_had_src : num;
-    A.x_rot = A.num_src >= 1 ? A_had : nullptr;                     // optional: used from five rows up
+    A.x_rot = A.num_src >= 1 ? A_had : nullptr;                     // optional
     return launch_gemv(A, stream);
 }
 

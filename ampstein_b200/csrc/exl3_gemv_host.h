@@ -32,7 +32,7 @@ struct GemvLaunch
     void* am_ws;         // >= 16 bytes, 8-byte aligned, zero before the first launch (key + block counter)
     void* am_ids; void* am_pos; void* am_log; long long am_log_cap;
     int am_vocab;
-    void* x_rot;         // optional scratch, (sources, m, k) fp16: with five rows or more the input is rotated
+    void* x_rot;         // optional scratch, (sources, m, k) fp16: from five rows on (large weights: fewer) the input is rotated
     int num_src;         // once by a launch of its own instead of by every CTA (sources: 1, or the bundle's)
 };
 

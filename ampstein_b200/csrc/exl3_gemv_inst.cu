@@ -34,7 +34,7 @@ gemv_fn AMP_CAT(gemv_kernel_k, AMP_GEMV_K)(int cb, int MB, int mode, int gin)
         { exl3_gemv_kernel<AMP_GEMV_K, 1, 1, 0, 1>, exl3_gemv_kernel<AMP_GEMV_K, 1, 2, 0, 1> },
         { exl3_gemv_kernel<AMP_GEMV_K, 2, 1, 0, 1>, exl3_gemv_kernel<AMP_GEMV_K, 2, 2, 0, 1> },
     };
-    // input already rotated (batches of five rows and more)
+    // input already rotated
     static const gemv_fn fnr[3][2] =
     {
         { exl3_gemv_kernel<AMP_GEMV_K, 0, 1, 0, 2>, exl3_gemv_kernel<AMP_GEMV_K, 0, 2, 0, 2> },

@@ -193,13 +193,18 @@ def exl3_gemm(A, B, C, suh, svh, mul1=False, mcg=False):
     K = _kcode("exl3_gemm", K, mul1)
     # the binding allocates the input-rotation scratch per call, as the reference's does
     # (src/torch/amp_torch.cpp:11282); the decode kernel (<= 16 rows) does not need it
-    # (from five rows on it lets the input be rotated once instead of by every CTA; the half-rate
-    # kernel always takes its input rotated)
-    A_had = torch.empty(A.shape, dtype=torch.float16, device=A.device) if (m >= 5 or bf16 or half_rate) else None
+    # (it lets the input be rotated once instead of by every CTA)
+    A_had = torch.empty(A.shape, dtype=torch.float16, device=A.device) if (bf16 or half_rate or _rotates_once(m, k, n)) else None
     _launch(A, "amp_exl3_gemm_bf16" if bf16 else "amp_exl3_gemm", A.data_ptr(), B.data_ptr(), C.data_ptr(),
                   suh.data_ptr(), A_had.data_ptr() if A_had is not None else None, svh.data_ptr(), m, k, n, K,
                   _cb(mul1, mcg), 1 if C.dtype == torch.float32 else 0)
     return C
+
+
+def _rotates_once(m, k, n):
+    """Whether the decode kernel may use a scratch for the rotated input: from five rows on, and with fewer where the
+    weight is large (the library decides by the device's size; this is its rule for 148 SMs, rounded down)."""
+    return m >= 5 or (m - 1) * k * n >= 200000000 or k * n >= 330000000
 
 
 class GemmPlan:
@@ -232,8 +237,8 @@ class GemmPlan:
         if k != self.k or m < 1 or dev < 0 or dev != t.get_device() or _get_device() != dev:
             return None
         y = x.new_empty((m, self.n))
-        had = x.new_empty((m, k)) if m >= 5 else None            # rotation scratch, as in exl3_gemm
-        _lib.call("amp_exl3_gemm", x.data_ptr(), t.data_ptr(), y.data_ptr(), s.data_ptr(), had.data_ptr() if m >= 5 else None, v.data_ptr(), m, k, self.n, self.K,
+        had = x.new_empty((m, k)) if _rotates_once(m, k, self.n) else None            # rotation scratch, as in exl3_gemm
+        _lib.call("amp_exl3_gemm", x.data_ptr(), t.data_ptr(), y.data_ptr(), s.data_ptr(), had.data_ptr() if had is not None else None, v.data_ptr(), m, k, self.n, self.K,
                   self.cb, 0, _raw_stream(dev))
         return y
 
@@ -533,7 +538,7 @@ def mgemm(x, B_ptrs, C, suh_ptrs, A_had, svh_ptrs, K, mcg, mul1, opts=None):
         if not x.is_contiguous():
             raise ValueError("mgemm: x must be contiguous")
     _launch(x, "amp_exl3_mgemm_bf16" if bf16 else "amp_exl3_mgemm", x.data_ptr(), B_ptrs.data_ptr(), C.data_ptr(), suh_ptrs.data_ptr(),
-                  A_had.data_ptr() if A_had is not None else None, svh_ptrs.data_ptr(), num, m, k, width,
+                  A_had.data_ptr() if A_had is not None and (m >= 5 or bf16) else None, svh_ptrs.data_ptr(), num, m, k, width,
                   int(K), _cb(mul1, mcg), 1 if C.dtype == torch.float32 else 0,
                   c_ptrs.data_ptr() if c_ptrs is not None else None,
                   n_stride.data_ptr() if n_stride is not None else None,

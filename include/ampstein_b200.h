@@ -279,7 +279,7 @@ int amp_exl3_mgemm_rms_norm_res(const void* x, const void* res, const void* norm
  *   c_ptrs[num] + n_stride_list[num]  per-slice output pointer and row width of the matrix it
  *                                     belongs to; both NULL = outputs stacked in C (num, m, width)
  * All slices share k, K, the codebook and the width (a multiple of 128). Up to 16 rows run on the
- * decode kernel (A_had, when given, receives the rotated input of every source from five rows up,
+ * decode kernel (A_had, when given, receives the rotated input of every source from five rows up, or fewer where the weight is large,
  * as for amp_exl3_gemm); more rows run as ONE tensor-core grid over all slices and A_had
  * ((sources, m, k) fp16, sources = num_had_src or num) is required.
  * Replaces: exl3_mgemm, Q/exl3_gemm.cu:351-735 (binding torch.mgemm,
@@ -538,8 +538,8 @@ int amp_comm_allreduce_fp16(const void* x, void* out, void* const* bufs, int* co
 int amp_exl3_gemv_allreduce(const void* x, const void* trellis, void* out, const void* suh, const void* svh,
                             int m, int k, int n, int K, int cb, void* const* bufs, int* const* ctls,
                             int rank, int N, long cap, cudaStream_t stream);
-/* The same with an optional scratch for the rotated input ((m, k) fp16 or NULL), used from five rows
- * on exactly as amp_exl3_gemm uses A_had. */
+/* The same with an optional scratch for the rotated input ((m, k) fp16 or NULL), used
+ * exactly as amp_exl3_gemm uses A_had. */
 int amp_exl3_gemv_allreduce_rot(const void* x, const void* trellis, void* out, const void* suh, const void* svh,
                                 int m, int k, int n, int K, int cb, void* const* bufs, int* const* ctls,
                                 int rank, int N, long cap, void* x_rot, cudaStream_t stream);

@@ -273,6 +273,26 @@ def test_mgemm_bundles_above_16_rows(amp, oracle, m, bf16):
     assert gemm_status() == 0
 
 
+@pytest.mark.parametrize("m,K,cb", [(1, 2, 0), (2, 2, 1), (3, 2, 2), (4, 3, 1)])
+def test_rows_1_to_4_of_a_large_weight_with_and_without_the_rotation_scratch(amp, m, K, cb):
+    """A weight large enough that one to four rows are rotated once too: the same bits either way."""
+    from ampstein_b200 import _lib
+    k, n = 2048, 230400
+    torch.manual_seed(6400 + m)
+    t = torch.randint(-32768, 32768, (k // 16, n // 16, 16 * K), dtype=torch.int16, device="cuda")
+    su, sv = ((torch.randint(0, 2, (w,), device="cuda") * 2 - 1).half() for w in (k, n))
+    x = torch.randn(m, k, device="cuda").half()
+    outs = []
+    for scratch in (None, torch.full((m, k), float("nan"), dtype=torch.float16, device="cuda")):
+        y = torch.full((m, n), float("nan"), dtype=torch.float32, device="cuda")
+        _lib.call("amp_exl3_gemm", x.data_ptr(), t.data_ptr(), y.data_ptr(), su.data_ptr(),
+                  scratch.data_ptr() if scratch is not None else None, sv.data_ptr(), m, k, n, K, cb, 1,
+                  torch.cuda.current_stream().cuda_stream)
+        outs.append(y)
+    torch.cuda.synchronize()
+    assert torch.equal(outs[0], outs[1]) and not scratch.isnan().any()
+
+
 @pytest.mark.parametrize("m,K,cb", [(5, 4, 0), (8, 5, 0), (8, 3, 2), (13, 4, 1), (16, 6, 0)])
 def test_rows_5_to_16_with_and_without_the_rotation_scratch(amp, oracle, m, K, cb):
     """From five rows on, exl3_gemm with A_had rotates the input once in a launch of its own; without
