@@ -234,7 +234,7 @@ int launch_gemv(const GemvLaunch& A, cudaStream_t stream)
     const bool prerot = !tc && !A.mode && !A.arin.N && !special_in && A.x_rot && A.x &&
                         (m >= GEMV_PREROTATE_MIN_M || (m >= 2 && (m - 1) * per >= GEMV_PREROTATE_MIN_PER) || (m == 1 && !i8 && per >= 100));
     gemv_fn fn = tc ? gemv_tc_kernel_for(K, A.cb, A.ar.N != 0)
-                    : gemv_kernel_for(K, i8 ? i8 : A.cb, MB, A.mode, A.mode ? (A.moe.inline_runs ? 7 : 0) : A.arin.N ? 1 : (norm_producer ? 5 : (norm_consumer ? 6 : (fused_norm ? 4 : (fused_act ? 3 : (prerot ? 2 : 0))))));
+                    : gemv_kernel_for(K, i8 ? i8 : A.cb, MB, A.mode, A.mode ? (A.moe.inline_runs ? 7 : 0) : A.arin.N ? 1 : (norm_producer ? 5 : (norm_consumer ? 6 : (fused_norm ? 4 : (fused_act ? 3 : (A.ar.N ? 8 : 0) + (prerot ? (A.ar.N ? 1 : 2) : 0))))));
     if (!fn) return fail(AMP_E_UNSUPPORTED, "exl3_gemv: no kernel for K=%d cb=%d", K, A.cb);
 
     // x~ rows resident at a time: at most 16 KB of shared memory (whole segments for small

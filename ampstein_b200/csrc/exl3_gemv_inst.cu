@@ -16,13 +16,16 @@ namespace amp {
 // half-integer bitrates (mul1 codebook): single matrices, fp16 activations
 gemv_fn AMP_CAT(gemv_kernel_k, AMP_GEMV_K)(int cb, int MB, int mode, int gin)
 {
-    static const gemv_fn fn[2][2] =
+    // plain input, input already rotated; the same with the fused all-reduce
+    static const gemv_fn fn[4][2] =
     {
         { exl3_gemv_kernel<AMP_GEMV_K, 2, 1>, exl3_gemv_kernel<AMP_GEMV_K, 2, 2> },
         { exl3_gemv_kernel<AMP_GEMV_K, 2, 1, 0, 2>, exl3_gemv_kernel<AMP_GEMV_K, 2, 2, 0, 2> },
+        { exl3_gemv_kernel<AMP_GEMV_K, 2, 1, 0, 8>, exl3_gemv_kernel<AMP_GEMV_K, 2, 2, 0, 8> },
+        { exl3_gemv_kernel<AMP_GEMV_K, 2, 1, 0, 9>, exl3_gemv_kernel<AMP_GEMV_K, 2, 2, 0, 9> },
     };
-    if (cb != 2 || mode || (gin != 0 && gin != 2) || MB < 1 || MB > 2) return nullptr;
-    return fn[gin / 2][MB - 1];
+    if (cb != 2 || mode || (gin != 0 && gin != 2 && gin != 8 && gin != 9) || MB < 1 || MB > 2) return nullptr;
+    return fn[gin >= 8 ? gin - 6 : gin / 2][MB - 1];
 }
 #else
 gemv_fn AMP_CAT(gemv_kernel_k, AMP_GEMV_K)(int cb, int MB, int mode, int gin)
@@ -74,6 +77,19 @@ gemv_fn AMP_CAT(gemv_kernel_k, AMP_GEMV_K)(int cb, int MB, int mode, int gin)
         { exl3_gemv_kernel<AMP_GEMV_K, 1, 1>, exl3_gemv_kernel<AMP_GEMV_K, 1, 2> },
         { exl3_gemv_kernel<AMP_GEMV_K, 2, 1>, exl3_gemv_kernel<AMP_GEMV_K, 2, 2> },
     };
+    // with the fused all-reduce: plain input (8), input already rotated (9)
+    static const gemv_fn far[3][2] =
+    {
+        { exl3_gemv_kernel<AMP_GEMV_K, 0, 1, 0, 8>, exl3_gemv_kernel<AMP_GEMV_K, 0, 2, 0, 8> },
+        { exl3_gemv_kernel<AMP_GEMV_K, 1, 1, 0, 8>, exl3_gemv_kernel<AMP_GEMV_K, 1, 2, 0, 8> },
+        { exl3_gemv_kernel<AMP_GEMV_K, 2, 1, 0, 8>, exl3_gemv_kernel<AMP_GEMV_K, 2, 2, 0, 8> },
+    };
+    static const gemv_fn farr[3][2] =
+    {
+        { exl3_gemv_kernel<AMP_GEMV_K, 0, 1, 0, 9>, exl3_gemv_kernel<AMP_GEMV_K, 0, 2, 0, 9> },
+        { exl3_gemv_kernel<AMP_GEMV_K, 1, 1, 0, 9>, exl3_gemv_kernel<AMP_GEMV_K, 1, 2, 0, 9> },
+        { exl3_gemv_kernel<AMP_GEMV_K, 2, 1, 0, 9>, exl3_gemv_kernel<AMP_GEMV_K, 2, 2, 0, 9> },
+    };
     // grouped experts: runs from a table, and a single token (gin 7)
     static const gemv_fn moe[3][2] =
     {
@@ -88,10 +104,11 @@ gemv_fn AMP_CAT(gemv_kernel_k, AMP_GEMV_K)(int cb, int MB, int mode, int gin)
         { exl3_gemv_kernel<AMP_GEMV_K, 2, 1, 1, 7>, exl3_gemv_kernel<AMP_GEMV_K, 2, 1, 2, 7> },
     };
     // cb 3 = the mul1 codebook with int8 activations: one batch row, plain launches only
-    if (cb == 3) return (MB == 1 && !mode && !gin) ? exl3_gemv_kernel<AMP_GEMV_K, 3, 1> : nullptr;
-    if (cb == 4) return (MB == 1 && !mode && !gin) ? exl3_gemv_kernel<AMP_GEMV_K, 4, 1> : nullptr;
+    if (cb == 3) return (MB == 1 && !mode && (!gin || gin == 8)) ? (gin ? exl3_gemv_kernel<AMP_GEMV_K, 3, 1, 0, 8> : exl3_gemv_kernel<AMP_GEMV_K, 3, 1>) : nullptr;
+    if (cb == 4) return (MB == 1 && !mode && (!gin || gin == 8)) ? (gin ? exl3_gemv_kernel<AMP_GEMV_K, 4, 1, 0, 8> : exl3_gemv_kernel<AMP_GEMV_K, 4, 1>) : nullptr;
     if (cb < 0 || cb > 2 || MB < 1 || MB > 2 || mode < 0 || mode > 2) return nullptr;
     if (mode) return (MB == 1 && (!gin || gin == 7)) ? (gin ? one : moe)[cb][mode - 1] : nullptr;
+    if (gin >= 8) return (gin == 8 ? far : farr)[cb][MB - 1];
     if (gin == 4) return fnn[cb][MB - 1];
     if (gin == 5) return fnp[cb][MB - 1];
     if (gin == 6) return fnc[cb][MB - 1];

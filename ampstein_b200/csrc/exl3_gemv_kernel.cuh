@@ -716,11 +716,15 @@ static __device__ __noinline__ void gemv_reduce_partials(float* part, const floa
 // 4: the input is RMSNorm(x + x2) * norm_w (residual add and norm in front of q|k|v, gate|up, lm_head).
 // 5 / 6: the same norm split between the producer of the residual contribution (its epilogue adds it to
 // the stream and leaves per-block sums of squares) and the consumer (its prologue only scales).
-template <int K, int CB, int MB, int MODE = 0, int GIN = 0>
+template <int K, int CB, int MB, int MODE = 0, int FORM = 0>
 __global__ __launch_bounds__(GEMV_THREADS, (MB == 1 ? AMP_GEMV_MINBLOCKS : 3))
 void exl3_gemv_kernel(const GemvParams P)
 {
     extern __shared__ __align__(128) unsigned char smem[];
+    // FORM: the input side (GIN), and for the plain and the rotated input whether the fused all-reduce is in it (8, 9)
+    // or not (0, 2): most launches have none, and carry neither its code nor its registers
+    constexpr int GIN = FORM == 8 ? 0 : (FORM == 9 ? 2 : FORM);
+    constexpr bool AR = MODE == 0 && FORM != 0 && FORM != 2;
     const GemvSmem L = gemv_smem_layout(K, P.m, P.xgroups, P.cluster, GIN == 1, (GIN == 4 || CB == 4) ? P.rowbuf : 0);
     int XPITCH = gemv_xpitch(P.xgroups);               // (grouped modes: per segment)
     int XG = P.xgroups;
@@ -1878,7 +1882,7 @@ void exl3_gemv_kernel(const GemvParams P)
                     half4 o;
                     o.x = __hmul2(__floats2half2_rn(h0, h1), sv.x);
                     o.y = __hmul2(__floats2half2_rn(h2, h3), sv.y);
-                    if constexpr (MODE == 0)
+                    if constexpr (AR)
                     {
                         if (P.ar.N)
                         {
@@ -1973,7 +1977,7 @@ void exl3_gemv_kernel(const GemvParams P)
                     }
                 }
             }
-            if constexpr (MODE == 0)
+            if constexpr (AR)
             {
                 if (P.ar.N)
                 {
