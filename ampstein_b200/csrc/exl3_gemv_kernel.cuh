@@ -716,13 +716,17 @@ static __device__ __noinline__ void gemv_reduce_partials(float* part, const floa
 // 4: the input is RMSNorm(x + x2) * norm_w (residual add and norm in front of q|k|v, gate|up, lm_head).
 // 5 / 6: the same norm split between the producer of the residual contribution (its epilogue adds it to
 // the stream and leaves per-block sums of squares) and the consumer (its prologue only scales).
+// 7: a single token of the grouped modes. 8 / 9: plain / rotated input with the fused all-reduce.
 template <int K, int CB, int MB, int MODE = 0, int FORM = 0>
 __global__ __launch_bounds__(GEMV_THREADS, (MB == 1 ? AMP_GEMV_MINBLOCKS : 3))
 void exl3_gemv_kernel(const GemvParams P)
 {
     extern __shared__ __align__(128) unsigned char smem[];
     // FORM: the input side (GIN), and for the plain and the rotated input whether the fused all-reduce is in it (8, 9)
-    // or not (0, 2): most launches have none, and carry neither its code nor its registers
+    // or not (0, 2): most launches have none, and carry neither its code nor its registers (with it in the plain instances:
+    // spills around the main loop, 5120 x 25600 at 8 rows 48.9 -> 54.7 us, the decode step 2286 -> 2336). No further
+    // split: with the cluster launch as an instance of its own, single shapes gained (4096 x 6144 9.5 -> 8.5 us) and the step
+    // lost (2479), as launches of changing functions start with cold instruction caches
     constexpr int GIN = FORM == 8 ? 0 : (FORM == 9 ? 2 : FORM);
     constexpr bool AR = MODE == 0 && FORM != 0 && FORM != 2;
     const GemvSmem L = gemv_smem_layout(K, P.m, P.xgroups, P.cluster, GIN == 1, (GIN == 4 || CB == 4) ? P.rowbuf : 0);
