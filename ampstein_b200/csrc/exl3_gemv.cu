@@ -174,10 +174,13 @@ int g_int8_max_k = int8_env("EXL3_INT8_GEMV_MAX_K", 6);
 
 int launch_gemv(const GemvLaunch& A, cudaStream_t stream)
 {
-    const int m = A.m, k = A.k, K = A.K;
-    const bool half_rate = K > GEMV_HALF;
-    AMP_REQUIRE((K >= 1 && K <= 8) || (K <= GEMV_HALF + 3 && half_rate && A.cb == 2 && !A.mode && !A.tables),
-                "exl3_gemv: unsupported EXL3 bitrate %d (integer 1..8)", K);
+    const int m = A.m, k = A.k;
+    // (A.K comes from the caller of an entry point: the code of the half-integer instances is formed here only, so that
+    // no value of it names one)
+    const bool half_rate = A.half_rate != 0;
+    AMP_REQUIRE(half_rate ? A.K >= 1 && A.K <= 3 && A.cb == 2 && !A.mode && !A.tables : A.K >= 1 && A.K <= 8,
+                "exl3_gemv: unsupported EXL3 bitrate %d (integer 1..8)", A.K);
+    const int K = half_rate ? GEMV_HALF + A.K : A.K;
     AMP_REQUIRE(A.cb >= 0 && A.cb <= 2, "exl3_gemv: codebook index %d out of range", A.cb);
     AMP_REQUIRE(m >= 1 && m <= 16, "exl3_gemv: m must be 1..16 (got %d)", m);
     AMP_REQUIRE(k > 0 && A.width > 0 && k % 128 == 0 && A.width % 128 == 0 && A.stride % 128 == 0,
@@ -824,10 +827,13 @@ static int gemm_any(const void* A, int a_bf16, const void* trellis, void* C, con
         AMP_REQUIRE(K <= 256 + 3 && cb == 2, "exl3_gemm: half-integer bitrates are 1.5 / 2.5 / 3.5 with the mul1 codebook");
         AMP_REQUIRE(m <= 16 && !a_bf16, "exl3_gemm: half-integer bitrates take up to 16 fp16 rows here");
         AMP_REQUIRE(A && suh && A_had && k > 0 && k % 128 == 0, "exl3_gemm: half-integer bitrates need the A_had scratch (same shape as A)");
-        GemvLaunch L = direct(A, trellis, C, suh, svh, m, k, n, GEMV_HALF + K - 256, cb, c_fp32, 0, 0);
+        GemvLaunch L = direct(A, trellis, C, suh, svh, m, k, n, K - 256, cb, c_fp32, 0, 0);
+        L.half_rate = 1;
         L.x_rot = A_had; L.num_src = 1;
         return launch_gemv(L, stream);
     }
+    // (before the rotation kernel of the many-rows path runs: what is refused is refused whatever the row count)
+    AMP_REQUIRE(K >= 1 && K <= 8, "exl3_gemm: unsupported EXL3 bitrate %d (integer 1..8, or AMP_EXL3_HALF_RATE)", K);
     if (m <= 16 && !a_bf16 && !(few_rows_on_tensor_cores(m, k, n) && ((uintptr_t) C & 15) == 0 && ((uintptr_t) A_had & 15) == 0))
     {
         GemvLaunch L = direct(A, trellis, C, suh, svh, m, k, n, K, cb, c_fp32, 0, 0);
@@ -875,6 +881,7 @@ static int mgemm_any(const void* x, int x_bf16, const void* trellis_ptrs, void* 
 {
     if (num == 0 || m == 0) return 0;
     AMP_REQUIRE(num > 0 && m > 0, "exl3_mgemm: negative matrix or row count");
+    AMP_REQUIRE(K >= 1 && K <= 8, "exl3_mgemm: unsupported EXL3 bitrate %d (integer 1..8)", K);
     const int sources = had_src_list ? num_had_src : num;
     const bool few = m <= 16 && !x_bf16;
     if (!few || (sources >= 1 && sources <= 3 && ((uintptr_t) C & 15) == 0 && ((uintptr_t) A_had & 15) == 0 && few_rows_on_tensor_cores(m, k, (long) num * width)))

@@ -4,6 +4,8 @@ import ctypes
 import os
 import re
 
+import pytest
+
 from conftest import ROOT
 
 
@@ -51,8 +53,42 @@ def test_bad_arguments_return_codes_without_a_gpu():
     assert L.amp_had_r_128(p, p, None, None, 0, 128, 0, 1.0, None) == 0
 
 
+@pytest.mark.parametrize("K", [0, 9, 16, 17, 18, 19, 20, -1, 256, 260])
+def test_no_entry_takes_an_internal_bitrate_code(K):
+    """The decode kernel's instances for half-integer rates have codes of their own (17..19); a caller's K of that value
+    is not a bitrate, at any row count and with any entry (amp_exl3_gemv_static asks for the device first and is left out).
+    The refusal comes before any CUDA call."""
+    from ampstein_b200 import _lib
+    L = _lib.lib()
+    buf = ctypes.create_string_buffer(4096)
+    p = ctypes.addressof(buf)
+    p += (-p) % 16
+    q = p + 1024                                             # (outputs that must not alias an input)
+    bufs = (ctypes.c_void_p * 2)(p, p)
+    k = n = 128
+    calls = [("amp_exl3_gemv", (p, p, q, p, p, 1, k, n, K, 2, 0, None)),
+             ("amp_exl3_gemv_cfg", (p, p, q, p, p, 1, k, n, K, 2, 0, 0, 0, None)),
+             ("amp_exl3_gemv_allreduce", (p, p, q, p, p, 1, k, n, K, 2, bufs, bufs, 0, 2, 4096, None)),
+             ("amp_exl3_gemv_allreduce_rot", (p, p, q, p, p, 1, k, n, K, 2, bufs, bufs, 0, 2, 4096, p, None)),
+             ("amp_exl3_gemv_push", (p, p, p, p, 1, k, n, K, 2, bufs, bufs, 0, 2, 4096, None)),
+             ("amp_exl3_gemv_gathered", (p, q, p, p, 1, k, n, K, 2, 0, p, p, 2, 4096, None)),
+             ("amp_exl3_gemv_silu_mul", (p, p, p, q, p, p, 1, k, n, K, 2, 0, None)),
+             ("amp_exl3_gemv_rms_norm_res", (p, p, p, 1e-5, q, p, q, p, p, 1, k, n, K, 2, 0, None)),
+             ("amp_exl3_gemv_add_res", (p, p, p, p, p, q, q, 1, k, n, K, 2, None)),
+             ("amp_exl3_gemv_normed", (p, p, p, 1e-5, p, q, p, p, 1, k, n, K, 2, 0, None)),
+             ("amp_exl3_mgemm_normed", (p, p, p, 1e-5, p, q, p, p, 1, 1, k, n, K, 2, 0, None, None, None, None))]
+    for m in (1, 8, 9, 16, 17, 600):
+        calls += [("amp_exl3_gemm", (p, p, q, p, p, p, m, k, n, K, 2, 0, None)),
+                  ("amp_exl3_mgemm", (p, p, q, p, p, p, 1, m, k, n, K, 2, 0, None, None, None, 0, None))]
+    for name, args in calls:
+        if name == "amp_exl3_gemm" and K > 256:
+            continue                                         # AMP_EXL3_HALF_RATE is this entry's own; its range: below
+        assert getattr(L, name)(*args) < 0, name
+        assert "bitrate" in _lib.last_error(), (name, _lib.last_error())
+    assert L.amp_exl3_gemm(p, p, q, p, p, p, 1, k, n, 260, 2, 0, None) < 0 and "half-integer" in _lib.last_error()
+
+
 def test_python_front_end_rejects_cpu_tensors():
-    import pytest
     import torch
     import ampstein_b200 as amp
     t = torch.zeros((8, 8, 64), dtype=torch.int16)
