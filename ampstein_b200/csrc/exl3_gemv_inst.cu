@@ -16,16 +16,14 @@ namespace amp {
 // half-integer bitrates (mul1 codebook): single matrices, fp16 activations
 gemv_fn AMP_CAT(gemv_kernel_k, AMP_GEMV_K)(int cb, int MB, int mode, int gin)
 {
-    // plain input, input already rotated; the same with the fused all-reduce
-    static const gemv_fn fn[4][2] =
+    // plain input, input already rotated (no fused all-reduce: no entry takes these rates with one)
+    static const gemv_fn fn[2][2] =
     {
         { exl3_gemv_kernel<AMP_GEMV_K, 2, 1>, exl3_gemv_kernel<AMP_GEMV_K, 2, 2> },
         { exl3_gemv_kernel<AMP_GEMV_K, 2, 1, 0, 2>, exl3_gemv_kernel<AMP_GEMV_K, 2, 2, 0, 2> },
-        { exl3_gemv_kernel<AMP_GEMV_K, 2, 1, 0, 8>, exl3_gemv_kernel<AMP_GEMV_K, 2, 2, 0, 8> },
-        { exl3_gemv_kernel<AMP_GEMV_K, 2, 1, 0, 9>, exl3_gemv_kernel<AMP_GEMV_K, 2, 2, 0, 9> },
     };
-    if (cb != 2 || mode || (gin != 0 && gin != 2 && gin != 8 && gin != 9) || MB < 1 || MB > 2) return nullptr;
-    return fn[gin >= 8 ? gin - 6 : gin / 2][MB - 1];
+    if (cb != 2 || mode || (gin != 0 && gin != 2) || MB < 1 || MB > 2) return nullptr;
+    return fn[gin / 2][MB - 1];
 }
 #else
 gemv_fn AMP_CAT(gemv_kernel_k, AMP_GEMV_K)(int cb, int MB, int mode, int gin)
