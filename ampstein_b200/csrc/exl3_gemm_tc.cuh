@@ -386,6 +386,7 @@ void exl3_gemm_tc_kernel(const TgParams S)
         s_bad = 0;
     }
     __syncwarp();
+    if (split > 1) cluster_arrive_started();
     if (warp == NDEC)
     {
         if constexpr (PAIR)
@@ -584,8 +585,8 @@ void exl3_gemm_tc_kernel(const TgParams S)
     if (warp < NDEC) wait_bar(b_done + ((nsteps - 1) % DS) * 8, (uint32_t) (((nsteps - 1) / DS) & 1));
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-    // peers write into this CTA's receive buffer from here on: where it overlaps the stages, everybody's MMAs
-    // must have read theirs
+    if (split > 1) cluster_wait_started();                   // the peers run: their shared memory is written from here on
+    // ... and they write into this CTA's receive buffer: where it overlaps the stages, everybody's MMAs must have read theirs
     if (split > 1 && S.recv_off == 0) cluster_sync_all();
     const int row = tg_row(split), n0 = S.n0;
     // passes of equal length, each CTA of the cluster finishing TS tokens of a pass

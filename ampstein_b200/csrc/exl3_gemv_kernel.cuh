@@ -526,6 +526,19 @@ __device__ __forceinline__ void cluster_st_f32(uint32_t addr, float v)
     asm volatile("st.shared::cluster.f32 [%0], %1;" :: "r"(addr), "f"(v) : "memory");
 }
 
+// A CTA's shared memory may be accessed by a peer only once that CTA is known to run: every thread arrives at the top of
+// the kernel and waits in front of its first access, by when the peers have long started (the wait costs nothing there). The
+// arrival releases what the thread wrote to its own shared memory before it.
+__device__ __forceinline__ void cluster_arrive_started()
+{
+    asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+}
+
+__device__ __forceinline__ void cluster_wait_started()
+{
+    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+
 __device__ __forceinline__ void cluster_sync_all()
 {
     asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
@@ -864,6 +877,7 @@ void exl3_gemv_kernel(const GemvParams P)
             u1 = u0 + per;
         }
     }
+    if (!RUNS && P.cluster) cluster_arrive_started();
 
     const uint32_t ring_s = smem_u32(smem + L.ring) + warp * (S * SLOT);      // this warp's ring
 
@@ -1713,7 +1727,11 @@ void exl3_gemv_kernel(const GemvParams P)
         // cluster form: the partial goes straight into the shared memory of the cluster's first CTA
         const bool clustered = !RUNS && P.cluster > 0;
         uint32_t xdst = 0;
-        if (clustered) xdst = cluster_map(smem_u32(smem + L.xchg), 0) + cluster_rank() * (m * 128 * 4);
+        if (clustered)
+        {
+            cluster_wait_started();                    // (the first CTA runs: its shared memory is written next; one segment per CTA)
+            xdst = cluster_map(smem_u32(smem + L.xchg), 0) + cluster_rank() * (m * 128 * 4);
+        }
         #pragma unroll
         for (int nt = 0; nt < NT; ++nt)
         #pragma unroll

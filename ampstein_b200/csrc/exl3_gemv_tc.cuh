@@ -163,6 +163,7 @@ void exl3_gemv_tc_kernel(const GemvParams P)
     split.q = U / ncta;
     split.r = U - split.q * ncta;
     const int u0 = split.begin(cta), u1 = split.begin(cta + 1);
+    if (P.cluster > 0) cluster_arrive_started();
 
     if (t == 0)
     {
@@ -541,7 +542,11 @@ void exl3_gemv_tc_kernel(const GemvParams P)
             float* dst = whole ? part : slots + (size_t) my_slot * m * 128;
             const bool clustered = P.cluster > 0;
             uint32_t xdst = 0;
-            if (clustered) xdst = cluster_map(smem_u32(smem + L.xchg), 0) + cluster_rank() * (m * 128 * 4);
+            if (clustered)
+            {
+                cluster_wait_started();                // (one segment per CTA)
+                xdst = cluster_map(smem_u32(smem + L.xchg), 0) + cluster_rank() * (m * 128 * 4);
+            }
             const int col = 32 * warp + lane;
             #pragma unroll
             for (int b = 0; b < TCV_MAX_M; ++b)
@@ -675,7 +680,7 @@ void exl3_gemv_tc_kernel(const GemvParams P)
         cp_async_wait_n<0>();
     }
     // the cluster barrier is a whole-CTA affair: the issuing warp joins it here
-    if (warp == TCV_WARPS && P.cluster > 0) cluster_sync_all();
+    if (warp == TCV_WARPS && P.cluster > 0) { cluster_wait_started(); cluster_sync_all(); }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
     if (warp == TCV_WARPS)
