@@ -10,8 +10,10 @@ import torch
 from . import _lib
 
 
-_raw_stream = torch._C._cuda_getCurrentRawStream       # (torch.cuda.current_stream builds a Stream object: 2 us)
-_get_device = torch._C._cuda_getDevice
+# The current stream's handle and device without the objects torch.cuda builds around them (2 us). Both are private to
+# torch and absent where it is built without CUDA: the public forms stand in.
+_raw_stream = getattr(torch._C, "_cuda_getCurrentRawStream", None) or (lambda dev: torch.cuda.current_stream(dev).cuda_stream)
+_get_device = getattr(torch._C, "_cuda_getDevice", None) or torch.cuda.current_device
 
 
 def _stream(t):

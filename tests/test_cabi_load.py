@@ -97,3 +97,17 @@ def test_python_front_end_rejects_cpu_tensors():
         amp.exl3_reconstruct(w, t, 4)
     with pytest.raises(TypeError):
         amp.exl3_gemm(w, t, w, None, None)
+
+
+def test_package_imports_on_a_torch_without_cuda():
+    """torch's private CUDA functions do not exist in a CPU build; the package imports there, and its operators refuse
+    host tensors as they do everywhere."""
+    import subprocess
+    import sys
+    code = ("import torch\n"
+            "for n in [n for n in dir(torch._C) if n.startswith('_cuda_')]: delattr(torch._C, n)\n"
+            "import ampstein_b200 as amp, ampstein_b200.models\n"
+            "try: amp.exl3_reconstruct(torch.zeros((128, 128), dtype=torch.float16), torch.zeros((8, 8, 64), dtype=torch.int16), 4)\n"
+            "except RuntimeError as e: print('refused', e)\n")
+    r = subprocess.run([sys.executable, "-c", code], cwd=ROOT, capture_output=True, text=True)
+    assert r.returncode == 0 and r.stdout.startswith("refused"), r.stderr[-2000:]
