@@ -210,38 +210,50 @@ def _rotates_once(m, k, n):
 
 
 class GemmPlan:
-    """A checked weight (trellis, suh, svh) as exl3_gemm takes it, for callers that apply it many times: run()
-    checks only the activations (the full check costs as much host time as a small launch). Holds the tensors it
-    was made from; matches() tells whether they are still the caller's."""
+    """A weight (trellis, suh, svh, codebook flags) as exl3_gemm's checks found it, for callers that apply it many times.
+    It describes the weight and holds none of its tensors: matches() compares the caller's, as they are now, with the
+    description (a tensor may have been resized, or given other storage, behind the same object), and run() then checks
+    the activations alone."""
 
-    __slots__ = ("tensors", "k", "n", "K", "cb")
+    __slots__ = ("shape", "k", "n", "K", "cb", "mul1", "mcg", "rotate_from")
 
     def __init__(self, trellis, suh, svh, mul1=False, mcg=False):
         _check_cuda("exl3_gemm", trellis, suh, svh)
-        self.k, self.n, self.K = _trellis_dims("exl3_gemm", trellis)
-        if suh.dtype != torch.float16 or svh.dtype != torch.float16 or suh.numel() != self.k or svh.numel() != self.n:
+        self.k, self.n, self.K = _trellis_dims("exl3_gemm", trellis, half_ok=True)
+        if suh.dtype != torch.float16 or svh.dtype != torch.float16:
+            raise TypeError("exl3_gemm: A must be float16 (or bfloat16), suh and svh float16")
+        if suh.numel() != self.k or svh.numel() != self.n:
             raise ValueError("exl3_gemm: incompatible shapes")
         self.cb = _cb(mul1, mcg)
-        self.tensors = (trellis, suh, svh)
+        self.shape, self.mul1, self.mcg = trellis.shape, mul1, mcg
+        # fewest rows that get a rotation scratch, as in exl3_gemm; half-integer bitrates: none of this path
+        self.rotate_from = next(m for m in range(1, 6) if _rotates_once(m, self.k, self.n)) if float(self.K) == int(self.K) else None
 
-    def matches(self, trellis, suh, svh):
-        t = self.tensors
-        return t[0] is trellis and t[1] is suh and t[2] is svh
+    def matches(self, trellis, suh, svh, mul1, mcg):
+        try:
+            return (trellis.shape == self.shape and mul1 == self.mul1 and mcg == self.mcg
+                    and (trellis.dtype is torch.int16 or trellis.dtype is torch.uint16) and trellis.is_contiguous()
+                    and suh.dtype is torch.float16 and suh.numel() == self.k and suh.is_contiguous()
+                    and svh.dtype is torch.float16 and svh.numel() == self.n and svh.is_contiguous())
+        except AttributeError:
+            return False                                     # not a tensor: the full check says so
 
-    def run(self, x):
-        """The (m, n) fp16 result for a contiguous (m, k) fp16 CUDA tensor of at least one row on the weight's
-        device; None where x is anything else (the caller then takes exl3_gemm, which says what is wrong)."""
-        t, s, v = self.tensors
-        if x.dtype is not torch.float16 or x.dim() != 2 or not x.is_contiguous():
+    def run(self, x, trellis, suh, svh):
+        """The (m, n) fp16 result for a contiguous (m, k) fp16 CUDA tensor of at least one row and tensors that match,
+        all on the current device; None for anything else (the caller then takes exl3_gemm, which says what is wrong),
+        half-integer bitrates among it."""
+        shape = x.shape
+        if x.dtype is not torch.float16 or len(shape) != 2 or not x.is_contiguous() or self.rotate_from is None:
             return None
-        m, k = x.shape
+        m, k = shape
         dev = x.get_device()
-        if k != self.k or m < 1 or dev < 0 or dev != t.get_device() or _get_device() != dev:
+        if (k != self.k or m < 1 or dev < 0 or dev != trellis.get_device() or dev != suh.get_device() or dev != svh.get_device()
+                or _get_device() != dev):
             return None
         y = x.new_empty((m, self.n))
-        had = x.new_empty((m, k)) if _rotates_once(m, k, self.n) else None            # rotation scratch, as in exl3_gemm
-        _lib.call("amp_exl3_gemm", x.data_ptr(), t.data_ptr(), y.data_ptr(), s.data_ptr(), had.data_ptr() if had is not None else None, v.data_ptr(), m, k, self.n, self.K,
-                  self.cb, 0, _raw_stream(dev))
+        had = x.new_empty(shape) if m >= self.rotate_from else None
+        _lib.call("amp_exl3_gemm", x.data_ptr(), trellis.data_ptr(), y.data_ptr(), suh.data_ptr(), had.data_ptr() if had is not None else None,
+                  svh.data_ptr(), m, k, self.n, self.K, self.cb, 0, _raw_stream(dev))
         return y
 
 
