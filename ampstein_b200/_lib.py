@@ -48,6 +48,7 @@ SIGNATURES = {
     "amp_exl3_mgemm_normed": [_vp, _vp, _vp, ctypes.c_float, _vp, _vp, _vp, _vp, _i, _i, _i, _i, _i, _i, _i, _vp, _vp, _vp, _vp],
     "amp_exl3_set_gemm_pair": [_i],
     "amp_exl3_set_gemm_plan": [_i, _i],
+    "amp_exl3_set_gemm_wait_limit": [_i, _i],
     "amp_exl3_set_int8_gemv": [_i, _i],
     "amp_exl3_set_gemm_relay_release": [_i],
     "amp_comm_allreduce_fp16": [_vp, _vp, _vp, _vp, _i, _i, _l, _l, _i, _i, _vp],

@@ -7,6 +7,7 @@ namespace amp {
 __device__ int g_tc_status;
 int g_tc_relay_release = 0;
 int g_tc_pair = 1;                            // see amp_exl3_set_gemm_pair
+unsigned g_tc_wait[2] = { TC_SPIN_LIMIT, TC_SPIN_LIMIT };       // see amp_exl3_set_gemm_wait_limit
 int g_tc_split = 0, g_tc_tile = 0;            // forced (0: by rule), see amp_exl3_set_gemm_plan
 
 // address of the status word, looked up once per device (under a lock: two host threads may make their first launch
@@ -183,6 +184,7 @@ int launch_gemm_tc(const void* xh, const void* trellis, void* c, const void* svh
     P.M = M; P.k = k; P.n = n; P.c_fp32 = c_fp32;
     P.tables = T ? 1 : 0;
     P.relay_release = g_tc_relay_release;
+    P.wait_limit = g_tc_wait[0]; P.wait_limit_last = g_tc_wait[1];
     if (T) { P.t_trellis = T->trellis; P.t_svh = T->svh; P.t_c = T->c; P.t_stride = T->stride; P.t_src = T->src; }
     if (int rc = tc_status_ptr(dev, &P.status)) return rc;
     S.pdl = g_pdl;
@@ -250,6 +252,7 @@ int launch_gemm_tc_grouped(const void* xt, void* c, long Mcap, int k, int n, int
     P.t_trellis = t_trellis; P.t_svh = t_svh;
     P.g_ntiles = G.ntiles; P.g_tile_e = G.tile_e; P.g_tile_row0 = G.tile_row0; P.g_tile_rows = G.tile_rows;
     P.g_experts = G.experts;
+    P.wait_limit = P.wait_limit_last = g_tc_wait[0];
     P.g_bits[0] = G.bits[0]; P.g_bits[1] = G.bits[1];
     if (int rc = tc_status_ptr(dev, &P.status)) return rc;
     tg_fn fn = tg_kernel(K, cb, TG_GROUPED);
@@ -306,5 +309,14 @@ AMP_API int amp_exl3_set_gemm_plan(int split, int tile)
 {
     g_tc_split = split < 0 || split > 8 ? 0 : split;
     g_tc_tile = tile < 0 || tile > 512 ? 0 : (tile + 15) & ~15;
+    return 0;
+}
+
+// Polls of a barrier wait before it is declared lost, and of the waits of the last CTA of a cluster or pair (a few
+// microseconds each; 0: the default, TC_SPIN_LIMIT). For tests of what a wait that runs out leaves behind.
+AMP_API int amp_exl3_set_gemm_wait_limit(int polls, int last)
+{
+    g_tc_wait[0] = polls > 0 ? (unsigned) polls : TC_SPIN_LIMIT;
+    g_tc_wait[1] = last > 0 ? (unsigned) last : TC_SPIN_LIMIT;
     return 0;
 }

@@ -28,7 +28,12 @@
 // Epilogue: the accumulator's rows are output columns, its columns tokens. Every CTA lays its partial sums out
 // token by token in its own shared memory and sends every CTA of the cluster the run of tokens that one
 // finishes; there four lanes per token add the partials in ascending k order (bitwise reproducible), run the 128-point
-// Hadamard, scale and store. Every mbarrier wait is bounded as in the other kernels.
+// Hadamard, scale and store.
+//
+// Every mbarrier wait is bounded. A role whose wait ran out hands nothing over any more (no copy, no tile, no MMA, no
+// arrival), so that every role that depends on it runs out as well, in the other CTA of
+// a pair too; the CTAs of a split tell each other before the partial sums are added. What was not computed from complete
+// operands is therefore not stored, the status word is set, and no CTA leaves before its own copies and MMAs are done.
 #pragma once
 #include "exl3_gemv_kernel.cuh"
 #include "exl3_gemv_host.h"
@@ -39,7 +44,7 @@ namespace amp {
 constexpr int TC_BM = 128;            // output columns per CTA (UMMA M)
 constexpr int TC_BN = 128;            // ... as the bundle and grouping code counts them
 constexpr int TC_BK = 64;             // k per step (one 128-byte swizzle row)
-constexpr unsigned TC_SPIN_LIMIT = 1u << 22;   // try_wait polls before a wait is declared lost
+constexpr unsigned TC_SPIN_LIMIT = 1u << 22;   // try_wait polls before a wait is declared lost (about 4 us each)
 
 struct TcParams
 {
@@ -49,6 +54,7 @@ struct TcParams
     void* c;                    // (M, n) fp16 or fp32
     int M, k, n, c_fp32;        // n: row width of the trellis / output (bundle: columns per slice)
     int* status;
+    unsigned wait_limit, wait_limit_last;   // polls of a barrier wait; of the last CTA of a cluster or pair (amp_exl3_set_gemm_wait_limit)
     int relay_release;          // pair form: the relay's remote arrival releases at cluster scope (slower; default relaxed)
     // bundle (tables == 1): several matrices or equal-width column slices in one grid, identified
     // by device pointer tables with one entry per slice, exactly as the decode kernel's table mode
@@ -227,7 +233,8 @@ __device__ __forceinline__ uint32_t tg_weights2(uint32_t sa, uint32_t sb)
 }
 
 // Whole-warp wait for an mbarrier phase, bounded, as straight-line code: the usual case (already there) is
-// one instruction and a branch not taken. Returns false when `limit` polls were not enough.
+// one instruction and a branch not taken. Returns false when a first look and `limit` more were not enough (a look at a
+// phase that is not there yet lasts about 4 us).
 // CLUSTER: acquires at cluster scope (the arrival comes from the other CTA of a pair).
 #define AMP_TG_WAIT(sem) \
     asm volatile( \
@@ -236,11 +243,11 @@ __device__ __forceinline__ uint32_t tg_weights2(uint32_t sa, uint32_t sb)
         "@p bra $TG_DONE_%=;\n\t" \
         "mov.u32 n, %3;\n" \
         "$TG_POLL_%=:\n\t" \
-        "mbarrier.try_wait.parity" sem ".shared::cta.b64 p, [%1], %2;\n\t" \
-        "@p bra $TG_DONE_%=;\n\t" \
+        "setp.eq.u32 q, n, 0;\n\t" \
+        "@q bra $TG_DONE_%=;\n\t" \
         "sub.u32 n, n, 1;\n\t" \
-        "setp.ne.u32 q, n, 0;\n\t" \
-        "@q bra $TG_POLL_%=;\n" \
+        "mbarrier.try_wait.parity" sem ".shared::cta.b64 p, [%1], %2;\n\t" \
+        "@!p bra $TG_POLL_%=;\n" \
         "$TG_DONE_%=:\n\t" \
         "selp.u32 %0, 1, 0, p;\n\t}" \
         : "=r"(r) : "r"(bar), "r"(parity), "r"(limit) : "memory")
@@ -302,6 +309,11 @@ __device__ __forceinline__ void tg_arrive_cluster(uint32_t cluster_bar, int rele
 {
     if (release) asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" :: "r"(cluster_bar) : "memory");
     else asm volatile("mbarrier.arrive.relaxed.cluster.shared::cluster.b64 _, [%0];" :: "r"(cluster_bar) : "memory");
+}
+
+__device__ __forceinline__ void tg_st_cluster_u32(uint32_t addr, uint32_t v)
+{
+    asm volatile("st.shared::cluster.u32 [%0], %1;" :: "r"(addr), "r"(v) : "memory");
 }
 
 __device__ __forceinline__ uint32_t tg_cluster_rank()
@@ -386,7 +398,6 @@ void exl3_gemm_tc_kernel(const TgParams S)
         s_bad = 0;
     }
     __syncwarp();
-    if (split > 1) cluster_arrive_started();
     if (warp == NDEC)
     {
         if constexpr (PAIR)
@@ -421,15 +432,18 @@ void exl3_gemm_tc_kernel(const TgParams S)
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
     if (PAIR) cluster_sync_all();                            // both CTAs' barriers exist before anyone arrives remotely
+    // (the issue warp has time: its arrival publishes s_bad = 0. From the decode warps a releasing arrival costs 0.5 us)
+    else if (split > 1) { if (warp == NDEC + 1) cluster_arrive_started<true>(); else cluster_arrive_started(); }
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     const uint32_t tmem = s_tmem;
 
-    // After a wait that ran out, later waits give up at once: the roles run on over stale data to their end
-    // (nothing is stored) and every barrier below is still reached.
-    unsigned limit = TC_SPIN_LIMIT;
+    // 0: a wait of this role ran out. It walks on to its end, looks at later barriers once each and hands nothing over any
+    // more; every barrier below is still reached.
+    auto full_limit = [&]() { return !GROUPED && (PAIR ? prank == 1 : crank == split - 1) ? P.wait_limit_last : P.wait_limit; };
+    unsigned limit = full_limit();
     auto wait_bar = [&](uint32_t bar, uint32_t parity)
     {
-        if (!tg_wait(bar, parity, limit)) { limit = 1; s_bad = 1; }
+        if (!tg_wait(bar, parity, limit)) { limit = 0; s_bad = 1; }
     };
     const uint32_t w_base = smem_u32(smem), b_x = smem_u32(x_full), b_w = smem_u32(w_full), b_done = smem_u32(done), b_peer = smem_u32(peer);
     (void) b_peer;
@@ -449,20 +463,31 @@ void exl3_gemm_tc_kernel(const TgParams S)
         const unsigned char* xs = W.xt + (((size_t) ks0 * P.M + m0 + prank * h0) << 7);
         const size_t to1 = ((size_t) (S.n0 + prank * h1 - prank * h0)) << 7;
         const int off1 = (PAIR ? S.n0 / 2 : S.n0) * (TC_BK * 2);
+        uint32_t phs = 0;
+        int issued = 0;
         for (int i = 0; i < nsteps; ++i)
         {
             wait_bar(b_done + sd * 8, phd);
-            if (tg_elect())
+            if (tg_elect() && limit)
             {
                 mbar_expect_tx(&x_full[s], (uint32_t) (e0 + e1) * 128);
                 if (e0 > 0) bulk_g2s(x_base + s * x_bytes, xs, (uint32_t) e0 * 128, &x_full[s]);
                 if (NG > 1 && e1 > 0) bulk_g2s(x_base + s * x_bytes + off1, xs + to1, (uint32_t) e1 * 128, &x_full[s]);
             }
+            if (limit == 0) continue;
+            ++issued;
             xs += (size_t) P.M << 7;
-            if (++s == XS) s = 0;
+            if (++s == XS) { s = 0; phs ^= 1; }
             if (++sd == DS) { sd = 0; phd ^= 1; }
         }
         __syncwarp();
+        // the last copies have landed before this warp leaves, whoever gave up waiting for them
+        for (int j = min(issued, XS); j > 0; --j)
+        {
+            if (s == 0) { s = XS; phs ^= 1; }
+            --s;
+            tg_wait(b_x + s * 8, phs, full_limit());
+        }
     }
     else if (warp == NDEC + 1)
     {
@@ -483,18 +508,19 @@ void exl3_gemm_tc_kernel(const TgParams S)
                 if (prank != 0)
                 {
                     // relay: tell the first CTA that this CTA's halves of the step are ready
-                    if (tg_elect()) tg_arrive_cluster(cluster_map(b_peer + sd * 8, 0), P.relay_release);
+                    if (tg_elect() && limit) tg_arrive_cluster(cluster_map(b_peer + sd * 8, 0), P.relay_release);
                     __syncwarp();
+                    if (limit == 0) continue;
                     if (++s == WS) { s = 0; ph ^= 1; }
                     if (++sx == XS) { sx = 0; phx ^= 1; }
-                    if (++sd == DS) sd = 0;
+                    if (++sd == DS) { sd = 0; phd ^= 1; }
                     continue;
                 }
-                if (!tg_wait<true>(b_peer + sd * 8, phd, limit)) { limit = 1; s_bad = 1; }
+                if (!tg_wait<true>(b_peer + sd * 8, phd, limit)) { limit = 0; s_bad = 1; }
             }
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
             const uint64_t dx = dx0 + (uint64_t) ((sx * x_bytes) >> 4), dwt = dw0 + (uint64_t) ((s * TG_W_BYTES) >> 4);
-            if (tg_elect())
+            if (tg_elect() && limit)
             {
                 #pragma unroll
                 for (int kk = 0; kk < TC_BK / 16; ++kk) tg_umma<PAIR>(tmem, dwt + 2 * kk, dx + 2 * kk, idesc, (i > 0 || kk > 0) ? 1u : 0u);
@@ -506,10 +532,14 @@ void exl3_gemm_tc_kernel(const TgParams S)
                 else umma_commit(&done[sd]);
             }
             __syncwarp();
+            if (limit == 0) continue;
             if (++sd == DS) { sd = 0; phd ^= 1; }
             if (++s == WS) { s = 0; ph ^= 1; }
             if (++sx == XS) { sx = 0; phx ^= 1; }
         }
+        // the MMAs of the steps that this CTA issued (second CTA of a pair: handed over) are done before it leaves (no step
+        // at all: the parity passes on the barrier nobody has arrived on)
+        tg_wait(b_done + (sd == 0 ? DS - 1 : sd - 1) * 8, sd == 0 ? phd ^ 1 : phd, full_limit());
     }
     else
     {
@@ -528,7 +558,7 @@ void exl3_gemm_tc_kernel(const TgParams S)
         {
             asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
             __syncwarp();
-            if (lane == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" :: "r"(publish) : "memory");
+            if (lane == 0 && limit) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" :: "r"(publish) : "memory");
         };
         while (--left >= 0)
         {
@@ -585,7 +615,12 @@ void exl3_gemm_tc_kernel(const TgParams S)
     if (warp < NDEC) wait_bar(b_done + ((nsteps - 1) % DS) * 8, (uint32_t) (((nsteps - 1) / DS) & 1));
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-    if (split > 1) cluster_wait_started();                   // the peers run: their shared memory is written from here on
+    if (split > 1)
+    {
+        cluster_wait_started();                              // the peers run: their shared memory is written from here on
+        // nobody adds up partial sums to which a wait that ran out has contributed (read behind the barrier of the exchange)
+        if (s_bad && t < split) tg_st_cluster_u32(cluster_map(smem_u32(const_cast<int*>(&s_bad)), (uint32_t) t), 1);
+    }
     // ... and they write into this CTA's receive buffer: where it overlaps the stages, everybody's MMAs must have read theirs
     if (split > 1 && S.recv_off == 0) cluster_sync_all();
     const int row = tg_row(split), n0 = S.n0;

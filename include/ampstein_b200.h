@@ -125,6 +125,12 @@ int amp_exl3_set_gemm_pair(int mode);
  */
 int amp_exl3_set_gemm_plan(int split, int tile);
 /*
+ * Polls (a few microseconds each) after which a barrier wait of the tensor-core GEMM is declared lost, and those of the
+ * last block of a cluster or pair; 0: the default (2^22). After a lost wait the outputs that depend on it are not stored
+ * and amp_exl3_gemm_status reports it. For tests. Returns 0. No counterpart in the reference.
+ */
+int amp_exl3_set_gemm_wait_limit(int polls, int last);
+/*
  * Int8-activation form of the one-row GEMV for mul1 (codebook 2) tensors up to max_k bits: the
  * rotated input is quantised to int8 with one scale per 128 rows of k and the dot product runs as
  * dp4a on the byte sum of the codebook's product, exact in int32 (about 6e-3 relative rms against

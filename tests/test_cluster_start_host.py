@@ -9,7 +9,7 @@ import pytest
 from conftest import ROOT
 
 CSRC = os.path.join(ROOT, "ampstein_b200", "csrc")
-ACCESS = re.compile(r"\bcluster_st_f32\(|\bmp_ld_cluster\(|\bcluster_st_u32\(")
+ACCESS = re.compile(r"\bcluster_st_f32\(|\bmp_ld_cluster\(|\btg_st_cluster_u32\(")
 
 
 def _kernels(name):
@@ -30,7 +30,7 @@ def test_peers_are_known_to_run_before_their_memory_is_accessed(name):
         if not access:
             continue
         before = body[:access.start()]
-        arrive, wait = before.find("cluster_arrive_started("), before.find("cluster_wait_started(")
+        arrive, wait = before.find("cluster_arrive_started"), before.find("cluster_wait_started(")
         whole = before.find("mp_cluster_sync(")              # the dispatch kernel: a whole barrier, on the only path
         assert whole >= 0 or 0 <= arrive < wait, kernel
 
