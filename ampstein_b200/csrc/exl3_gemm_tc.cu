@@ -5,7 +5,6 @@
 namespace amp {
 
 __device__ int g_tc_status;
-int g_tc_relay_release = 0;
 int g_tc_pair = 1;                            // see amp_exl3_set_gemm_pair
 unsigned g_tc_wait[2] = { TC_SPIN_LIMIT, TC_SPIN_LIMIT };       // see amp_exl3_set_gemm_wait_limit
 int g_tc_split = 0, g_tc_tile = 0;            // forced (0: by rule), see amp_exl3_set_gemm_plan
@@ -183,7 +182,6 @@ int launch_gemm_tc(const void* xh, const void* trellis, void* c, const void* svh
     P.xt = (const unsigned char*) xh; P.trellis = (const uint16_t*) trellis; P.svh = (const __half*) svh; P.c = c;
     P.M = M; P.k = k; P.n = n; P.c_fp32 = c_fp32;
     P.tables = T ? 1 : 0;
-    P.relay_release = g_tc_relay_release;
     P.wait_limit = g_tc_wait[0]; P.wait_limit_last = g_tc_wait[1];
     if (T) { P.t_trellis = T->trellis; P.t_svh = T->svh; P.t_c = T->c; P.t_stride = T->stride; P.t_src = T->src; }
     if (int rc = tc_status_ptr(dev, &P.status)) return rc;
@@ -197,7 +195,7 @@ int launch_gemm_tc(const void* xh, const void* trellis, void* c, const void* svh
     if (cudaError_t e = ensure_smem(fn, smem, dev)) return cuda_rc(e, "exl3_gemm smem attribute");
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned) (blocks * S.split), (unsigned) mblk, 1);
-    cfg.blockDim = dim3(tg_threads(2), 1, 1);
+    cfg.blockDim = dim3(tg_threads(2, form == TG_PAIR), 1, 1);
     cfg.dynamicSmemBytes = smem;
     cfg.stream = stream;
     cudaLaunchAttribute attr[2];
@@ -285,13 +283,10 @@ AMP_API int amp_exl3_gemm_status(int* out)
     return 0;
 }
 
-// The pair form's remote arrival: 0 = relaxed (default), 1 = release at cluster scope (what the PTX memory model asks
-// for on paper). Returns the previous setting.
-AMP_API int amp_exl3_set_gemm_relay_release(int enable)
+// The pair form's remote arrivals release at cluster scope, always; this used to select it. Returns 1, the setting.
+AMP_API int amp_exl3_set_gemm_relay_release(int)
 {
-    const int old = g_tc_relay_release;
-    g_tc_relay_release = enable ? 1 : 0;
-    return old;
+    return 1;
 }
 
 // Pair (cta_group::2) form: 0 = never, 1 = by plan (default), 2 / 3 = pairs of 512 / 256 tokens whenever n is a

@@ -22,7 +22,8 @@
 // 0.75 us per step whatever the batch.
 //
 // Warps 0 .. 8 NG - 1 decode, in groups of four that take alternate 64-row steps (a warp owns two 16-column tile
-// columns); one warp fetches x~ with bulk copies, one issues the MMAs. A step's stages (decoded weights, x~) are
+// columns); one warp fetches x~ with bulk copies, one issues the MMAs (second CTA of a pair: three report its operands
+// to the first CTA instead). A step's stages (decoded weights, x~) are
 // freed by one tcgen05.commit.
 //
 // Epilogue: the accumulator's rows are output columns, its columns tokens. Every CTA lays its partial sums out
@@ -55,7 +56,6 @@ struct TcParams
     int M, k, n, c_fp32;        // n: row width of the trellis / output (bundle: columns per slice)
     int* status;
     unsigned wait_limit, wait_limit_last;   // polls of a barrier wait; of the last CTA of a cluster or pair (amp_exl3_set_gemm_wait_limit)
-    int relay_release;          // pair form: the relay's remote arrival releases at cluster scope (slower; default relaxed)
     // bundle (tables == 1): several matrices or equal-width column slices in one grid, identified
     // by device pointer tables with one entry per slice, exactly as the decode kernel's table mode
     int tables;
@@ -177,7 +177,13 @@ struct TgParams
 // warps that decode a step together (each 8 / 4 = 2 of the eight 16-column tiles of the block): per step a warp
 // pays about 60 instructions of bookkeeping, so that it should not be shorter
 constexpr int TG_GROUP_WARPS = 4;
-__host__ __device__ constexpr int tg_threads(int ng) { return 32 * (8 * ng + 2); }
+// Warps of a pair's second CTA that tell the first one that a step's operands are ready. The arrival releases at cluster
+// scope, which takes about 1 us (it waits for what the SM has in flight): one relay paces the pair at 1.1 us per step,
+// three taking every third step each cost nothing (2048 rows, sustained, us, one relay / three / one whose arrival was
+// relaxed, which no rule of the memory model covers: 4096 x 14336 at 3 bits 295 / 236 / 234, 14336 x 4096 at 4 bits 284 / 247 /
+// 240, 4096 x 6144 at 5 bits 152 / 114 / 117). Two warps more fit: registers are granted to groups of four warps.
+constexpr int TG_RELAYS = 3;
+__host__ __device__ constexpr int tg_threads(int ng, bool pair = false) { return 32 * (8 * ng + 2 + (pair ? TG_RELAYS - 1 : 0)); }
 
 // K words of one lane from global memory, widest loads the alignment allows. Where that takes several loads,
 // each touches the same sectors of the warp's rows again and has to find them in L1 (with L1::no_allocate 5 bits
@@ -297,18 +303,13 @@ __device__ __forceinline__ void tg_commit_both(uint64_t* bar)
                  :: "r"(smem_u32(bar)), "h"((unsigned short) 3) : "memory");
 }
 
-// The second CTA's arrival on the first CTA's barrier, one per step. Relaxed by default: with release semantics at
-// cluster scope the instruction waits for everything the SM has in flight (over a thousand cycles) and sets the
-// pace of the pair. What the arrival publishes is already in place when it is sent: the x~ bytes were written by
-// the bulk copy whose completion this warp observed with an acquire, the weight tile by warps that each ran
-// fence.proxy.async and a releasing arrive on the barrier this warp acquired; both live in this SM's shared memory,
-// which the pair's tensor cores read in place. This leans on a property of the hardware, not on a rule of the PTX
-// memory model (on paper the chain needs a releasing arrival), and is therefore selectable
-// (amp_exl3_set_gemm_relay_release); a test requires identical bits from both forms.
-__device__ __forceinline__ void tg_arrive_cluster(uint32_t cluster_bar, int release)
+// An arrival on a barrier of the first CTA of a pair: publishes what this thread wrote or observed (releasing arrivals of
+// the decode warps, completed bulk copies) to whoever acquires the phase at cluster scope. What the pair's MMAs read in this
+// CTA's shared memory: x~ bytes whose bulk copy completed on the barrier the relay has acquired, and weight tiles whose
+// writers each ran fence.proxy.async and a releasing arrive on another one; the first CTA's issue warp acquires this phase.
+__device__ __forceinline__ void tg_arrive_cluster(uint32_t cluster_bar)
 {
-    if (release) asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" :: "r"(cluster_bar) : "memory");
-    else asm volatile("mbarrier.arrive.relaxed.cluster.shared::cluster.b64 _, [%0];" :: "r"(cluster_bar) : "memory");
+    asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" :: "r"(cluster_bar) : "memory");
 }
 
 __device__ __forceinline__ void tg_st_cluster_u32(uint32_t addr, uint32_t v)
@@ -324,7 +325,7 @@ __device__ __forceinline__ uint32_t tg_cluster_rank()
 }
 
 template <int K, int CB, int NG, bool GROUPED, bool PAIR = false>
-__global__ __launch_bounds__(tg_threads(NG), NG == 1 ? 2 : 1)
+__global__ __launch_bounds__(tg_threads(NG, PAIR), NG == 1 ? 2 : 1)
 void exl3_gemm_tc_kernel(const TgParams S)
 {
     const TcParams& P = S.t;
@@ -489,6 +490,32 @@ void exl3_gemm_tc_kernel(const TgParams S)
             tg_wait(b_x + s * 8, phs, full_limit());
         }
     }
+    else if (PAIR && prank != 0 && warp > NDEC)
+    {
+        // ---- relay (second CTA of a pair): tell the first CTA that this CTA's halves of a step are ready; see TG_RELAYS ----
+        const int r = warp - (NDEC + 1), held = min(XS, WS);
+        int s = r % WS, sx = r % XS, sd = r % DS, sq = r + DS - held, last = -1;
+        uint32_t ph = (r / WS) & 1, phx = (r / XS) & 1, phd = (r / DS) & 1, phq = 1, phl = 0;
+        if (sq >= DS) { sq -= DS; phq = 0; }
+        for (int i = r; i < nsteps; i += TG_RELAYS)
+        {
+            // The stages' barriers have passed the phases of the steps in front (other relays'): a phase that is two behind
+            // has the same parity as the one waited for. (And no further than this step's: done needs this arrival.)
+            wait_bar(b_done + sq * 8, phq);
+            wait_bar(b_x + sx * 8, phx);
+            wait_bar(b_w + s * 8, ph);
+            if (tg_elect() && limit) tg_arrive_cluster(cluster_map(b_peer + sd * 8, 0));
+            __syncwarp();
+            if (limit == 0) continue;
+            last = sd; phl = phd;
+            s += TG_RELAYS; while (s >= WS) { s -= WS; ph ^= 1; }
+            sx += TG_RELAYS; while (sx >= XS) { sx -= XS; phx ^= 1; }
+            sd += TG_RELAYS; while (sd >= DS) { sd -= DS; phd ^= 1; }
+            sq += TG_RELAYS; while (sq >= DS) { sq -= DS; phq ^= 1; }
+        }
+        // the MMAs of the steps handed over have read this CTA's shared memory before it leaves
+        if (last >= 0) tg_wait(b_done + last * 8, phl, full_limit());
+    }
     else if (warp == NDEC + 1)
     {
         // ---- MMA issue: D (128 columns x N tokens) += W^T (128 x 16) x~^T (16 x N). The whole warp walks
@@ -505,17 +532,6 @@ void exl3_gemm_tc_kernel(const TgParams S)
             wait_bar(b_w + s * 8, ph);
             if constexpr (PAIR)
             {
-                if (prank != 0)
-                {
-                    // relay: tell the first CTA that this CTA's halves of the step are ready
-                    if (tg_elect() && limit) tg_arrive_cluster(cluster_map(b_peer + sd * 8, 0), P.relay_release);
-                    __syncwarp();
-                    if (limit == 0) continue;
-                    if (++s == WS) { s = 0; ph ^= 1; }
-                    if (++sx == XS) { sx = 0; phx ^= 1; }
-                    if (++sd == DS) { sd = 0; phd ^= 1; }
-                    continue;
-                }
                 if (!tg_wait<true>(b_peer + sd * 8, phd, limit)) { limit = 0; s_bad = 1; }
             }
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
@@ -537,11 +553,11 @@ void exl3_gemm_tc_kernel(const TgParams S)
             if (++s == WS) { s = 0; ph ^= 1; }
             if (++sx == XS) { sx = 0; phx ^= 1; }
         }
-        // the MMAs of the steps that this CTA issued (second CTA of a pair: handed over) are done before it leaves (no step
-        // at all: the parity passes on the barrier nobody has arrived on)
+        // the MMAs of the steps that this CTA issued are done before it leaves (no step at all: the parity passes on the
+        // barrier nobody has arrived on)
         tg_wait(b_done + (sd == 0 ? DS - 1 : sd - 1) * 8, sd == 0 ? phd ^ 1 : phd, full_limit());
     }
-    else
+    else if (warp < NDEC)
     {
         // ---- decode ----
         const int ncol = dw * (16 * NT) + gq;
@@ -603,6 +619,8 @@ void exl3_gemm_tc_kernel(const TgParams S)
                 sts128(b + o1 + 1024, colB[4], colB[5], colB[6], colB[7]);
             }
             publish = wbar;
+            // (second CTA of a pair: at once, the way to the first CTA's MMA is a microsecond longer)
+            if (PAIR && prank != 0) { hand_over(); publish = 0; }
             wst += NGR * TG_W_BYTES; wbar += NGR * 8;
             if (wst >= w_base + WS * TG_W_BYTES) { wst -= WS * TG_W_BYTES; wbar -= WS * 8; }
             sd += NGR;

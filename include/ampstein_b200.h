@@ -145,10 +145,8 @@ int amp_exl3_set_gemm_wait_limit(int polls, int last);
  */
 int amp_exl3_set_int8_gemv(int mode, int max_k);
 /*
- * Pair form only: the one remote mbarrier arrival per k step that tells the first CTA of a pair that
- * the second CTA's operands are ready is `relaxed` by default; 1 selects `release.cluster`, the form
- * the PTX memory model asks for on paper (slower; results are identical, which a test checks).
- * Returns the previous setting. No counterpart in the reference.
+ * Without effect, kept for its callers: the remote arrivals of the pair form release at cluster scope, always. Returns 1.
+ * No counterpart in the reference.
  */
 int amp_exl3_set_gemm_relay_release(int enable);
 

@@ -731,7 +731,7 @@ def test_prefill_gemm_bench_shapes_repeatable(amp, k, n, K):
     assert gemm_status() == 0
     for y in outs[1:]:
         assert torch.equal(y, outs[0])
-    # the releasing form of the pair's remote arrival must give the same bits as the relaxed default
+    # (the arrivals between the blocks of a pair always release: the entry that used to select it changes nothing)
     prev = _lib.lib().amp_exl3_set_gemm_relay_release(1)
     try:
         for _ in range(12):
