@@ -38,3 +38,12 @@ def test_peers_are_known_to_run_before_their_memory_is_accessed(name):
 def test_the_search_finds_the_kernels():
     found = {k for f in os.listdir(CSRC) if f.endswith((".cu", ".cuh")) for k, b in _kernels(f) if ACCESS.search(b)}
     assert found >= {"exl3_gemv_kernel", "exl3_gemv_tc_kernel", "exl3_gemm_tc_kernel", "moe_dispatch_kernel"}
+
+
+def test_arrivals_on_a_peers_barrier_release_at_cluster_scope():
+    """An arrival on another block's mbarrier publishes what its block wrote: only a release at cluster scope does."""
+    remote = []
+    for name in sorted(os.listdir(CSRC)):
+        text = re.sub(r"/\*.*?\*/|//[^\n]*", "", open(os.path.join(CSRC, name)).read(), flags=re.S)
+        remote += re.findall(r"mbarrier\.arrive[\w.:]*\.shared::cluster[\w.]*", text)
+    assert remote and all(".release.cluster." in r for r in remote), remote
