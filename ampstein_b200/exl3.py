@@ -14,6 +14,7 @@ from . import _lib
 # torch and absent where it is built without CUDA: the public forms stand in.
 _raw_stream = getattr(torch._C, "_cuda_getCurrentRawStream", None) or (lambda dev: torch.cuda.current_stream(dev).cuda_stream)
 _get_device = getattr(torch._C, "_cuda_getDevice", None) or torch.cuda.current_device
+_F16 = torch.float16
 
 
 def _stream(t):
@@ -211,11 +212,10 @@ def _rotates_once(m, k, n):
 
 class GemmPlan:
     """A weight (trellis, suh, svh, codebook flags) as exl3_gemm's checks found it, for callers that apply it many times.
-    It describes the weight and holds none of its tensors: matches() compares the caller's, as they are now, with the
-    description (a tensor may have been resized, or given other storage, behind the same object), and run() then checks
-    the activations alone."""
+    It describes the weight and holds none of its tensors: every run() compares the caller's, as they are now, with the
+    description (a tensor may have been resized, or given other storage, behind the same object)."""
 
-    __slots__ = ("shape", "k", "n", "K", "cb", "mul1", "mcg", "rotate_from")
+    __slots__ = ("shape", "dtype", "k", "n", "K", "cb", "mul1", "mcg", "rotate_from")
 
     def __init__(self, trellis, suh, svh, mul1=False, mcg=False):
         _check_cuda("exl3_gemm", trellis, suh, svh)
@@ -225,34 +225,33 @@ class GemmPlan:
         if suh.numel() != self.k or svh.numel() != self.n:
             raise ValueError("exl3_gemm: incompatible shapes")
         self.cb = _cb(mul1, mcg)
-        self.shape, self.mul1, self.mcg = trellis.shape, mul1, mcg
+        self.shape, self.dtype, self.mul1, self.mcg = trellis.shape, trellis.dtype, mul1, mcg
         # fewest rows that get a rotation scratch, as in exl3_gemm; half-integer bitrates: none of this path
         self.rotate_from = next(m for m in range(1, 6) if _rotates_once(m, self.k, self.n)) if float(self.K) == int(self.K) else None
 
     def matches(self, trellis, suh, svh, mul1, mcg):
         try:
-            return (trellis.shape == self.shape and mul1 == self.mul1 and mcg == self.mcg
-                    and (trellis.dtype is torch.int16 or trellis.dtype is torch.uint16) and trellis.is_contiguous()
-                    and suh.dtype is torch.float16 and suh.numel() == self.k and suh.is_contiguous()
-                    and svh.dtype is torch.float16 and svh.numel() == self.n and svh.is_contiguous())
+            return (trellis.shape == self.shape and trellis.dtype is self.dtype and trellis.is_contiguous()
+                    and suh.numel() == self.k and suh.dtype is _F16 and suh.is_contiguous()
+                    and svh.numel() == self.n and svh.dtype is _F16 and svh.is_contiguous()
+                    and mul1 == self.mul1 and mcg == self.mcg)
         except AttributeError:
             return False                                     # not a tensor: the full check says so
 
-    def run(self, x, trellis, suh, svh):
-        """The (m, n) fp16 result for a contiguous (m, k) fp16 CUDA tensor of at least one row and tensors that match,
+    def run(self, x, trellis, suh, svh, mul1, mcg):
+        """The (m, n) fp16 result for a contiguous (m, k) fp16 CUDA tensor of at least one row and a weight that matches,
         all on the current device; None for anything else (the caller then takes exl3_gemm, which says what is wrong),
         half-integer bitrates among it."""
-        shape = x.shape
-        if x.dtype is not torch.float16 or len(shape) != 2 or not x.is_contiguous() or self.rotate_from is None:
+        shape, dev, from_ = x.shape, x.get_device(), self.rotate_from
+        if len(shape) != 2 or x.dtype is not _F16 or not x.is_contiguous() or from_ is None or dev < 0 or _get_device() != dev:
             return None
         m, k = shape
-        dev = x.get_device()
-        if (k != self.k or m < 1 or dev < 0 or dev != trellis.get_device() or dev != suh.get_device() or dev != svh.get_device()
-                or _get_device() != dev):
+        if (k != self.k or m < 1 or not self.matches(trellis, suh, svh, mul1, mcg)
+                or dev != trellis.get_device() or dev != suh.get_device() or dev != svh.get_device()):
             return None
-        y = x.new_empty((m, self.n))
-        had = x.new_empty(shape) if m >= self.rotate_from else None
-        _lib.call("amp_exl3_gemm", x.data_ptr(), trellis.data_ptr(), y.data_ptr(), suh.data_ptr(), had.data_ptr() if had is not None else None,
+        y = x.new_empty(m, self.n)                           # (0.4 us less than with a tuple)
+        had = x.new_empty(m, k) if m >= from_ else None
+        _lib.call("amp_exl3_gemm", x.data_ptr(), trellis.data_ptr(), y.data_ptr(), suh.data_ptr(), None if had is None else had.data_ptr(),
                   svh.data_ptr(), m, k, self.n, self.K, self.cb, 0, _raw_stream(dev))
         return y
 
