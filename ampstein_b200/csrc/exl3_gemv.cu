@@ -786,11 +786,12 @@ AMP_API int amp_exl3_set_pdl(int enable)
 extern "C" int amp_had_r_128(const void* in, void* out, const void* pre, const void* post,
                              long rows, int cols, int dtype, float scale, cudaStream_t stream);
 
-// C = had(A*suh) @ W_hat -> had(.)*svh for any m. Up to 16 rows run on the decode kernel (the input
+// C = had(A*suh) @ W_hat -> had(.)*svh for any m. Up to eight rows run on the decode kernel (the input
 // transform lives in the kernel's prologue; from five rows on, large weights from fewer, when A_had is given,
 // a small launch of its own rotates the input into A_had once); more rows take the
-// tensor-core path: x~ is written into A_had (same shape as A, fp16: required) by the Hadamard
-// kernel and the tcgen05 GEMM consumes it. a_bf16: A holds bf16 instead of fp16 (m > 16 only).
+// tensor-core path: x~ is written into A_had (same shape as A, fp16: required above 16 rows, below it the
+// stream's workspace serves) by the Hadamard kernel and the tcgen05 GEMM consumes it. a_bf16: A holds bf16
+// instead of fp16 (tensor-core path at any m).
 // Nine to sixteen rows: the decode kernel repeats the MMA of every weight for the second eight rows, the short-batch
 // tensor-core kernel takes the same time from 2 to 16 rows. Measured (us, tensor cores / decode kernel): 4096 x 4096
 // at 4 bits 9 rows 13.9 / 32.1, 16 rows 14.0 / 39.0; 4096 x 14336 8 rows 30.3 / 23.3, 9 rows 30.1 / 41.6; 25600 x
@@ -823,7 +824,8 @@ static int gemm_any(const void* A, int a_bf16, const void* trellis, void* C, con
     if (K > 256)
     {
         // half-integer bitrate KA + 0.5 (K = AMP_EXL3_HALF_RATE(KA)), mul1 codebook: up to 16 rows on the decode
-        // kernel (the many-rows operator reconstructs the weight once instead, see exl3_gemm_recon)
+        // kernel (the many-rows operator reconstructs the weight once instead, see exl3_gemm_recon). A_had is part of
+        // this form's contract at every row count, also where a few rows are rotated in the kernel.
         AMP_REQUIRE(K <= 256 + 3 && cb == 2, "exl3_gemm: half-integer bitrates are 1.5 / 2.5 / 3.5 with the mul1 codebook");
         AMP_REQUIRE(m <= 16 && !a_bf16, "exl3_gemm: half-integer bitrates take up to 16 fp16 rows here");
         AMP_REQUIRE(A && suh && A_had && k > 0 && k % 128 == 0, "exl3_gemm: half-integer bitrates need the A_had scratch (same shape as A)");
@@ -870,10 +872,10 @@ AMP_API int amp_exl3_gemm_bf16(const void* A, const void* trellis, void* C, cons
 // them (int64 device arrays). num entries in trellis_ptrs / svh_ptrs (and c_ptrs, n_stride_list,
 // had_src_list when given); suh_ptrs has one entry per source (num_had_src, or num when
 // had_src_list is null). Outputs go to c_ptrs[i] with row width n_stride_list[i], or stacked
-// into C as (num, m, width) when c_ptrs is null. Up to 16 rows run on the decode kernel (A_had
-// unused); more rows take the tensor-core path as ONE grid over all slices: the rotated input of
-// every source is written into A_had ((sources, m, k) fp16, required), then the bundle form of the
-// prefill GEMM runs over num * width columns.
+// into C as (num, m, width) when c_ptrs is null. Up to eight rows, and up to 16 of more than three sources, run on the
+// decode kernel; more rows take the tensor-core path as ONE grid over all slices: the rotated input of
+// every source is written into A_had ((sources, m, k) fp16, required above 16 rows), then the bundle form of the
+// GEMM runs over num * width columns.
 static int mgemm_any(const void* x, int x_bf16, const void* trellis_ptrs, void* C, const void* suh_ptrs,
                      void* A_had, const void* svh_ptrs, int num, int m, int k, int width,
                      int K, int cb, int c_fp32, const void* c_ptrs, const void* n_stride_list,

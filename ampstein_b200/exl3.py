@@ -195,8 +195,7 @@ def exl3_gemm(A, B, C, suh, svh, mul1=False, mcg=False):
         return C
     K = _kcode("exl3_gemm", K, mul1)
     # the binding allocates the input-rotation scratch per call, as the reference's does
-    # (src/torch/amp_torch.cpp:11282); the decode kernel (<= 16 rows) does not need it
-    # (it lets the input be rotated once instead of by every CTA)
+    # (src/torch/amp_torch.cpp:11282). Few rows do without where nothing is rotated into it.
     A_had = torch.empty(A.shape, dtype=torch.float16, device=A.device) if (bf16 or half_rate or _rotates_once(m, k, n)) else None
     _launch(A, "amp_exl3_gemm_bf16" if bf16 else "amp_exl3_gemm", A.data_ptr(), B.data_ptr(), C.data_ptr(),
                   suh.data_ptr(), A_had.data_ptr() if A_had is not None else None, svh.data_ptr(), m, k, n, K,
@@ -459,7 +458,9 @@ def mgemm_rms_norm_res(x, res, norm_w, eps, y, B_ptrs, C, suh_ptrs, svh_ptrs, K,
 # (twice as many where k is 16384: the decode costs that form a pass over memory, the trellis GEMM's k split
 # hides it). Measured on B200 (us, trellis GEMM / reconstruct + matmul): 4096 x 1024 at 512 rows 19 / 21, 1024
 # rows 27 / 23, 2048 rows 39 / 27; 4096 x 2048 at 512 rows 25 / 30, 1024 rows 33 / 34, 2048 rows 48 / 44;
-# 14336 x 2048 at 1024 rows 80 / 105. Above 2048 columns the trellis GEMM wins or is level.
+# 14336 x 2048 at 1024 rows 80 / 105. Above 2048 columns the trellis GEMM wins or is level. The two forms round in
+# different places (reconstruct: both Hadamards and the scales folded into fp16 weights; trellis GEMM: the rotated input
+# alone) and differ by about 1e-3 of the largest value.
 RECON_MM_MAX_N = 2048
 
 
@@ -504,8 +505,8 @@ def mgemm(x, B_ptrs, C, suh_ptrs, A_had, svh_ptrs, K, mcg, mul1, opts=None):
     CUDA pointer tables; C (num, m, n) stacked output. opts selects sliced mode:
     {size_n_list, c_ptrs, n_stride_list, had_src_list, num_had_src}; C is then only a
     (num_slices, m, width) descriptor. A_had is a (sources, m, k) fp16 scratch, sources =
-    num_had_src or num: unused up to 4 rows, optional up to 16 (when given, the input is rotated once
-    by a launch of its own), required above (one tensor-core grid over all slices). x may
+    num_had_src or num: not passed on up to 4 rows, optional up to 16 (when given, the input is rotated once
+    by a launch of its own), required above (nine rows and more: one tensor-core grid over all slices). x may
     be bfloat16 (tensor-core path at any row count; not in the reference). Returns C."""
     for name, t in (("B_ptrs", B_ptrs), ("suh_ptrs", suh_ptrs), ("svh_ptrs", svh_ptrs)):
         if not isinstance(t, torch.Tensor) or t.dtype != torch.int64 or not t.is_cuda:
@@ -550,6 +551,9 @@ def mgemm(x, B_ptrs, C, suh_ptrs, A_had, svh_ptrs, K, mcg, mul1, opts=None):
             raise ValueError("mgemm: A_had must be a contiguous float16 tensor of (sources, m, k)")
         if not x.is_contiguous():
             raise ValueError("mgemm: x must be contiguous")
+    # (two to four rows without the scratch, although the library's rule would use it for wide bundles: level. Measured, us, rotated
+    # in the CTAs / once, 2, 3, 4 rows: 5120 -> 2 x 25600 at 5 bits 68.1 / 65.5, 72.9 / 73.1, 76.0 / 72.9, at 3 bits 66.8 / 67.1,
+    # 71.5 / 74.1, 74.6 / 75.3; 4096 -> 2 x 14336 at 4 bits 29.9 / 29.8, 32.1 / 31.9, 34.3 / 33.5)
     _launch(x, "amp_exl3_mgemm_bf16" if bf16 else "amp_exl3_mgemm", x.data_ptr(), B_ptrs.data_ptr(), C.data_ptr(), suh_ptrs.data_ptr(),
                   A_had.data_ptr() if A_had is not None and (m >= 5 or bf16) else None, svh_ptrs.data_ptr(), num, m, k, width,
                   int(K), _cb(mul1, mcg), 1 if C.dtype == torch.float32 else 0,

@@ -90,12 +90,14 @@ int amp_had_r_128(const void* in, void* out, const void* pre, const void* post,
 
 /*
  * EXL3 linear, any m: C (m, n) fp16 (c_fp32 = 0) or fp32 (c_fp32 = 1) = A (m, k) fp16 through
- * the quantized weight. suh and svh are required. k and n multiples of 128. Up to 16 rows run on
- * the decode kernel; more rows on the tensor-core (tcgen05) prefill kernel, which needs A_had:
- * the reference's scratch argument, m * k halves, 16-byte aligned (it receives the rotated input
- * in an internal order; its contents mean nothing to the caller). With 5..16 rows A_had is optional:
- * when given, the input is rotated into it once by a small launch of its own instead of by every
- * CTA of the decode kernel (about 10 % faster at eight rows); NULL keeps the single launch.
+ * the quantized weight. suh and svh are required. k and n multiples of 128. Up to 8 rows run on
+ * the decode kernel, more rows on the tensor-core (tcgen05) GEMM (half-integer rates: the decode kernel up to
+ * 16 rows). A_had is the reference's scratch argument, m * k halves (it receives the rotated input in an
+ * internal order; its contents mean nothing to the caller). Required above 16 rows (16-byte aligned) and,
+ * whatever the row count, with half-integer rates; optional otherwise: up to 8 rows, when given, the
+ * input is rotated into it once by a small launch of its own instead of by every CTA of the decode
+ * kernel, from five rows on or fewer where the weight is large (about 10 % faster at eight rows; NULL keeps the
+ * single launch); from 9 to 16 rows the stream's workspace stands in for it. The result does not depend on it.
  * Replaces: exl3_gemm, Q/exl3_gemm.cu:114-349 (binding torch.exl3_gemm,
  * src/torch/amp_torch.cpp:11250-11293), including its GEMV dispatch Q/exl3_gemv.cu:92-184, and,
  * above 144 rows, the reconstruct + cuBLAS path of torch.exl3_gemm_recon
@@ -275,17 +277,17 @@ int amp_exl3_mgemm_rms_norm_res(const void* x, const void* res, const void* norm
 
 /*
  * Several EXL3 matrices -- or equal-width column slices of matrices -- against ONE shared input
- * x (m, k) in a single launch, m <= 16. Matrices are named by DEVICE pointer tables (int64
+ * x (m, k) in a single grid. Matrices are named by DEVICE pointer tables (int64
  * device arrays), exactly as the reference takes them, so no host synchronisation is needed:
  *   trellis_ptrs[num], svh_ptrs[num]  per slice (already offset to the slice's first column)
  *   suh_ptrs[num_had_src]             per source matrix; had_src_list[num] (int32) maps a slice
  *                                     to its source, NULL = identity
  *   c_ptrs[num] + n_stride_list[num]  per-slice output pointer and row width of the matrix it
  *                                     belongs to; both NULL = outputs stacked in C (num, m, width)
- * All slices share k, K, the codebook and the width (a multiple of 128). Up to 16 rows run on the
+ * All slices share k, K, the codebook and the width (a multiple of 128). Up to 8 rows run on the
  * decode kernel (A_had, when given, receives the rotated input of every source from five rows up, or fewer where the weight is large,
- * as for amp_exl3_gemm); more rows run as ONE tensor-core grid over all slices and A_had
- * ((sources, m, k) fp16, sources = num_had_src or num) is required.
+ * as for amp_exl3_gemm), and so do 9 to 16 rows of more than three sources; more rows run as ONE tensor-core grid
+ * over all slices, with A_had ((sources, m, k) fp16, sources = num_had_src or num) required above 16 rows.
  * Replaces: exl3_mgemm, Q/exl3_gemm.cu:351-735 (binding torch.mgemm,
  * src/torch/amp_torch.cpp:10193-10322; bundle builders src/ucode/ampstein/models.uc:338-432).
  * size_n_list of the reference's signature has no counterpart here: every slice is `width` columns
