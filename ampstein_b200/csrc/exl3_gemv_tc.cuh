@@ -449,6 +449,8 @@ void exl3_gemv_tc_kernel(const GemvParams P)
                     prefetched = true;
                 }
 
+                // every decode warp reads the sums of all rows, which the warps of the tasks have just written
+                if constexpr (CB == 2) wait_bar(x_s + 8 * buf, (uint32_t) (((ev - 1) >> 1) & 1));
                 const int c0 = max(cg0, g0);
                 for (int g = c0; g < cg1; ++g)
                 {

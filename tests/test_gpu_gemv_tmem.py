@@ -79,3 +79,19 @@ def test_bundles(amp_tmem, oracle):
     torch.cuda.synchronize()
     for o, (t, su, sv) in zip(outs, (q_np, k_np, v_np)):
         check_close(o[0].cpu().numpy(), oracle.linear(x, t, su, sv, 0, fp32_out=True))
+
+
+@pytest.mark.parametrize("m,k,K", [(3, 512, 7), (1, 256, 4), (8, 1280, 5)])
+def test_mul1_row_sums_are_complete_when_read(amp_tmem, oracle, m, k, K):
+    """The mul1 codebook adds a multiple of the rotated rows' sums, which each decode warp reads as the others have just
+    written them: every one of many launches gives the same bits."""
+    from ampstein_b200 import _lib
+    trellis, suh, svh, x = make_linear(k, 256, K, seed=5100 + m, m=m)
+    t, s, v, xx = dev(trellis), dev(suh), dev(svh), dev(x)
+    outs = torch.full((300, m, 256), float("nan"), dtype=torch.float32, device="cuda")
+    for y in outs:
+        _lib.call("amp_exl3_gemv", xx.data_ptr(), t.data_ptr(), y.data_ptr(), s.data_ptr(), v.data_ptr(), m, k, 256, K, 2, 1,
+                  torch.cuda.current_stream().cuda_stream)
+    torch.cuda.synchronize()
+    check_close(outs[0].cpu().numpy(), oracle.linear(x, trellis, suh, svh, 2, fp32_out=True))
+    assert torch.equal(outs, outs[:1].expand_as(outs))
