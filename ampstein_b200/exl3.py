@@ -196,23 +196,26 @@ def exl3_gemm(A, B, C, suh, svh, mul1=False, mcg=False):
     K = _kcode("exl3_gemm", K, mul1)
     # the binding allocates the input-rotation scratch per call, as the reference's does
     # (src/torch/amp_torch.cpp:11282). Few rows do without where nothing is rotated into it.
-    A_had = torch.empty(A.shape, dtype=torch.float16, device=A.device) if (bf16 or half_rate or _rotates_once(m, k, n)) else None
+    A_had = torch.empty(A.shape, dtype=torch.float16, device=A.device) if (bf16 or half_rate or m >= _rotate_from(k, n)) else None
     _launch(A, "amp_exl3_gemm_bf16" if bf16 else "amp_exl3_gemm", A.data_ptr(), B.data_ptr(), C.data_ptr(),
                   suh.data_ptr(), A_had.data_ptr() if A_had is not None else None, svh.data_ptr(), m, k, n, K,
                   _cb(mul1, mcg), 1 if C.dtype == torch.float32 else 0)
     return C
 
 
-def _rotates_once(m, k, n):
-    """Whether the decode kernel may use a scratch for the rotated input: from five rows on, and with fewer where the
-    weight is large (the library decides by the device's size; this is its rule for 148 SMs, rounded down)."""
-    return m >= 5 or (m - 1) * k * n >= 200000000 or k * n >= 330000000
+def _rotate_from(k, n):
+    """Fewest rows from which the decode kernel may use a scratch for the rotated input: five, and fewer where the
+    weight is large (the library decides by the device's size; this is its rule for 148 SMs, rounded down: one row
+    from 330 M weights on, else (m - 1) times the weights from 200 M)."""
+    kn = k * n
+    return 1 if kn >= 330000000 else (min(5, 1 - -200000000 // kn) if kn else 5)
 
 
 class GemmPlan:
     """A weight (trellis, suh, svh, codebook flags) as exl3_gemm's checks found it, for callers that apply it many times.
-    It describes the weight and holds none of its tensors: every run() compares the caller's, as they are now, with the
-    description (a tensor may have been resized, or given other storage, behind the same object)."""
+    It describes the weight and holds none of its tensors: matches() compares the caller's, as they are now, with the
+    description (a tensor may have been resized, or given other storage, behind the same object), and run() then checks
+    the activations alone."""
 
     __slots__ = ("shape", "dtype", "k", "n", "K", "cb", "mul1", "mcg", "rotate_from")
 
@@ -226,7 +229,7 @@ class GemmPlan:
         self.cb = _cb(mul1, mcg)
         self.shape, self.dtype, self.mul1, self.mcg = trellis.shape, trellis.dtype, mul1, mcg
         # fewest rows that get a rotation scratch, as in exl3_gemm; half-integer bitrates: none of this path
-        self.rotate_from = next(m for m in range(1, 6) if _rotates_once(m, self.k, self.n)) if float(self.K) == int(self.K) else None
+        self.rotate_from = _rotate_from(self.k, self.n) if type(self.K) is int else None
 
     def matches(self, trellis, suh, svh, mul1, mcg):
         try:
@@ -237,16 +240,15 @@ class GemmPlan:
         except AttributeError:
             return False                                     # not a tensor: the full check says so
 
-    def run(self, x, trellis, suh, svh, mul1, mcg):
-        """The (m, n) fp16 result for a contiguous (m, k) fp16 CUDA tensor of at least one row and a weight that matches,
+    def run(self, x, trellis, suh, svh):
+        """The (m, n) fp16 result for a contiguous (m, k) fp16 CUDA tensor of at least one row and tensors that match,
         all on the current device; None for anything else (the caller then takes exl3_gemm, which says what is wrong),
         half-integer bitrates among it."""
         shape, dev, from_ = x.shape, x.get_device(), self.rotate_from
         if len(shape) != 2 or x.dtype is not _F16 or not x.is_contiguous() or from_ is None or dev < 0 or _get_device() != dev:
             return None
         m, k = shape
-        if (k != self.k or m < 1 or not self.matches(trellis, suh, svh, mul1, mcg)
-                or dev != trellis.get_device() or dev != suh.get_device() or dev != svh.get_device()):
+        if k != self.k or m < 1 or dev != trellis.get_device() or dev != suh.get_device() or dev != svh.get_device():
             return None
         y = x.new_empty(m, self.n)                           # (0.4 us less than with a tuple)
         had = x.new_empty(m, k) if m >= from_ else None

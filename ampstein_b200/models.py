@@ -36,10 +36,9 @@ class LinearEXL3:
         if out is None and m <= RECON_ROWS:
             # the per-token call: the weight is checked in full when it is not what it was
             plan = self._plan
-            out = plan.run(x, self.trellis, self.suh, self.svh, self.mul1, self.mcg) if plan is not None else None
-            if out is None and (plan is None or not plan.matches(self.trellis, self.suh, self.svh, self.mul1, self.mcg)):
+            if plan is None or not plan.matches(self.trellis, self.suh, self.svh, self.mul1, self.mcg):
                 plan = self._plan = exl3.GemmPlan(self.trellis, self.suh, self.svh, self.mul1, self.mcg)
-                out = plan.run(x, self.trellis, self.suh, self.svh, self.mul1, self.mcg)
+            out = plan.run(x, self.trellis, self.suh, self.svh)
             if out is not None:
                 return out if self.bias is None else out.add(self.bias)
         if out is None and m > RECON_ROWS and self.out_features <= RECON_MAX_N:
