@@ -190,6 +190,77 @@ void had_tiled_kernel(const void* __restrict__ in, __half* __restrict__ out, con
     *reinterpret_cast<half4*>(dst) = o;
 }
 
+// The same rotation for many rows: a warp takes the same 128-value chunk of eight rows, four lanes each (quad_had128: the same
+// bits), so that a 64-k step of its rows is written as 1 KB in one place, and with several sources (a bundle's scale
+// vectors) the input is read once. Bound by HBM where input and output exceed the L2, by instruction issue otherwise
+// (about 9 instructions per 32 values against 25 of the one-warp form). Rows beyond M compute on row M - 1 and store nothing.
+// Measured, us, one-warp form / this: 333 x 4096 3.5 / 3.1, 333 x 14336 9.2 / 7.3, 2048 x 4096 14.5 / 10.5, with three sources 38.2 /
+// 17.7, 2048 x 14336 45.0 / 28.1 (4.2 TB/s).
+template <bool BF16>
+__global__ __launch_bounds__(256, 3)
+void had_tiled_rows_kernel(const void* __restrict__ in, __half* __restrict__ out, const __half* __restrict__ pre,
+                           const long long* __restrict__ pre_table, int sources, long groups, int chunks_per_row, long M)
+{
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    const int lane = threadIdx.x & 31, pc = lane & 3;
+    const long task = (long) blockIdx.x * 8 + (threadIdx.x >> 5);
+    if (task >= groups * chunks_per_row) return;
+    const long group = task / chunks_per_row, row = group * 8 + (lane >> 2);
+    const int cb = (int) (task - group * chunks_per_row);
+    const bool live = row < M;
+    const uint4* src = reinterpret_cast<const uint4*>(reinterpret_cast<const unsigned char*>(in) +
+                                                      ((((live ? row : M - 1) * chunks_per_row + cb) << 8) + (pc << 4)));
+    uint4 raw[4];                                            // elements 8 (pc + 4 j) .. of the chunk
+    #pragma unroll
+    for (int j = 0; j < 4; ++j) raw[j] = src[4 * j];
+    #pragma unroll 1
+    for (int i = blockIdx.y; i < sources; i += gridDim.y)
+    {
+        // (8-byte loads: a scale vector of a bundle's table is only known to be 8-byte aligned)
+        const uint2* sv = reinterpret_cast<const uint2*>((pre_table ? reinterpret_cast<const __half*>(pre_table[i]) : pre) + cb * 128 + 8 * pc);
+        f32x2 h[16];
+        #pragma unroll
+        for (int j = 0; j < 4; ++j)
+        {
+            const uint2 s01 = sv[8 * j], s23 = sv[8 * j + 1];
+            const uint32_t sc[4] = { s01.x, s01.y, s23.x, s23.y }, x[4] = { raw[j].x, raw[j].y, raw[j].z, raw[j].w };
+            #pragma unroll
+            for (int q = 0; q < 4; ++q)
+            {
+                const __half2 s = *reinterpret_cast<const __half2*>(&sc[q]);
+                if constexpr (BF16)
+                {
+                    const __nv_bfloat162 v = *reinterpret_cast<const __nv_bfloat162*>(&x[q]);
+                    h[4 * j + q] = pack_f32x2(__low2float(v) * __low2float(s), __high2float(v) * __high2float(s));
+                }
+                else
+                {
+                    const float2 v = __half22float2(__hmul2(*reinterpret_cast<const __half2*>(&x[q]), s));
+                    h[4 * j + q] = pack_f32x2(v.x, v.y);
+                }
+            }
+        }
+        quad_had128(h, pc);
+        if (!live) continue;
+        unsigned char* dst = reinterpret_cast<unsigned char*>(out) + (((size_t) i * chunks_per_row + cb) * 2 * M + row) * 128;
+        #pragma unroll
+        for (int j = 0; j < 4; ++j)                          // piece pc + 4 j of the chunk: k step 2 cb + j / 2
+        {
+            uint4 o;
+            __half2* o2 = reinterpret_cast<__half2*>(&o);
+            #pragma unroll
+            for (int q = 0; q < 4; ++q) o2[q] = __float22half2_rn(unpack_f32x2(mul_f32x2(h[4 * j + q], pack_f32x2(kRScale, kRScale))));
+            *reinterpret_cast<uint4*>(dst + (size_t) (j >> 1) * M * 128 + (((pc + 4 * (j & 1)) ^ (int) (row & 7)) << 4)) = o;
+        }
+    }
+}
+
+// 128-value chunks from which the eight-row form is the faster one: below, its longer chain per warp shows (us, one-warp
+// form / eight-row form: 128 x 4096 2.2 / 2.5, 200 x 4096 2.7 / 2.5, 77 x 4096 with three sources 2.9 / 2.6), above it has a
+// third of the instructions. Tasks (eight rows x 128 values) from which one block walks all sources of a bundle instead of
+// one each (three sources, one each / walking: 333 x 4096 5.8 / 6.3, 700 x 4096 9.2 / 9.2, 2048 x 4096 21.1 / 17.7).
+constexpr long HAD_ROWS_MIN = 6400, HAD_WALK_MIN = 2560;
+
 // (M, k) fp16 or bf16 -> tiled x~ (M * k halves). Internal to the prefill path.
 int launch_had_tiled(const void* in, void* out, const void* pre, long M, int k, int bf16, cudaStream_t stream,
                      const long long* pre_table, int sources)
@@ -200,6 +271,17 @@ int launch_had_tiled(const void* in, void* out, const void* pre, long M, int k, 
     const long chunks = M * (k / 128);
     const long blocks = (chunks + 7) / 8;
     AMP_REQUIRE(blocks <= 0x7fffffffL, "exl3_gemm: too many rows");
+    if (!pre_table) sources = 1;
+    // (16-byte loads of the input; one that is only 8-byte aligned stays on the one-warp form)
+    const long groups = (M + 7) / 8, tasks = groups * (k / 128);
+    if (((uintptr_t) in & 15) == 0 && chunks * sources >= HAD_ROWS_MIN)
+    {
+        // one block walks all sources where that alone fills the device
+        const dim3 grid((unsigned) ((tasks + 7) / 8), tasks >= HAD_WALK_MIN ? 1u : (unsigned) sources);
+        if (bf16) had_tiled_rows_kernel<true><<<grid, 256, 0, stream>>>(in, (__half*) out, (const __half*) pre, pre_table, sources, groups, k / 128, M);
+        else had_tiled_rows_kernel<false><<<grid, 256, 0, stream>>>(in, (__half*) out, (const __half*) pre, pre_table, sources, groups, k / 128, M);
+        return cuda_rc(cudaGetLastError(), "exl3_gemm input rotation");
+    }
     const dim3 grid((unsigned) blocks, pre_table ? (unsigned) sources : 1u);
     if (bf16) had_tiled_kernel<true><<<grid, 256, 0, stream>>>(in, (__half*) out, (const __half*) pre, pre_table, chunks, k / 128, M, kRScale);
     else had_tiled_kernel<false><<<grid, 256, 0, stream>>>(in, (__half*) out, (const __half*) pre, pre_table, chunks, k / 128, M, kRScale);

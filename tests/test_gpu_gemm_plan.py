@@ -37,3 +37,30 @@ def test_forced_plans(amp, oracle, m, k, n, K, cb, split, tile):
         assert np.array_equal(got, again)                # fixed order of the partial sums
     finally:
         _lib.lib().amp_exl3_set_gemm_plan(0, 0)
+
+
+# Either form of the rotation kernel in front of the GEMM (one warp per chunk; eight rows per warp from 6400 chunks on, walking all
+# sources from 2560 tasks on), read back from the caller's scratch: bit-exact against the stand-alone Hadamard. Row counts around
+# multiples of eight; an input that is only 8-byte aligned.
+@pytest.mark.parametrize("m,k,sources,bf16,offset", [
+    (17, 4096, 1, False, 0), (199, 4096, 1, False, 0), (201, 4096, 1, True, 0), (207, 4096, 1, False, 4), (81, 4096, 3, False, 0),
+    (70, 4096, 3, True, 0), (641, 4096, 3, False, 0), (639, 4096, 2, True, 0), (1025, 1024, 1, True, 4), (6401, 128, 1, False, 0)])
+def test_rotation_forms(amp, m, k, sources, bf16, offset):
+    dt = torch.bfloat16 if bf16 else torch.float16
+    x = torch.randn(m * k + offset, device="cuda").to(dt)[offset:].view(1, m, k)
+    n, K = 128, 4
+    tr = torch.randint(-32768, 32768, (sources, k // 16, n // 16, 16 * K), dtype=torch.int16, device="cuda")
+    suh = torch.randn(sources, k, device="cuda").to(torch.float16)
+    svh = torch.ones(sources, n, dtype=torch.float16, device="cuda")
+    had = torch.empty(sources, m, k, dtype=torch.float16, device="cuda")
+    out = torch.empty(sources, m, n, dtype=torch.float16, device="cuda")
+    tables = [amp.ptr_array([t[i].data_ptr() for i in range(sources)]) for t in (tr, suh, svh)]
+    amp.mgemm(x, tables[0], out, tables[1], had, tables[2], K, False, False)
+    assert gemm_status() == 0
+    row, piece = torch.arange(m, device="cuda").view(1, m, 1), torch.arange(8, device="cuda")
+    for i in range(sources):
+        ref = torch.empty(m, k, dtype=torch.float16, device="cuda")
+        amp.had_r_128(x[0].float() if bf16 else x[0], ref, pre_scale=suh[i])      # (bf16 rows: scaled and rotated in fp32)
+        got = had[i].view(k // 64, m, 8, 8)                  # (k step, row, 16-byte piece, value); piece p lies at p ^ (row & 7)
+        got = got.gather(2, (piece ^ (row & 7)).view(1, m, 8, 1).expand(k // 64, m, 8, 8))
+        assert torch.equal(got.permute(1, 0, 2, 3).reshape(m, k).view(torch.int16), ref.view(torch.int16))
