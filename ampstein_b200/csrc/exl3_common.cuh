@@ -20,24 +20,44 @@ constexpr float kRScale = 0.088388347648f;   // 1/sqrt(128), spelled as the refe
 // Codebooks
 // ------------------------------------------------------------------------------------------
 
-// cb 0 / cb 1: the 32-bit word whose two fp16 halves SUM to the weight. Keeping the halves
-// apart lets a tensor-core k-pair do the final add (see exl3_gemv.cu).
-template <int CB>
-__device__ __forceinline__ uint32_t cb_halves(uint32_t s)
+// The 32-bit product behind a weight (codebooks 0 / 1: its two fp16 halves are masked next, 2 and its int8 forms: its
+// bytes are summed). DUP: the state stands in both halves of r (r = s * 65537) and the multiplier is M / 65537 mod 2^32 =
+// M - (M << 16): a byte permute that has no zero to fill the upper half with needs no mask.
+template <int CB, bool DUP = false>
+__device__ __forceinline__ uint32_t cb_product(uint32_t r)
 {
-    static_assert(CB == 0 || CB == 1, "cb_halves: cb 0 or 1");
-    uint32_t x = (CB == 0) ? s * 89226354u + 64248484u : s * 0xCBAC1FEDu;
+    constexpr uint32_t M = CB == 0 ? 89226354u : (CB == 1 ? 0xCBAC1FEDu : 0x83DCD12Du);
+    const uint32_t x = r * (DUP ? M - (M << 16) : M);
+    return CB == 0 ? x + 64248484u : x;
+}
+
+// cb 0 / cb 1: the 32-bit word whose two fp16 halves SUM to the weight, of its product. Keeping the halves
+// apart lets a tensor-core k-pair do the final add (see exl3_gemv.cu).
+__device__ __forceinline__ uint32_t cb_halves_of(uint32_t x)
+{
     uint32_t y;
     // (x & 0x8fff8fff) ^ 0x3b603b60 in one LOP3: f(a,b,c) = (a & b) ^ c  -> LUT 0x6a
     asm("lop3.b32 %0, %1, 0x8fff8fff, 0x3b603b60, 0x6a;" : "=r"(y) : "r"(x));
     return y;
 }
 
-// cb 2: fp16 bit pattern of 1024 + bytesum(s * M) (upper half of the word is zero); the weight
+template <int CB>
+__device__ __forceinline__ uint32_t cb_halves(uint32_t s)
+{
+    static_assert(CB == 0 || CB == 1, "cb_halves: cb 0 or 1");
+    return cb_halves_of(cb_product<CB>(s));
+}
+
+// cb 2: fp16 bit pattern of 1024 + bytesum(s * M) (upper half of the word is zero), of its product; the weight
 // is that value * k_inv + k_bias
+__device__ __forceinline__ uint32_t cb2_raw_of(uint32_t x)
+{
+    return __dp4a(x, 0x01010101u, 0x6400u);
+}
+
 __device__ __forceinline__ uint32_t cb2_raw(uint32_t s)
 {
-    return __dp4a(s * 0x83DCD12Du, 0x01010101u, 0x6400u);
+    return cb2_raw_of(cb_product<2>(s));
 }
 
 // Exact fp16 weight of a state, bit-identical to the reference's decode_3inst<cb>
@@ -119,13 +139,6 @@ __device__ __forceinline__ uint32_t window_end_ct(const uint32_t (&w)[NW], uint3
         const uint32_t v = __funnelshift_r(w[j1], hi, sh);
         return FMA ? mask16_fma(v) : (v & 0xffffu);
     }
-}
-
-// window of weight I of the chunk at K bits per weight
-template <int K, int I, int NW, bool FMA = true>
-__device__ __forceinline__ uint32_t window_ct(const uint32_t (&w)[NW], uint32_t prev)
-{
-    return window_end_ct<(I + 1) * K - 1, NW, FMA>(w, prev);
 }
 
 // ------------------------------------------------------------------------------------------

@@ -132,26 +132,12 @@ __device__ __forceinline__ void umma_commit(uint64_t* bar)
                  :: "r"(smem_u32(bar)) : "memory");
 }
 
-// two states -> two exact fp16 weights packed (a in the low half), bit-identical to the reference
-template <int CB>
-__device__ __forceinline__ uint32_t weights2(uint32_t sa, uint32_t sb)
-{
-    if constexpr (CB == 2)
-    {
-        const uint32_t raw = __byte_perm(cb2_raw(sa), cb2_raw(sb), 0x5410);
-        const __half2 kinv = __half2half2(__ushort_as_half((unsigned short) 0x1eee));
-        const __half2 kbias = __half2half2(__ushort_as_half((unsigned short) 0xc931));
-        const __half2 w = __hfma2(*reinterpret_cast<const __half2*>(&raw), kinv, kbias);
-        return *reinterpret_cast<const uint32_t*>(&w);
-    }
-    else
-    {
-        const uint32_t ya = cb_halves<CB>(sa), yb = cb_halves<CB>(sb);
-        const uint32_t lo = __byte_perm(ya, yb, 0x5410), hi = __byte_perm(ya, yb, 0x7632);
-        const __half2 w = __hadd2(*reinterpret_cast<const __half2*>(&lo), *reinterpret_cast<const __half2*>(&hi));
-        return *reinterpret_cast<const uint32_t*>(&w);
-    }
-}
+// Shared shifts (window_product) where they take load off the integer ALU, which also packs here: at 3 and 6 bits a shift and a
+// mask on the other pipe per window leave it less to do, except for codebook 2, whose masks are ALU work too (us, one each /
+// shared: 59 tokens x top-8 of 128 experts at 3 bits 190.9 / 197.8; 600 x 4096 x 14336 at 6 bits 81.5 / 82.4, codebook 2 at 3 bits
+// 78.8 / 75.6, at 6 bits 78.3 / 75.6)
+template <int K, int CB>
+constexpr bool tg_shared_phase = shared_phase<K> && (CB == 2 || (K != 3 && K != 6));
 
 constexpr int TG_MAX_N = 256;                 // tokens per accumulator (UMMA N)
 constexpr int TG_MAX_TOKENS = 512;            // tokens per tile: two accumulators, with 16 decode warps only
@@ -223,16 +209,23 @@ __device__ __forceinline__ void lds_f32x2(uint32_t addr, f32x2& a, f32x2& b)
     asm volatile("ld.shared.v2.b64 {%0, %1}, [%2];" : "=l"(a), "=l"(b) : "r"(addr) : "memory");
 }
 
-// Two states -> two exact fp16 weights, packed. As weights2, with the halves of each word added by one
-// instruction per weight on the half-precision pipe and one byte permute per pair (weights2: two permutes
-// and one addition): the integer ALU is the busier pipe.
+// Products of two weights (cb_product) -> two exact fp16 weights, packed (a in the low half), bit-identical to the reference.
+// Codebooks 0 / 1: the halves of each word are added by one instruction per weight on the half-precision pipe and
+// packed by one byte permute per pair (two permutes and one addition: the integer ALU is the busier pipe).
 template <int CB>
-__device__ __forceinline__ uint32_t tg_weights2(uint32_t sa, uint32_t sb)
+__device__ __forceinline__ uint32_t tg_weights2(uint32_t xa, uint32_t xb)
 {
-    if constexpr (CB == 2) return weights2<2>(sa, sb);
+    if constexpr (CB == 2)
+    {
+        const uint32_t raw = __byte_perm(cb2_raw_of(xa), cb2_raw_of(xb), 0x5410);
+        const __half2 kinv = __half2half2(__ushort_as_half((unsigned short) 0x1eee));
+        const __half2 kbias = __half2half2(__ushort_as_half((unsigned short) 0xc931));
+        const __half2 w = __hfma2(*reinterpret_cast<const __half2*>(&raw), kinv, kbias);
+        return *reinterpret_cast<const uint32_t*>(&w);
+    }
     else
     {
-        const uint32_t ya = cb_halves<CB>(sa), yb = cb_halves<CB>(sb);
+        const uint32_t ya = cb_halves_of(xa), yb = cb_halves_of(xb);
         const __half2 ha = *reinterpret_cast<const __half2*>(&ya), hb = *reinterpret_cast<const __half2*>(&yb);
         const __half2 wa = __hadd2(__low2half2(ha), __high2half2(ha)), wb = __hadd2(__low2half2(hb), __high2half2(hb));
         return __byte_perm(*reinterpret_cast<const uint32_t*>(&wa), *reinterpret_cast<const uint32_t*>(&wb), 0x5410);
@@ -600,7 +593,7 @@ void exl3_gemm_tc_kernel(const TgParams S)
                     constexpr int R = decltype(rtag)::value;
                     uint32_t st[8];
                     // (codebook 2 already has two instructions per weight on the FMA pipe: its fields are cut on the ALU)
-                    states8<K, R, CB != 2>(w[c], prev[c], st);
+                    products8<K, R, CB, CB != 2, tg_shared_phase<K, CB>>(w[c], prev[c], st);
                     colA[R] = tg_weights2<CB>(st[0], st[1]);     colA[4 + R] = tg_weights2<CB>(st[2], st[3]);
                     colB[R] = tg_weights2<CB>(st[4], st[5]);     colB[4 + R] = tg_weights2<CB>(st[6], st[7]);
                 };

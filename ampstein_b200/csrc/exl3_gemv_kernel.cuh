@@ -350,13 +350,13 @@ __device__ __forceinline__ void load_chunk_s(uint32_t addr, uint32_t (&w)[K])
     }
 }
 
-// A-operand word of one weight: codebooks 0/1 give (lo, hi) halves, codebook 2 the raw
+// A-operand word of one weight from its product: codebooks 0/1 give (lo, hi) halves, codebook 2 the raw
 // 1024+bytesum pattern with a zero upper half (affine part applied in the epilogue)
 template <int CB>
-__device__ __forceinline__ uint32_t a_word(uint32_t s)
+__device__ __forceinline__ uint32_t a_word(uint32_t x)
 {
-    if constexpr (CB == 2) return cb2_raw(s);
-    else return cb_halves<CB>(s);
+    if constexpr (CB == 2) return cb2_raw_of(x);
+    else return cb_halves_of(x);
 }
 
 // 16-bit field extraction on the FMA-heavy pipe: dp2a with a one-hot byte vector is
@@ -378,79 +378,94 @@ __device__ __forceinline__ uint32_t hi16_fma(uint32_t r)
     return d;
 }
 
-#ifndef AMP_GEMV_HI_FMA_MASK
-#define AMP_GEMV_HI_FMA_MASK 0x6      // which of a word's (up to four) pairs take their high state on the FMA pipe
-#endif
-#ifndef AMP_GEMV_LO_FMA_MASK
-#define AMP_GEMV_LO_FMA_MASK 0xf      // ... and their low state
-#endif
+// Bitrates whose windows share shifted words (below): windows that end at the same bit of a byte are at most 24 bits apart
+template <int K>
+constexpr bool shared_phase = K == 1 || K == 2 || K == 3 || K == 4 || K == 6 || K == 8;
 
-// The eight 16-bit states of virtual lane R (positions 8R..8R+7 of the lane's chunk).
-// When K divides 16, windows 16/K positions apart are exactly 16 bits apart, so one 32-bit
-// word cut from the stream holds two states (high and low half): one funnel shift serves two
-// weights. Other bitrates cut each window on its own (shift on the ALU, mask on the FMA pipe).
-template <int K, int R, bool FMA = true>
-__device__ __forceinline__ void states8(const uint32_t (&w)[gemv_words(K)], uint32_t prev, uint32_t (&s)[8])
+// Product (cb_product) of the weight whose window ends with bit LAST of the lane's chunk w[0..NW), preceded by `prev`.
+// SHARE: the stream is cut into 32-bit words shifted by 0 .. 7 bits so that the window ends with a byte; the compiler computes
+// a shifted word once for all windows in it, and a window is then one instruction: a half of the word (on the
+// FMA-heavy pipe with FMA), its middle (byte permute), or the last byte of the word in front and the first of this one
+// (byte permute, twice over: see cb_product). Shifts and fields per weight: 1.16 at 4 bits (1.38 when a funnel shift served the two
+// windows 16 bits apart), 1.56 at 6 and 1.66 at 3 bits (1.9 with a shift and a mask each), 1 at 8. At 5 and 7 bits the windows that end at the same bit
+// of a byte are more than a word apart: a shift and a mask each.
+// The decode GEMV is bound by issue (its slots and the cycles in which an mma.sync blocks them add up to all cycles): 4.80 -> 4.42
+// warp instructions per 32 weights at 4 bits. One row, us: 4096 x 229376 at 4 bits 184.8 -> 175.6 (2.67 TB/s), 4096 x 128256 at 6
+// bits 115.4 -> 110.8, 4096 x 28672 at 2 / 4 / 8 bits 27.4 / 27.4 / 29.2 -> 25.4 / 26.3 / 28.1, 3 bits (bound by the integer ALU)
+// 29.1 -> 29.0; tensor-core GEMM, 200 x 4096 x 28672 at 4 bits 71.1 -> 69.4 (3 and 6 bits: see tg_shared_phase).
+template <int CB, int LAST, int NW, bool FMA, bool SHARE>
+__device__ __forceinline__ uint32_t window_product(const uint32_t (&w)[NW], uint32_t prev)
 {
-    if constexpr (K > 8)
-    {
-        // half-integer rate: pairs of positions of 2 KA + 1 bits, the first of a pair KA bits long
-        auto cut = [&](auto tag)
-        {
-            constexpr int I = R * 8 + decltype(tag)::value, KA = K - GEMV_HALF, B2 = 2 * KA + 1;
-            return window_end_ct<(I & 1) ? (I / 2 + 1) * B2 - 1 : (I / 2) * B2 + KA - 1, gemv_words(K), FMA>(w, prev);
-        };
-        s[0] = cut(std::integral_constant<int, 0>()); s[1] = cut(std::integral_constant<int, 1>());
-        s[2] = cut(std::integral_constant<int, 2>()); s[3] = cut(std::integral_constant<int, 3>());
-        s[4] = cut(std::integral_constant<int, 4>()); s[5] = cut(std::integral_constant<int, 5>());
-        s[6] = cut(std::integral_constant<int, 6>()); s[7] = cut(std::integral_constant<int, 7>());
-    }
-    else if constexpr (K == 4 || K == 8)
-    {
-        constexpr int D = 16 / K;                       // pair distance in positions
-        int pair = 0;
-        #pragma unroll
-        for (int j = 0; j < 8; ++j)
-        {
-            if ((j / D) % 2 != 0) continue;             // j is the earlier (high-half) member of its pair
-            const int i_lo = R * 8 + j + D;             // later member: its window ends the 32-bit word
-            const int last = (i_lo + 1) * K - 1;
-            const int j1 = last / 32, sh = 31 - (last % 32);
-            uint32_t r;
-            if (sh == 0) r = w[j1];
-            else r = __funnelshift_r(w[j1], j1 == 0 ? prev : w[j1 > 0 ? j1 - 1 : 0], sh);
-            s[j] = (FMA && ((AMP_GEMV_HI_FMA_MASK >> pair) & 1)) ? hi16_fma(r) : (r >> 16);
-            s[j + D] = (FMA && ((AMP_GEMV_LO_FMA_MASK >> pair) & 1)) ? lo16_fma(r) : (r & 0xffffu);
-            ++pair;
-        }
-    }
+    constexpr int p = (7 - LAST % 8) % 8, E = LAST + p, j = E / 32, b = E % 32 / 8;
+    static_assert(j < NW, "window outside the chunk");
+    if constexpr (p != 0 && !SHARE) return cb_product<CB>(window_end_ct<LAST, NW, FMA>(w, prev));
     else
     {
-        s[0] = window_ct<K, R * 8 + 0, K, FMA>(w, prev); s[1] = window_ct<K, R * 8 + 1, K, FMA>(w, prev);
-        s[2] = window_ct<K, R * 8 + 2, K, FMA>(w, prev); s[3] = window_ct<K, R * 8 + 3, K, FMA>(w, prev);
-        s[4] = window_ct<K, R * 8 + 4, K, FMA>(w, prev); s[5] = window_ct<K, R * 8 + 5, K, FMA>(w, prev);
-        s[6] = window_ct<K, R * 8 + 6, K, FMA>(w, prev); s[7] = window_ct<K, R * 8 + 7, K, FMA>(w, prev);
+        const uint32_t before = j > 0 ? w[j > 0 ? j - 1 : 0] : prev, f = p ? __funnelshift_r(w[j], before, p) : w[j];
+        if constexpr (b == 1) return cb_product<CB>(FMA ? hi16_fma(f) : f >> 16);
+        else if constexpr (b == 3) return cb_product<CB>(FMA ? lo16_fma(f) : f & 0xffffu);
+        else if constexpr (b == 2) return cb_product<CB>(__byte_perm(f, 0u, 0x4421));
+        else
+        {
+            // (of the shifted word in front only the last byte)
+            const uint32_t g = !p ? before : (j > 0 ? __funnelshift_r(before, j > 1 ? w[j > 1 ? j - 2 : 0] : prev, p) : prev >> p);
+            return cb_product<CB, true>(__byte_perm(f, g, 0x4343));
+        }
     }
+}
+
+// The products of the eight weights of virtual lane R (positions 8R..8R+7 of the lane's chunk)
+template <int K, int R, int CB, bool FMA = true, bool SHARE = shared_phase<K>>
+__device__ __forceinline__ void products8(const uint32_t (&w)[gemv_words(K)], uint32_t prev, uint32_t (&x)[8])
+{
+    auto cut = [&](auto tag)
+    {
+        constexpr int I = R * 8 + decltype(tag)::value;
+        if constexpr (K > 8)
+        {
+            // half-integer rate: pairs of positions of 2 KA + 1 bits, the first of a pair KA bits long
+            constexpr int KA = K - GEMV_HALF, B2 = 2 * KA + 1;
+            return cb_product<CB>(window_end_ct<(I & 1) ? (I / 2 + 1) * B2 - 1 : (I / 2) * B2 + KA - 1, gemv_words(K), FMA>(w, prev));
+        }
+        else return window_product<CB, (I + 1) * K - 1, gemv_words(K), FMA, SHARE>(w, prev);
+    };
+    x[0] = cut(std::integral_constant<int, 0>()); x[1] = cut(std::integral_constant<int, 1>());
+    x[2] = cut(std::integral_constant<int, 2>()); x[3] = cut(std::integral_constant<int, 3>());
+    x[4] = cut(std::integral_constant<int, 4>()); x[5] = cut(std::integral_constant<int, 5>());
+    x[6] = cut(std::integral_constant<int, 6>()); x[7] = cut(std::integral_constant<int, 7>());
 }
 
 // Decode the lane's 8 weights of virtual lane R of one tile and issue the two MMAs (into two
 // accumulators, so that they do not wait for each other). w/prev: the lane's K words and the
 // word before them. xb: duplicated activations of the tile's 16 rows for this lane's batch
-// row(s), xb[r] = row r.
-template <int K, int CB, int MB, int R>
+// row(s), xb[r] = row r. PACK (codebook 2): see there.
+template <int K, int CB, int MB, int R, bool PACK>
 __device__ __forceinline__ void decode_mma_r(const uint32_t (&w)[gemv_words(K)], uint32_t prev, const uint32_t (&xb)[MB][16],
                                              float (&acc0)[MB][4], float (&acc1)[MB][4])
 {
-    uint32_t s[8], a[8];
+    uint32_t x[8], a[8];
     // (codebook 2 already has the multiply and the byte sum on the FMA-heavy pipe: its fields are cut on the ALU)
-    states8<K, R, CB != 2>(w, prev, s);
+    products8<K, R, CB, CB != 2>(w, prev, x);
     #pragma unroll
-    for (int j = 0; j < 8; ++j) a[j] = a_word<CB>(s[j]);
+    for (int j = 0; j < 8; ++j) a[j] = a_word<CB>(x[j]);
+    // positions j and j+4 are the same row in columns c and c+8 -> MMA rows g and g+8;
+    // positions (0,1) are tile rows (2R, 2R+1), positions (2,3) rows (2R+8, 2R+9)
+    if constexpr (PACK)
+    {
+        // one fp16 value per weight: two weights share a register and one MMA takes all eight (half a permute per weight
+        // against the eight issue cycles of every second MMA); the duplicated activations are taken apart again (eight
+        // permutes a unit)
+        #pragma unroll
+        for (int j = 0; j < 8; j += 2) a[j] = __byte_perm(a[j], a[j + 1], 0x5410);
+        #pragma unroll
+        for (int mb = 0; mb < MB; ++mb)
+            mma_16816((R & 1) ? acc1[mb] : acc0[mb], a[0], a[4], a[2], a[6], __byte_perm(xb[mb][2 * R], xb[mb][2 * R + 1], 0x5410),
+                      __byte_perm(xb[mb][2 * R + 8], xb[mb][2 * R + 9], 0x5410));
+        return;
+    }
     #pragma unroll
     for (int mb = 0; mb < MB; ++mb)
     {
-        // positions j and j+4 are the same row in columns c and c+8 -> MMA rows g and g+8;
-        // positions (0,1) are tile rows (2R, 2R+1), positions (2,3) rows (2R+8, 2R+9)
         mma_16816(acc0[mb], a[0], a[4], a[1], a[5], xb[mb][2 * R], xb[mb][2 * R + 1]);
         mma_16816(acc1[mb], a[2], a[6], a[3], a[7], xb[mb][2 * R + 8], xb[mb][2 * R + 9]);
     }
@@ -473,16 +488,16 @@ template <int K, int R>
 __device__ __forceinline__ void decode_dp4a_r(const uint32_t (&w)[gemv_words(K)], uint32_t prev, const uint32_t (&xs)[16],
                                               int (&a0)[2], int (&a1)[2])
 {
-    uint32_t s[8];
-    states8<K, R, false>(w, prev, s);
-    a0[0] = dp4a_us(s[0] * 0x83DCD12Du, xs[2 * R], a0[0]);
-    a0[1] = dp4a_us(s[2] * 0x83DCD12Du, xs[2 * R + 8], a0[1]);
-    a1[0] = dp4a_us(s[4] * 0x83DCD12Du, xs[2 * R], a1[0]);
-    a1[1] = dp4a_us(s[6] * 0x83DCD12Du, xs[2 * R + 8], a1[1]);
-    a0[0] = dp4a_us(s[1] * 0x83DCD12Du, xs[2 * R + 1], a0[0]);
-    a0[1] = dp4a_us(s[3] * 0x83DCD12Du, xs[2 * R + 9], a0[1]);
-    a1[0] = dp4a_us(s[5] * 0x83DCD12Du, xs[2 * R + 1], a1[0]);
-    a1[1] = dp4a_us(s[7] * 0x83DCD12Du, xs[2 * R + 9], a1[1]);
+    uint32_t x[8];
+    products8<K, R, 2, false>(w, prev, x);
+    a0[0] = dp4a_us(x[0], xs[2 * R], a0[0]);
+    a0[1] = dp4a_us(x[2], xs[2 * R + 8], a0[1]);
+    a1[0] = dp4a_us(x[4], xs[2 * R], a1[0]);
+    a1[1] = dp4a_us(x[6], xs[2 * R + 8], a1[1]);
+    a0[0] = dp4a_us(x[1], xs[2 * R + 1], a0[0]);
+    a0[1] = dp4a_us(x[3], xs[2 * R + 9], a0[1]);
+    a1[0] = dp4a_us(x[5], xs[2 * R + 1], a1[0]);
+    a1[1] = dp4a_us(x[7], xs[2 * R + 9], a1[1]);
 }
 
 // The same with a second set of activation codes (the int8 rounding error of the first set, quantised
@@ -491,18 +506,16 @@ template <int K, int R>
 __device__ __forceinline__ void decode_dp4a2_r(const uint32_t (&w)[gemv_words(K)], uint32_t prev, const uint32_t (&xs)[16], const uint32_t (&xr)[16],
                                                int (&a0)[2], int (&a1)[2], int (&b0)[2], int (&b1)[2])
 {
-    uint32_t s[8];
-    states8<K, R, false>(w, prev, s);
-    #pragma unroll
-    for (int i = 0; i < 8; ++i) s[i] *= 0x83DCD12Du;
-    a0[0] = dp4a_us(s[0], xs[2 * R], a0[0]);         b0[0] = dp4a_us(s[0], xr[2 * R], b0[0]);
-    a0[1] = dp4a_us(s[2], xs[2 * R + 8], a0[1]);     b0[1] = dp4a_us(s[2], xr[2 * R + 8], b0[1]);
-    a1[0] = dp4a_us(s[4], xs[2 * R], a1[0]);         b1[0] = dp4a_us(s[4], xr[2 * R], b1[0]);
-    a1[1] = dp4a_us(s[6], xs[2 * R + 8], a1[1]);     b1[1] = dp4a_us(s[6], xr[2 * R + 8], b1[1]);
-    a0[0] = dp4a_us(s[1], xs[2 * R + 1], a0[0]);     b0[0] = dp4a_us(s[1], xr[2 * R + 1], b0[0]);
-    a0[1] = dp4a_us(s[3], xs[2 * R + 9], a0[1]);     b0[1] = dp4a_us(s[3], xr[2 * R + 9], b0[1]);
-    a1[0] = dp4a_us(s[5], xs[2 * R + 1], a1[0]);     b1[0] = dp4a_us(s[5], xr[2 * R + 1], b1[0]);
-    a1[1] = dp4a_us(s[7], xs[2 * R + 9], a1[1]);     b1[1] = dp4a_us(s[7], xr[2 * R + 9], b1[1]);
+    uint32_t x[8];
+    products8<K, R, 2, false>(w, prev, x);
+    a0[0] = dp4a_us(x[0], xs[2 * R], a0[0]);         b0[0] = dp4a_us(x[0], xr[2 * R], b0[0]);
+    a0[1] = dp4a_us(x[2], xs[2 * R + 8], a0[1]);     b0[1] = dp4a_us(x[2], xr[2 * R + 8], b0[1]);
+    a1[0] = dp4a_us(x[4], xs[2 * R], a1[0]);         b1[0] = dp4a_us(x[4], xr[2 * R], b1[0]);
+    a1[1] = dp4a_us(x[6], xs[2 * R + 8], a1[1]);     b1[1] = dp4a_us(x[6], xr[2 * R + 8], b1[1]);
+    a0[0] = dp4a_us(x[1], xs[2 * R + 1], a0[0]);     b0[0] = dp4a_us(x[1], xr[2 * R + 1], b0[0]);
+    a0[1] = dp4a_us(x[3], xs[2 * R + 9], a0[1]);     b0[1] = dp4a_us(x[3], xr[2 * R + 9], b0[1]);
+    a1[0] = dp4a_us(x[5], xs[2 * R + 1], a1[0]);     b1[0] = dp4a_us(x[5], xr[2 * R + 1], b1[0]);
+    a1[1] = dp4a_us(x[7], xs[2 * R + 9], a1[1]);     b1[1] = dp4a_us(x[7], xr[2 * R + 9], b1[1]);
 }
 
 // thread-block cluster helpers: rank of this CTA, address of a shared-memory location in another
@@ -1703,13 +1716,18 @@ void exl3_gemv_kernel(const GemvParams P)
                 }
                 else
                 {
+                    // Two mul1 weights per register, us before / now: 5120 x 25600 at 8 rows, 4 bits 53.9 / 50.6, 3 bits 57.2 / 53.8;
+                    // 4096 x 28672 at 4 bits, 4 rows 35.6 / 33.9 (5 % of that from the shared shifts); 4096 x 14336 at 3.5 bits, one row 19.3 / 18.7. Not where
+                    // the fields already fill the integer pipe: 5 and 7 bits (5120 x 25600 at 5 bits, 8 rows 55.3 / 57.2), half
+                    // rates behind a rotation launch (4096 x 14336 at 2.5 bits, 8 rows 26.6 / 27.4)
+                    constexpr bool PACK = CB == 2 && (shared_phase<K> || (K > 8 && (GIN != 2 || MB == 2)));
                     #pragma unroll
                     for (int nt = 0; nt < NT; ++nt)
                     {
-                        decode_mma_r<K, CB, MB, 0>(w[nt], prev[nt], xb, acc0[nt], acc1[nt]);
-                        decode_mma_r<K, CB, MB, 1>(w[nt], prev[nt], xb, acc0[nt], acc1[nt]);
-                        decode_mma_r<K, CB, MB, 2>(w[nt], prev[nt], xb, acc0[nt], acc1[nt]);
-                        decode_mma_r<K, CB, MB, 3>(w[nt], prev[nt], xb, acc0[nt], acc1[nt]);
+                        decode_mma_r<K, CB, MB, 0, PACK>(w[nt], prev[nt], xb, acc0[nt], acc1[nt]);
+                        decode_mma_r<K, CB, MB, 1, PACK>(w[nt], prev[nt], xb, acc0[nt], acc1[nt]);
+                        decode_mma_r<K, CB, MB, 2, PACK>(w[nt], prev[nt], xb, acc0[nt], acc1[nt]);
+                        decode_mma_r<K, CB, MB, 3, PACK>(w[nt], prev[nt], xb, acc0[nt], acc1[nt]);
                     }
                 }
 

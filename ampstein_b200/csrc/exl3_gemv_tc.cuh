@@ -474,10 +474,10 @@ void exl3_gemv_tc_kernel(const GemvParams P)
                     for (int h = 0; h < 2; ++h)
                     {
                         uint32_t st8[8], a0[8], a1[8];
-                        if (h == 0) states8<K, 0>(w[0], prev[0], st8); else states8<K, 2>(w[0], prev[0], st8);
+                        if (h == 0) products8<K, 0, CB>(w[0], prev[0], st8); else products8<K, 2, CB>(w[0], prev[0], st8);
                         #pragma unroll
                         for (int j = 0; j < 8; ++j) a0[j] = a_word<CB>(st8[j]);
-                        if (h == 0) states8<K, 1>(w[0], prev[0], st8); else states8<K, 3>(w[0], prev[0], st8);
+                        if (h == 0) products8<K, 1, CB>(w[0], prev[0], st8); else products8<K, 3, CB>(w[0], prev[0], st8);
                         #pragma unroll
                         for (int j = 0; j < 8; ++j) a1[j] = a_word<CB>(st8[j]);
                         // the previous stage's stores have had half a stage of arithmetic to land
@@ -498,11 +498,11 @@ void exl3_gemv_tc_kernel(const GemvParams P)
                         const uint32_t t_st = t_lane + 32 * st;
                         tcv_st_tile(t_st, a0);
                         tcv_st_tile(t_st + 16, a1);
-                        if (h == 0) states8<K, 0>(w[1], prev[1], st8); else states8<K, 2>(w[1], prev[1], st8);
+                        if (h == 0) products8<K, 0, CB>(w[1], prev[1], st8); else products8<K, 2, CB>(w[1], prev[1], st8);
                         #pragma unroll
                         for (int j = 0; j < 8; ++j) a0[j] = a_word<CB>(st8[j]);
                         tcv_st_tile(t_st + (16u << 16), a0);
-                        if (h == 0) states8<K, 1>(w[1], prev[1], st8); else states8<K, 3>(w[1], prev[1], st8);
+                        if (h == 0) products8<K, 1, CB>(w[1], prev[1], st8); else products8<K, 3, CB>(w[1], prev[1], st8);
                         #pragma unroll
                         for (int j = 0; j < 8; ++j) a1[j] = a_word<CB>(st8[j]);
                         tcv_st_tile(t_st + (16u << 16) + 16, a1);
