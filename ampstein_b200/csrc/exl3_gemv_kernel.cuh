@@ -605,6 +605,14 @@ __device__ __forceinline__ void cp_async16_s(uint32_t dst, const void* src)
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" :: "r"(dst), "l"(src) : "memory");
 }
 
+// 8 bytes of constant data, requested here and not where the compiler would rather have it
+__device__ __forceinline__ uint2 ldg_v2(const void* p)
+{
+    uint2 v;
+    asm volatile("ld.global.nc.v2.u32 {%0, %1}, [%2];" : "=r"(v.x), "=r"(v.y) : "l"(p));
+    return v;
+}
+
 template <int N>
 __device__ __forceinline__ void cp_async_wait_n()
 {
@@ -1746,6 +1754,11 @@ void exl3_gemv_kernel(const GemvParams P)
         float* slots = P.scratch;                      // [cta][2][m][128]
         const int my_slot = 2 * cta + (blk * G > u0 ? 1 : 0);
         float* dst = whole ? part : slots + (size_t) my_slot * m * 128;
+        // The block's output scales are requested ahead of the exchange: behind it they are one more round trip to the L2 at the
+        // end of the launch (one row, us: 4096 x 1024 at 4 bits 5.54 -> 5.25, 4096 x 28672 27.2 -> 27.0, a one-token MoE layer at
+        // 4 bits 25.8 -> 21.4; 8 rows 4096 x 28672 36.5 -> 35.9). The instances with the all-reduce or a fused neighbour spill already.
+        uint2 sv_raw;
+        if constexpr (!AR) sv_raw = ldg_v2(svh + (size_t) nb * 128 + lane * 4);
         // cluster form: the partial goes straight into the shared memory of the cluster's first CTA
         const bool clustered = !RUNS && P.cluster > 0;
         uint32_t xdst = 0;
@@ -1872,7 +1885,10 @@ void exl3_gemv_kernel(const GemvParams P)
                 float h0 = v.x, h1 = v.y, h2 = v.z, h3 = v.w;
                 warp_had128(h0, h1, h2, h3, lane);
                 h0 *= kRScale; h1 *= kRScale; h2 *= kRScale; h3 *= kRScale;
-                const half4 sv = reinterpret_cast<const half4*>(svh + (size_t) nb * 128)[lane];
+                if constexpr (AR) sv_raw = ldg_v2(svh + (size_t) nb * 128 + lane * 4);
+                half4 sv;
+                sv.x = *reinterpret_cast<const __half2*>(&sv_raw.x);
+                sv.y = *reinterpret_cast<const __half2*>(&sv_raw.y);
                 if constexpr (MODE != 0)
                 {
                     // fp32 scale, optional bias, scattered to the slot's row
