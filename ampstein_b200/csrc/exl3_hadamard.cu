@@ -6,6 +6,7 @@
 #include "exl3_common.cuh"
 #include <cuda_bf16.h>
 #include "host_common.h"
+#include "exl3_gemv_host.h"
 
 namespace amp {
 
@@ -137,6 +138,17 @@ void had_r_128_kernel(const void* __restrict__ in, void* __restrict__ out,
     }
 }
 
+// Start of the rotation kernels. Themselves dependent launches (pdl): their blocks move in as those of the grid in front (a
+// GEMM as a rule) leave, and wait here until that grid is done -- its output is read, and it may still read the x~ that is
+// overwritten. Only then is the GEMM behind released: it allocates its tensor memory and starts its weight stream under this
+// kernel, as ever after everything in front of this kernel, and waits (griddepcontrol.wait in its fetch warp) before it reads
+// the first rotated row. (No __restrict__ in these kernels: it would let a load move up across the wait.)
+__device__ __forceinline__ void had_tiled_begin(int pdl)
+{
+    if (pdl) asm volatile("griddepcontrol.wait;" ::: "memory");
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+
 // Rotated prefill activations in the layout the tensor-core GEMM fetches them in: x~ =
 // fp16(H(x * suh) / sqrt(128)) of an (M, k) matrix, stored k-step-major -- [k / 64][M] rows of 64
 // halves (128 bytes) -- with the 16-byte pieces of a row already XOR-swizzled by (row & 7). A
@@ -145,19 +157,16 @@ void had_r_128_kernel(const void* __restrict__ in, void* __restrict__ out,
 // as the plain kernels above (fp16 input: scaled in fp16; bf16 input: scaled in fp32).
 template <bool BF16>
 __global__ __launch_bounds__(256)
-void had_tiled_kernel(const void* __restrict__ in, __half* __restrict__ out, const __half* __restrict__ pre,
-                      const long long* __restrict__ pre_table, long chunks, int chunks_per_row, long M, float r_scale)
+void had_tiled_kernel(const void* in, __half* out, const __half* pre,
+                      const long long* pre_table, long chunks, int chunks_per_row, long M, float r_scale, int pdl)
 {
+    had_tiled_begin(pdl);
     // bundle: blockIdx.y = source; each source has its own scale vector and its own x~
     if (pre_table)
     {
         pre = reinterpret_cast<const __half*>(pre_table[blockIdx.y]);
         out += (size_t) blockIdx.y * (size_t) chunks * 128;
     }
-    // the GEMM that consumes this kernel's output may be scheduled from now on: it allocates its
-    // tensor memory and starts its weight stream under this kernel, and waits (griddepcontrol.wait
-    // in its fetch thread) before it reads the first rotated row
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     const int lane = threadIdx.x & 31;
     const long chunk = (long) blockIdx.x * 8 + (threadIdx.x >> 5);
     if (chunk >= chunks) return;
@@ -198,10 +207,10 @@ void had_tiled_kernel(const void* __restrict__ in, __half* __restrict__ out, con
 // 17.7, 2048 x 14336 45.0 / 28.1 (4.2 TB/s).
 template <bool BF16>
 __global__ __launch_bounds__(256, 3)
-void had_tiled_rows_kernel(const void* __restrict__ in, __half* __restrict__ out, const __half* __restrict__ pre,
-                           const long long* __restrict__ pre_table, int sources, long groups, int chunks_per_row, long M)
+void had_tiled_rows_kernel(const void* in, __half* out, const __half* pre,
+                           const long long* pre_table, int sources, long groups, int chunks_per_row, long M, int pdl)
 {
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    had_tiled_begin(pdl);
     const int lane = threadIdx.x & 31, pc = lane & 3;
     const long task = (long) blockIdx.x * 8 + (threadIdx.x >> 5);
     if (task >= groups * chunks_per_row) return;
@@ -261,6 +270,22 @@ void had_tiled_rows_kernel(const void* __restrict__ in, __half* __restrict__ out
 // one each (three sources, one each / walking: 333 x 4096 5.8 / 6.3, 700 x 4096 9.2 / 9.2, 2048 x 4096 21.1 / 17.7).
 constexpr long HAD_ROWS_MIN = 6400, HAD_WALK_MIN = 2560;
 
+// 256 threads a block, as a programmatic dependent of the launch in front
+template <typename... Par, typename... Arg>
+static cudaError_t launch_dependent(void (*kernel)(Par...), dim3 grid, cudaStream_t stream, Arg... args)
+{
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = dim3(256, 1, 1);
+    cfg.stream = stream;
+    cudaLaunchAttribute attr;
+    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr.val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = &attr;
+    cfg.numAttrs = g_pdl ? 1 : 0;
+    return cudaLaunchKernelEx(&cfg, kernel, static_cast<Par>(args)...);
+}
+
 // (M, k) fp16 or bf16 -> tiled x~ (M * k halves). Internal to the prefill path.
 int launch_had_tiled(const void* in, void* out, const void* pre, long M, int k, int bf16, cudaStream_t stream,
                      const long long* pre_table, int sources)
@@ -278,14 +303,12 @@ int launch_had_tiled(const void* in, void* out, const void* pre, long M, int k, 
     {
         // one block walks all sources where that alone fills the device
         const dim3 grid((unsigned) ((tasks + 7) / 8), tasks >= HAD_WALK_MIN ? 1u : (unsigned) sources);
-        if (bf16) had_tiled_rows_kernel<true><<<grid, 256, 0, stream>>>(in, (__half*) out, (const __half*) pre, pre_table, sources, groups, k / 128, M);
-        else had_tiled_rows_kernel<false><<<grid, 256, 0, stream>>>(in, (__half*) out, (const __half*) pre, pre_table, sources, groups, k / 128, M);
-        return cuda_rc(cudaGetLastError(), "exl3_gemm input rotation");
+        return cuda_rc(launch_dependent(bf16 ? had_tiled_rows_kernel<true> : had_tiled_rows_kernel<false>, grid, stream, in, (__half*) out,
+                                        (const __half*) pre, pre_table, sources, groups, k / 128, M, g_pdl), "exl3_gemm input rotation");
     }
     const dim3 grid((unsigned) blocks, pre_table ? (unsigned) sources : 1u);
-    if (bf16) had_tiled_kernel<true><<<grid, 256, 0, stream>>>(in, (__half*) out, (const __half*) pre, pre_table, chunks, k / 128, M, kRScale);
-    else had_tiled_kernel<false><<<grid, 256, 0, stream>>>(in, (__half*) out, (const __half*) pre, pre_table, chunks, k / 128, M, kRScale);
-    return cuda_rc(cudaGetLastError(), "exl3_gemm input rotation");
+    return cuda_rc(launch_dependent(bf16 ? had_tiled_kernel<true> : had_tiled_kernel<false>, grid, stream, in, (__half*) out,
+                                    (const __half*) pre, pre_table, chunks, k / 128, M, kRScale, g_pdl), "exl3_gemm input rotation");
 }
 
 }  // namespace amp

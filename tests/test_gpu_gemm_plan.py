@@ -64,3 +64,35 @@ def test_rotation_forms(amp, m, k, sources, bf16, offset):
         got = had[i].view(k // 64, m, 8, 8)                  # (k step, row, 16-byte piece, value); piece p lies at p ^ (row & 7)
         got = got.gather(2, (piece ^ (row & 7)).view(1, m, 8, 1).expand(k // 64, m, 8, 8))
         assert torch.equal(got.permute(1, 0, 2, 3).reshape(m, k).view(torch.int16), ref.view(torch.int16))
+
+
+# The rotation kernel moves in under the GEMM in front of it: a chain of linears that read each other's output through ONE
+# scratch for the rotated input gives the bits of the same chain without dependent launches. Either rotation form (6400 chunks),
+# every GEMM form, and decode launches (8 rows) in between.
+@pytest.mark.parametrize("rows", [(17, 17, 17), (77, 8, 77), (300, 600, 300), (900, 900, 900)])
+def test_dependent_rotations(amp, rows):
+    from ampstein_b200 import _lib
+    k, K = 1024, 4
+    g = torch.Generator(device="cuda").manual_seed(5)
+    tr = torch.randint(-32768, 32768, (3, k // 16, k // 16, 16 * K), dtype=torch.int16, device="cuda", generator=g)
+    suh = torch.randint(0, 2, (3, k), device="cuda", generator=g).to(torch.float16) * 2 - 1
+    svh = torch.full((3, k), 1.0 / (1.2437 * k ** 0.5), dtype=torch.float16, device="cuda")
+    x = torch.randn(1000, k, device="cuda", generator=g).to(torch.float16)
+    had = torch.empty_like(x)
+
+    def chain():
+        a, b = x.clone(), torch.zeros_like(x)
+        for _ in range(8):
+            for i, m in enumerate(rows):
+                amp.exl3_gemm(a[:m], tr[i], b[:m], suh[i], svh[i], had[:m])
+                a, b = b, a
+        return a, b
+
+    got = chain()
+    _lib.lib().amp_exl3_set_pdl(0)
+    try:
+        ref = chain()
+    finally:
+        _lib.lib().amp_exl3_set_pdl(1)
+    assert gemm_status() == 0
+    assert all(torch.equal(p.view(torch.int16), q.view(torch.int16)) for p, q in zip(got, ref))
