@@ -84,7 +84,8 @@ def test_dependent_rotations(amp, rows):
         a, b = x.clone(), torch.zeros_like(x)
         for _ in range(8):
             for i, m in enumerate(rows):
-                amp.exl3_gemm(a[:m], tr[i], b[:m], suh[i], svh[i], had[:m])
+                _lib.call("amp_exl3_gemm", a.data_ptr(), tr[i].data_ptr(), b.data_ptr(), suh[i].data_ptr(), had.data_ptr(), svh[i].data_ptr(),
+                          m, k, k, K, 0, 0, torch.cuda.current_stream().cuda_stream)
                 a, b = b, a
         return a, b
 
