@@ -132,12 +132,12 @@ __device__ __forceinline__ void umma_commit(uint64_t* bar)
                  :: "r"(smem_u32(bar)) : "memory");
 }
 
-// Shared shifts (window_product) where they take load off the integer ALU, which also packs here: at 3 and 6 bits a shift and a
+// Shared shifts (window_product) where they take load off the integer ALU, which also packs here: at 2, 3 and 6 bits a shift and a
 // mask on the other pipe per window leave it less to do, except for codebook 2, whose masks are ALU work too (us, one each /
-// shared: 59 tokens x top-8 of 128 experts at 3 bits 190.9 / 197.8; 600 x 4096 x 14336 at 6 bits 81.5 / 82.4, codebook 2 at 3 bits
+// shared: 24 x 4096 x 14336 at 2 bits 28.8 / 29.4, 77 x 4096 x 14336 30.6 / 31.3; 59 tokens x top-8 of 128 experts at 3 bits 190.9 / 197.8; 600 x 4096 x 14336 at 6 bits 81.5 / 82.4, codebook 2 at 3 bits
 // 78.8 / 75.6, at 6 bits 78.3 / 75.6)
 template <int K, int CB>
-constexpr bool tg_shared_phase = shared_phase<K> && (CB == 2 || (K != 3 && K != 6));
+constexpr bool tg_shared_phase = shared_phase<K> && (CB == 2 || (K != 2 && K != 3 && K != 6));
 
 constexpr int TG_MAX_N = 256;                 // tokens per accumulator (UMMA N)
 constexpr int TG_MAX_TOKENS = 512;            // tokens per tile: two accumulators, with 16 decode warps only
