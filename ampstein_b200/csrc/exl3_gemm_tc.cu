@@ -75,13 +75,14 @@ static int tg_layout(TgParams& S, int tile, int ng, bool pair = false)
 // Tokens a CTA finishes per epilogue pass and where their partial sums ((source, token) rows of 512 bytes) are
 // received: behind the stages where that leaves three x~ stages (no barrier between the k loop and the exchange
 // then), else over the stages, in several passes if need be. Returns the dynamic shared memory.
-static int tg_exchange(TgParams& S, int smem)
+static int tg_exchange(TgParams& S, int smem, bool pair)
 {
+    const int xr = pair ? S.tile / 2 : S.tile;
     int ts = (S.tile + S.split - 1) / S.split;
     S.recv_off = 0;
     if (S.split > 1)
     {
-        const int budget = smem - tg_smem(0, S.wstages, 0), recv = S.split * ts * tg_row(S.split), x = S.tile * TC_BK * 2;
+        const int budget = smem - tg_smem(0, S.wstages, 0), recv = S.split * ts * tg_row(S.split), x = xr * TC_BK * 2;
         const int left = (budget - recv) / x;
         if (budget > recv && left >= 3)
         {
@@ -92,7 +93,7 @@ static int tg_exchange(TgParams& S, int smem)
     const int room = smem / tg_row(S.split);
     if (!S.recv_off && ts * S.split > room) ts = room / S.split & ~15;
     S.share = ts;
-    return S.recv_off ? tg_smem(S.tile, S.wstages, S.xstages) + S.split * ts * tg_row(S.split) : smem;
+    return S.recv_off ? tg_smem(xr, S.wstages, S.xstages) + S.split * ts * tg_row(S.split) : smem;
 }
 
 // Clusters of c CTAs (one CTA per SM) the device holds at once: the SMs of a GPC come in no multiple of c
@@ -122,22 +123,21 @@ static int tg_max_clusters(int c, int sms, int dev)
     return v;
 }
 
-// Tile height, decode groups and k split for M rows x `blocks` column blocks: the cheapest by a model (us) that ranks
-// plans. A 64-row step takes the slowest of the decode (0.40 per 8192 weights), the tensor pipe's own time (0.28
-// per 256 tokens; the whole step of a 512-token pair takes 0.65) and the x~ tiles of all CTAs out of L2 (8.5 TB/s); a
-// CTA costs 4 + 0.02 per token around its k loop, the exchange of a split 1.5 and 0.035 (clusters of more than four: 0.07)
-// per token that crosses to a peer. The sums are not times: the median plan of a single CTA comes out at 1.12 x its
-// measured time, pairs at 0.88, 512-token pairs at 0.6 - 0.8. The ranking is what was measured: over 74 pairs of a shape (eight, 2048 x
-// 5120 .. 14336 x 4096) and a row count (24 .. 2048), every tile height and split forced in turn, the plan taken is on
-// average within 1.4 % of the best one in short bursts and 0.7 % under sustained load (where the GPU runs at 1.45 GHz); the
-// worst ones are 8192 x 2048 at 1500 rows (80.6 us with tiles of 192 tokens, 68.3 with 384 and k cut in two) and 4096 x
-// 28672 at 256 rows (81.5 as pairs, 69.6 as single CTAs; sustained 78.2 / 76.5).
+// Tile height, form and k split for M rows x `blocks` column blocks: the cheapest by a model (us) that ranks plans. A 64-row
+// step takes the slowest of the decode (0.40 per 8192 weights, 0.52 in a pair with its hand-over), the tensor pipe
+// (0.46 per 256 tokens, 0.56 per 512 of a pair) and the x~ tiles of all CTAs out of L2 (8.5 TB/s; the CTAs of a pair fetch half
+// each); a CTA costs 4 + 0.0115 per token (a pair 1.2 more) around its k loop, the exchange of a split 0.7 and 0.034 per token
+// that crosses to a peer. The sums are not times, the ranking is what was measured: 224 pairs of a shape (24, k 1024 .. 25600, n 512
+// .. 28672, 4 bits) and a row count (17 .. 2048), every form, tile height and split forced in turn; the plan taken is on average within
+// 0.7 % of the best one, nine in ten within 1.0 % (the constants before this fit: 1.3 and 4.8 %; without splits of pairs 0.8 and
+// 1.1 %). The worst: 410 x 16256 x 1664 with k cut in five 57.5 us, in four 41.5; 372 x
+// 14336 x 4096 58.7 / 52.5.
 // One CTA of sixteen decode warps per SM: two of eight take as long per step and longer per exchange.
 static int tg_plan(TgParams& S, int M, long blocks, bool pairs, int ksteps, int sms, int dev, int* form)
 {
     // forced by tests and sweeps: pairs of 512- / 256-token tiles (modes 2, 3), no pairs (0), a tile height, a split
     const int tile_forced = g_tc_tile ? g_tc_tile : (pairs && g_tc_pair == 2 ? 512 : (pairs && g_tc_pair == 3 ? 256 : 0));
-    const bool only_pairs = pairs && g_tc_pair >= 2 && !g_tc_split, no_pairs = !pairs || !g_tc_pair || g_tc_split;
+    const bool only_pairs = pairs && g_tc_pair >= 2, no_pairs = !pairs || !g_tc_pair || (g_tc_split && g_tc_pair < 2);
     double best = 1e30;
     int best_smem = 0;
     TgParams T = S;
@@ -146,20 +146,20 @@ static int tg_plan(TgParams& S, int M, long blocks, bool pairs, int ksteps, int 
         {
             const int smem = tg_layout(T, tile_forced ? tile_forced : ((M + tiles - 1) / tiles + 15) & ~15, 2, pair), xs = T.xstages;
             if (!smem) continue;
-            for (int c = 1; c <= (pair ? 1 : 8) && c <= ksteps; ++c)
+            for (int c = 1; c <= (pair ? 4 : 8) && c <= ksteps; ++c)
             {
                 T.split = c;
                 T.xstages = xs;
                 if (g_tc_split && c != g_tc_split) continue;
-                const int need = tg_exchange(T, smem);
+                const int need = tg_exchange(T, smem, pair);
                 if (T.share < 1) continue;
                 const long clusters = (pair ? blocks / 2 : blocks) * ((M + T.tile - 1) / T.tile);
-                const long fit = c > 1 || pair ? tg_max_clusters(pair ? 2 : c, sms, dev) : sms;
-                const long waves = (clusters + fit - 1) / fit, live = c * (clusters < fit ? clusters : fit);
-                const double mma = 0.28 * T.tile / 256, l2 = pair ? 0.0 : T.tile * 128.0 * live / 8.5e6;
-                const double step = mma > l2 ? (mma > 0.40 ? mma : 0.40) : (l2 > 0.40 ? l2 : 0.40);
-                const double cost = waves * ((double) ((ksteps + c - 1) / c) * step + 4.0 + 0.02 * T.tile + (pair ? 1.0 : 0.0)
-                                             + (c > 1 ? 1.5 + (c > 4 ? 0.07 : 0.035) * T.tile * (c - 1) / c : 0.0));
+                const long fit = c > 1 || pair ? tg_max_clusters(pair ? 2 * c : c, sms, dev) : sms;
+                const long waves = (clusters + fit - 1) / fit, live = (pair ? 2 : 1) * c * (clusters < fit ? clusters : fit);
+                const double mma = (pair ? 0.0011 : 0.0018) * T.tile, l2 = T.tile * (pair ? 64.0 : 128.0) * live / 8.5e6, decode = pair ? 0.52 : 0.40;
+                const double feed = mma > l2 ? mma : l2, step = feed > decode ? feed : decode;
+                const double cost = waves * ((double) ((ksteps + c - 1) / c) * step + 4.0 + 0.0115 * T.tile + (pair ? 1.2 : 0.0)
+                                             + (c > 1 ? 0.7 + 0.034 * T.tile * (c - 1) / c : 0.0));
                 if (cost < best * 0.99) { best = cost; best_smem = need; S = T; *form = pair ? TG_PAIR : TG_DENSE; }
             }
         }
@@ -206,7 +206,7 @@ int launch_gemm_tc(const void* xh, const void* trellis, void* c, const void* svh
     cfg.stream = stream;
     cudaLaunchAttribute attr[2];
     int na = 0;
-    const int cluster = form == TG_PAIR ? 2 : S.split;
+    const int cluster = form == TG_PAIR ? 2 * S.split : S.split;
     if (cluster > 1)
     {
         attr[na].id = cudaLaunchAttributeClusterDimension;

@@ -12,7 +12,8 @@
 //   * dense: one CTA of 16 decode warps per SM; k is split over the CTAs of a thread-block cluster, so that a small
 //     matrix or a short batch still spreads over the device (partial sums meet through distributed shared memory);
 //   * pair: two CTAs (two SMs) with tcgen05 cta_group::2, 256 columns x up to 512 tokens. Each CTA decodes its 128
-//     columns and fetches half of the x~ rows; the tensor cores of both read both halves. For many rows;
+//     columns and fetches half of the x~ rows; the tensor cores of both read both halves. For many rows. k may be split
+//     over up to four pairs of a cluster (x~ then crosses the L2 once per 256 columns also where the grid needs the split);
 //   * grouped: one CTA of 8 decode warps per (expert tile, projection, 128 columns), two per SM, so that one CTA's
 //     set-up and epilogue run under the other's decode.
 //
@@ -152,7 +153,7 @@ struct TgParams
     TcParams t;                 // pointers, sizes, bundle tables, expert tile table
     int tile;                   // tokens per tile: a multiple of 16, at most 512
     int n0;                     // tokens of the first accumulator: a multiple of 16, at most 256 (the rest: the second, at column 256)
-    int split;                  // CTAs per cluster = slices of k (1: no cluster)
+    int split;                  // slices of k: CTAs per cluster (1: no cluster), pairs per cluster in the pair form
     int wstages, xstages;       // stages of decoded weights and of x~: wstages >= 2 NG
     int x_area;                 // expert groups: bytes of all x~ stages together (xstages then follows from the tile's rows)
     int tmem_cols;              // tensor-memory columns to allocate: a power of two >= tile, >= 32 (two accumulators: 512)
@@ -291,10 +292,10 @@ __device__ __forceinline__ void tg_umma(uint32_t d, uint64_t a, uint64_t b, uint
 
 // Arrives, once every tcgen05.mma issued so far by this thread has completed, on the barrier at this shared-memory
 // offset in both CTAs of a pair (an arrival multicast, not a load)
-__device__ __forceinline__ void tg_commit_both(uint64_t* bar)
+__device__ __forceinline__ void tg_commit_both(uint64_t* bar, unsigned short pair_mask)
 {
     asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;"
-                 :: "r"(smem_u32(bar)), "h"((unsigned short) 3) : "memory");
+                 :: "r"(smem_u32(bar)), "h"(pair_mask) : "memory");
 }
 
 // An arrival on a barrier of the first CTA of a pair: publishes what this thread wrote or observed (releasing arrivals of
@@ -347,9 +348,11 @@ void exl3_gemm_tc_kernel(const TgParams S)
     // anything); a grouped launch is followed by kernels that do not wait themselves
     if constexpr (!GROUPED) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     const int t = threadIdx.x, lane = t & 31, warp = __shfl_sync(0xffffffffu, t >> 5, 0);
-    const int split = GROUPED || PAIR ? 1 : S.split;
-    const int prank = PAIR ? (int) tg_cluster_rank() : 0;    // CTA of a pair
-    const int crank = split > 1 ? (int) tg_cluster_rank() : 0;
+    const int split = GROUPED ? 1 : S.split;
+    // place in the cluster: slice of k (crank), CTA of a pair (prank); the CTA that holds the same columns in slice i
+    const int rank = PAIR || split > 1 ? (int) tg_cluster_rank() : 0;
+    const int prank = PAIR ? rank & 1 : 0, crank = PAIR ? rank >> 1 : rank;
+    auto peer_of = [&](int i) { return (uint32_t) (PAIR ? 2 * i + prank : i); };
     TcSlice W;
     int m0, rows;
     if constexpr (GROUPED)
@@ -367,7 +370,7 @@ void exl3_gemm_tc_kernel(const TgParams S)
     }
     else
     {
-        W = tc_slice<TC_BN>(P, (int) blockIdx.x / split);
+        W = tc_slice<TC_BN>(P, PAIR ? (int) blockIdx.x / (2 * split) * 2 + prank : (int) blockIdx.x / split);
         m0 = (int) blockIdx.y * S.tile;
         rows = min(S.tile, P.M - m0);
     }
@@ -437,7 +440,7 @@ void exl3_gemm_tc_kernel(const TgParams S)
 
     // 0: a wait of this role ran out. It walks on to its end, looks at later barriers once each and hands nothing over any
     // more; every barrier below is still reached.
-    auto full_limit = [&]() { return !GROUPED && (PAIR ? prank == 1 : crank == split - 1) ? P.wait_limit_last : P.wait_limit; };
+    auto full_limit = [&]() { return !GROUPED && crank == split - 1 && (!PAIR || prank == 1) ? P.wait_limit_last : P.wait_limit; };
     unsigned limit = full_limit();
     auto wait_bar = [&](uint32_t bar, uint32_t parity)
     {
@@ -501,7 +504,7 @@ void exl3_gemm_tc_kernel(const TgParams S)
             wait_bar(b_done + sq * 8, phq);
             wait_bar(b_x + sx * 8, phx);
             wait_bar(b_w + s * 8, ph);
-            if (tg_elect() && limit) tg_arrive_cluster(cluster_map(b_peer + sd * 8, 0));
+            if (tg_elect() && limit) tg_arrive_cluster(cluster_map(b_peer + sd * 8, (uint32_t) rank & ~1u));
             __syncwarp();
             if (limit == 0) continue;
             last = sd; phl = phd;
@@ -541,7 +544,7 @@ void exl3_gemm_tc_kernel(const TgParams S)
                     #pragma unroll
                     for (int kk = 0; kk < TC_BK / 16; ++kk)
                         tg_umma<PAIR>(tmem + TG_MAX_N, dwt + 2 * kk, dx + to1 + 2 * kk, idesc1, (i > 0 || kk > 0) ? 1u : 0u);
-                if constexpr (PAIR) tg_commit_both(&done[sd]);
+                if constexpr (PAIR) tg_commit_both(&done[sd], (unsigned short) (3u << (rank & ~1)));
                 else umma_commit(&done[sd]);
             }
             __syncwarp();
@@ -632,9 +635,9 @@ void exl3_gemm_tc_kernel(const TgParams S)
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     if (split > 1)
     {
-        cluster_wait_started();                              // the peers run: their shared memory is written from here on
+        if constexpr (!PAIR) cluster_wait_started();         // the peers run: their shared memory is written from here on
         // nobody adds up partial sums to which a wait that ran out has contributed (read behind the barrier of the exchange)
-        if (s_bad && t < split) tg_st_cluster_u32(cluster_map(smem_u32(const_cast<int*>(&s_bad)), (uint32_t) t), 1);
+        if (s_bad && t < split) tg_st_cluster_u32(cluster_map(smem_u32(const_cast<int*>(&s_bad)), peer_of(t)), 1);
     }
     // ... and they write into this CTA's receive buffer: where it overlaps the stages, everybody's MMAs must have read theirs
     if (split > 1 && S.recv_off == 0) cluster_sync_all();
@@ -675,7 +678,7 @@ void exl3_gemm_tc_kernel(const TgParams S)
                     {
                         const uint32_t a = col + (uint32_t) (tl * row);
                         if (dest == crank) asm volatile("st.shared.u32 [%0], %1;" :: "r"(a), "r"(v[j]) : "memory");
-                        else cluster_st_f32(cluster_map(a, (uint32_t) dest), __uint_as_float(v[j]));
+                        else cluster_st_f32(cluster_map(a, peer_of(dest)), __uint_as_float(v[j]));
                     }
                     if (++tl == TS) { tl = 0; ++dest; }
                 }

@@ -39,6 +39,29 @@ def test_forced_plans(amp, oracle, m, k, n, K, cb, split, tile):
         _lib.lib().amp_exl3_set_gemm_plan(0, 0)
 
 
+# Pairs with k split over two to four of them: few rows, two accumulators, slices of unequal length, several passes of the
+# epilogue, several tiles, more than one pair of column blocks
+@pytest.mark.parametrize("m,k,n,K,cb,split,tile", [
+    (17, 256, 256, 4, 0, 2, 32), (33, 640, 512, 3, 2, 3, 48), (300, 1152, 256, 5, 1, 4, 304), (512, 512, 256, 2, 0, 2, 512),
+    (500, 896, 768, 6, 0, 4, 256), (1030, 256, 256, 4, 2, 4, 512), (47, 1024, 1280, 8, 1, 3, 16)])
+def test_forced_pair_splits(amp, oracle, m, k, n, K, cb, split, tile):
+    from ampstein_b200 import _lib
+    trellis, suh, svh, x = make_linear(k, n, K, seed=9100 + m + K, m=m)
+    svh = (svh.astype(np.float32) / (1.2437 * np.sqrt(k))).astype(np.float16)
+    ref = oracle.linear(x, trellis, suh, svh, cb, fp32_out=True)
+    old = _lib.lib().amp_exl3_set_gemm_pair(2)
+    _lib.lib().amp_exl3_set_gemm_plan(split, tile)
+    try:
+        for fp32 in (False, True):
+            got = run_gemm(amp, trellis, suh, svh, x, cb, fp32=fp32)
+            assert gemm_status() == 0
+            check_close(got, ref)
+        assert np.array_equal(got, run_gemm(amp, trellis, suh, svh, x, cb, fp32=True))
+    finally:
+        _lib.lib().amp_exl3_set_gemm_plan(0, 0)
+        _lib.lib().amp_exl3_set_gemm_pair(old)
+
+
 # Either form of the rotation kernel in front of the GEMM (one warp per chunk; eight rows per warp from 6400 chunks on, walking all
 # sources from 2560 tasks on), read back from the caller's scratch: bit-exact against the stand-alone Hadamard. Row counts around
 # multiples of eight; an input that is only 8-byte aligned.
