@@ -257,43 +257,47 @@ __device__ __forceinline__ void ms_scale(const uint4 (&v)[4], const uint4 (&s)[4
     }
 }
 
-// One row per warp; a warp takes eight 128-value chunks of its row per pass, four lanes each.
-// Bound by instruction issue (two rotations per assignment): the packed butterflies took 12000 rows of 2048 from
-// 47 to 29 us.
+// A warp takes one 8-row group (rows of one expert) and MS_IN_CHUNKS consecutive 128-value chunks of it, four lanes to a row: the
+// chain of loads from the group to its rows (group, expert, token, row) is walked once for all of them, a scale vector's piece is
+// loaded for eight rows at once, and a 64-k step of the rows is written as 1 KB in one place. Two rotations per assignment.
+// Bound by instruction issue (0.51 of the slots, 376 instructions per 8 rotations) and the few warps its registers leave: 12000 rows of
+// 2048 in 36 us (38 with a row per warp); loads requested one chunk ahead at four blocks per SM 40.
+constexpr int MS_IN_CHUNKS = 4;
 __global__ __launch_bounds__(128, 5)
 void moe_sorted_rotate_in_kernel(const MsRot P)
 {
     // (the GEMM behind this launch may set itself up and start its weight stream; its fetch warp waits for this grid)
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, pc = lane & 3, cl = lane >> 2;
-    const int nrows = P.hdr[1], chunks = P.H >> 7;
-    for (int p = (int) blockIdx.x * 4 + warp; p < nrows; p += (int) gridDim.x * 4)
+    const int chunks = P.H >> 7, parts = (chunks + MS_IN_CHUNKS - 1) / MS_IN_CHUNKS, ntasks = (P.hdr[1] >> 3) * parts;
+    for (int task = (int) blockIdx.x * 4 + warp; task < ntasks; task += (int) gridDim.x * 4)
     {
-        const int rec = P.grp[p >> 3], e = rec & 0xffffff;
-        if ((p & 7) >= (rec >> 24)) continue;
+        const int g = task / parts, c0 = (task - g * parts) * MS_IN_CHUNKS, p = 8 * g + cl;
+        const int rec = P.grp[g], e = rec & 0xffffff;
+        if (rec >> 24 == 0) continue;
         const int s = P.sstart[e] + (p - P.pstart[e]);
-        const long long tok = (s >= 0 && s < P.A) ? P.tok_sorted[s] : -1;
         const __half* gs = P.g_suh ? reinterpret_cast<const __half*>(P.g_suh[e]) : nullptr;
         const __half* us = reinterpret_cast<const __half*>(P.u_suh[e]);
-        if (tok < 0 || tok >= P.T)
+        bool live = cl < (rec >> 24);
+        const long long tok = (live && s >= 0 && s < P.A) ? P.tok_sorted[s] : -1;
+        if (live && (tok < 0 || tok >= P.T))
         {
-            if (lane == 0) atomicOr(P.status, MS_E_TOKEN);
-            continue;                                      // the row keeps whatever it held; it is never summed
+            if (pc == 0) atomicOr(P.status, MS_E_TOKEN);
+            live = false;                                  // the row keeps whatever it held; it is never summed
         }
-        if (lane == 0)
+        if (live && pc == 0 && c0 == 0)
         {
             const int j = atomicAdd(&P.fill[tok], 1);
             if (j < P.topk) P.list[(size_t) tok * P.topk + j] = make_int2(p, s);
             else atomicOr(P.status, MS_E_TOPK);
         }
-        const __half* src = P.y + (size_t) tok * P.H;
+        const __half* src = P.y + (size_t) (live ? tok : 0) * P.H;         // (idle lanes still take part in the shuffles)
         unsigned char* xu = P.xt + (gs ? (size_t) P.mcap * P.H * 2 : 0);
+        const int c1 = min(c0 + MS_IN_CHUNKS, chunks);
         #pragma unroll 1
-        for (int c0 = 0; c0 < chunks; c0 += 8)
+        for (int cb = c0; cb < c1; ++cb)
         {
-            const int cb = c0 + cl;
-            const bool live = cb < chunks;                 // (idle lanes still take part in the shuffles)
-            const int off = (live ? cb : 0) * 128;
+            const int off = cb * 128;
             uint4 v[4], sc[4];
             f32x2 h[16];
             ms_load_pieces(src + off, pc, v);
@@ -312,47 +316,48 @@ void moe_sorted_rotate_in_kernel(const MsRot P)
     }
 }
 
-// task = 128-value chunks of a row: a warp takes eight consecutive (row, chunk) pairs of an expert's 8-row group, four
-// lanes each
+// A warp takes one 128-value chunk of an 8-row group, four lanes to a row. SILU: the gated SiLU without a limit, as an instance
+// of its own: chosen at run time for
+// every value the activation took most of the kernel's 39 instructions per value. The layer of 1500 tokens x top-8, us: 357 with eight chunks of a row per
+// warp, 352 in this order, 346 with the instance.
+template <bool SILU>
 __global__ __launch_bounds__(256, 3)
 void moe_sorted_rotate_act_kernel(const MsRot P)
 {
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, pc = lane & 3, cl = lane >> 2;
-    const int ngroups = P.hdr[1] >> 3, chunks = P.I >> 7;
+    const int chunks = P.I >> 7, ntasks = (P.hdr[1] >> 3) * chunks;
     const __half* gbase = P.gu;                                                     // gate outputs (projection 0)
     const __half* ubase = P.gu + (P.gated ? (size_t) P.mcap * P.I : 0);              // up outputs
-    for (int g = blockIdx.x; g < ngroups; g += gridDim.x)
+    for (int task = (int) blockIdx.x * 8 + warp; task < ntasks; task += (int) gridDim.x * 8)
     {
-        const int rec = P.grp[g], e = rec & 0xffffff, rows = rec >> 24;
-        if (rows == 0) continue;
-        const __half* ds = reinterpret_cast<const __half*>(P.d_suh[e]);
-        #pragma unroll 1
-        for (int cb = warp; cb < chunks; cb += 8)          // lane group cl: row cl of the group, chunk cb
+        const int g = task / chunks, cb = task - g * chunks, p = 8 * g + cl;
+        const int rec = P.grp[g];
+        // (rows beyond the group's own are computed on whatever the workspace holds there, and not stored)
+        const __half* ur = ubase + (size_t) p * P.I + cb * 128;
+        const __half* gr = gbase + (size_t) p * P.I + cb * 128;
+        uint4 u[4], gt[4], sc[4];
+        f32x2 h[16];
+        ms_load_pieces(ur, pc, u);
+        ms_load_pieces(SILU || P.gated ? gr : ur, pc, gt);
+        if (rec >> 24 == 0) continue;
+        ms_load_pieces(reinterpret_cast<const __half*>(P.d_suh[rec & 0xffffff]) + cb * 128, pc, sc);
+        #pragma unroll
+        for (int j = 0; j < 4; ++j)
         {
-            const bool live = cl < rows;                   // (idle lanes still take part in the shuffles)
-            const int p = 8 * g + (live ? cl : 0);
-            const __half* ur = ubase + (size_t) p * P.I + cb * 128;
-            const __half* gr = gbase + (size_t) p * P.I + cb * 128;
-            uint4 u[4], gt[4], sc[4];
-            f32x2 h[16];
-            ms_load_pieces(ur, pc, u);
-            ms_load_pieces(P.gated ? gr : ur, pc, gt);
-            ms_load_pieces(ds + cb * 128, pc, sc);
+            const __half2* a = reinterpret_cast<const __half2*>(&gt[j]);
+            const __half2* b = reinterpret_cast<const __half2*>(&u[j]);
+            const __half2* c = reinterpret_cast<const __half2*>(&sc[j]);
             #pragma unroll
-            for (int j = 0; j < 4; ++j)
+            for (int q = 0; q < 4; ++q)
             {
-                const __half2* a = reinterpret_cast<const __half2*>(&gt[j]);
-                const __half2* b = reinterpret_cast<const __half2*>(&u[j]);
-                const __half2* c = reinterpret_cast<const __half2*>(&sc[j]);
-                #pragma unroll
-                for (int q = 0; q < 4; ++q)
-                    h[4 * j + q] = pack_f32x2(moe_act_gate(P.act, P.gated, __low2float(a[q]), __low2float(b[q]), P.act_limit) * __low2float(c[q]),
-                                               moe_act_gate(P.act, P.gated, __high2float(a[q]), __high2float(b[q]), P.act_limit) * __high2float(c[q]));
+                auto act1 = [&](float g1, float u1) { return SILU ? moe_act_gate(MOE_ACT_SILU, true, g1, u1, 0.0f) : moe_act_gate(P.act, P.gated, g1, u1, P.act_limit); };
+                h[4 * j + q] = pack_f32x2(act1(__low2float(a[q]), __low2float(b[q])) * __low2float(c[q]),
+                                           act1(__high2float(a[q]), __high2float(b[q])) * __high2float(c[q]));
             }
-            quad_had128(h, pc);
-            if (live) ms_store_pieces(P.xt, P.mcap, p, cb, pc, h);
         }
+        quad_had128(h, pc);
+        if (cl < (rec >> 24)) ms_store_pieces(P.xt, P.mcap, p, cb, pc, h);
     }
 }
 
@@ -557,7 +562,7 @@ AMP_API int amp_exl3_moe_sorted(const amp_moe_sorted_args* a, cudaStream_t strea
     R.g_suh = gated ? (const long long*) a->g_suh : nullptr; R.u_suh = (const long long*) a->u_suh;
     R.xt = ws + L.xt_gu; R.mcap = (int) L.mcap;
     R.fill = Pp.fill; R.list = (int2*) (ws + L.list);
-    const long in_blocks = L.mcap / 4;                 // (a row per warp)
+    const long in_blocks = (groups_max * ((a->H / 128 + MS_IN_CHUNKS - 1) / MS_IN_CHUNKS) + 3) / 4;       // four tasks a block
     moe_sorted_rotate_in_kernel<<<(unsigned) (in_blocks < (long) sms * 20 ? in_blocks : (long) sms * 20), 128, 0, stream>>>(R);
     if (cudaError_t e = cudaGetLastError()) return cuda_rc(e, "exl3_moe_sorted input rotation launch");
 
@@ -596,7 +601,10 @@ AMP_API int amp_exl3_moe_sorted(const amp_moe_sorted_args* a, cudaStream_t strea
     MsRot D = R;
     D.gu = gu; D.I = a->I; D.d_suh = (const long long*) a->d_suh; D.act = a->act; D.gated = gated ? 1 : 0; D.act_limit = a->act_limit;
     D.xt = ws + L.xt_d;
-    moe_sorted_rotate_act_kernel<<<rot_blocks, 256, 0, stream>>>(D);
+    const long act_blocks = (groups_max * (a->I / 128) + 7) / 8;                                              // eight tasks a block
+    const unsigned act_grid = (unsigned) (act_blocks < (long) sms * 12 ? act_blocks : (long) sms * 12);
+    if (gated && a->act == MOE_ACT_SILU && a->act_limit == 0.0f) moe_sorted_rotate_act_kernel<true><<<act_grid, 256, 0, stream>>>(D);
+    else moe_sorted_rotate_act_kernel<false><<<act_grid, 256, 0, stream>>>(D);
     if (cudaError_t e = cudaGetLastError()) return cuda_rc(e, "exl3_moe_sorted activation launch");
 
     G.kinds = 1;
