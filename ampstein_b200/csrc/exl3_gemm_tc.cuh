@@ -344,9 +344,9 @@ void exl3_gemm_tc_kernel(const TgParams S)
     __shared__ __align__(16) uint2 s_svh[32];                    // the block's output scales
     constexpr int NDEC = 8 * NG, NGR = NDEC / TG_GROUP_WARPS;    // decode warps; groups of them that take alternate steps
 
-    // the rotation kernel of the next linear may move in as this grid's CTAs leave (it waits for all of them before it does
-    // anything); a grouped launch is followed by kernels that do not wait themselves
-    if constexpr (!GROUPED) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    // the kernel behind (as a rule the rotation of the next linear, or of the expert layer's activations) may move in as this
+    // grid's CTAs leave; it waits for all of them before it does anything
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     const int t = threadIdx.x, lane = t & 31, warp = __shfl_sync(0xffffffffu, t >> 5, 0);
     const int split = GROUPED ? 1 : S.split;
     // place in the cluster: slice of k (crank), CTA of a pair (prank); the CTA that holds the same columns in slice i

@@ -72,4 +72,21 @@ int launch_gemm_tc_grouped(const void* xt, void* c, long Mcap, int k, int n, int
 
 extern int g_pdl;
 
+// Launch as a programmatic dependent of the launch in front (g_pdl): the kernel waits (griddepcontrol.wait) before it touches
+// anything that launch reads or writes
+template <typename... Par, typename... Arg>
+inline cudaError_t launch_dependent(void (*kernel)(Par...), dim3 grid, int threads, cudaStream_t stream, Arg... args)
+{
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = dim3((unsigned) threads, 1, 1);
+    cfg.stream = stream;
+    cudaLaunchAttribute attr;
+    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr.val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = &attr;
+    cfg.numAttrs = g_pdl ? 1 : 0;
+    return cudaLaunchKernelEx(&cfg, kernel, static_cast<Par>(args)...);
+}
+
 }  // namespace amp

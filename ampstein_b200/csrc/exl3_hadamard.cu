@@ -270,22 +270,6 @@ void had_tiled_rows_kernel(const void* in, __half* out, const __half* pre,
 // one each (three sources, one each / walking: 333 x 4096 5.8 / 6.3, 700 x 4096 9.2 / 9.2, 2048 x 4096 21.1 / 17.7).
 constexpr long HAD_ROWS_MIN = 6400, HAD_WALK_MIN = 2560;
 
-// 256 threads a block, as a programmatic dependent of the launch in front
-template <typename... Par, typename... Arg>
-static cudaError_t launch_dependent(void (*kernel)(Par...), dim3 grid, cudaStream_t stream, Arg... args)
-{
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = grid;
-    cfg.blockDim = dim3(256, 1, 1);
-    cfg.stream = stream;
-    cudaLaunchAttribute attr;
-    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr.val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = &attr;
-    cfg.numAttrs = g_pdl ? 1 : 0;
-    return cudaLaunchKernelEx(&cfg, kernel, static_cast<Par>(args)...);
-}
-
 // (M, k) fp16 or bf16 -> tiled x~ (M * k halves). Internal to the prefill path.
 int launch_had_tiled(const void* in, void* out, const void* pre, long M, int k, int bf16, cudaStream_t stream,
                      const long long* pre_table, int sources)
@@ -303,11 +287,11 @@ int launch_had_tiled(const void* in, void* out, const void* pre, long M, int k, 
     {
         // one block walks all sources where that alone fills the device
         const dim3 grid((unsigned) ((tasks + 7) / 8), tasks >= HAD_WALK_MIN ? 1u : (unsigned) sources);
-        return cuda_rc(launch_dependent(bf16 ? had_tiled_rows_kernel<true> : had_tiled_rows_kernel<false>, grid, stream, in, (__half*) out,
+        return cuda_rc(launch_dependent(bf16 ? had_tiled_rows_kernel<true> : had_tiled_rows_kernel<false>, grid, 256, stream, in, (__half*) out,
                                         (const __half*) pre, pre_table, sources, groups, k / 128, M, g_pdl), "exl3_gemm input rotation");
     }
     const dim3 grid((unsigned) blocks, pre_table ? (unsigned) sources : 1u);
-    return cuda_rc(launch_dependent(bf16 ? had_tiled_kernel<true> : had_tiled_kernel<false>, grid, stream, in, (__half*) out,
+    return cuda_rc(launch_dependent(bf16 ? had_tiled_kernel<true> : had_tiled_kernel<false>, grid, 256, stream, in, (__half*) out,
                                     (const __half*) pre, pre_table, chunks, k / 128, M, kRScale, g_pdl), "exl3_gemm input rotation");
 }
 

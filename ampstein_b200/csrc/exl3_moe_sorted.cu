@@ -129,9 +129,19 @@ __device__ __forceinline__ int block_excl_scan_1024(int v, int* s_warp, int& tot
     return wbase + inc - v;
 }
 
+// Every kernel of the chain is a dependent launch: its blocks move in as those of the one in front leave, and wait for that grid
+// here. Each waits before it releases the next, so that what a kernel reads or overwrites belongs to grids that are done,
+// however far in front; the GEMMs behind the rotations, too, read the tile table before their own wait.
+__device__ __forceinline__ void ms_begin()
+{
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+
 __global__ __launch_bounds__(1024)
 void moe_sorted_prep_kernel(const MsPrep P)
 {
+    ms_begin();
     __shared__ int s_warp[32];
     const int t = threadIdx.x;
     for (int i = t; i < P.T; i += 1024) P.fill[i] = 0;
@@ -266,8 +276,7 @@ constexpr int MS_IN_CHUNKS = 4;
 __global__ __launch_bounds__(128, 5)
 void moe_sorted_rotate_in_kernel(const MsRot P)
 {
-    // (the GEMM behind this launch may set itself up and start its weight stream; its fetch warp waits for this grid)
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    ms_begin();         // (the GEMM behind may set itself up and start its weight stream; its fetch warp waits for this grid)
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, pc = lane & 3, cl = lane >> 2;
     const int chunks = P.H >> 7, parts = (chunks + MS_IN_CHUNKS - 1) / MS_IN_CHUNKS, ntasks = (P.hdr[1] >> 3) * parts;
     for (int task = (int) blockIdx.x * 4 + warp; task < ntasks; task += (int) gridDim.x * 4)
@@ -324,7 +333,7 @@ template <bool SILU>
 __global__ __launch_bounds__(256, 3)
 void moe_sorted_rotate_act_kernel(const MsRot P)
 {
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    ms_begin();
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, pc = lane & 3, cl = lane >> 2;
     const int chunks = P.I >> 7, ntasks = (P.hdr[1] >> 3) * chunks;
     const __half* gbase = P.gu;                                                     // gate outputs (projection 0)
@@ -364,10 +373,9 @@ void moe_sorted_rotate_act_kernel(const MsRot P)
 // One block per token: its (row, sorted position) entries in ascending row order (= ascending
 // expert), weight * row summed in fp32, added to the output row.
 __global__ __launch_bounds__(256)
-void moe_sorted_combine_kernel(const int* __restrict__ fill, const int2* __restrict__ list, int topk,
-                               const __half* __restrict__ w_sorted, const float* __restrict__ dout,
-                               float* __restrict__ out, int H)
+void moe_sorted_combine_kernel(const int* fill, const int2* list, int topk, const __half* w_sorted, const float* dout, float* out, int H)
 {
+    ms_begin();         // (no __restrict__: it would let a load move up across the wait)
     __shared__ int s_row[MS_MAX_TOPK];
     __shared__ float s_w[MS_MAX_TOPK];
     const int tok = blockIdx.x, t = threadIdx.x;
@@ -544,8 +552,7 @@ AMP_API int amp_exl3_moe_sorted(const amp_moe_sorted_args* a, cudaStream_t strea
     Pp.src[2] = gated ? (const long long*) a->g_svh : nullptr;     Pp.src[3] = (const long long*) a->u_svh;
     Pp.src[4] = (const long long*) a->d_trellis;                   Pp.src[5] = (const long long*) a->d_svh;
     Pp.tab = (long long*) (ws + L.tab);
-    moe_sorted_prep_kernel<<<1, 1024, 0, stream>>>(Pp);
-    if (cudaError_t e = cudaGetLastError()) return cuda_rc(e, "exl3_moe_sorted prep launch");
+    if (cudaError_t e = launch_dependent(moe_sorted_prep_kernel, 1, 1024, stream, Pp)) return cuda_rc(e, "exl3_moe_sorted prep launch");
 
     int dev = 0, sms = 148;
     if (cudaError_t e = cudaGetDevice(&dev)) return cuda_rc(e, "cudaGetDevice");
@@ -563,8 +570,7 @@ AMP_API int amp_exl3_moe_sorted(const amp_moe_sorted_args* a, cudaStream_t strea
     R.xt = ws + L.xt_gu; R.mcap = (int) L.mcap;
     R.fill = Pp.fill; R.list = (int2*) (ws + L.list);
     const long in_blocks = (groups_max * ((a->H / 128 + MS_IN_CHUNKS - 1) / MS_IN_CHUNKS) + 3) / 4;       // four tasks a block
-    moe_sorted_rotate_in_kernel<<<(unsigned) (in_blocks < (long) sms * 20 ? in_blocks : (long) sms * 20), 128, 0, stream>>>(R);
-    if (cudaError_t e = cudaGetLastError()) return cuda_rc(e, "exl3_moe_sorted input rotation launch");
+    if (cudaError_t e = launch_dependent(moe_sorted_rotate_in_kernel, (unsigned) (in_blocks < (long) sms * 20 ? in_blocks : (long) sms * 20), 128, stream, R)) return cuda_rc(e, "exl3_moe_sorted input rotation launch");
 
     TcGroups G = {};
     G.ntiles = Pp.hdr; G.tile_e = Pp.tile_e; G.tile_row0 = Pp.tile_row0; G.tile_rows = Pp.tile_rows;
@@ -603,9 +609,8 @@ AMP_API int amp_exl3_moe_sorted(const amp_moe_sorted_args* a, cudaStream_t strea
     D.xt = ws + L.xt_d;
     const long act_blocks = (groups_max * (a->I / 128) + 7) / 8;                                              // eight tasks a block
     const unsigned act_grid = (unsigned) (act_blocks < (long) sms * 12 ? act_blocks : (long) sms * 12);
-    if (gated && a->act == MOE_ACT_SILU && a->act_limit == 0.0f) moe_sorted_rotate_act_kernel<true><<<act_grid, 256, 0, stream>>>(D);
-    else moe_sorted_rotate_act_kernel<false><<<act_grid, 256, 0, stream>>>(D);
-    if (cudaError_t e = cudaGetLastError()) return cuda_rc(e, "exl3_moe_sorted activation launch");
+    const bool silu = gated && a->act == MOE_ACT_SILU && a->act_limit == 0.0f;
+    if (cudaError_t e = launch_dependent(silu ? moe_sorted_rotate_act_kernel<true> : moe_sorted_rotate_act_kernel<false>, act_grid, 256, stream, D)) return cuda_rc(e, "exl3_moe_sorted activation launch");
 
     G.kinds = 1;
     G.bits[0] = G.bits[1] = mixed ? (const unsigned char*) a->d_bits : nullptr;
@@ -619,9 +624,8 @@ AMP_API int amp_exl3_moe_sorted(const amp_moe_sorted_args* a, cudaStream_t strea
                                                                  (float*) a->scratch, (const long long*) a->slot_base, a->scratch_rows);
         return cuda_rc(cudaGetLastError(), "exl3_moe_sorted slot launch");
     }
-    moe_sorted_combine_kernel<<<a->T, 256, 0, stream>>>(Pp.fill, (const int2*) (ws + L.list), R.topk, (const __half*) a->w_sorted,
-                                                        (const float*) (ws + L.dout), (float*) a->out, a->H);
-    return cuda_rc(cudaGetLastError(), "exl3_moe_sorted combine launch");
+    return cuda_rc(launch_dependent(moe_sorted_combine_kernel, a->T, 256, stream, Pp.fill, (const int2*) (ws + L.list), R.topk, (const __half*) a->w_sorted,
+                                    (const float*) (ws + L.dout), (float*) a->out, a->H), "exl3_moe_sorted combine launch");
 }
 
 AMP_API int amp_exl3_moe_gather(float* out, const float* scratch, const void* flat_expert, const void* inv_order,
