@@ -125,13 +125,12 @@ static int tg_max_clusters(int c, int sms, int dev)
 
 // Tile height, form and k split for M rows x `blocks` column blocks: the cheapest by a model (us) that ranks plans. A 64-row
 // step takes the slowest of the decode (0.40 per 8192 weights, 0.52 in a pair with its hand-over), the tensor pipe
-// (0.46 per 256 tokens, 0.56 per 512 of a pair) and the x~ tiles of all CTAs out of L2 (8.5 TB/s; the CTAs of a pair fetch half
-// each); a CTA costs 4 + 0.0115 per token (a pair 1.2 more) around its k loop, the exchange of a split 0.7 and 0.034 per token
-// that crosses to a peer. The sums are not times, the ranking is what was measured: 224 pairs of a shape (24, k 1024 .. 25600, n 512
+// (0.46 per 256 tokens, 0.69 per 512 of a pair) and the x~ tiles of all CTAs out of L2 (8.5 TB/s; the CTAs of a pair fetch half
+// each); a CTA costs 4 + 0.0138 per token (a pair 1.2 more) around its k loop, the exchange of a split 0.7 and 0.032 per token
+// that crosses to a peer. The sums are not times, the ranking is what was measured: 296 pairs of a shape (24, k 1024 .. 25600, n 512
 // .. 28672, 4 bits) and a row count (17 .. 2048), every form, tile height and split forced in turn; the plan taken is on average within
-// 0.7 % of the best one, nine in ten within 1.0 % (the constants before this fit: 1.3 and 4.8 %; without splits of pairs 0.8 and
-// 1.1 %). The worst: 410 x 16256 x 1664 with k cut in five 57.5 us, in four 41.5; 372 x
-// 14336 x 4096 58.7 / 52.5.
+// 0.5 % of the best one, nine in ten within 0.7 % (the constants before this fit: 1.1 and 3.8 %; without splits of pairs 0.7 and
+// 0.9 %). The worst: 410 x 16256 x 1664 with k cut in five 57.5 us, in four 41.5; 372 x 14336 x 4096 58.7 / 52.5.
 // One CTA of sixteen decode warps per SM: two of eight take as long per step and longer per exchange.
 static int tg_plan(TgParams& S, int M, long blocks, bool pairs, int ksteps, int sms, int dev, int* form)
 {
@@ -156,10 +155,10 @@ static int tg_plan(TgParams& S, int M, long blocks, bool pairs, int ksteps, int 
                 const long clusters = (pair ? blocks / 2 : blocks) * ((M + T.tile - 1) / T.tile);
                 const long fit = c > 1 || pair ? tg_max_clusters(pair ? 2 * c : c, sms, dev) : sms;
                 const long waves = (clusters + fit - 1) / fit, live = (pair ? 2 : 1) * c * (clusters < fit ? clusters : fit);
-                const double mma = (pair ? 0.0011 : 0.0018) * T.tile, l2 = T.tile * (pair ? 64.0 : 128.0) * live / 8.5e6, decode = pair ? 0.52 : 0.40;
+                const double mma = (pair ? 0.00134 : 0.0018) * T.tile, l2 = T.tile * (pair ? 64.0 : 128.0) * live / 8.5e6, decode = pair ? 0.52 : 0.40;
                 const double feed = mma > l2 ? mma : l2, step = feed > decode ? feed : decode;
-                const double cost = waves * ((double) ((ksteps + c - 1) / c) * step + 4.0 + 0.0115 * T.tile + (pair ? 1.2 : 0.0)
-                                             + (c > 1 ? 0.7 + 0.034 * T.tile * (c - 1) / c : 0.0));
+                const double cost = waves * ((double) ((ksteps + c - 1) / c) * step + 4.0 + 0.0138 * T.tile + (pair ? 1.2 : 0.0)
+                                             + (c > 1 ? 0.7 + 0.032 * T.tile * (c - 1) / c : 0.0));
                 if (cost < best * 0.99) { best = cost; best_smem = need; S = T; *form = pair ? TG_PAIR : TG_DENSE; }
             }
         }
