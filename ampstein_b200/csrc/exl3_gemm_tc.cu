@@ -295,7 +295,7 @@ AMP_API int amp_exl3_set_gemm_relay_release(int)
 }
 
 // Pair (cta_group::2) form: 0 = never, 1 = by plan (default), 2 / 3 = pairs of 512 / 256 tokens whenever n is a
-// multiple of 256 (tests). Returns the previous setting.
+// multiple of 256, with a forced split over up to four pairs (tests). Returns the previous setting.
 AMP_API int amp_exl3_set_gemm_pair(int mode)
 {
     const int old = g_tc_pair;

@@ -117,12 +117,12 @@ int amp_exl3_gemm_bf16(const void* A, const void* trellis, void* C, const void* 
 
 /*
  * Pair form of the tensor-core GEMM (two CTAs per 256 columns, tcgen05 cta_group::2): 0 = never, 1 = by plan (default),
- * 2 / 3 = pairs of 512 / 256 tokens whenever n is a multiple of 256 (for tests). Returns the previous setting. No
- * counterpart in the reference.
+ * 2 / 3 = pairs of 512 / 256 tokens whenever n is a multiple of 256, with the split of amp_exl3_set_gemm_plan where one is
+ * forced, up to four pairs (for tests). Returns the previous setting. No counterpart in the reference.
  */
 int amp_exl3_set_gemm_pair(int mode);
 /*
- * Plan of the tensor-core GEMM for tests and sweeps: the number of k slices (1..8) and / or the tokens per tile (a
+ * Plan of the tensor-core GEMM for tests and sweeps: the number of k slices (1..8; of single CTAs unless pairs are forced) and / or the tokens per tile (a
  * multiple of 16, up to 512); 0: by rule (default). Returns 0. No counterpart in the reference.
  */
 int amp_exl3_set_gemm_plan(int split, int tile);
