@@ -245,9 +245,9 @@ int launch_gemm_tc_grouped(const void* xt, void* c, long Mcap, int k, int n, int
     S.x_area = smem - tg_smem(0, S.wstages, 0);
     S.split = 1;
     S.share = smem / tg_row(1) & ~15;
-    // Dependent launch only where every grid that does anything waits for the rotation kernel: with one launch per
-    // bit width a launch whose experts all have another width would be over before that kernel, and the next
-    // launch's wait would be for it alone.
+    // Dependent launch only where the first CTA of the grid waits for the rotation kernel: with one launch per bit width a
+    // launch whose experts all have another width would be over before that kernel, and the next launch's wait would be
+    // for it alone.
     S.pdl = g_pdl && !G.bits[0];
     TcParams& P = S.t;
     P.xt = (const unsigned char*) xt; P.c = c;

@@ -326,8 +326,13 @@ void exl3_gemm_tc_kernel(const TgParams S)
     const TcParams& P = S.t;
     if constexpr (GROUPED)
     {
-        // the whole CTA leaves, before any barrier or allocation
-        if ((int) blockIdx.y >= *P.g_ntiles || P.g_tile_rows[blockIdx.y] <= 0) return;
+        // the whole CTA leaves, before any barrier or allocation (the first one of the grid not before the grid in front is done:
+        // a grid without any tile is over only then, see ms_begin)
+        if ((int) blockIdx.y >= *P.g_ntiles || P.g_tile_rows[blockIdx.y] <= 0)
+        {
+            if (S.pdl && blockIdx.x == 0 && blockIdx.y == 0) pdl_wait();
+            return;
+        }
         const unsigned char* bits = P.g_bits[(int) blockIdx.x / (P.n / TC_BN)];
         if (bits && bits[P.g_tile_e[blockIdx.y]] != K) return;
     }
@@ -336,6 +341,7 @@ void exl3_gemm_tc_kernel(const TgParams S)
     if (smem_u32(smem_raw) & 1023)                           // (the swizzle needs the alignment the declaration asks for)
     {
         if (threadIdx.x == 0) atomicExch(P.status, 2);
+        if (S.pdl) pdl_wait();
         return;
     }
     __shared__ uint64_t x_full[TG_MAX_STAGES], w_full[TG_MAX_STAGES], done[TG_MAX_STAGES], peer[PAIR ? TG_MAX_STAGES : 1];

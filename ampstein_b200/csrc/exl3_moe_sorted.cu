@@ -131,7 +131,8 @@ __device__ __forceinline__ int block_excl_scan_1024(int v, int* s_warp, int& tot
 
 // Every kernel of the chain is a dependent launch: its blocks move in as those of the one in front leave, and wait for that grid
 // here. Each waits before it releases the next, so that what a kernel reads or overwrites belongs to grids that are done,
-// however far in front; the GEMMs behind the rotations, too, read the tile table before their own wait.
+// however far in front; the GEMMs behind the rotations, too, read the tile table before their own wait. A grid is done once its
+// blocks have left, whether they have waited or not: in every grid at least one block waits, in a GEMM without any tile too.
 __device__ __forceinline__ void ms_begin()
 {
     asm volatile("griddepcontrol.wait;" ::: "memory");

@@ -252,6 +252,54 @@ def test_sorted_moe_replays_from_a_cuda_graph_with_new_routing(amp, oracle):
         check(out.cpu().numpy(), oracle.moe_coop(x, sel, rw, ex, gu_f16=True))
 
 
+@pytest.mark.parametrize("kg,ku", [(3, 3), (3, 4)])
+def test_sorted_moe_without_any_tile_in_front_of_another_call(amp, kg, ku):
+    """Calls that no expert falls into (a row range, an expert-parallel shard without picks) launch GEMMs without a tile; the next
+    call on the same workspace, directly behind in one graph, rewrites tables that the launches in front of those GEMMs read.
+    Bit-equal to the same calls with dependent launches off."""
+    from ampstein_b200 import _lib
+    E, H, I, topk = 8, 256, 128, 2
+    ex = [dict(zip(("gate", "up", "down"), (one[kind] for kind, one in zip(("gate", "up", "down"), group))))
+          for group in zip(make_experts(E, H, I, H, kg, 4100), make_experts(E, H, I, H, ku, 4200), make_experts(E, H, I, H, 4, 4300))]
+    cfg = build_cfg(amp, ex, H, I, H, H, 0, 1, topk)
+    cfg.update({"Kg": kg, "Ku": ku, "Kd": 4, "I": I})
+    rng = np.random.default_rng(91)
+    calls = []
+    for T, e0, lo, hi in ((900, 0, 1, 0), (900, 0, 5000, 0), (40, 0, 1, 0), (900, 100, 1, 0), (500, 0, 1, 0), (40, 0, 5000, 0), (40, 100, 1, 0), (900, 0, 1, 0)):
+        sel, rw = routing(rng, T, E, topk)
+        x = dev(rng.standard_normal((T, H)).astype(np.float16))
+        calls.append((x, torch.zeros((T, H), dtype=torch.float32, device="cuda")) + tuple(amp.moe_sort_routing(dev(sel), dev(rw), E, e0)) + (lo, hi))
+
+    def run_all():
+        for x, out, count, tok, wts, lo, hi in calls:
+            amp.moe_fused(x, out, count, tok, wts, cfg, -1, lo, hi, 16)
+
+    def replay():
+        for c in calls:
+            c[1].zero_()
+        st, gr = torch.cuda.Stream(), torch.cuda.CUDAGraph()
+        torch.cuda.synchronize()
+        with torch.cuda.stream(st):
+            run_all()                                        # warm-up: the workspace exists before capture
+        torch.cuda.synchronize()
+        with torch.cuda.stream(st), torch.cuda.graph(gr, stream=st):
+            run_all()
+        for _ in range(20):
+            gr.replay()
+        torch.cuda.synchronize()
+        assert amp.moe_fused_status(cfg) == 0
+        return [c[1].clone() for c in calls]
+
+    got = replay()
+    _lib.lib().amp_exl3_set_pdl(0)
+    try:
+        want = replay()
+    finally:
+        _lib.lib().amp_exl3_set_pdl(1)
+    for g, w, c in zip(got, want, calls):
+        assert torch.equal(g, w) and bool(g.any()) == (c[5] == 1 and int(c[2][:E].sum()) > 0)
+
+
 def test_sorted_moe_reports_bad_routing_without_touching_memory(amp):
     """A token index outside [0, T) and counts that describe more rows than the list holds set the
     status word; the entries in error are left out."""
