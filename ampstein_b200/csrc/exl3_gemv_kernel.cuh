@@ -872,7 +872,13 @@ void exl3_gemv_kernel(const GemvParams P)
         if (ONE && inline_active == 0 && cta == 0 && P.moe.first_down)
             for (int c = warp; c < (P.moe.Ho >> 7); c += GEMV_WARPS) moe_combine_chunk(P.moe, 0, c, lane);
     }
-    if (cta >= ncta) return;                           // an exited CTA counts as having released its dependents
+    if (cta >= ncta)                                   // an exited CTA counts as having released its dependents
+    {
+        // a launch without any run (no local pick, no pick of this bit width): it is over once its CTAs have left, and the
+        // next launch waits for it alone; so the first one leaves only behind the grid in front
+        if (MODE == 2 && cta == 0 && P.pdl) pdl_wait();
+        return;
+    }
     GemvSplit split;
     split.q = U / ncta;
     split.r = U - split.q * ncta;

@@ -14,6 +14,7 @@ WAIT = re.compile(r"griddepcontrol\.wait|\bpdl_wait\(|\bms_begin\(|\bhad_tiled_b
 NOT_FIRST = {
     "gemv_prerotate_kernel": {"if (task >= m * per_row) return;"},
     "exl3_gemv_tc_kernel": {"if (cta >= ncta) return;"},     # (its work is known on the host, and not empty)
+    "exl3_gemv_kernel": {"if (u0 >= u1) return;", "if (cblk * G >= U) return;"},       # behind cta >= ncta: the first of ncta ranges is not empty
     # (a CTA whose expert has another bit width: such launches are not dependent)
     "exl3_gemm_tc_kernel": {"if (bits && bits[P.g_tile_e[blockIdx.y]] != K) return;"},
 }
@@ -38,7 +39,7 @@ def _early_returns(body):
 
 
 DEPENDENT = [(name, kernel, body) for name in sorted(f for f in os.listdir(CSRC) if f.endswith((".cu", ".cuh")))
-             for kernel, body in _kernels(name) if WAIT.search(body) and kernel != "exl3_gemv_kernel"]
+             for kernel, body in _kernels(name) if WAIT.search(body)]
 
 
 @pytest.mark.parametrize("name,kernel", [d[:2] for d in DEPENDENT])
@@ -50,5 +51,5 @@ def test_first_block_waits_before_it_leaves(name, kernel):
 
 def test_the_search_finds_the_kernels():
     found = {k for _, k, _ in DEPENDENT}
-    assert found >= {"exl3_gemv_tc_kernel", "exl3_gemm_tc_kernel", "moe_prep_kernel", "moe_sorted_combine_kernel",
+    assert found >= {"exl3_gemv_kernel", "exl3_gemv_tc_kernel", "exl3_gemm_tc_kernel", "moe_prep_kernel", "moe_sorted_combine_kernel",
                      "had_tiled_kernel", "had_tiled_rows_kernel", "gemv_prerotate_kernel"}

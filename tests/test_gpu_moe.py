@@ -193,6 +193,57 @@ def test_moe_experts_of_different_bit_widths(amp, oracle, T):
     assert cfg["_kmask"] == (0b11100, 0b101010)
 
 
+@pytest.mark.parametrize("T", [1, 5])
+def test_moe_launches_without_a_run_in_front_of_another_call(amp, T):
+    """Launches that find no work (a bit width that no pick has, a call without local picks) directly followed, in one graph, by
+    the launches of another width and by the next call on the same scratch: bit-equal to the same calls with dependent
+    launches off."""
+    from ampstein_b200 import _lib
+    E, H, I, topk = 8, 512, 256, 3
+    kgu, kd = [3, 4, 4, 3, 5, 4, 3, 5], [4, 4, 2, 2, 4, 6, 6, 2]
+    at = {K: make_experts(E, H, I, H, K, seed=1700 + 50 * K) for K in sorted(set(kgu + kd))}
+    ex = [{"gate": at[kgu[e]][e]["gate"], "up": at[kgu[e]][e]["up"], "down": at[kd[e]][e]["down"]} for e in range(E)]
+    rng = np.random.default_rng(45 + T)
+    bits = lambda v: torch.tensor(v, dtype=torch.uint8, device="cuda")
+    cfg = build_cfg(amp, ex, H, I, H, H, 0, 8, topk, g_bits=bits(kgu), u_bits=bits(kgu), d_bits=bits(kd), min_expert=8, max_expert=16)
+    x = [dev(rng.standard_normal((T, H)).astype(np.float16)) for _ in range(6)]
+    rw = dev(rng.uniform(0.2, 0.6, (T, topk)).astype(np.float16))
+    # experts 8 .. 15 are local. Down: all widths; 2 bits alone (the 4 and 6 bits launches behind are empty); none at all; 6 bits alone
+    picks = [[8, 10, 13], [10, 11, 15], [0, 1, 2], [13, 14, 3], [8, 9, 12], [1, 20, 7]]
+    sel = [dev(np.stack([rng.permutation(p) for _ in range(T)]).astype(np.int64)) for p in picks]
+    outs = [torch.zeros_like(cfg["out"]) for _ in picks]
+
+    def run_all():
+        for xi, si, oi in zip(x, sel, outs):
+            cfg["out"] = oi
+            amp.moe_coop(xi, si, rw, cfg)
+
+    def replay():
+        st, gr = torch.cuda.Stream(), torch.cuda.CUDAGraph()
+        torch.cuda.synchronize()
+        with torch.cuda.stream(st):
+            run_all()
+        torch.cuda.synchronize()
+        with torch.cuda.stream(st), torch.cuda.graph(gr, stream=st):
+            run_all()
+        for o in outs:
+            o.fill_(float("nan"))
+        torch.cuda.synchronize()
+        for _ in range(20):
+            gr.replay()
+        torch.cuda.synchronize()
+        return [o[:T].clone() for o in outs]
+
+    got = replay()
+    _lib.lib().amp_exl3_set_pdl(0)
+    try:
+        want = replay()
+    finally:
+        _lib.lib().amp_exl3_set_pdl(1)
+    for g, w, p in zip(got, want, picks):
+        assert torch.equal(g, w) and bool(g.any()) == any(8 <= e < 16 for e in p)
+
+
 def test_moe_and_a_plain_gemv_on_two_streams_at_once(amp, oracle):
     """The reference runs the shared expert's linears on a side stream while moe_coop runs
     (src/ucode/ampstein/glm5.uc:970,998): launches that overlap on the GPU must not share arrival
