@@ -123,14 +123,27 @@ static int tg_max_clusters(int c, int sms, int dev)
     return v;
 }
 
+// Share of a wave that clusters of an odd size take longer when they fill the device (`left` more would fit) behind a rotation
+// kernel whose blocks are still leaving (a dependent launch). What the occupancy query counts fits at once only on free SMs: clusters
+// that move in one by one as SMs free up leave single SMs over, and the last ones start late. Measured, us, with dependent launches /
+// in plain order: 400 x 2304 with k cut in three, 41 clusters 28.7 / 33.0, 44: 34.6 / 33.0, 45 (all that fit) 43.1 / 33.0; 400 x 3840 cut
+// in five, 23: 30.3 / 33.0, 25: 36.6 / 33.1, 26 (all) 46.4 / 33.3. Rotations of up to a block per SM leave no trace (40 rows: 12.2 at any
+// count), nor do even sizes, nor seven (105 of 148 SMs).
+static double tg_late(int c, long left, long chunks, int sms)
+{
+    return (c != 3 && c != 5) || chunks <= 8L * sms || left > 2 ? 0.0 : (left == 0 ? 0.4 : (left == 1 ? 0.15 : 0.04));
+}
+
 // Tile height, form and k split for M rows x `blocks` column blocks: the cheapest by a model (us) that ranks plans. A 64-row
-// step takes the slowest of the decode (0.40 per 8192 weights, 0.52 in a pair with its hand-over), the tensor pipe
-// (0.46 per 256 tokens, 0.69 per 512 of a pair) and the x~ tiles of all CTAs out of L2 (8.5 TB/s; the CTAs of a pair fetch half
-// each); a CTA costs 4 + 0.0138 per token (a pair 1.2 more) around its k loop, the exchange of a split 0.7 and 0.032 per token
-// that crosses to a peer. The sums are not times, the ranking is what was measured: 296 pairs of a shape (24, k 1024 .. 25600, n 512
-// .. 28672, 4 bits) and a row count (17 .. 2048), every form, tile height and split forced in turn; the plan taken is on average within
-// 0.5 % of the best one, nine in ten within 0.7 % (the constants before this fit: 1.1 and 3.8 %; without splits of pairs 0.7 and
-// 0.9 %). The worst: 410 x 16256 x 1664 with k cut in five 57.5 us, in four 41.5; 372 x 14336 x 4096 58.7 / 52.5.
+// step takes the slowest of the decode (0.44 per 8192 weights, 0.48 in a pair with its hand-over), the tensor pipe
+// (0.50 per 256 tokens, 0.66 per 512 of a pair) and the x~ tiles of all CTAs out of L2 (9.7 TB/s; the CTAs of a pair fetch half
+// each); a CTA costs 3.6 + 0.0155 per token (a pair 2.8 more) around its k loop, the exchange of a split 0.72 and 0.0354 per token
+// that crosses to a peer. One set of constants: over 1 .. 8 bits and the three codebooks a step's decode differs by a tenth (0.32 ..
+// 0.37, pairs 0.34 .. 0.40). The sums are not times, the ranking is what was measured: fitted on 984 pairs of a shape (k 1024 .. 25600,
+// n 512 .. 28672, 2 .. 8 bits, every codebook) and a row count (17 .. 2048), every form, tile height and split forced in turn. On 357
+// others, on another machine, the plan taken is on average within 0.4 % of the best one, nineteen in twenty within 1.9 % (before tg_late
+// and with constants fitted at 4 bits: 1.2 and 7.5 %, at worst 1.52 x); twelve are more than 5 % above it, at worst 133 x 1792 x 3584
+// 14.2 us / 12.7, 1756 x 10368 x 13952 472 / 432, 698 x 14336 x 2048 59.5 / 55.1.
 // One CTA of sixteen decode warps per SM: two of eight take as long per step and longer per exchange.
 static int tg_plan(TgParams& S, int M, long blocks, bool pairs, int ksteps, int sms, int dev, int* form)
 {
@@ -155,10 +168,11 @@ static int tg_plan(TgParams& S, int M, long blocks, bool pairs, int ksteps, int 
                 const long clusters = (pair ? blocks / 2 : blocks) * ((M + T.tile - 1) / T.tile);
                 const long fit = c > 1 || pair ? tg_max_clusters(pair ? 2 * c : c, sms, dev) : sms;
                 const long waves = (clusters + fit - 1) / fit, live = (pair ? 2 : 1) * c * (clusters < fit ? clusters : fit);
-                const double mma = (pair ? 0.00134 : 0.0018) * T.tile, l2 = T.tile * (pair ? 64.0 : 128.0) * live / 8.5e6, decode = pair ? 0.52 : 0.40;
+                const double late = S.pdl && !pair ? tg_late(c, waves * fit - clusters, (long) M * ksteps / 2, sms) : 0.0;
+                const double mma = (pair ? 0.00128 : 0.00195) * T.tile, l2 = T.tile * (pair ? 64.0 : 128.0) * live / 9.67e6, decode = pair ? 0.48 : 0.44;
                 const double feed = mma > l2 ? mma : l2, step = feed > decode ? feed : decode;
-                const double cost = waves * ((double) ((ksteps + c - 1) / c) * step + 4.0 + 0.0138 * T.tile + (pair ? 1.2 : 0.0)
-                                             + (c > 1 ? 0.7 + 0.032 * T.tile * (c - 1) / c : 0.0));
+                const double cost = (waves + late) * ((double) ((ksteps + c - 1) / c) * step + 3.6 + 0.0155 * T.tile + (pair ? 2.8 : 0.0)
+                                             + (c > 1 ? 0.72 + 0.0354 * T.tile * (c - 1) / c : 0.0));
                 if (cost < best * 0.99) { best = cost; best_smem = need; S = T; *form = pair ? TG_PAIR : TG_DENSE; }
             }
         }

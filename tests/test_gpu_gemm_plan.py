@@ -120,3 +120,30 @@ def test_dependent_rotations(amp, rows):
         _lib.lib().amp_exl3_set_pdl(1)
     assert gemm_status() == 0
     assert all(torch.equal(p.view(torch.int16), q.view(torch.int16)) for p, q in zip(got, ref))
+
+
+# Splits whose clusters of three or five fill the device: behind a rotation kernel that is still leaving, the last ones start late
+# (410 x 16256 x 1664: 57 us against 41). The plan is not one of them: the result has the bits of the plan named, not of that one.
+@pytest.mark.parametrize("m,k,n,K,late,plan", [(410, 16256, 1664, 4, (5, 208), (4, 208)), (736, 10496, 1408, 6, (3, 192), (4, 256)),
+                                               (716, 8320, 640, 4, (5, 144), (6, 192))])
+def test_clusters_that_start_late_are_not_planned(amp, m, k, n, K, late, plan):
+    from ampstein_b200 import _lib
+    g = torch.Generator(device="cuda").manual_seed(7)
+    tr = torch.randint(-32768, 32768, (k // 16, n // 16, 16 * K), dtype=torch.int16, device="cuda", generator=g)
+    suh, svh = torch.ones(k, dtype=torch.float16, device="cuda"), torch.ones(n, dtype=torch.float16, device="cuda")
+    x = torch.randn(m, k, device="cuda", generator=g).to(torch.float16)
+    had = torch.empty_like(x)
+
+    def run(split, tile):
+        y = torch.empty(m, n, dtype=torch.float32, device="cuda")
+        _lib.lib().amp_exl3_set_gemm_plan(split, tile)
+        try:
+            _lib.call("amp_exl3_gemm", x.data_ptr(), tr.data_ptr(), y.data_ptr(), suh.data_ptr(), had.data_ptr(), svh.data_ptr(), m, k, n, K, 0, 1,
+                      torch.cuda.current_stream().cuda_stream)
+        finally:
+            _lib.lib().amp_exl3_set_gemm_plan(0, 0)
+        return y
+
+    got = run(0, 0)
+    assert torch.equal(got, run(*plan)) and not torch.equal(got, run(*late))
+    assert gemm_status() == 0
