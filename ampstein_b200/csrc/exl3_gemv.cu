@@ -133,9 +133,10 @@ constexpr int GEMV_CLUSTER = 8, GEMV_CLUSTER_MAX_M = 8, GEMV_CLUSTER_MAX_UNITS =
 // rounding). Runs right before a GEMV of five or more rows, which then only copies x~ into
 // fragment order instead of rotating all rows of its range in every CTA.
 __global__ __launch_bounds__(256)
-void gemv_prerotate_kernel(const __half* __restrict__ x, __half* __restrict__ out, const __half* __restrict__ suh,
+void gemv_prerotate_kernel(const __half* x, __half* out, const __half* __restrict__ suh,
                            const long long* __restrict__ t_suh, int m, int k, int pdl)
 {
+    // (x and out without __restrict__: it would let a load move up across the wait)
     // the GEMV behind this launch may start its weight stream now; it waits for this grid before it
     // reads x~, and this grid waits for the producer of x
     if (pdl) pdl_launch_dependents();

@@ -4,7 +4,8 @@
 // exist so that the fused forms can be tested and timed against the same arithmetic as separate
 // launches inside one CUDA graph (the reference keeps its own kernels for them:
 // src/torch/amp_kernels.cu:235-251, 279-360, 823-901). Each takes part in programmatic dependent
-// launch like the GEMV kernels do.
+// launch like the GEMV kernels do. (No __restrict__ on what the kernel in front writes: it would let a load move up across the
+// wait.)
 #include "exl3_common.cuh"
 #include "exl3_gemv_host.h"
 #include "host_common.h"
@@ -17,8 +18,8 @@ namespace amp {
 // registers between the two passes (rows up to 4096 wide; wider rows re-read y), so one L2 round trip
 // follows the wait.
 __global__ __launch_bounds__(256)
-void rms_norm_res_kernel(const __half* __restrict__ x, const __half* __restrict__ r, const __half* __restrict__ w,
-                         __half* __restrict__ y, __half* __restrict__ n, int dim, float eps, int pdl)
+void rms_norm_res_kernel(const __half* x, const __half* r, const __half* __restrict__ w,
+                         __half* y, __half* n, int dim, float eps, int pdl)
 {
     __shared__ float s_red[8];
     __shared__ float s_scale;
@@ -93,7 +94,7 @@ void rms_norm_res_kernel(const __half* __restrict__ x, const __half* __restrict_
 
 // out = fp16(silu(g) * u), fp32 math
 __global__ __launch_bounds__(256)
-void silu_mul_kernel(const __half* __restrict__ g, const __half* __restrict__ u, __half* __restrict__ out, long count4, int pdl)
+void silu_mul_kernel(const __half* g, const __half* u, __half* out, long count4, int pdl)
 {
     if (pdl) { pdl_launch_dependents(); pdl_wait(); }
     for (long c = (long) blockIdx.x * 256 + threadIdx.x; c < count4; c += (long) gridDim.x * 256)
@@ -111,7 +112,7 @@ void silu_mul_kernel(const __half* __restrict__ g, const __half* __restrict__ u,
 // advance log[pos] = ids; ids = pick; pos += 1, by the block that arrives last. key / count: zero
 // between launches.
 __global__ __launch_bounds__(256)
-void argmax_advance_kernel(const __half* __restrict__ logits, int n, long long* ids, long long* pos, long long* log,
+void argmax_advance_kernel(const __half* logits, int n, long long* ids, long long* pos, long long* log,
                            long long log_cap, unsigned long long* key_out, unsigned int* count, int pdl)
 {
     if (pdl) { pdl_launch_dependents(); pdl_wait(); }

@@ -1,6 +1,7 @@
 """A launch behind a dependent launch waits for that grid alone, and a grid is over once its blocks have left. So that a wait
 covers everything in front, the first block of every dependent grid waits (griddepcontrol.wait) on every path before it leaves:
-the early returns in the source. No run could show a violation, the grids' overlap is a matter of timing."""
+the early returns in the source. And no load is allowed to move up across the wait. No run could show a violation, the grids'
+overlap is a matter of timing."""
 import os
 import re
 
@@ -47,6 +48,20 @@ def test_first_block_waits_before_it_leaves(name, kernel):
     body = next(b for n, k, b in DEPENDENT if (n, k) == (name, kernel))
     for statement in _early_returns(body):
         assert WAIT.search(statement) or statement in NOT_FIRST.get(kernel, ()), statement
+
+
+def test_nothing_in_front_of_the_wait_is_declared_unaliased():
+    """A load through a const __restrict__ pointer may be moved across the wait (the compiler takes what it points to as constant
+    for the whole kernel): only static operands are declared so in a dependent kernel."""
+    kernels = {k for _, k, _ in DEPENDENT}
+    seen = set()
+    for name in sorted({n for n, _, _ in DEPENDENT}):
+        text = re.sub(r"/\*.*?\*/|//[^\n]*", "", open(os.path.join(CSRC, name)).read(), flags=re.S)
+        for m in re.finditer(r"__global__[^;{]*?(\w+)\s*\(([^)]*)\)\s*\{", text):
+            if m.group(1) in kernels:
+                seen.add(m.group(1))
+                assert set(re.findall(r"__restrict__\s+(\w+)", m.group(2))) <= {"suh", "t_suh", "w"}, m.group(1)
+    assert seen == kernels
 
 
 def test_the_search_finds_the_kernels():
