@@ -13,12 +13,15 @@ torch = pytest.importorskip("torch")
 pytestmark = pytest.mark.gpu
 
 
-@pytest.mark.parametrize("m,n,pair,split,tile", [(64, 18944, 0, 1, 0), (64, 9472, 0, 2, 0), (40, 4608, 0, 4, 0), (512, 2304, 0, 8, 512),
-                                                 (64, 18944, 2, 0, 0), (300, 9472, 3, 0, 0)])
-def test_nothing_is_stored_after_a_lost_wait(m, n, pair, split, tile):
+# (the last three: pairs with a k split, where a pair that gave up tells the others of its cluster; longer slices of k, so that
+# each runs over several fetches from the host)
+@pytest.mark.parametrize("m,n,pair,split,tile,k", [(64, 18944, 0, 1, 0, 1024), (64, 9472, 0, 2, 0, 1024), (40, 4608, 0, 4, 0, 1024), (512, 2304, 0, 8, 512, 1024),
+                                                   (64, 18944, 2, 0, 0, 1024), (300, 9472, 3, 0, 0, 1024),
+                                                   (64, 9472, 2, 2, 64, 2048), (200, 4608, 2, 4, 208, 8192), (512, 9472, 2, 2, 512, 4096)])
+def test_nothing_is_stored_after_a_lost_wait(m, n, pair, split, tile, k):
     from ampstein_b200 import _lib
     L = _lib.lib()
-    k, K = 1024, 8
+    K = 8
     trellis, suh, svh, x = make_linear(k, n, K, seed=8800 + m + split, m=m)
     svh = (svh.astype(np.float32) / (1.2437 * np.sqrt(k))).astype(np.float16)
     host = torch.from_numpy(trellis.view(np.int16)).pin_memory()

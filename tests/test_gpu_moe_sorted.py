@@ -94,7 +94,7 @@ def test_sorted_moe_row_tiers_shard_range_and_accumulation(amp, oracle):
     assert np.array_equal(out.cpu().numpy(), one + np.float32(1.5))
 
 
-@pytest.mark.parametrize("act,gated,limit,cbname", [(1, True, 0.0, None), (3, True, 7.0, "mcg"), (0, False, 0.0, "mul1")])
+@pytest.mark.parametrize("act,gated,limit,cbname", [(1, True, 0.0, None), (3, True, 7.0, "mcg"), (0, False, 0.0, "mul1"), (0, True, 0.75, None)])
 def test_sorted_moe_activations_codebooks_and_no_gate(amp, oracle, act, gated, limit, cbname):
     E, H, I, K, topk, T = 4, 128, 256, 4, 2, 150
     ex = make_experts(E, H, I, H, K, seed=2500 + act)
@@ -108,6 +108,20 @@ def test_sorted_moe_activations_codebooks_and_no_gate(amp, oracle, act, gated, l
     cb = {"mcg": 1, "mul1": 2}.get(cbname, 0)
     ref = oracle.moe_coop(x, sel, rw, ex, act=act, act_limit=limit, gated=gated, cb=cb, gu_f16=True)
     check(got, ref)
+
+
+# Hidden widths whose 128-value chunks the input rotation cuts into parts of four with a shorter last one (5, 9, 10 chunks)
+@pytest.mark.parametrize("H,I,T,gated", [(640, 128, 90, True), (1152, 384, 150, True), (1280, 128, 33, False)])
+def test_sorted_moe_widths_with_a_short_last_part(amp, oracle, H, I, T, gated):
+    E, K, topk = 4, 3, 2
+    ex = make_experts(E, H, I, H, K, seed=4500 + H)
+    rng = np.random.default_rng(H)
+    x = rng.standard_normal((T, H)).astype(np.float16)
+    sel, rw = routing(rng, T, E, topk)
+    cfg = build_cfg(amp, ex, H, I, H, H, K, 1, topk, gated=gated)
+    cfg["I"] = I
+    got, _ = run_sorted(amp, cfg, x, sel, rw, E)
+    check(got, oracle.moe_coop(x, sel, rw, ex, gated=gated, gu_f16=True))
 
 
 def test_sorted_moe_deferred_slots_and_gather(amp, oracle):
