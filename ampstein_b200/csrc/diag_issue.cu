@@ -5,16 +5,13 @@
 // and (d) the two mma.sync alone. Measurement infrastructure, not part of the hot path: it backs the
 // statement that on sm_100 a legacy mma.sync keeps its scheduler from issuing other instructions
 // for most of the eight cycles the tensor pipe works on it. No counterpart in the reference.
-#include "exl3_common.cuh"
+#include "exl3_gemv_kernel.cuh"
 #include "host_common.h"
 #include <vector>
 
 namespace amp {
 
 constexpr int DIAG_ITERS = 1024;
-
-__device__ __forceinline__ uint32_t diag_lo16(uint32_t r) { uint32_t d; asm("dp2a.lo.u32.u32 %0, %1, %2, %3;" : "=r"(d) : "r"(r), "r"(0x00000001u), "r"(0u)); return d; }
-__device__ __forceinline__ uint32_t diag_hi16(uint32_t r) { uint32_t d; asm("dp2a.lo.u32.u32 %0, %1, %2, %3;" : "=r"(d) : "r"(r), "r"(0x00000100u), "r"(0u)); return d; }
 
 // V: 0 decode + two mma.sync, 1 decode + tcgen05.st (8 registers), 2 decode + checksum (four lop3),
 // 3 two mma.sync on undecoded words
@@ -36,54 +33,55 @@ __global__ void __launch_bounds__(128) diag_issue_kernel(uint32_t* out, long lon
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         tmem = s_tmem + ((uint32_t) (warp * 32) << 16);
     }
-    uint32_t cur = seed * (threadIdx.x + 1) + blockIdx.x, prev = cur ^ 0x9e3779b9u, sink = 0;
+    uint32_t w[4], prev = seed ^ 0x9e3779b9u, cur = seed * (threadIdx.x + 1) + blockIdx.x, sink = 0;
     float d0[4] = {0, 0, 0, 0}, d1[4] = {0, 0, 0, 0};
     const uint32_t b0 = seed | 0x3c003c00u, b1 = b0 + 1;
     __syncthreads();
     const long long t0 = clock64();
-    #pragma unroll 4
-    for (int it = 0; it < DIAG_ITERS; ++it)
+    // four iterations per turn: the 32 weights of a lane's chunk of four words, as the kernel walks a tile
+    for (int it = 0; it < DIAG_ITERS; it += 4)
     {
-        uint32_t a[8];
-        if (V == 3)
+        #pragma unroll
+        for (int j = 0; j < 4; ++j) { w[j] = cur; cur = cur * 1664525u + 1013904223u; }
+        auto quarter = [&](auto rtag)
         {
-            #pragma unroll
-            for (int j = 0; j < 8; ++j) a[j] = cur + j;
-        }
-        else
-        {
-            // the kernel's K = 4 decode: three funnel shifts, eight 16-bit extractions split between
-            // the ALU and the FMA-heavy pipe, eight multiply-adds, eight lop3
-            #pragma unroll
-            for (int c = 0; c < 4; ++c)
+            constexpr int R = decltype(rtag)::value;
+            uint32_t a[8];
+            if (V == 3)
             {
-                const uint32_t r = c ? __funnelshift_r(cur, prev, 4 * c) : cur;
-                const uint32_t h = (c == 1 || c == 2) ? diag_hi16(r) : (r >> 16);
-                const uint32_t l = diag_lo16(r);
-                a[3 - c] = cb_halves<0>(h);
-                a[7 - c] = cb_halves<0>(l);
+                #pragma unroll
+                for (int j = 0; j < 8; ++j) a[j] = w[R] + j;
             }
-        }
-        if (V == 0 || V == 3)
-        {
-            mma_16816(d0, a[0], a[4], a[1], a[5], b0, b1);
-            mma_16816(d1, a[2], a[6], a[3], a[7], b1, b0);
-        }
-        if (V == 1)
-        {
-            asm volatile("tcgen05.st.sync.aligned.16x256b.x2.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};"
-                :: "r"(tmem + (uint32_t) ((it & 1) * 16)), "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(a[4]), "r"(a[5]), "r"(a[6]), "r"(a[7]) : "memory");
-            if ((it & 7) == 7) asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
-        }
-        if (V == 2)
-        {
-            asm volatile("lop3.b32 %0, %0, %1, %2, 0x96;" : "+r"(sink) : "r"(a[0]), "r"(a[1]));
-            asm volatile("lop3.b32 %0, %0, %1, %2, 0x96;" : "+r"(sink) : "r"(a[2]), "r"(a[3]));
-            asm volatile("lop3.b32 %0, %0, %1, %2, 0x96;" : "+r"(sink) : "r"(a[4]), "r"(a[5]));
-            asm volatile("lop3.b32 %0, %0, %1, %2, 0x96;" : "+r"(sink) : "r"(a[6]), "r"(a[7]));
-        }
-        prev = cur;
-        cur = cur * 1664525u + 1013904223u;
+            else
+            {
+                // the decode GEMV's own decode at 4 bits, codebook 0
+                uint32_t x[8];
+                products8<4, R, 0>(w, prev, x);
+                #pragma unroll
+                for (int j = 0; j < 8; ++j) a[j] = a_word<0>(x[j]);
+            }
+            if (V == 0 || V == 3)
+            {
+                mma_16816(d0, a[0], a[4], a[1], a[5], b0, b1);
+                mma_16816(d1, a[2], a[6], a[3], a[7], b1, b0);
+            }
+            if (V == 1)
+            {
+                asm volatile("tcgen05.st.sync.aligned.16x256b.x2.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};"
+                    :: "r"(tmem + (uint32_t) ((R & 1) * 16)), "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(a[4]), "r"(a[5]), "r"(a[6]), "r"(a[7]) : "memory");
+                if (R == 3 && (it & 4)) asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+            }
+            if (V == 2)
+            {
+                asm volatile("lop3.b32 %0, %0, %1, %2, 0x96;" : "+r"(sink) : "r"(a[0]), "r"(a[1]));
+                asm volatile("lop3.b32 %0, %0, %1, %2, 0x96;" : "+r"(sink) : "r"(a[2]), "r"(a[3]));
+                asm volatile("lop3.b32 %0, %0, %1, %2, 0x96;" : "+r"(sink) : "r"(a[4]), "r"(a[5]));
+                asm volatile("lop3.b32 %0, %0, %1, %2, 0x96;" : "+r"(sink) : "r"(a[6]), "r"(a[7]));
+            }
+        };
+        quarter(std::integral_constant<int, 0>()); quarter(std::integral_constant<int, 1>());
+        quarter(std::integral_constant<int, 2>()); quarter(std::integral_constant<int, 3>());
+        prev = w[3];
     }
     const long long t1 = clock64();
     out[blockIdx.x * blockDim.x + threadIdx.x] = __float_as_uint(d0[0] + d0[1] + d0[2] + d0[3] + d1[0] + d1[1] + d1[2] + d1[3]) + cur + sink;

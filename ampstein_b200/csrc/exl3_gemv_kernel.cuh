@@ -1730,11 +1730,15 @@ void exl3_gemv_kernel(const GemvParams P)
                 }
                 else
                 {
-                    // Two mul1 weights per register, us before / now: 5120 x 25600 at 8 rows, 4 bits 53.9 / 50.6, 3 bits 57.2 / 53.8;
-                    // 4096 x 28672 at 4 bits, 4 rows 35.6 / 33.9 (5 % of that from the shared shifts); 4096 x 14336 at 3.5 bits, one row 19.3 / 18.7. Not where
-                    // the fields already fill the integer pipe: 5 and 7 bits (5120 x 25600 at 5 bits, 8 rows 55.3 / 57.2), half
-                    // rates behind a rotation launch (4096 x 14336 at 2.5 bits, 8 rows 26.6 / 27.4)
-                    constexpr bool PACK = CB == 2 && (shared_phase<K> || (K > 8 && (GIN != 2 || MB == 2)));
+                    // Two mul1 weights per register. 40 shapes (k 1024 .. 25600, n 512 .. 128256) at 2, 3, 4, 6 and 8 bits, two to
+                    // eight rows: 1.9 % faster on average, 1.6 % slower at worst but for 4096 x 6144 at 8 bits (11.2 / 10.4 us two
+                    // rows), e.g. us before / now: 5120 x 25600 at 4 bits, 8 rows 53.9 / 50.6, 13184 x 7040 at 8 bits, 4 rows 34.2 /
+                    // 32.3. Not where the fields already fill the integer pipe: 5 and 7 bits (5120 x 25600 at 5 bits, 8 rows 55.3 /
+                    // 57.2) and half rates of up to eight rows (the same shapes at 1.5, 2.5 and 3.5 bits, one to four rows: 2.6 %
+                    // slower on average, 5120 x 25600 at 3.5 bits, one row 37.4 / 39.0, 4096 x 4096 9.7 / 10.2; behind a rotation
+                    // launch, five to eight rows, between 7 % faster and 6 % slower). Nine to sixteen rows (MB 2) at half
+                    // rates gain: 14336 x 4096 at 2.5 bits, 12 rows 56.7 / 54.2.
+                    constexpr bool PACK = CB == 2 && (shared_phase<K> || (K > 8 && MB == 2));
                     #pragma unroll
                     for (int nt = 0; nt < NT; ++nt)
                     {
