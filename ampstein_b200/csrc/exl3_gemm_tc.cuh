@@ -133,12 +133,15 @@ __device__ __forceinline__ void umma_commit(uint64_t* bar)
                  :: "r"(smem_u32(bar)) : "memory");
 }
 
-// Shared shifts (window_product) where they take load off the integer ALU, which also packs here: at 2, 3 and 6 bits a shift and a
-// mask on the other pipe per window leave it less to do, except for codebook 2, whose masks are ALU work too (us, one each /
-// shared: 24 x 4096 x 14336 at 2 bits 28.8 / 29.4, 77 x 4096 x 14336 30.6 / 31.3; 59 tokens x top-8 of 128 experts at 3 bits 190.9 / 197.8; 600 x 4096 x 14336 at 6 bits 81.5 / 82.4, codebook 2 at 3 bits
-// 78.8 / 75.6, at 6 bits 78.3 / 75.6)
-template <int K, int CB>
-constexpr bool tg_shared_phase = shared_phase<K> && (CB == 2 || (K != 2 && K != 3 && K != 6));
+// Shared shifts (window_product) where they take load off the integer ALU, which also packs here. At 2, 3 and 6 bits a shift and a
+// mask on the other pipe per window leave it less to do in most instances. us, one each / shared (24 to 333 rows x 4096 x 14336,
+// 14336 x 4096, 5120 x 25600, 2048 x 5120; expert layers of 59, 300 and 1500 tokens x top-8 of 128):
+//   2 bits   24 x 4096 x 14336 27.6 / 28.4 (codebook 2 27.3 / 28.4), 200 x 5120 x 25600 74.0 / 75.4, from 333 rows on between 2 %
+//            more and 1 % less (92.0 / 90.2); experts 239 / 230, 244 / 235, 318 / 310 (codebook 2 216 / 217, 225 / 224, 308 / 305)
+//   3, 6     codebooks 0, 1: dense 30.2 / 30.4 and 30.4 / 32.1, experts of 59 tokens 236 / 240 and 240 / 246; codebook 2, whose masks are
+//            ALU work too: 59 tokens 221 / 218 and 232 / 231, 5120 x 25600 at 6 bits, 333 rows 92.3 / 91.0, 3 bits dense level
+template <int K, int CB, bool GROUPED>
+constexpr bool tg_shared_phase = shared_phase<K> && (K == 2 ? GROUPED : CB == 2 || (K != 3 && K != 6));
 
 constexpr int TG_MAX_N = 256;                 // tokens per accumulator (UMMA N)
 constexpr int TG_MAX_TOKENS = 512;            // tokens per tile: two accumulators, with 16 decode warps only
@@ -605,7 +608,7 @@ void exl3_gemm_tc_kernel(const TgParams S)
                     constexpr int R = decltype(rtag)::value;
                     uint32_t st[8];
                     // (codebook 2 already has two instructions per weight on the FMA pipe: its fields are cut on the ALU)
-                    products8<K, R, CB, CB != 2, tg_shared_phase<K, CB>>(w[c], prev[c], st);
+                    products8<K, R, CB, CB != 2, tg_shared_phase<K, CB, GROUPED>>(w[c], prev[c], st);
                     colA[R] = tg_weights2<CB>(st[0], st[1]);     colA[4 + R] = tg_weights2<CB>(st[2], st[3]);
                     colB[R] = tg_weights2<CB>(st[4], st[5]);     colB[4 + R] = tg_weights2<CB>(st[6], st[7]);
                 };
