@@ -386,13 +386,13 @@ constexpr bool shared_phase = K == 1 || K == 2 || K == 3 || K == 4 || K == 6 || 
 // SHARE: the stream is cut into 32-bit words shifted by 0 .. 7 bits so that the window ends with a byte; the compiler computes
 // a shifted word once for all windows in it, and a window is then one instruction: a half of the word (on the
 // FMA-heavy pipe with FMA), its middle (byte permute), or the last byte of the word in front and the first of this one
-// (byte permute, twice over: see cb_product). Shifts and fields per weight: 1.16 at 4 bits (1.38 when a funnel shift served the two
-// windows 16 bits apart), 1.56 at 6 and 1.66 at 3 bits (1.9 with a shift and a mask each), 1 at 8. At 5 and 7 bits the windows that end at the same bit
-// of a byte are more than a word apart: a shift and a mask each.
+// (byte permute, twice over: see cb_product). Shifts and fields per weight: 1.16 at 4 bits (1.38 when a funnel shift served the
+// two windows 16 bits apart), 1.56 at 6 and 1.66 at 3 bits (1.9 with a shift and a mask each), 1 at 8. At 5 and 7 bits the
+// windows that end at the same bit of a byte are more than a word apart: a shift and a mask each.
 // The decode GEMV is bound by issue (its slots and the cycles in which an mma.sync blocks them add up to all cycles): 4.80 -> 4.42
-// warp instructions per 32 weights at 4 bits. One row, us: 4096 x 229376 at 4 bits 184.8 -> 175.6 (2.67 TB/s), 4096 x 128256 at 6
-// bits 115.4 -> 110.8, 4096 x 28672 at 2 / 4 / 8 bits 27.4 / 27.4 / 29.2 -> 25.4 / 26.3 / 28.1, 3 bits (bound by the integer ALU)
-// 29.1 -> 29.0; tensor-core GEMM, 200 x 4096 x 28672 at 4 bits 71.1 -> 69.4 (3 and 6 bits: see tg_shared_phase).
+// warp instructions per weight and lane at 4 bits. One row, us: 4096 x 229376 at 4 bits 184.8 -> 175.6 (2.67 TB/s), 4096 x 128256
+// at 6 bits 115.4 -> 110.8, 4096 x 28672 at 2 / 4 / 8 bits 27.4 / 27.4 / 29.2 -> 25.4 / 26.3 / 28.1, 3 bits (bound by the integer
+// ALU) 29.1 -> 29.0; tensor-core GEMM, 200 x 4096 x 28672 at 4 bits 71.1 -> 69.4 (2, 3 and 6 bits: see tg_shared_phase).
 template <int CB, int LAST, int NW, bool FMA, bool SHARE>
 __device__ __forceinline__ uint32_t window_product(const uint32_t (&w)[NW], uint32_t prev)
 {
@@ -1734,17 +1734,20 @@ void exl3_gemv_kernel(const GemvParams P)
                     // eight rows: 1.9 % faster on average, 1.6 % slower at worst but for 4096 x 6144 at 8 bits (11.2 / 10.4 us two
                     // rows), e.g. us before / now: 5120 x 25600 at 4 bits, 8 rows 53.9 / 50.6, 13184 x 7040 at 8 bits, 4 rows 34.2 /
                     // 32.3. Not where the fields already fill the integer pipe: 5 and 7 bits (5120 x 25600 at 5 bits, 8 rows 55.3 /
-                    // 57.2) and half rates of up to eight rows (the same shapes at 1.5, 2.5 and 3.5 bits, one to four rows: 2.6 %
-                    // slower on average, 5120 x 25600 at 3.5 bits, one row 37.4 / 39.0, 4096 x 4096 9.7 / 10.2; behind a rotation
-                    // launch, five to eight rows, between 7 % faster and 6 % slower). Nine to sixteen rows (MB 2) at half
-                    // rates gain: 14336 x 4096 at 2.5 bits, 12 rows 56.7 / 54.2.
+                    // 57.2). At half rates the permutes of all weights cost that pipe more than the MMAs save, those of every
+                    // second quarter do not; one row, us, none / half / all of them: 4096 x 14336 at 2.5 bits 19.2 / 18.4 / 19.0, at
+                    // 3.5 bits 19.3 / 18.8 / 18.8, 5120 x 25600 at 3.5 bits 37.5 / 37.7 / 38.8, 4096 x 4096 9.8 / 9.9 / 10.3, 4480 x
+                    // 13568 at 2.5 bits 21.3 / 21.5 / 22.3, 4096 x 6144 at 1.5 bits 10.4 / 10.3 / 10.6. None behind a rotation launch
+                    // of up to eight rows (23680 x 25216 at 1.5 bits 135.7 / 138.3); all from nine rows on (MB 2; 14336 x 4096 at
+                    // 2.5 bits, 12 rows 56.7 / 54.2 none / all).
                     constexpr bool PACK = CB == 2 && (shared_phase<K> || (K > 8 && MB == 2));
+                    constexpr bool SOME = PACK || (CB == 2 && K > 8 && GIN != 2);
                     #pragma unroll
                     for (int nt = 0; nt < NT; ++nt)
                     {
-                        decode_mma_r<K, CB, MB, 0, PACK>(w[nt], prev[nt], xb, acc0[nt], acc1[nt]);
+                        decode_mma_r<K, CB, MB, 0, SOME>(w[nt], prev[nt], xb, acc0[nt], acc1[nt]);
                         decode_mma_r<K, CB, MB, 1, PACK>(w[nt], prev[nt], xb, acc0[nt], acc1[nt]);
-                        decode_mma_r<K, CB, MB, 2, PACK>(w[nt], prev[nt], xb, acc0[nt], acc1[nt]);
+                        decode_mma_r<K, CB, MB, 2, SOME>(w[nt], prev[nt], xb, acc0[nt], acc1[nt]);
                         decode_mma_r<K, CB, MB, 3, PACK>(w[nt], prev[nt], xb, acc0[nt], acc1[nt]);
                     }
                 }
