@@ -201,10 +201,10 @@ void had_tiled_kernel(const void* in, __half* out, const __half* pre,
 
 // The same rotation for many rows: a warp takes the same 128-value chunk of eight rows, four lanes each (quad_had128: the same
 // bits), so that a 64-k step of its rows is written as 1 KB in one place, and with several sources (a bundle's scale
-// vectors) the input is read once. Bound by HBM where input and output exceed the L2, by instruction issue otherwise
-// (about 9 instructions per 32 values against 25 of the one-warp form). Rows beyond M compute on row M - 1 and store nothing.
+// vectors) the input is read once. 13.6 warp instructions per 32 values (45 in the one-warp form) at 0.47 of the issue slots; what it
+// waits for are its loads. Rows beyond M compute on row M - 1 and store nothing.
 // Measured, us, one-warp form / this: 333 x 4096 3.5 / 3.1, 333 x 14336 9.2 / 7.3, 2048 x 4096 14.5 / 10.5, with three sources 38.2 /
-// 17.7, 2048 x 14336 45.0 / 28.1 (4.2 TB/s).
+// 17.7, 2048 x 14336 45.0 / 28.1 (4.2 TB/s in and out; 59 MB of it read from HBM, 15 written back, the rest stays in L2).
 template <bool BF16>
 __global__ __launch_bounds__(256, 3)
 void had_tiled_rows_kernel(const void* in, __half* out, const __half* pre,

@@ -326,10 +326,9 @@ void moe_sorted_rotate_in_kernel(const MsRot P)
     }
 }
 
-// A warp takes one 128-value chunk of an 8-row group, four lanes to a row. SILU: the gated SiLU without a limit, as an instance
-// of its own: chosen at run time for
-// every value the activation took most of the kernel's 39 instructions per value. The layer of 1500 tokens x top-8, us: 357 with eight chunks of a row per
-// warp, 352 in this order, 346 with the instance.
+// A warp takes one 128-value chunk of an 8-row group, four lanes to a row. SILU: the gated SiLU without a limit, as an instance of
+// its own: chosen at run time for every value the activation took most of the kernel's 39 instructions per value. The layer of
+// 1500 tokens x top-8, us: 357 with eight chunks of a row per warp, 352 in this order, 346 with the instance.
 template <bool SILU>
 __global__ __launch_bounds__(256, 3)
 void moe_sorted_rotate_act_kernel(const MsRot P)
@@ -361,7 +360,10 @@ void moe_sorted_rotate_act_kernel(const MsRot P)
             #pragma unroll
             for (int q = 0; q < 4; ++q)
             {
-                auto act1 = [&](float g1, float u1) { return SILU ? moe_act_gate(MOE_ACT_SILU, true, g1, u1, 0.0f) : moe_act_gate(P.act, P.gated, g1, u1, P.act_limit); };
+                auto act1 = [&](float g1, float u1)
+                {
+                    return SILU ? moe_act_gate(MOE_ACT_SILU, true, g1, u1, 0.0f) : moe_act_gate(P.act, P.gated, g1, u1, P.act_limit);
+                };
                 h[4 * j + q] = pack_f32x2(act1(__low2float(a[q]), __low2float(b[q])) * __low2float(c[q]),
                                            act1(__high2float(a[q]), __high2float(b[q])) * __high2float(c[q]));
             }
@@ -571,7 +573,9 @@ AMP_API int amp_exl3_moe_sorted(const amp_moe_sorted_args* a, cudaStream_t strea
     R.xt = ws + L.xt_gu; R.mcap = (int) L.mcap;
     R.fill = Pp.fill; R.list = (int2*) (ws + L.list);
     const long in_blocks = (groups_max * ((a->H / 128 + MS_IN_CHUNKS - 1) / MS_IN_CHUNKS) + 3) / 4;       // four tasks a block
-    if (cudaError_t e = launch_dependent(moe_sorted_rotate_in_kernel, (unsigned) (in_blocks < (long) sms * 20 ? in_blocks : (long) sms * 20), 128, stream, R)) return cuda_rc(e, "exl3_moe_sorted input rotation launch");
+    const unsigned in_grid = (unsigned) (in_blocks < (long) sms * 20 ? in_blocks : (long) sms * 20);
+    if (cudaError_t e = launch_dependent(moe_sorted_rotate_in_kernel, in_grid, 128, stream, R))
+        return cuda_rc(e, "exl3_moe_sorted input rotation launch");
 
     TcGroups G = {};
     G.ntiles = Pp.hdr; G.tile_e = Pp.tile_e; G.tile_row0 = Pp.tile_row0; G.tile_rows = Pp.tile_rows;
@@ -611,7 +615,8 @@ AMP_API int amp_exl3_moe_sorted(const amp_moe_sorted_args* a, cudaStream_t strea
     const long act_blocks = (groups_max * (a->I / 128) + 7) / 8;                                              // eight tasks a block
     const unsigned act_grid = (unsigned) (act_blocks < (long) sms * 12 ? act_blocks : (long) sms * 12);
     const bool silu = gated && a->act == MOE_ACT_SILU && a->act_limit == 0.0f;
-    if (cudaError_t e = launch_dependent(silu ? moe_sorted_rotate_act_kernel<true> : moe_sorted_rotate_act_kernel<false>, act_grid, 256, stream, D)) return cuda_rc(e, "exl3_moe_sorted activation launch");
+    if (cudaError_t e = launch_dependent(silu ? moe_sorted_rotate_act_kernel<true> : moe_sorted_rotate_act_kernel<false>, act_grid, 256, stream, D))
+        return cuda_rc(e, "exl3_moe_sorted activation launch");
 
     G.kinds = 1;
     G.bits[0] = G.bits[1] = mixed ? (const unsigned char*) a->d_bits : nullptr;
@@ -625,8 +630,9 @@ AMP_API int amp_exl3_moe_sorted(const amp_moe_sorted_args* a, cudaStream_t strea
                                                                  (float*) a->scratch, (const long long*) a->slot_base, a->scratch_rows);
         return cuda_rc(cudaGetLastError(), "exl3_moe_sorted slot launch");
     }
-    return cuda_rc(launch_dependent(moe_sorted_combine_kernel, a->T, 256, stream, Pp.fill, (const int2*) (ws + L.list), R.topk, (const __half*) a->w_sorted,
-                                    (const float*) (ws + L.dout), (float*) a->out, a->H), "exl3_moe_sorted combine launch");
+    return cuda_rc(launch_dependent(moe_sorted_combine_kernel, a->T, 256, stream, Pp.fill, (const int2*) (ws + L.list), R.topk,
+                                    (const __half*) a->w_sorted, (const float*) (ws + L.dout), (float*) a->out, a->H),
+                   "exl3_moe_sorted combine launch");
 }
 
 AMP_API int amp_exl3_moe_gather(float* out, const float* scratch, const void* flat_expert, const void* inv_order,

@@ -474,8 +474,9 @@ int amp_exl3_set_moe_sorted_tile(int sub);
 int amp_exl3_moe_sorted_status(const void* workspace, int* out, cudaStream_t stream);
 
 /*
- * Programmatic dependent launch of the decode kernels (default on): each kernel starts its
- * weight stream before waiting for the kernel in front of it. Returns the previous setting.
+ * Programmatic dependent launch (default on): the kernels move in as those in front leave, and a decode kernel starts its weight
+ * stream before it waits for the kernel in front of it. So a kernel that writes packed weights or scale vectors on the same
+ * stream must not itself release its dependents early (an ordinary kernel or a copy does not). Returns the previous setting.
  * The reference has no counterpart (it launches cooperative kernels back to back).
  */
 int amp_exl3_set_pdl(int enable);
