@@ -21,7 +21,8 @@ def amp():
 @pytest.mark.parametrize("m,k,n,K,cb,split,tile", [
     (17, 128, 128, 4, 0, 1, 0), (17, 128, 128, 1, 1, 2, 0), (33, 640, 256, 3, 2, 3, 32), (18, 512, 384, 5, 0, 8, 0),
     (129, 896, 128, 6, 1, 5, 128), (256, 256, 128, 8, 2, 4, 256), (257, 384, 256, 2, 0, 1, 272), (500, 1024, 128, 7, 0, 4, 512),
-    (300, 256, 640, 4, 1, 2, 304), (512, 512, 128, 3, 0, 8, 512), (97, 1152, 128, 5, 1, 7, 16), (1030, 256, 128, 4, 2, 1, 0)])
+    (300, 256, 640, 4, 1, 2, 304), (512, 512, 128, 3, 0, 8, 512), (97, 1152, 128, 5, 1, 7, 16), (1030, 256, 128, 4, 2, 1, 0),
+    (65, 384, 256, 2, 2, 3, 0), (130, 640, 128, 2, 1, 2, 0)])
 def test_forced_plans(amp, oracle, m, k, n, K, cb, split, tile):
     from ampstein_b200 import _lib
     trellis, suh, svh, x = make_linear(k, n, K, seed=8300 + m + K, m=m)

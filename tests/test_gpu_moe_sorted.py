@@ -110,6 +110,20 @@ def test_sorted_moe_activations_codebooks_and_no_gate(amp, oracle, act, gated, l
     check(got, ref)
 
 
+# 2 bits: the grouped instances cut their windows otherwise than the dense ones
+@pytest.mark.parametrize("cbname", [None, "mcg", "mul1"])
+def test_sorted_moe_at_two_bits(amp, oracle, cbname):
+    E, H, I, K, topk, T = 4, 256, 128, 2, 2, 70
+    ex = make_experts(E, H, I, H, K, seed=4700)
+    rng = np.random.default_rng(47)
+    x = rng.standard_normal((T, H)).astype(np.float16)
+    sel, rw = routing(rng, T, E, topk)
+    cfg = build_cfg(amp, ex, H, I, H, H, K, 1, topk, **({cbname: True} if cbname else {}))
+    cfg["I"] = I
+    got, _ = run_sorted(amp, cfg, x, sel, rw, E)
+    check(got, oracle.moe_coop(x, sel, rw, ex, cb={"mcg": 1, "mul1": 2}.get(cbname, 0), gu_f16=True))
+
+
 # Hidden widths whose 128-value chunks the input rotation cuts into parts of four with a shorter last one (5, 9, 10 chunks)
 @pytest.mark.parametrize("H,I,T,gated", [(640, 128, 90, True), (1152, 384, 150, True), (1280, 128, 33, False)])
 def test_sorted_moe_widths_with_a_short_last_part(amp, oracle, H, I, T, gated):
